@@ -11,6 +11,12 @@ for p in (ROOT, os.path.join(ROOT, "oracle"), GOLDEN):
         sys.path.insert(0, p)
 
 
+# The adapter tests run where the reference tree is present; an empty mount
+# point is not a tree.
+if "QCMG_REFERENCE_DIR" not in os.environ and not os.path.isfile("/root/reference/src_qcm/CPT.cpp"):
+    os.environ["QCMG_REFERENCE_DIR"] = os.path.join(ROOT, "oracle", "no_reference")
+
+
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (GB300) and the built libqcmg")
 
