@@ -8,7 +8,9 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "qcmg.h"
@@ -819,6 +821,31 @@ int qcmg_self_energy(int L, int M, const double* e, const double* v, int nb, con
   });
 }
 
+// Whether V(-K) = V(K)^T and Hdiff = Hdiff^T: every element real, the sums of
+// the elements at (r, c, R) and (c, r, -R) equal, Hdiff real and symmetric;
+// integer translations, so that a grid's wavevector 1 - K stands for -K.
+static bool transposed_at_minus_k(int L, const double* R, int nel, const int32_t* el_r,
+                                  const int32_t* el_c, const int32_t* el_n, const double* el_v,
+                                  const double* hdiff) {
+  std::map<std::tuple<int, int, double, double, double>, double> sum;
+  for (int k = 0; k < nel; ++k) {
+    if (el_v[2 * k + 1] != 0.0) return false;
+    const double* r = R + 3 * el_n[k];
+    if (r[0] != std::rint(r[0]) || r[1] != std::rint(r[1]) || r[2] != std::rint(r[2])) return false;
+    sum[{el_r[k], el_c[k], r[0] + 0.0, r[1] + 0.0, r[2] + 0.0}] += el_v[2 * k];
+  }
+  for (const auto& [key, v] : sum) {
+    const auto& [r, c, x, y, z] = key;
+    const auto it = sum.find({c, r, 0.0 - x, 0.0 - y, 0.0 - z});
+    if (it == sum.end() || !(it->second == v)) return false;
+  }
+  for (int r = 0; r < L; ++r)
+    for (int c = 0; c < L; ++c)
+      if (hdiff[2 * (r * L + c) + 1] != 0.0 || !(hdiff[2 * (r * L + c)] == hdiff[2 * (c * L + r)]))
+        return false;
+  return true;
+}
+
 int qcmg_lattice_create(int L, int nR, const double* R, int nel, const int32_t* el_r,
                         const int32_t* el_c, const int32_t* el_n, const double* el_v,
                         const double* hdiff, const double* gpos, qcmg_lattice** out) {
@@ -870,6 +897,33 @@ int qcmg_lattice_create(int L, int nR, const double* R, int nel, const int32_t* 
         t.el_n.upload(n.data(), nel, t.stream);
         t.el_v.upload(v.data(), (size_t)2 * nel, t.stream);
       }
+      // the same elements by matrix position, for the V tables
+      std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+        return el_r[p] * L + el_c[p] < el_r[q] * L + el_c[q];
+      });
+      std::vector<short> vidx((size_t)L * L, -1);
+      std::vector<int> ps, pn(nel);
+      std::vector<double> pv((size_t)2 * nel);
+      for (int k = 0; k < nel; ++k) {
+        const int o = order[k];
+        short& q = vidx[(size_t)el_r[o] * L + el_c[o]];
+        if (q < 0) {
+          q = (short)ps.size();
+          ps.push_back(k);
+        }
+        pn[k] = el_n[o];
+        pv[2 * k] = el_v[2 * o];
+        pv[2 * k + 1] = el_v[2 * o + 1];
+      }
+      t.nnz = (int)ps.size();
+      ps.push_back(nel);
+      t.vidx.upload(vidx.data(), vidx.size(), t.stream);
+      t.pos_start.upload(ps.data(), ps.size(), t.stream);
+      if (nel) {
+        t.pe_n.upload(pn.data(), nel, t.stream);
+        t.pe_v.upload(pv.data(), (size_t)2 * nel, t.stream);
+      }
+      t.el_sym = transposed_at_minus_k(L, R, nel, el_r, el_c, el_n, el_v, hdiff);
       QCMG_CUDA(cudaStreamSynchronize(t.stream));
     } catch (...) {
       if (h->lat.stream) cudaStreamDestroy(h->lat.stream);
@@ -902,6 +956,12 @@ int qcmg_lattice_set_green(qcmg_lattice* h, int M, const double* e, const double
     Lattice& t = h->lat;
     QCMG_CUDA(cudaSetDevice(t.device));
     t.M = M;
+    auto real = [](const double* a, size_t n) {
+      for (size_t k = 0; k < n; ++k)
+        if (a[2 * k + 1] != 0.0) return false;
+      return true;
+    };
+    t.green_real = real(v, (size_t)t.L * M) && real(tcb, (size_t)t.L * nb);
     if (M) {
       t.e.upload(e, M, t.stream);
       t.v.upload(v, (size_t)2 * t.L * M, t.stream);

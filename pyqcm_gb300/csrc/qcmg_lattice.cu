@@ -13,20 +13,19 @@
 //   CPT   Gcpt = G (1 - V G)^-1 = M^-1                       (CPT.cpp:76-86)
 //         g(K) = (1/L) sum_ab Gcpt_ab e^{2 pi i K.(x_b - x_a)} (lattice_model.cpp:724-740)
 //   CDMFT PGF(z) = mean_K Gcpt(K, z)                          (CPT.cpp:283-345)
-// G^-1 and log|det G| are computed once per frequency; each (K, z) point then
-// costs one LU factorization of an L x L complex matrix, done by one thread
-// with its matrix in shared memory (interleaved across threads, no bank
-// conflicts).
+// G^-1 and |det G| are computed once per frequency; each (K, z) point then
+// costs one LU factorization of an L x L complex matrix, done by one thread:
+// up to L = 16 by the kernels of qcmg_points.cuh, else (and for the K means)
+// with its matrix in shared memory, interleaved across threads.  Sums over a
+// K grid take one point of each pair (K, -K) where V(-K) = V(K)^T.
+#include <algorithm>
 #include <cmath>
-#include <cstdio>
-#include <cstdlib>
-#include <map>
-#include <mutex>
 #include <vector>
 
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
 #include "qcmg_lattice.h"
+#include "qcmg_points.h"
 
 namespace qcmg {
 
@@ -34,8 +33,8 @@ struct cdbl {
   double x, y;
 };
 __device__ __forceinline__ cdbl cmul(cdbl a, cdbl b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
-__device__ __forceinline__ cdbl cfma_sub(cdbl acc, cdbl a, cdbl b) {  // acc - a*b
-  return {acc.x - (a.x * b.x - a.y * b.y), acc.y - (a.x * b.y + a.y * b.x)};
+__device__ __forceinline__ cdbl cfma_sub(cdbl acc, cdbl a, cdbl b) {  // acc - a*b, four FMAs
+  return {fma(a.y, b.y, fma(-a.x, b.x, acc.x)), fma(-a.y, b.x, fma(-a.x, b.y, acc.y))};
 }
 __device__ __forceinline__ cdbl cinv(cdbl a) {
   double d = a.x * a.x + a.y * a.y;
@@ -50,11 +49,13 @@ __device__ __forceinline__ cdbl cinv(cdbl a) {
 __global__ void k_freq_prep(int L, int nw, const double2* __restrict__ G,  // nw x L x L (G[b + a L] = G(b,a))
                             const double2* __restrict__ z, int nb, const double2* __restrict__ tcb,
                             const double* __restrict__ eb, const double2* __restrict__ Hdiff,
-                            double2* __restrict__ base, double* __restrict__ logdetG) {
+                            double2* __restrict__ base, double* __restrict__ logdetG,
+                            double* __restrict__ det2, int* __restrict__ dexp) {
   extern __shared__ double2 sm[];
   double2* A = sm;              // L x 2L augmented [G | I], row-major A[r*2L + c]
   __shared__ int piv;
-  __shared__ double ldet;
+  double dm = 1.0;  // thread 0: |det G|^2 = dm 2^de
+  int de = 0;
   const int w = blockIdx.x;
   const int L2 = 2 * L;
   // G(r, c) with numpy orientation: G stored as G[b + a L] = G(b, a)  ->  G(r,c) = Gw[r + c L]
@@ -63,7 +64,6 @@ __global__ void k_freq_prep(int L, int nw, const double2* __restrict__ G,  // nw
     int r = idx / L2, c = idx % L2;
     A[idx] = c < L ? Gw[r + c * L] : make_double2(c - L == r ? 1.0 : 0.0, 0.0);
   }
-  if (threadIdx.x == 0) ldet = 0.0;
   __syncthreads();
   for (int p = 0; p < L; ++p) {
     if (threadIdx.x == 0) {
@@ -78,7 +78,7 @@ __global__ void k_freq_prep(int L, int nw, const double2* __restrict__ G,  // nw
         }
       }
       piv = best;
-      ldet += 0.5 * log(bv);
+      det_mul(dm, de, bv);
     }
     __syncthreads();
     if (piv != p)
@@ -128,7 +128,13 @@ __global__ void k_freq_prep(int L, int nw, const double2* __restrict__ G,  // nw
     }
     B[idx] = make_double2(gx, gy);
   }
-  if (threadIdx.x == 0) logdetG[w] = ldet;  // the pivots are those of G itself
+  if (threadIdx.x == 0) {  // the pivots are those of G itself
+    logdetG[w] = 0.5 * (log(dm) + (double)de * 0.6931471805599453094);
+    if (det2) {
+      det2[w] = dm;
+      dexp[w] = de;
+    }
+  }
 }
 
 // Sigma(z) = z - base with base = G^-1 + Gamma + t_c (k_freq_prep with the
@@ -184,7 +190,7 @@ void self_energy_batch(int L, int M, const double* e, const double* v, int nb, c
   const size_t smem = (size_t)L * 2 * L * sizeof(double2);
   k_freq_prep<<<nz, 128, smem, s>>>(L, nz, (const double2*)G.p, (const double2*)z, nb,
                                     (const double2*)tcb, eb, (const double2*)mtc.p,
-                                    (double2*)sigma, ldg.p);
+                                    (double2*)sigma, ldg.p, nullptr, nullptr);
   k_sigma_from_base<<<nz, 128, 0, s>>>(L, nz, (const double2*)z, (double2*)sigma);
   if (gamma)
     k_gamma<<<nz, 128, 0, s>>>(L, nz, (const double2*)z, nb, (const double2*)tcb, eb,
@@ -389,9 +395,8 @@ __global__ void k_points(PointArgs A) {
 
 // Sum of each row of vals (nrow x ncol), one block of kSumThreads per row:
 // thread t adds the elements t, t + kSumThreads, ... in order, then a fixed
-// tree adds the threads' sums.  The order depends on neither the point
-// kernel's block size nor its grid, so the Potthoff functional is the same
-// number whatever block size the tuner picks.
+// tree adds the threads' sums: an order that does not depend on the point
+// kernel's grid.
 constexpr int kSumThreads = 256;
 __global__ void __launch_bounds__(kSumThreads) k_row_sums(const double* __restrict__ vals,
                                                           int ncol, double* __restrict__ sums) {
@@ -412,92 +417,163 @@ __global__ void __launch_bounds__(kSumThreads) k_row_sums(const double* __restri
 // host side
 
 static int point_threads(int L) {
-  // one L x L complex matrix per thread in shared memory, up to 224 KB a
-  // block (one block per SM at L = 12: 96 points)
+  // one L x L complex matrix per thread in shared memory, up to 224 KB a block
   const size_t per = (size_t)2 * L * L * 8;  // bytes per point
   int T = (int)((224 * 1024) / per);
-  if (const char* e = std::getenv("QCMG_POINT_THREADS")) {  // tuning override
-    const int v = std::atoi(e);
-    if (v >= 32 && (size_t)v * per <= 224 * 1024) T = v;
-  }
   T = (T / 32) * 32;
   if (T > 256) T = 256;
   if (T < 32) T = 32;
   return T;
 }
 
-// Block size of the SEF point kernel, tuned once per matrix dimension L and
-// process: each candidate (multiples of 32 whose matrices fit the shared
-// memory budget, at most four, largest first) runs the same launch on the
-// caller's first frequencies (as many as one launch of that shape takes),
-// timed with CUDA events after one untimed run; the least time per
-// frequency is kept.  QCMG_POINT_THREADS overrides the choice;
-// QCMG_VERBOSE reports it on stderr.
-static std::mutex g_tune_mu;
-static std::map<int, int> g_tuned_sef;
-
-template <class Launch>
-static int tuned_sef_threads(int L, Launch&& launch, cudaStream_t s) {
-  if (std::getenv("QCMG_POINT_THREADS")) return point_threads(L);
-  {
-    std::lock_guard<std::mutex> lock(g_tune_mu);
-    auto it = g_tuned_sef.find(L);
-    if (it != g_tuned_sef.end()) return it->second;
-  }
-  const int tmax = point_threads(L);
-  std::vector<int> cand;
-  for (int T = tmax; T >= 32 && cand.size() < 4; T -= 32) cand.push_back(T);
-  cudaEvent_t e0, e1;
-  QCMG_CUDA(cudaEventCreate(&e0));
-  QCMG_CUDA(cudaEventCreate(&e1));
-  int best = tmax;
-  float best_ms = 0.0f;
-  for (int T : cand) {
-    launch(T);  // untimed: first-launch costs
-    QCMG_CUDA(cudaEventRecord(e0, s));
-    const int nf = launch(T);  // frequencies this launch covered
-    QCMG_CUDA(cudaEventRecord(e1, s));
-    QCMG_CUDA(cudaEventSynchronize(e1));
-    float ms = 0.0f;
-    QCMG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    ms /= (float)nf;
-    if (T == cand.front() || ms < best_ms) {
-      best_ms = ms;
-      best = T;
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (std::getenv("QCMG_VERBOSE"))
-    std::fprintf(stderr,
-                 "qcmg: SEF point kernel, L = %d: %d threads per block (%.3f ms per frequency)\n",
-                 L, best, best_ms);
-  std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_tuned_sef[L] = best;
-  return best;
-}
-
 void Lattice::prepare(int nw, const double* z, cudaStream_t s) {
   QCMG_CHECK_ARG(L > 0 && L <= 32, "lattice Green function dimension must be 1..32");
   QCMG_CHECK_ARG(M >= 0, "Q-matrix not set");
-  DevBuf<double> dz;
-  dz.upload(z, (size_t)2 * nw, s);
-  DevBuf<double> G;
-  G.alloc((size_t)2 * L * L * nw);
+  ws_z.upload(z, (size_t)2 * nw, s);
+  ws_G.alloc((size_t)2 * L * L * nw);
   if (M > 0) {
-    green_function_batch(L, M, e.p, v.p, nw, dz.p, G.p, s);
+    green_function_batch(L, M, e.p, v.p, nw, ws_z.p, ws_G.p, s);
   } else {
-    QCMG_CUDA(cudaMemsetAsync(G.p, 0, G.n * 8, s));
+    QCMG_CUDA(cudaMemsetAsync(ws_G.p, 0, (size_t)2 * L * L * nw * 8, s));
   }
   base.alloc((size_t)2 * L * L * nw);
   logdetG.alloc(nw);
+  det2.alloc(nw);
+  dexp.alloc(nw);
   size_t smem = (size_t)L * 2 * L * sizeof(double2);
-  k_freq_prep<<<nw, 128, smem, s>>>(L, nw, (const double2*)G.p, (const double2*)dz.p, nb,
+  k_freq_prep<<<nw, 128, smem, s>>>(L, nw, (const double2*)ws_G.p, (const double2*)ws_z.p, nb,
                                     (const double2*)tcb.p, eb.p, (const double2*)hdiff.p,
-                                    (double2*)base.p, logdetG.p);
+                                    (double2*)base.p, logdetG.p, det2.p, dexp.p);
   QCMG_CUDA(cudaGetLastError());
-  QCMG_CUDA(cudaStreamSynchronize(s));
   prepared_nw = nw;
+}
+
+// ---------------------------------------------------------------------------
+// tables over the wavevectors
+
+// Rows of V(K) at nk points: vk[q nk + h] = sum of the elements at position q
+// times e^{2 pi i K_h.R}; the phases come from the grid's axis tables (rep:
+// the points' flat grid indices) or, for explicit wavevectors, a sincos.
+__global__ void k_vk(int nk, const int* __restrict__ rep, const double2* __restrict__ tab, int gx,
+                     int gy, const double* __restrict__ K, int nR, const double* __restrict__ R,
+                     const int* __restrict__ pos_start, const int* __restrict__ pe_n,
+                     const double2* __restrict__ pe_v, double2* __restrict__ vk) {
+  const int h = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  if (h >= nk) return;
+  double sr = 0.0, si = 0.0;
+  for (int e = pos_start[q]; e < pos_start[q + 1]; ++e) {
+    const int n = pe_n[e];
+    double c, s;
+    if (rep) {
+      const int ik = rep[h];
+      const int ix = ik % gx, iy = (ik / gx) % gy, iz = ik / (gx * gy);
+      const double2 tx = tab[(size_t)ix * nR + n];
+      const double2 ty = tab[(size_t)(gx + iy) * nR + n];
+      const double2 tz = tab[(size_t)(gx + gy + iz) * nR + n];
+      const double xr = tx.x * ty.x - tx.y * ty.y, xi = tx.x * ty.y + tx.y * ty.x;
+      c = xr * tz.x - xi * tz.y;
+      s = xr * tz.y + xi * tz.x;
+    } else {
+      const double* k = K + 3 * (size_t)h;
+      sincos(2.0 * M_PI * (k[0] * R[3 * n] + k[1] * R[3 * n + 1] + k[2] * R[3 * n + 2]), &s, &c);
+    }
+    const double2 v = pe_v[e];
+    sr += v.x * c - v.y * s;
+    si += v.x * s + v.y * c;
+  }
+  vk[(size_t)q * nk + h] = make_double2(sr, si);
+}
+
+// uk[a nk + h] = e^{2 pi i K_h.x_a}
+__global__ void k_uk(int nk, const double* __restrict__ K, const double* __restrict__ gpos,
+                     double2* __restrict__ uk) {
+  const int h = blockIdx.x * blockDim.x + threadIdx.x, a = blockIdx.y;
+  if (h >= nk) return;
+  const double* k = K + 3 * (size_t)h;
+  const double* x = gpos + 3 * a;
+  double s, c;
+  sincos(2.0 * M_PI * (k[0] * x[0] + k[1] * x[1] + k[2] * x[2]), &s, &c);
+  uk[(size_t)a * nk + h] = make_double2(c, s);
+}
+
+int Lattice::grid_points(int gx, int gy, int gz, double off, cudaStream_t s) {
+  // pairing needs -K on the grid: offsets 0 and 1/2 (axes of one point other
+  // than the first have K = 0)
+  const bool pair = paired() && (off == 0.0 || off == 0.5);
+  if (rep.p && gx == rep_gx && gy == rep_gy && gz == rep_gz && off == rep_off && pair == rep_paired)
+    return nrep;
+  auto minus = [&](int i, int g, bool first) {
+    if (g == 1 && !first) return 0;
+    return off == 0.0 ? (g - i) % g : g - 1 - i;
+  };
+  std::vector<int> r;
+  std::vector<double> w;
+  const int nk = gx * gy * gz;
+  for (int ik = 0; ik < nk; ++ik) {
+    int p = ik;
+    if (pair) {
+      const int i = ik % gx, j = (ik / gx) % gy, l = ik / (gx * gy);
+      p = minus(i, gx, true) + gx * (minus(j, gy, false) + gy * minus(l, gz, false));
+    }
+    if (ik > p) continue;
+    r.push_back(ik);
+    w.push_back(ik < p ? 2.0 : 1.0);
+  }
+  rep_off = -1.0;
+  rep.upload(r.data(), r.size(), s);
+  wgt.upload(w.data(), w.size(), s);
+  QCMG_CUDA(cudaStreamSynchronize(s));  // r and w go out of scope
+  nrep = (int)r.size();
+  rep_gx = gx;
+  rep_gy = gy;
+  rep_gz = gz;
+  rep_off = off;
+  rep_paired = pair;
+  return nrep;
+}
+
+void Lattice::point_tables(int h0, int nk, const double* K, int gx, int gy, int gz, double off,
+                           bool u, cudaStream_t s) {
+  const dim3 grid((unsigned)((nk + 127) / 128), (unsigned)std::max(nnz, 1));
+  ws_v.alloc((size_t)2 * std::max(nnz, 1) * nk);
+  if (nnz) {
+    const double2* tb = K ? nullptr : (const double2*)phase_tables(gx, gy, gz, off, s);
+    k_vk<<<grid, 128, 0, s>>>(nk, K ? nullptr : rep.p + h0, tb, gx, gy, K ? K + 3 * (size_t)h0 : nullptr,
+                              nR, R.p, pos_start.p, pe_n.p, (const double2*)pe_v.p,
+                              (double2*)ws_v.p);
+  }
+  if (u) {
+    ws_u.alloc((size_t)2 * L * nk);
+    k_uk<<<dim3(grid.x, L), 128, 0, s>>>(nk, K + 3 * (size_t)h0, gpos.p, (double2*)ws_u.p);
+  }
+  QCMG_CUDA(cudaGetLastError());
+}
+
+// Workspaces up to this size stay with the handle.
+constexpr size_t kKeepBytes = (size_t)64 << 20;
+
+void Lattice::trim_workspaces() {
+  for (DevBuf<double>* b : {&ws_z, &ws_G, &ws_K, &ws_v, &ws_u, &ws_part, &ws_out, &base})
+    if (b->n * 8 > kKeepBytes) b->release();
+}
+
+// Wavevectors per launch of the point kernels: a multiple of 32, the tables
+// (rows of 16 bytes per wavevector) at most 256 MB.
+static int points_per_launch(int rows, int nk) {
+  const size_t most = ((size_t)256 << 20) / ((size_t)16 * std::max(rows, 1));
+  return (int)std::min<size_t>((size_t)nk, std::max<size_t>(most / 32 * 32, 32));
+}
+
+static LuArgs lu_args(const Lattice& lat, int nw) {
+  LuArgs A;
+  A.nw = nw;
+  A.base = (const double2*)lat.base.p;
+  A.vidx = lat.vidx.p;
+  A.vk = (const double2*)lat.ws_v.p;
+  A.uk = (const double2*)lat.ws_u.p;
+  A.det2 = lat.det2.p;
+  A.dexp = lat.dexp.p;
+  return A;
 }
 
 static PointArgs point_args(const Lattice& lat, int nw) {
@@ -554,92 +630,104 @@ const double* Lattice::phase_tables(int gx, int gy, int gz, double off, cudaStre
 
 double Lattice::sef_grid(int nw, const double* w, const double* wt, int nkx, int nky, int nkz,
                          cudaStream_t s) {
-  std::vector<double> z(2 * nw);
+  std::vector<double> z(2 * nw), hs(nw);
   for (int i = 0; i < nw; ++i) {
     z[2 * i] = 0.0;
     z[2 * i + 1] = w[i];
   }
-  double total = 0.0;
   const int nk = nkx * nky * nkz;
-  // frequencies are processed one by one so the per-frequency weight is
-  // applied exactly; each launch covers the whole K grid
   prepare(nw, z.data(), s);
-  const double2* phases = (const double2*)phase_tables(nkx, nky, nkz, 0.0, s);
-  // Several frequencies per launch (enough blocks for many waves on every
-  // SM), each block working on the points of one frequency; every point's
-  // log|det| is stored, and each frequency's sum is then taken in a fixed
-  // order (k_row_sums), so the weights apply to whole per-frequency sums and
-  // the result does not depend on the block size.
-  auto shape = [&](int T, unsigned& bpf, int& fpl) {
-    bpf = (unsigned)std::max<size_t>(1, std::min<size_t>((nk + T - 1) / T, 152 * 4));
-    fpl = std::max(1, std::min(nw, (int)((152u * 16u + bpf - 1) / bpf)));
+  // each frequency's K sum is taken in a fixed order (k_row_sums over the
+  // points, or over the warps' sums), so the weights apply to whole
+  // per-frequency sums
+  auto sums = [&](const double* rows, int ncol, int i0, int nf) {
+    ws_out.alloc(nw);
+    k_row_sums<<<nf, kSumThreads, 0, s>>>(rows, ncol, ws_out.p + i0);
+    QCMG_CUDA(cudaGetLastError());
   };
-  DevBuf<double> vals, sums;
-  auto launch = [&](int T, int i0, int nf, unsigned bpf) {
+  if (L <= kMaxPointL) {
+    const int np = grid_points(nkx, nky, nkz, 0.0, s), nkb = (np + 31) / 32;
+    ws_part.alloc((size_t)nw * nkb);
+    const int step = points_per_launch(nnz, np);
+    for (int h0 = 0; h0 < np; h0 += step) {
+      const int n = std::min(step, np - h0);
+      point_tables(h0, n, nullptr, nkx, nky, nkz, 0.0, false, s);
+      LuArgs A = lu_args(*this, nw);
+      A.nk = n;
+      A.wgt = wgt.p + h0;
+      A.part = ws_part.p + h0 / 32;
+      A.part_ld = nkb;
+      launch_sef_points(L, A, s);
+    }
+    sums(ws_part.p, nkb, 0, nw);
+  } else {
+    // a full matrix per thread in shared memory, several frequencies per
+    // launch (enough blocks for many waves on every SM)
+    const double2* phases = (const double2*)phase_tables(nkx, nky, nkz, 0.0, s);
+    const int T = point_threads(L);
+    const unsigned bpf = (unsigned)std::max<size_t>(1, std::min<size_t>((nk + T - 1) / T, 152 * 4));
+    const int fpl = std::max(1, std::min(nw, (int)((152u * 16u + bpf - 1) / bpf)));
     const size_t smem = (size_t)2 * L * L * T * 8;
     QCMG_CUDA(cudaFuncSetAttribute(k_points<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
-    if (vals.n < (size_t)nf * nk) vals.alloc((size_t)nf * nk);
-    PointArgs A = point_args(*this, nf);
-    A.base = (const double2*)base.p + (size_t)i0 * L * L;
-    A.nk = nk;
-    A.gx = nkx;
-    A.gy = nky;
-    A.gz = nkz;
-    A.off = 0.0;
-    A.vals = vals.p;
-    A.bpf = (int)bpf;
-    A.ldg = logdetG.p + i0;
-    A.tab = phases;
-    k_points<0><<<bpf * nf, T, smem, s>>>(A);
-    QCMG_CUDA(cudaGetLastError());
-  };
-  const int T = tuned_sef_threads(
-      L,
-      [&](int Tc) {
-        unsigned b;
-        int f;
-        shape(Tc, b, f);
-        const int nf = std::min(f, nw);
-        launch(Tc, 0, nf, b);
-        return nf;
-      },
-      s);
-  unsigned bpf;
-  int fpl;
-  shape(T, bpf, fpl);
-  if (sums.n < (size_t)fpl) sums.alloc((size_t)fpl);
-  std::vector<double> hs((size_t)fpl);
-  for (int i0 = 0; i0 < nw; i0 += fpl) {
-    const int nf = std::min(fpl, nw - i0);
-    launch(T, i0, nf, bpf);
-    k_row_sums<<<nf, kSumThreads, 0, s>>>(vals.p, nk, sums.p);
-    QCMG_CUDA(cudaGetLastError());
-    QCMG_CUDA(cudaMemcpyAsync(hs.data(), sums.p, (size_t)nf * 8, cudaMemcpyDeviceToHost, s));
-    QCMG_CUDA(cudaStreamSynchronize(s));
-    for (int f = 0; f < nf; ++f) total += wt[i0 + f] * (hs[f] / nk);
+    ws_part.alloc((size_t)fpl * nk);
+    for (int i0 = 0; i0 < nw; i0 += fpl) {
+      const int nf = std::min(fpl, nw - i0);
+      PointArgs A = point_args(*this, nf);
+      A.base = (const double2*)base.p + (size_t)i0 * L * L;
+      A.nk = nk;
+      A.gx = nkx;
+      A.gy = nky;
+      A.gz = nkz;
+      A.off = 0.0;
+      A.vals = ws_part.p;
+      A.bpf = (int)bpf;
+      A.ldg = logdetG.p + i0;
+      A.tab = phases;
+      k_points<0><<<bpf * nf, T, smem, s>>>(A);
+      QCMG_CUDA(cudaGetLastError());
+      sums(ws_part.p, nk, i0, nf);
+    }
   }
+  QCMG_CUDA(cudaMemcpyAsync(hs.data(), ws_out.p, (size_t)nw * 8, cudaMemcpyDeviceToHost, s));
+  QCMG_CUDA(cudaStreamSynchronize(s));
+  trim_workspaces();
+  double total = 0.0;
+  for (int i = 0; i < nw; ++i) total += wt[i] * (hs[i] / nk);
   return total;
 }
 
 void Lattice::cpt(int nz, const double* z, int nk, const double* K, double* g, cudaStream_t s) {
   prepare(nz, z, s);
-  PointArgs A = point_args(*this, nz);
-  DevBuf<double> dK, out;
-  dK.upload(K, (size_t)3 * nk, s);
-  out.alloc((size_t)2 * nz * nk);
-  A.nk = nk;
-  A.K = dK.p;
-  A.out = (double2*)out.p;
-  const int T = point_threads(L);
-  const size_t smem = (size_t)2 * L * L * T * 8;
-  QCMG_CUDA(cudaFuncSetAttribute(k_points<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const size_t npts = (size_t)nz * nk;
-  unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((npts + T - 1) / T, 152 * 8));
-  k_points<1><<<gr, T, smem, s>>>(A);
-  QCMG_CUDA(cudaGetLastError());
-  QCMG_CUDA(cudaMemcpyAsync(g, out.p, (size_t)2 * nz * nk * 8, cudaMemcpyDeviceToHost, s));
+  ws_K.upload(K, (size_t)3 * nk, s);
+  ws_out.alloc((size_t)2 * nz * nk);
+  if (L <= kMaxPointL) {
+    const int step = points_per_launch(nnz + L, nk);
+    for (int h0 = 0; h0 < nk; h0 += step) {
+      const int n = std::min(step, nk - h0);
+      point_tables(h0, n, ws_K.p, 1, 1, 1, 0.0, true, s);
+      LuArgs A = lu_args(*this, nz);
+      A.nk = n;
+      A.out = (double2*)ws_out.p + h0;
+      A.out_ld = nk;
+      launch_cpt_points(L, A, s);
+    }
+  } else {
+    PointArgs A = point_args(*this, nz);
+    A.nk = nk;
+    A.K = ws_K.p;
+    A.out = (double2*)ws_out.p;
+    const int T = point_threads(L);
+    const size_t smem = (size_t)2 * L * L * T * 8;
+    QCMG_CUDA(cudaFuncSetAttribute(k_points<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t npts = (size_t)nz * nk;
+    unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((npts + T - 1) / T, 152 * 8));
+    k_points<1><<<gr, T, smem, s>>>(A);
+    QCMG_CUDA(cudaGetLastError());
+  }
+  QCMG_CUDA(cudaMemcpyAsync(g, ws_out.p, (size_t)2 * nz * nk * 8, cudaMemcpyDeviceToHost, s));
   QCMG_CUDA(cudaStreamSynchronize(s));
+  trim_workspaces();
 }
 
 // K means of the per-point inverses, per frequency and moment:
@@ -767,6 +855,7 @@ void Lattice::kmoments(int nz, const double* z, int gx, int gy, int gz, double o
                               (size_t)2 * nc * nm * LL * 8, cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaStreamSynchronize(s));
   }
+  trim_workspaces();
 }
 
 }  // namespace qcmg

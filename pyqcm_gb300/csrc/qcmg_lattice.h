@@ -25,14 +25,42 @@ struct Lattice {
   int tab_gx = 0, tab_gy = 0, tab_gz = 0;
   double tab_off = -1.0;
   const double* phase_tables(int gx, int gy, int gz, double off, cudaStream_t s);
+  // the nonzero entries of V(K): vidx[r L + c] is the entry's row in the V
+  // tables (or -1); entry q sums the elements [pos_start[q], pos_start[q + 1])
+  int nnz = 0;
+  DevBuf<short> vidx;
+  DevBuf<int> pos_start, pe_n;
+  DevBuf<double> pe_v;  // complex
+  // V(-K) = V(K)^T (real elements, every one with its transposed partner, and
+  // a real symmetric Hdiff), and a real Q-matrix and bath: then every
+  // K-dependent matrix at -K is the transpose of the one at K
+  bool el_sym = false, green_real = false;
+  bool paired() const { return el_sym && green_real; }
+  // the points of a grid that a sum over K needs: all of them, or (paired)
+  // one of each pair (K, -K); cached for the last grid asked for
+  DevBuf<int> rep;      // flat grid index
+  DevBuf<double> wgt;   // 1, or 2 for a pair
+  int nrep = 0, rep_gx = 0, rep_gy = 0, rep_gz = 0;
+  double rep_off = -1.0;
+  bool rep_paired = false;
+  int grid_points(int gx, int gy, int gz, double off, cudaStream_t s);
   int M = -1;
   DevBuf<double> e;      // M poles
   DevBuf<double> v;      // L x M complex, column-major
   int nb = 0;
   DevBuf<double> tcb;    // L x nb complex, column-major
   DevBuf<double> eb;     // nb
-  DevBuf<double> base, logdetG;
+  DevBuf<double> base, logdetG, det2;
+  DevBuf<int> dexp;  // |det G|^2 = det2 2^dexp
   int prepared_nw = 0;
+  // workspaces kept between calls (released at the end of a call that needed
+  // more than kKeepBytes of one)
+  DevBuf<double> ws_z, ws_G, ws_K, ws_v, ws_u, ws_part, ws_out;
+  void trim_workspaces();
+  // rows of the V table (and with u set, of e^{2 pi i K.x}) for nk points
+  // from h0 of the grid's list (K null) or of the explicit K list
+  void point_tables(int h0, int nk, const double* K, int gx, int gy, int gz, double off, bool u,
+                    cudaStream_t s);
   cudaStream_t stream = nullptr;
 
   void prepare(int nw, const double* z, cudaStream_t s);
