@@ -15,11 +15,12 @@
 //   CDMFT PGF(z) = mean_K Gcpt(K, z)                          (CPT.cpp:283-345)
 // G^-1 and |det G| are computed once per frequency; each (K, z) point then
 // costs one LU factorization of an L x L complex matrix, done by one thread:
-// up to L = 16 by the kernels of qcmg_points.cuh, else (and for the K means)
+// up to L = 16 by the kernels of qcmg_points.cuh and qcmg_points_inv.cu, else
 // with its matrix in shared memory, interleaved across threads.  Sums over a
 // K grid take one point of each pair (K, -K) where V(-K) = V(K)^T.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "qcmg_internal.h"
@@ -496,10 +497,10 @@ __global__ void k_uk(int nk, const double* __restrict__ K, const double* __restr
   uk[(size_t)a * nk + h] = make_double2(c, s);
 }
 
-int Lattice::grid_points(int gx, int gy, int gz, double off, cudaStream_t s) {
+int Lattice::grid_points(int gx, int gy, int gz, double off, cudaStream_t s, bool may_pair) {
   // pairing needs -K on the grid: offsets 0 and 1/2 (axes of one point other
   // than the first have K = 0)
-  const bool pair = paired() && (off == 0.0 || off == 0.5);
+  const bool pair = may_pair && paired() && (off == 0.0 || off == 0.5);
   if (rep.p && gx == rep_gx && gy == rep_gy && gz == rep_gz && off == rep_off && pair == rep_paired)
     return nrep;
   auto minus = [&](int i, int g, bool first) {
@@ -524,6 +525,7 @@ int Lattice::grid_points(int gx, int gy, int gz, double off, cudaStream_t s) {
   wgt.upload(w.data(), w.size(), s);
   QCMG_CUDA(cudaStreamSynchronize(s));  // r and w go out of scope
   nrep = (int)r.size();
+  rep_host.swap(r);
   rep_gx = gx;
   rep_gy = gy;
   rep_gz = gz;
@@ -804,9 +806,127 @@ void Lattice::kmean(int nz, const double* z, int gx, int gy, int gz, double off,
   kmoments(nz, z, gx, gy, gz, off, 0, nullptr, out_host, s);
 }
 
+// The means of the translations `which` of Rm (empty: the plain mean) into
+// their places of out_host, nz x max(nmom, 1) x L x L.
+void Lattice::inverse_means(int nz, const double* z, int gx, int gy, int gz, double off, int nmom,
+                            const std::vector<int>& which, const double* Rm, double* out_host,
+                            cudaStream_t s) {
+  const int nk = gx * gy * gz, LL = L * L, nm = std::max<int>(1, (int)which.size());
+  bool integer = true;  // pairing takes e^{2 pi i (1 - K).R} for e^{-2 pi i K.R}
+  for (int m : which)
+    for (int a = 0; a < 3; ++a) integer = integer && Rm[3 * m + a] == std::rint(Rm[3 * m + a]);
+  const int np = grid_points(gx, gy, gz, off, s, integer);
+  const bool pair = rep_paired;
+  // rows: with translations, the points of each (ky, kz); else equal parts,
+  // about 4,096 warps over all frequencies but whole batches of 32
+  std::vector<int> rows{0}, fx(nm, 0);
+  std::vector<double> yz, wx, ax;
+  if (which.empty()) {
+    const int batches = (np + 31) / 32;
+    const int per = std::max(1, std::min(batches, (int)((size_t)batches * nz / 4096)));
+    for (int b = per; b < batches; b += per) rows.push_back(32 * b);
+    rows.push_back(np);
+  } else {
+    for (int h = 1; h < np; ++h)
+      if (rep_host[h] / gx != rep_host[h - 1] / gx) rows.push_back(h);
+    rows.push_back(np);
+    for (size_t q = 0; q < which.size(); ++q) {
+      const double r = Rm[3 * which[q]];
+      if (r == 0.0) continue;
+      size_t u = std::find(ax.begin(), ax.end(), std::fabs(r)) - ax.begin();
+      if (u == ax.size()) ax.push_back(std::fabs(r));
+      fx[q] = (r < 0 ? -1 : 1) * (int)(2 * u + 1);
+    }
+    for (double r : ax)
+      for (int part = 0; part < 2; ++part)
+        for (int i = 0; i < gx; ++i) {
+          const double a = 2.0 * M_PI * ((i + off) / gx) * r;
+          wx.push_back(part ? std::sin(a) : std::cos(a));
+        }
+    for (int m : which)
+      for (size_t r = 0; r + 1 < rows.size(); ++r) {
+        const int yzi = rep_host[rows[r]] / gx, j = yzi % gy, l = yzi / gy;
+        const double a = 2.0 * M_PI * ((gy > 1 ? (j + off) / gy : 0.0) * Rm[3 * m + 1] +
+                                       (gz > 1 ? (l + off) / gz : 0.0) * Rm[3 * m + 2]);
+        yz.push_back(std::cos(a));
+        yz.push_back(std::sin(a));
+      }
+  }
+  const int nrow = (int)rows.size() - 1, nf = 1 + 2 * (int)ax.size();
+  DevBuf<int> d_rows, d_fx;
+  DevBuf<double> d_yz, d_wx;
+  d_rows.upload(rows.data(), rows.size(), s);
+  if (!which.empty()) {
+    d_fx.upload(fx.data(), fx.size(), s);
+    d_yz.upload(yz.data(), yz.size(), s);
+    if (!wx.empty()) d_wx.upload(wx.data(), wx.size(), s);
+  }
+  point_tables(0, np, nullptr, gx, gy, gz, off, false, s);
+  // frequencies in chunks whose row sums fit in ~512 MB
+  const size_t per_z = (size_t)nrow * nf * LL * 16;
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(nz, ((size_t)512 << 20) / per_z));
+  ws_part.alloc((size_t)2 * chunk * nrow * nf * LL);
+  ws_out.alloc((size_t)2 * chunk * nm * LL);
+  std::vector<double> host((size_t)2 * nz * nm * LL);
+  for (int z0 = 0; z0 < nz; z0 += chunk) {
+    const int nc = std::min(chunk, nz - z0);
+    prepare(nc, z + 2 * (size_t)z0, s);
+    InvArgs A;
+    A.nk = np;
+    A.nw = nc;
+    A.nrow = nrow;
+    A.base = (const double2*)base.p;
+    A.vidx = vidx.p;
+    A.vk = (const double2*)ws_v.p;
+    A.wgt = wgt.p;
+    A.scale = pair ? 0.5 : 1.0;  // a pair's weight 2 is shared by the inverse and its transpose
+    A.row_start = d_rows.p;
+    A.rep = rep.p;
+    A.gx = gx;
+    A.nf = nf;
+    A.wx = d_wx.p;
+    A.part = (double2*)ws_part.p;
+    launch_inverse_means(L, A, nm, which.empty() ? nullptr : d_fx.p,
+                         which.empty() ? nullptr : (const double2*)d_yz.p, pair, 1.0 / nk,
+                         (double2*)ws_out.p, s);
+    QCMG_CUDA(cudaMemcpyAsync(host.data() + (size_t)2 * z0 * nm * LL, ws_out.p,
+                              (size_t)2 * nc * nm * LL * 8, cudaMemcpyDeviceToHost, s));
+    QCMG_CUDA(cudaStreamSynchronize(s));
+  }
+  trim_workspaces();
+  const int ld = std::max(nmom, 1);
+  for (int w = 0; w < nz; ++w)
+    for (int q = 0; q < nm; ++q)
+      std::memcpy(out_host + ((size_t)w * ld + (which.empty() ? 0 : which[q])) * 2 * LL,
+                  host.data() + ((size_t)w * nm + q) * 2 * LL, (size_t)2 * LL * 8);
+}
+
 void Lattice::kmoments(int nz, const double* z, int gx, int gy, int gz, double off, int nmom,
                        const double* Rm, double* out_host, cudaStream_t s) {
   QCMG_CHECK_ARG(nmom >= 0 && nmom <= kMaxMoments, "at most 16 translations per call");
+  if (L <= kMaxPointL) {
+    // translations in groups of at most (kMaxInvFuncs - 1)/2 distinct |R_x|
+    if (nmom == 0) return inverse_means(nz, z, gx, gy, gz, off, 0, {}, nullptr, out_host, s);
+    std::vector<int> todo(nmom);
+    for (int m = 0; m < nmom; ++m) todo[m] = m;
+    while (!todo.empty()) {
+      std::vector<int> now, later;
+      std::vector<double> ax;
+      for (int m : todo) {
+        const double a = std::fabs(Rm[3 * m]);
+        const bool known = a == 0.0 || std::find(ax.begin(), ax.end(), a) != ax.end();
+        if (!known && (int)ax.size() >= (kMaxInvFuncs - 1) / 2) {
+          later.push_back(m);
+          continue;
+        }
+        if (!known) ax.push_back(a);
+        now.push_back(m);
+      }
+      inverse_means(nz, z, gx, gy, gz, off, nmom, now, Rm, out_host, s);
+      todo.swap(later);
+    }
+    return;
+  }
   const int nk = gx * gy * gz, LL = L * L;
   const int T = point_threads(L);
   const size_t smem = (size_t)2 * L * L * T * 8;
@@ -830,9 +950,8 @@ void Lattice::kmoments(int nz, const double* z, int gx, int gy, int gz, double o
   // frequencies in chunks whose per-point inverses fit in ~512 MB
   const size_t per_z = (size_t)nk * LL * 16;
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>(nz, ((size_t)512 << 20) / per_z));
-  DevBuf<double> inv, out;
-  inv.alloc((size_t)2 * chunk * nk * LL);
-  out.alloc((size_t)2 * chunk * nm * LL);
+  ws_part.alloc((size_t)2 * chunk * nk * LL);
+  ws_out.alloc((size_t)2 * chunk * nm * LL);
   for (int z0 = 0; z0 < nz; z0 += chunk) {
     const int nc = std::min(chunk, nz - z0);
     prepare(nc, z + 2 * (size_t)z0, s);
@@ -843,15 +962,15 @@ void Lattice::kmoments(int nz, const double* z, int gx, int gy, int gz, double o
     A.nk = nk;
     A.off = off;
     A.tab = (const double2*)phase_tables(gx, gy, gz, off, s);
-    A.out = (double2*)inv.p;
+    A.out = (double2*)ws_part.p;
     const size_t npts = (size_t)nc * nk;
     unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((npts + T - 1) / T, 152 * 8));
     k_points<2><<<gr, T, smem, s>>>(A);
     k_mean_moments<<<dim3(nc, (LL + 31) / 32), 32 * kMomWarps, 0, s>>>(
-        (const double2*)inv.p, nc, nk, LL, nm, nmom > 0 ? (const double2*)ph.p : nullptr,
-        (double2*)out.p);
+        (const double2*)ws_part.p, nc, nk, LL, nm, nmom > 0 ? (const double2*)ph.p : nullptr,
+        (double2*)ws_out.p);
     QCMG_CUDA(cudaGetLastError());
-    QCMG_CUDA(cudaMemcpyAsync(out_host + (size_t)2 * z0 * nm * LL, out.p,
+    QCMG_CUDA(cudaMemcpyAsync(out_host + (size_t)2 * z0 * nm * LL, ws_out.p,
                               (size_t)2 * nc * nm * LL * 8, cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaStreamSynchronize(s));
   }

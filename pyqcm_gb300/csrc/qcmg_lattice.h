@@ -43,7 +43,11 @@ struct Lattice {
   int nrep = 0, rep_gx = 0, rep_gy = 0, rep_gz = 0;
   double rep_off = -1.0;
   bool rep_paired = false;
-  int grid_points(int gx, int gy, int gz, double off, cudaStream_t s);
+  std::vector<int> rep_host;
+  int grid_points(int gx, int gy, int gz, double off, cudaStream_t s, bool may_pair = true);
+  void inverse_means(int nz, const double* z, int gx, int gy, int gz, double off, int nmom,
+                     const std::vector<int>& which, const double* Rm, double* out_host,
+                     cudaStream_t s);
   int M = -1;
   DevBuf<double> e;      // M poles
   DevBuf<double> v;      // L x M complex, column-major

@@ -29,6 +29,31 @@ void launch_sef_points(int L, const LuArgs& A, cudaStream_t s);
 // out[w][k] = (1/L) u^+ (base_w - V(K))^-1 u
 void launch_cpt_points(int L, const LuArgs& A, cudaStream_t s);
 
+// The sums over K of the inverses. The points (their tables as in LuArgs) are
+// grouped in rows [row_start[r], row_start[r + 1]); with nf > 1 a row's points
+// share (ky, kz).
+struct InvArgs {
+  int nk = 0, nw = 0, nrow = 0;
+  const double2* base = nullptr;
+  const short* vidx = nullptr;
+  const double2* vk = nullptr;
+  const double* wgt = nullptr;
+  double scale = 1.0;               // on the weights
+  const int* row_start = nullptr;   // nrow + 1
+  const int* rep = nullptr;         // flat grid index of each point
+  int gx = 1;
+  int nf = 1;                       // weight functions: 1 and the rows of wx
+  const double* wx = nullptr;       // (nf - 1) x gx: cosine, sine of each distinct |R_x|
+  double2* part = nullptr;          // nw x nrow x nf x L x L
+};
+constexpr int kMaxInvFuncs = 9;
+
+// out (nw x nm x L x L row-major): the means with the phases of nm
+// translations. fx[m]: 0, or +-(the cosine's function) by the sign of R_x;
+// yz: nm x nrow, the rest of each phase (null: one plain mean).
+void launch_inverse_means(int L, const InvArgs& A, int nm, const int* fx, const double2* yz,
+                          bool paired, double inv_nk, double2* out, cudaStream_t s);
+
 // |det|^2 as mantissa and exponent: m 2^e *= bv (a squared modulus).  Zeros,
 // subnormals and non-finite values go into the mantissa unchanged.
 __device__ __forceinline__ void det_mul(double& m, int& e, double bv) {

@@ -90,3 +90,34 @@ def test_periodized_points(L, kind, nk):
     u = np.exp(2j * np.pi * (K @ p.gpos.T))
     ref = np.einsum("ka,zkab,kb->zk", u.conj(), np.linalg.inv(A), u) / L
     assert np.max(np.abs(g.view(np.complex128).reshape(len(z), nk) - ref)) < TOL * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("L", [1, 2, 4, 7, 8, 13, 16, 17])
+@pytest.mark.parametrize("kind", ["real", "complex", "onesided"])
+@pytest.mark.parametrize("g", [(1, 1, 1, 0.0), (7, 5, 1, 0.0), (8, 6, 2, 0.5), (33, 1, 1, 0.5), (40, 3, 1, 0.25)])
+@pytest.mark.parametrize("moments", ["none", "few", "many"])
+def test_inverse_means(L, kind, g, moments):
+    """Plain means and means with translations' phases: few translations, and
+    16 with more distinct x components than one pass takes."""
+    from pyqcm_gb300 import _lib
+    p = Problem(L, kind, 3)
+    z = np.array([0.3 + 0.3j, -1.2 + 0.5j, 2.0j])
+    R = {"none": np.zeros((0, 3)), "few": p.R.copy(),
+         "many": np.array([[(-1) ** m * m, m % 3 - 1, m % 2] for m in range(16)], float)}[moments]
+    if moments == "few" and g[0] == 33:
+        R[3] = [0.5, 0.0, 0.0]  # not a lattice translation: no pairing
+    blk = p.block()
+    nm = max(1, len(R))
+    out = np.zeros(2 * len(z) * nm * L * L)
+    if len(R):
+        _lib.check(_lib.lib().qcmg_lattice_kmoments(blk._h, len(z), _lib.ptr(z.view(np.float64)), *g[:3], g[3], nm,
+                                                    _lib.ptr(np.ascontiguousarray(R)), _lib.ptr(out)))
+    else:
+        _lib.check(_lib.lib().qcmg_lattice_kmean(blk._h, len(z), _lib.ptr(z.view(np.float64)), *g[:3], g[3], _lib.ptr(out)))
+    K = grid(*g)
+    A, _ = p.matrices(z, K)
+    X = np.linalg.inv(A)
+    ph = np.exp(2j * np.pi * (K @ R.T)) if len(R) else np.ones((len(K), 1))
+    ref = np.einsum("km,zkab->zmab", ph, X) / len(K)
+    got = out.view(np.complex128).reshape(len(z), nm, L, L)
+    assert np.max(np.abs(got - ref)) < TOL * max(1.0, np.max(np.abs(X)))
