@@ -771,6 +771,13 @@ int qcmg_apply_c(int L, int orb, int pm, int n_up, int n_dn, const double* x, do
   });
 }
 
+// Whether n complex numbers (re, im pairs) are all real.
+static bool all_real(const double* a, size_t n) {
+  for (size_t k = 0; k < n; ++k)
+    if (a[2 * k + 1] != 0.0) return false;
+  return true;
+}
+
 int qcmg_green_function(int L, int M, const double* e, const double* v, int nz, const double* z,
                         double* G) {
   return guarded([&] {
@@ -787,7 +794,7 @@ int qcmg_green_function(int L, int M, const double* e, const double* v, int nz, 
     dv.upload(v, (size_t)2 * L * M, 0);
     dz.upload(z, (size_t)2 * nz, 0);
     dG.alloc((size_t)2 * L * L * nz);
-    green_function_batch(L, M, de.p, dv.p, nz, dz.p, dG.p, 0);
+    green_function_batch(L, M, de.p, dv.p, all_real(v, (size_t)L * M), nz, dz.p, dG.p, 0);
     QCMG_CUDA(cudaMemcpy(G, dG.p, (size_t)2 * L * L * nz * 8, cudaMemcpyDeviceToHost));
   });
 }
@@ -814,7 +821,7 @@ int qcmg_self_energy(int L, int M, const double* e, const double* v, int nb, con
     dz.upload(z, (size_t)2 * nz, 0);
     ds.alloc((size_t)2 * L * L * nz);
     if (gamma) dg.alloc((size_t)2 * L * L * nz);
-    self_energy_batch(L, M, de.p, dv.p, nb, dtcb.p, deb.p, dtc.p, nz, dz.p, ds.p,
+    self_energy_batch(L, M, de.p, dv.p, M && all_real(v, (size_t)L * M), nb, dtcb.p, deb.p, dtc.p, nz, dz.p, ds.p,
                       gamma ? dg.p : nullptr, 0);
     QCMG_CUDA(cudaMemcpy(sigma, ds.p, (size_t)2 * L * L * nz * 8, cudaMemcpyDeviceToHost));
     if (gamma) QCMG_CUDA(cudaMemcpy(gamma, dg.p, (size_t)2 * L * L * nz * 8, cudaMemcpyDeviceToHost));
@@ -956,12 +963,8 @@ int qcmg_lattice_set_green(qcmg_lattice* h, int M, const double* e, const double
     Lattice& t = h->lat;
     QCMG_CUDA(cudaSetDevice(t.device));
     t.M = M;
-    auto real = [](const double* a, size_t n) {
-      for (size_t k = 0; k < n; ++k)
-        if (a[2 * k + 1] != 0.0) return false;
-      return true;
-    };
-    t.green_real = real(v, (size_t)t.L * M) && real(tcb, (size_t)t.L * nb);
+    t.v_real = all_real(v, (size_t)t.L * M);
+    t.bath_real = all_real(tcb, (size_t)t.L * nb);
     if (M) {
       t.e.upload(e, M, t.stream);
       t.v.upload(v, (size_t)2 * t.L * M, t.stream);

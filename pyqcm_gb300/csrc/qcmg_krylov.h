@@ -62,7 +62,8 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
 void launch_apply_c(int L, int orb, int spin, int pm, int nup, int ndn, const double* x, double* y,
                     double z, bool accumulate, cudaStream_t s);
 
-void green_function_batch(int L, int M, const double* e, const double* v, int nz, const double* z,
-                          double* G, cudaStream_t s);
+// real: every imaginary part of v (L x M complex) is zero
+void green_function_batch(int L, int M, const double* e, const double* v, bool real, int nz,
+                          const double* z, double* G, cudaStream_t s);
 
 }  // namespace qcmg

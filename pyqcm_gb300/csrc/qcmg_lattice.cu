@@ -44,8 +44,13 @@ __device__ __forceinline__ cdbl cinv(cdbl a) {
 
 // ---------------------------------------------------------------------------
 // Per-frequency preparation: Base(z) = G(z)^-1 + Gamma(z) - Hdiff and
-// log|det G(z)|, one block per frequency, Gauss-Jordan with partial pivoting
-// in shared memory.
+// |det G(z)|, one block per frequency: in-place Gauss-Jordan elimination with
+// row pivoting in shared memory. Two copies of the matrix take turns, so a
+// pivot costs one barrier: every warp finds the pivot row by itself, and the
+// row exchange, the scaling and the elimination are one expression per
+// element (a latency-bound chain of L steps; an augmented matrix with a
+// serial pivot search and seven barriers a step took 62 us for 256
+// frequencies at L = 12, 26 us now).
 
 __global__ void k_freq_prep(int L, int nw, const double2* __restrict__ G,  // nw x L x L (G[b + a L] = G(b,a))
                             const double2* __restrict__ z, int nb, const double2* __restrict__ tcb,
@@ -53,70 +58,57 @@ __global__ void k_freq_prep(int L, int nw, const double2* __restrict__ G,  // nw
                             double2* __restrict__ base, double* __restrict__ logdetG,
                             double* __restrict__ det2, int* __restrict__ dexp) {
   extern __shared__ double2 sm[];
-  double2* A = sm;              // L x 2L augmented [G | I], row-major A[r*2L + c]
-  __shared__ int piv;
+  __shared__ int row_of[32];  // matrix row in each place
+  const int LL = L * L, lane = threadIdx.x & 31;
+  double2 *A = sm, *B1 = sm + LL;
   double dm = 1.0;  // thread 0: |det G|^2 = dm 2^de
   int de = 0;
   const int w = blockIdx.x;
-  const int L2 = 2 * L;
   // G(r, c) with numpy orientation: G stored as G[b + a L] = G(b, a)  ->  G(r,c) = Gw[r + c L]
-  const double2* Gw = G + (size_t)w * L * L;
-  for (int idx = threadIdx.x; idx < L * L2; idx += blockDim.x) {
-    int r = idx / L2, c = idx % L2;
-    A[idx] = c < L ? Gw[r + c * L] : make_double2(c - L == r ? 1.0 : 0.0, 0.0);
-  }
+  const double2* Gw = G + (size_t)w * LL;
+  for (int idx = threadIdx.x; idx < LL; idx += blockDim.x) A[idx] = Gw[idx / L + (idx % L) * L];
+  if (threadIdx.x < 32) row_of[threadIdx.x] = threadIdx.x;
   __syncthreads();
   for (int p = 0; p < L; ++p) {
+    const bool in = lane >= p && lane < L;
+    const double2 mine = in ? A[lane * L + p] : make_double2(0.0, 0.0);
+    const unsigned key = in ? pivot_key(mine.x, mine.y) : 0u;
+    const unsigned most = __reduce_max_sync(0xffffffffu, key);
+    const int piv = __ffs(__ballot_sync(0xffffffffu, in && key == most)) - 1;
+    const double2 pp = A[piv * L + p];
+    const double d2 = fma(pp.x, pp.x, pp.y * pp.y), rd = 1.0 / d2;
+    const cdbl ip = {pp.x * rd, -pp.y * rd};
+    for (int idx = threadIdx.x; idx < LL; idx += blockDim.x) {
+      const int r = idx / L, c = idx - r * L;
+      const double2 pc = A[piv * L + c];
+      const cdbl t = c == p ? ip : cmul({pc.x, pc.y}, ip);  // the pivot row of the result
+      cdbl v = t;
+      if (r != p) {
+        const int src = r == piv ? p : r;
+        const double2 f = A[src * L + p];
+        const double2 a = A[src * L + c];
+        v = cfma_sub(c == p ? cdbl{0.0, 0.0} : cdbl{a.x, a.y}, {f.x, f.y}, t);
+      }
+      B1[idx] = make_double2(v.x, v.y);
+    }
     if (threadIdx.x == 0) {
-      int best = p;
-      double bv = -1.0;
-      for (int r = p; r < L; ++r) {
-        double2 a = A[r * L2 + p];
-        double m = a.x * a.x + a.y * a.y;
-        if (m > bv) {
-          bv = m;
-          best = r;
-        }
-      }
-      piv = best;
-      det_mul(dm, de, bv);
+      det_mul(dm, de, d2);
+      const int t = row_of[p];
+      row_of[p] = row_of[piv];
+      row_of[piv] = t;
     }
     __syncthreads();
-    if (piv != p)
-      for (int c = threadIdx.x; c < L2; c += blockDim.x) {
-        double2 t = A[p * L2 + c];
-        A[p * L2 + c] = A[piv * L2 + c];
-        A[piv * L2 + c] = t;
-      }
-    __syncthreads();
-    const double2 pp = A[p * L2 + p];
-    const cdbl ip = cinv({pp.x, pp.y});
-    __syncthreads();
-    for (int c = threadIdx.x; c < L2; c += blockDim.x) {
-      cdbl v = cmul({A[p * L2 + c].x, A[p * L2 + c].y}, ip);
-      A[p * L2 + c] = make_double2(v.x, v.y);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < L * L2; idx += blockDim.x) {
-      int r = idx / L2, c = idx % L2;
-      if (r == p) continue;
-      double2 f = A[r * L2 + p];
-      double2 a = A[p * L2 + c];
-      if (c == p) continue;  // column p is cleared below
-      cdbl v = cfma_sub({A[idx].x, A[idx].y}, {f.x, f.y}, {a.x, a.y});
-      A[idx] = make_double2(v.x, v.y);
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < L; r += blockDim.x)
-      if (r != p) A[r * L2 + p] = make_double2(0.0, 0.0);
-    __syncthreads();
+    double2* t = A;
+    A = B1;
+    B1 = t;
   }
+  // A is (P G)^-1 = G^-1 P^T: its column k is column row_of[k] of G^-1
   // Base = G^-1 + Gamma - Hdiff, row-major base[r*L + c]
   const double2 zw = z[w];
   double2* B = base + (size_t)w * L * L;
-  for (int idx = threadIdx.x; idx < L * L; idx += blockDim.x) {
-    int r = idx / L, c = idx % L;
-    double2 gi = A[r * L2 + L + c];
+  for (int at = threadIdx.x; at < LL; at += blockDim.x) {
+    const int r = at / L, c = row_of[at % L], idx = r * L + c;
+    double2 gi = A[at];
     double gx = gi.x - Hdiff[idx].x, gy = gi.y - Hdiff[idx].y;
     for (int i = 0; i < nb; ++i) {
       // Gamma(r,c) += tcb(r,i) conj(tcb(c,i)) / (z - eb_i)
@@ -171,14 +163,14 @@ __global__ void k_gamma(int L, int nw, const double2* __restrict__ z, int nb,
   }
 }
 
-void self_energy_batch(int L, int M, const double* e, const double* v, int nb, const double* tcb,
+void self_energy_batch(int L, int M, const double* e, const double* v, bool v_real, int nb, const double* tcb,
                        const double* eb, const double* tc, int nz, const double* z, double* sigma,
                        double* gamma, cudaStream_t s) {
   QCMG_CHECK_ARG(L > 0 && L <= 32, "Green function dimension must be 1..32");
   DevBuf<double> G, ldg, mtc;
   G.alloc((size_t)2 * L * L * nz);
   if (M > 0)
-    green_function_batch(L, M, e, v, nz, z, G.p, s);
+    green_function_batch(L, M, e, v, v_real, nz, z, G.p, s);
   else
     QCMG_CUDA(cudaMemsetAsync(G.p, 0, G.n * 8, s));
   // constant block -t_c
@@ -188,7 +180,7 @@ void self_energy_batch(int L, int M, const double* e, const double* v, int nb, c
   for (double& x : h) x = -x;
   mtc.upload(h.data(), h.size(), s);
   ldg.alloc(nz);
-  const size_t smem = (size_t)L * 2 * L * sizeof(double2);
+  const size_t smem = (size_t)2 * L * L * sizeof(double2);
   k_freq_prep<<<nz, 128, smem, s>>>(L, nz, (const double2*)G.p, (const double2*)z, nb,
                                     (const double2*)tcb, eb, (const double2*)mtc.p,
                                     (double2*)sigma, ldg.p, nullptr, nullptr);
@@ -433,7 +425,7 @@ void Lattice::prepare(int nw, const double* z, cudaStream_t s) {
   ws_z.upload(z, (size_t)2 * nw, s);
   ws_G.alloc((size_t)2 * L * L * nw);
   if (M > 0) {
-    green_function_batch(L, M, e.p, v.p, nw, ws_z.p, ws_G.p, s);
+    green_function_batch(L, M, e.p, v.p, v_real, nw, ws_z.p, ws_G.p, s);
   } else {
     QCMG_CUDA(cudaMemsetAsync(ws_G.p, 0, (size_t)2 * L * L * nw * 8, s));
   }
@@ -441,7 +433,7 @@ void Lattice::prepare(int nw, const double* z, cudaStream_t s) {
   logdetG.alloc(nw);
   det2.alloc(nw);
   dexp.alloc(nw);
-  size_t smem = (size_t)L * 2 * L * sizeof(double2);
+  const size_t smem = (size_t)2 * L * L * sizeof(double2);
   k_freq_prep<<<nw, 128, smem, s>>>(L, nw, (const double2*)ws_G.p, (const double2*)ws_z.p, nb,
                                     (const double2*)tcb.p, eb.p, (const double2*)hdiff.p,
                                     (double2*)base.p, logdetG.p, det2.p, dexp.p);

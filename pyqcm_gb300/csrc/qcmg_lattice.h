@@ -34,8 +34,8 @@ struct Lattice {
   // V(-K) = V(K)^T (real elements, every one with its transposed partner, and
   // a real symmetric Hdiff), and a real Q-matrix and bath: then every
   // K-dependent matrix at -K is the transpose of the one at K
-  bool el_sym = false, green_real = false;
-  bool paired() const { return el_sym && green_real; }
+  bool el_sym = false, v_real = false, bath_real = false;
+  bool paired() const { return el_sym && v_real && bath_real; }
   // the points of a grid that a sum over K needs: all of them, or (paired)
   // one of each pair (K, -K); cached for the last grid asked for
   DevBuf<int> rep;      // flat grid index
@@ -88,9 +88,10 @@ struct Lattice {
 // Cluster self-energy Sigma(z) = z - t_c - Gamma(z) - G(z)^-1 for nz complex
 // frequencies, with G(z) from the Q-matrix (L x M, column-major a + L i) and
 // Gamma(z) from the cluster-bath block tcb (column-major r + L i) and the
-// bath energies eb; t_c row-major; all arrays on the device; sigma (and
-// gamma when not null) nz x L x L row-major.
-void self_energy_batch(int L, int M, const double* e, const double* v, int nb, const double* tcb,
+// bath energies eb; t_c row-major; all arrays on the device (v_real: v's
+// imaginary parts are all zero); sigma (and gamma when not null) nz x L x L
+// row-major.
+void self_energy_batch(int L, int M, const double* e, const double* v, bool v_real, int nb, const double* tcb,
                        const double* eb, const double* tc, int nz, const double* z, double* sigma,
                        double* gamma, cudaStream_t s);
 

@@ -121,3 +121,19 @@ def test_inverse_means(L, kind, g, moments):
     ref = np.einsum("km,zkab->zmab", ph, X) / len(K)
     got = out.view(np.complex128).reshape(len(z), nm, L, L)
     assert np.max(np.abs(got - ref)) < TOL * max(1.0, np.max(np.abs(X)))
+
+
+@pytest.mark.parametrize("L", [1, 2, 5, 12, 32])
+@pytest.mark.parametrize("M", [1, 31, 32, 33, 500])
+@pytest.mark.parametrize("nz", [1, 3, 4, 37])
+@pytest.mark.parametrize("real", [True, False])
+def test_green_function_sums(L, M, nz, real):
+    """G(z) at the tile edges of the pole sum, real (symmetric) and complex."""
+    import pyqcm_gb300 as pg
+    rng = np.random.default_rng([L, M, nz])
+    v = rng.normal(size=(L, M)) + (0 if real else 1j * rng.normal(size=(L, M)))
+    e, z = rng.normal(size=M), rng.normal(size=nz) + 1j * rng.uniform(0.2, 1, nz)
+    ref = np.einsum("ai,zi,bi->zba", v, 1.0 / (z[:, None] - e), v.conj())
+    # M products of size |v|^2 / Im z, each with a few roundings
+    bound = 8 * np.finfo(float).eps * M * np.max(np.abs(v)) ** 2 / np.min(z.imag)
+    assert np.max(np.abs(pg.green_function(e, v, z) - ref)) < bound
