@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <vector>
 
 #include "qcmg_fx.cuh"
@@ -133,35 +134,68 @@ __global__ void k_fx_to_host(const int64_t* __restrict__ q, double* __restrict__
 }
 
 constexpr int kRedBlocksFx = 1024;
+constexpr int kFinalThreads = 512;
 
-// Exact <a, b> partials, two elements per 16-byte load (the fixed-point
-// vectors come from cudaMalloc, so even indices are 16-byte aligned); the
-// integer sums are exact, so the summation order does not matter.
-__global__ void __launch_bounds__(256) k_fx_dot(const int64_t* __restrict__ a,
-                                                const int64_t* __restrict__ b, size_t n,
-                                                I128* __restrict__ part) {
-  I128 s = {0, 0};
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const size_t n2 = n / 2;
-  const longlong2* a2 = reinterpret_cast<const longlong2*>(a);
-  const longlong2* b2 = reinterpret_cast<const longlong2*>(b);
-#pragma unroll 2
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n2; j += stride) {
-    const longlong2 x = __ldcs(a2 + j), y = __ldcs(b2 + j);
-    s = add128(s, shr128(mul_s64(x.x, y.x), kDotShift));
-    s = add128(s, shr128(mul_s64(x.y, y.y), kDotShift));
-  }
-  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0)
-    s = add128(s, shr128(mul_s64(a[n - 1], b[n - 1]), kDotShift));
-  block_store128(s, part);
+// log2 rounded up, as ceil_log2 (x > 0)
+__device__ __forceinline__ int ceil_log2_dev(double x) {
+  if (!(x > 0.0)) return 0;
+  int ex;
+  const double m = frexp(x, &ex);
+  return m == 0.5 ? ex - 1 : ex;
 }
 
-// Sum of the block partials by one warp (launched with 32 threads).
-__global__ void k_fx_final(const I128* __restrict__ part, int np, I128* __restrict__ out) {
+// Sum of one block's share of the 128-bit partials, complete in thread 0.
+__device__ __forceinline__ I128 final_sum128(const I128* __restrict__ part, int np) {
+  __shared__ I128 total;
   I128 s = {0, 0};
-  for (int i = threadIdx.x; i < np; i += blockDim.x) s = add128(s, part[i]);
-  s = warp_sum128(s);
-  if (threadIdx.x == 0) *out = s;
+  for (int i = threadIdx.x; i < np; i += kFinalThreads) s = add128(s, part[i]);
+  block_store128(s, &total - blockIdx.x);
+  __syncthreads();
+  return total;
+}
+
+// alpha = <v, w> from pass D's partials, and from it the coefficients of the
+// update w - alpha v - beta p: the same IEEE operations in the same order as
+// on the host (explicit roundings, no contraction), so the host need not
+// wait between the product and the update.  A single warp walking the ~1,000
+// partials took 12.1 us, this block 5.2 us (the norm's 3.8 us).
+__global__ void __launch_bounds__(kFinalThreads)
+    k_fx_alpha(const I128* __restrict__ part, int np, double vc, int vE, int vmb, double wc, int wE,
+               int wmb, double bp, long long mb, int pEe, FxStep* __restrict__ st) {
+  const I128 h = final_sum128(part, np);
+  if (threadIdx.x != 0) return;
+  const double r = __dadd_rn(ldexp((double)h.hi, 64), (double)h.lo);
+  const double alpha = __dmul_rn(__dmul_rn(vc, wc), ldexp(r, kDotShift + vE + wE));
+  const double k = __ddiv_rn(__dmul_rn(alpha, vc), wc);
+  const double bw = ldexp(1.0, wE + wmb), bv = __dmul_rn(fabs(k), ldexp(1.0, vE + vmb));
+  const int Eo = ceil_log2_dev(__dadd_rn(__dadd_rn(bw, bv), bp)) - kFxBits;
+  long long ma = 0;
+  int e = 0;
+  if (k != 0.0 && isfinite(k)) {
+    int ex;
+    const double m = frexp(k, &ex);
+    ma = llrint(ldexp(m, 53));  // an integer already
+    e = ex - 53;
+  }
+  st->alpha = alpha;
+  st->ma = ma;
+  st->mb = mb;
+  st->sw = Eo - wE;
+  st->sa = Eo - vE - e;
+  st->sb = Eo - pEe;
+  st->Eo = Eo;
+  st->qmax = 0;
+}
+
+// The update's norm from its partials.
+__global__ void __launch_bounds__(kFinalThreads) k_fx_norm(const I128* __restrict__ part, int np,
+                                                          const int* __restrict__ err,
+                                                          FxStep* __restrict__ st) {
+  const I128 h = final_sum128(part, np);
+  if (threadIdx.x != 0) return;
+  st->n_hi = h.hi;
+  st->n_lo = h.lo;
+  st->err = err ? *err : 0;
 }
 
 // Fused Lanczos update:
@@ -169,10 +203,12 @@ __global__ void k_fx_final(const I128* __restrict__ part, int np, I128* __restri
 // written over q_w, with exact |q_o|^2 partials and max|q_o|.
 __global__ void __launch_bounds__(256) k_fx_update(int64_t* __restrict__ w,
                                                    const int64_t* __restrict__ v,
-                                                   const int64_t* __restrict__ p, size_t n, int sw,
-                                                   int64_t ma, int sa, int64_t mb, int sb,
-                                                   I128* __restrict__ part,
-                                                   unsigned long long* __restrict__ qmax) {
+                                                   const int64_t* __restrict__ p, size_t n,
+                                                   FxStep* __restrict__ st,
+                                                   I128* __restrict__ part) {
+  const int sw = st->sw, sa = st->sa, sb = st->sb;
+  const int64_t ma = st->ma, mb = st->mb;
+  unsigned long long* qmax = &st->qmax;
   I128 s = {0, 0};
   unsigned long long m = 0;
   auto one = [&](int64_t wi, int64_t vi, int64_t pi) {
@@ -350,11 +386,19 @@ bool fx_prepare(qcmg_hamiltonian* H) {
   }
   T.bound = dmax + T.t_up * T.maxdeg_up + T.t_dn * T.maxdeg_dn;
   T.b = ceil_log2(std::max(T.bound, 1.0));
-  // rows per band of pass D: ~48 MB of x per band (QCMG_FX_BAND_MB overrides)
+  // Rows per band of pass D: ~48 MB of x per band (QCMG_FX_BAND_MB
+  // overrides).  A band of a down state is one warp's work, and a sector
+  // that fits in one such band has too few of them (924 warps for 924 x 924
+  // states): small sectors take shorter bands, down to one 64-row sweep, so
+  // that the items fill the chip's resident warps (48 per SM) twice.  x is
+  // L2-resident there whatever the band.  924 x 924, with the dot product:
+  // 49.5 us -> 14.3 us (cold).
   double band_mb = 48.0;
   if (const char* v = std::getenv("QCMG_FX_BAND_MB")) band_mb = std::max(1.0, std::atof(v));
   size_t band = (size_t)(band_mb * 1.0e6 / (8.0 * std::max<uint32_t>(H->dd, 1)));
   band = std::max<size_t>(256, (band / 256) * 256);
+  const size_t fill = (size_t)H->du * H->dd / ((size_t)2 * 48 * 152) / 64 * 64;
+  band = std::min(band, std::max<size_t>(64, fill));
   T.band = (uint32_t)std::min<size_t>(band, H->du);
   T.state = 1;
   return true;
@@ -396,19 +440,14 @@ void fx_to_f64(const FxVec& v, double* x, cudaStream_t s) {
   QCMG_CUDA(cudaGetLastError());
 }
 
-// exact <a, b> as a double
-double FxReducer::dot(const FxVec& a, const FxVec& b, cudaStream_t s) {
-  part.alloc(kRedBlocksFx);
-  out.alloc(1);
-  unsigned g = (unsigned)std::min<size_t>(kRedBlocksFx, std::max<size_t>(1, (a.n + 255) / 256));
-  k_fx_dot<<<g, 256, 0, s>>>(a.buf.p, b.buf.p, a.n, part.p);
-  k_fx_final<<<1, 32, 0, s>>>(part.p, (int)g, out.p);
-  QCMG_CUDA(cudaGetLastError());
-  I128 h;
-  QCMG_CUDA(cudaMemcpyAsync(&h, out.p, sizeof(I128), cudaMemcpyDeviceToHost, s));
-  QCMG_CUDA(cudaStreamSynchronize(s));
-  double r = std::ldexp((double)h.hi, 64) + (double)h.lo;
-  return a.c * b.c * std::ldexp(r, kDotShift + a.E + b.E);
+FxReducer::~FxReducer() {
+  if (host) cudaFreeHost(host);
+}
+
+void FxReducer::init(size_t partials) {
+  part.alloc(partials);
+  step.alloc(1);
+  if (!host) QCMG_CUDA(cudaMallocHost(&host, sizeof(FxStep)));
 }
 
 // ---------------------------------------------------------------------------
@@ -417,8 +456,8 @@ double FxReducer::dot(const FxVec& a, const FxVec& b, cudaStream_t s) {
 // y = H x  (or y = H x + gamma * yin with yin != nullptr, yin may be &y).
 // The output exponent follows from the bound |H|_inf (T.b) and the input's
 // largest component; c_y = c_x.
-void fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
-               FxReducer* dot, double* dot_out) {
+unsigned fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
+                   FxReducer* dot) {
   FxTables& T = H->fx;
   cudaStream_t s = H->stream;
   const size_t n = H->dim;
@@ -488,10 +527,6 @@ void fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, 
   A.dot_x = nullptr;
   A.dot_part = nullptr;
   if (dot) {
-    int sms = 0;
-    QCMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device));
-    dot->part.alloc(std::max<size_t>(kRedBlocksFx, product_dot_partials(sms)));
-    dot->out.alloc(1);
     A.dot_x = x.buf.p;
     A.dot_part = dot->part.p;
   }
@@ -499,15 +534,7 @@ void fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, 
   y.E = Eo;
   y.mb = kFxBits;
   y.c = x.c;
-  if (dot) {
-    k_fx_final<<<1, 32, 0, s>>>(dot->part.p, (int)np, dot->out.p);
-    QCMG_CUDA(cudaGetLastError());
-    I128 h;
-    QCMG_CUDA(cudaMemcpyAsync(&h, dot->out.p, sizeof(I128), cudaMemcpyDeviceToHost, s));
-    QCMG_CUDA(cudaStreamSynchronize(s));
-    const double r = std::ldexp((double)h.hi, 64) + (double)h.lo;
-    *dot_out = x.c * y.c * std::ldexp(r, kDotShift + x.E + y.E);
-  }
+  return np;
 }
 
 void fx_check_error(qcmg_hamiltonian* H) {
@@ -558,105 +585,169 @@ void fx_matvec_to_host(qcmg_hamiltonian* H, const double* x, double* yh, bool ac
 // Lanczos on FX vectors: the reference's recurrence (Lanczos.hpp:64-93)
 // written with normalized vectors, w = H v_j - alpha v_j - beta v_{j-1}.
 
-static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec* p, double alpha,
-                      double beta, FxReducer& red, double* norm2) {
+// w <- w - alpha v - beta p with alpha = <v, w> from the np partials that the
+// product left in red.part; returns alpha and |w|^2.
+static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec* p, unsigned np,
+                      double beta, FxReducer& red, double* alpha, double* norm2) {
   cudaStream_t s = H->stream;
   const size_t n = w.n;
-  // bound of the result in units of c_w
-  double bw = std::ldexp(1.0, w.E + w.mb);
-  double bv = std::fabs(alpha * v.c / w.c) * std::ldexp(1.0, v.E + v.mb);
-  double bp = p ? std::fabs(beta * p->c / w.c) * std::ldexp(1.0, p->E + p->mb) : 0.0;
-  int Eo = ceil_log2(bw + bv + bp) - kFxBits;
-  int e;
-  int64_t ma = 0, mb = 0;
-  int sa = 0, sb = 0;
-  split_double(alpha * v.c / w.c, &ma, &e);
-  sa = Eo - v.E - e;
+  double bp = 0.0;  // bound of the beta term, in units of c_w
+  int64_t mb = 0;
+  int e = 0;
   if (p) {
+    bp = std::fabs(beta * p->c / w.c) * std::ldexp(1.0, p->E + p->mb);
     split_double(beta * p->c / w.c, &mb, &e);
-    sb = Eo - p->E - e;
+    e += p->E;
   }
-  red.part.alloc(kRedBlocksFx);
-  red.out.alloc(1);
-  red.umax.alloc(1);
-  QCMG_CUDA(cudaMemsetAsync(red.umax.p, 0, 8, s));
+  k_fx_alpha<<<1, kFinalThreads, 0, s>>>(red.part.p, (int)np, v.c, v.E, v.mb, w.c, w.E, w.mb, bp,
+                                         (long long)mb, e, red.step.p);
   unsigned g = (unsigned)std::min<size_t>(kRedBlocksFx, std::max<size_t>(1, (n + 255) / 256));
-  k_fx_update<<<g, 256, 0, s>>>(w.buf.p, v.buf.p, p ? p->buf.p : nullptr, n, Eo - w.E, ma, sa, mb,
-                                sb, red.part.p, red.umax.p);
-  k_fx_final<<<1, 32, 0, s>>>(red.part.p, (int)g, red.out.p);
+  k_fx_update<<<g, 256, 0, s>>>(w.buf.p, v.buf.p, p ? p->buf.p : nullptr, n, red.step.p, red.part.p);
+  k_fx_norm<<<1, kFinalThreads, 0, s>>>(red.part.p, (int)g, H->fx.err.p, red.step.p);
   QCMG_CUDA(cudaGetLastError());
-  I128 h;
-  unsigned long long um = 0;
-  int err = 0;
-  QCMG_CUDA(cudaMemcpyAsync(&h, red.out.p, sizeof(I128), cudaMemcpyDeviceToHost, s));
-  QCMG_CUDA(cudaMemcpyAsync(&um, red.umax.p, 8, cudaMemcpyDeviceToHost, s));
-  if (H->fx.err.p) QCMG_CUDA(cudaMemcpyAsync(&err, H->fx.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  QCMG_CUDA(cudaMemcpyAsync(red.host, red.step.p, sizeof(FxStep), cudaMemcpyDeviceToHost, s));
   QCMG_CUDA(cudaStreamSynchronize(s));
-  if (err) throw Error(QCMG_ERR_CUDA, "a bulk copy into shared memory did not complete in time");
-  w.E = Eo;
-  w.mb = bitlen(um);
-  double r = std::ldexp((double)h.hi, 64) + (double)h.lo;
-  *norm2 = w.c * w.c * std::ldexp(r, kDotShift + 2 * Eo);
+  const FxStep& h = *red.host;
+  if (h.err) throw Error(QCMG_ERR_CUDA, "a bulk copy into shared memory did not complete in time");
+  w.E = h.Eo;
+  w.mb = bitlen(h.qmax);
+  *alpha = h.alpha;
+  const double r = std::ldexp((double)h.n_hi, 64) + (double)h.n_lo;
+  *norm2 = w.c * w.c * std::ldexp(r, kDotShift + 2 * h.Eo);
 }
+
+// One stored vector's term of the ground state.
+struct FxTerm {
+  const int64_t* q;
+  int64_t m;
+  int s;
+};
+
+// psi_i = 2^E sum_k round(q_k,i m_k 2^-s_k): the integer sum that adding the
+// terms one by one gives, in any order.  Every vector is read once.
+__global__ void __launch_bounds__(256) k_fx_combine(const FxTerm* __restrict__ t, int nt, size_t n,
+                                                    int E, double* __restrict__ psi) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int64_t g = 0;
+#pragma unroll 8
+  for (int k = 0; k < nt; ++k) g += mul_fix(__ldcs(t[k].q + i), t[k].m, t[k].s);
+  psi[i] = fx_to_f64(g, E);
+}
+
+// Device memory for the Lanczos vectors of one solve: slots of n elements,
+// 16-byte aligned, allocated many at a time.  get() returns null when the
+// next allocation would take more than a quarter of the memory that was free
+// at the start, or fails.
+struct FxSlots {
+  std::deque<DevBuf<int64_t>> blocks;
+  size_t stride = 0, left = 0, budget = 0;
+  int64_t* next = nullptr;
+  explicit FxSlots(size_t n) : stride((n + 1) & ~(size_t)1) {}
+  void measure() {
+    size_t fr = 0, total = 0;
+    QCMG_CUDA(cudaMemGetInfo(&fr, &total));
+    budget = std::max(fr / 4, 3 * stride * 8);
+  }
+  bool room_for(size_t cnt) const { return cnt <= budget / (stride * 8); }
+  int64_t* get(size_t want) {
+    if (left == 0) {
+      const size_t bytes = stride * 8;
+      const size_t cnt = std::max<size_t>(std::min(want, ((size_t)1 << 30) / bytes), blocks.empty() ? 3 : 1);
+      if (cnt * bytes > budget) return nullptr;
+      blocks.emplace_back();
+      try {
+        blocks.back().alloc(cnt * stride);
+      } catch (const Error& e) {
+        if (e.code != QCMG_ERR_NOMEM || blocks.size() == 1) throw;
+        cudaGetLastError();
+        return nullptr;
+      }
+      budget -= cnt * bytes;
+      left = cnt;
+      next = blocks.back().p;
+    }
+    int64_t* r = next;
+    next += stride;
+    --left;
+    return r;
+  }
+};
 
 LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, int max_iter,
                          double* psi_dev) {
   LanczosResult res;
   cudaStream_t s = H->stream;
+  const size_t n = H->dim;
   FxReducer red;
+  int sms = 0;
+  QCMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device));
+  red.init(std::max<size_t>(kRedBlocksFx, product_dot_partials(sms)));
   DevBuf<unsigned long long> tmp;
-  FxVec vbuf[3];
-  FxVec x0;
-  fx_from_f64(x0_dev, H->dim, x0, s, tmp);
-  auto run = [&](bool replay, const std::vector<double>* z, FxVec* gs) {
+  FxSlots slots(n);
+  // The Lanczos vectors are kept when the ground state is wanted and 300 of
+  // them (a solve takes 80 to 250) fit in a quarter of the free memory: psi
+  // is then one pass over them instead of a second run of the recurrence
+  // (3x4 cluster, 220 steps: a product and an update per step against 1.5 GB
+  // read once).
+  slots.measure();
+  bool keep = psi_dev != nullptr && slots.room_for((size_t)std::min(max_iter + 2, 300));
+  const size_t want = keep ? 64 : 3;
+  FxVec x0, vbuf[3];
+  vbuf[0].buf.borrow(slots.get(want), n);
+  for (FxVec& b : vbuf) b.n = n;
+  x0.buf.borrow(vbuf[0].buf.p, n);
+  x0.n = n;
+  fx_from_f64(x0_dev, n, x0, s, tmp);
+  struct Kept {
+    const int64_t* q;
+    int E;
+    double c;
+  };
+  std::vector<Kept> kept;
+  std::vector<double> z;
+  // the recurrence; replay: on the recorded coefficients, accumulating gs
+  auto run = [&](bool replay, FxVec* gs) {
     FxVec* v = &vbuf[0];
     FxVec* p = &vbuf[1];
     FxVec* w = &vbuf[2];
-    v->alloc(H->dim);
-    QCMG_CUDA(cudaMemcpyAsync(v->buf.p, x0.buf.p, H->dim * 8, cudaMemcpyDeviceToDevice, s));
+    if (replay) fx_from_f64(x0_dev, n, *v, s, tmp);
     v->E = x0.E;
     v->mb = x0.mb;
     v->c = x0.c;
     bool have_p = false;
     double beta_prev = 0.0;
-    std::vector<double> zz;
-    const int nsteps = replay ? (int)z->size() : max_iter + 1;
+    const int nsteps = replay ? (int)z.size() : max_iter + 1;
     for (int j = 0; j < nsteps; ++j) {
       if (replay) {
         // gs += z_j v_j
-        if (j == 0) {
-          gs->alloc(H->dim);
-          QCMG_CUDA(cudaMemsetAsync(gs->buf.p, 0, H->dim * 8, s));
-          double bnd = 0.0;
-          for (double zj : *z) bnd += std::fabs(zj);
-          gs->E = ceil_log2(bnd) - kFxBits;  // |psi_i| <= sum_j |z_j| |v_j|_max <= sum |z_j|
-          gs->c = 1.0;
-          gs->mb = kFxBits;
-        }
         int64_t m;
         int e;
-        split_double((*z)[j] * v->c, &m, &e);
-        k_fx_axpy<<<grid_ew(H->dim), 256, 0, s>>>(gs->buf.p, v->buf.p, H->dim, 0, m,
-                                                  gs->E - v->E - e);
+        split_double(z[j] * v->c, &m, &e);
+        k_fx_axpy<<<grid_ew(n), 256, 0, s>>>(gs->buf.p, v->buf.p, n, 0, m, gs->E - v->E - e);
         QCMG_CUDA(cudaGetLastError());
         if (j + 1 == nsteps) break;
+      } else if (keep) {
+        kept.push_back({v->buf.p, v->E, v->c});
+        int64_t* q = slots.get(want);
+        if (!q) {  // no room for more: a replay will follow
+          keep = false;
+          q = const_cast<int64_t*>(kept[0].q);  // neither v nor p: j >= 2 here
+        }
+        w->buf.borrow(q, n);
+      } else if (j < 2 && !w->buf.p) {
+        w->buf.borrow(slots.get(want), n);
       }
       // alpha = <v, H v> comes out of the product's second pass
-      double a = 0.0;
-      if (replay) {
-        fx_matvec(H, *v, *w, nullptr, 0.0);
-        a = res.alpha[j];
-      } else {
-        fx_matvec(H, *v, *w, nullptr, 0.0, &red, &a);
-      }
-      double n2 = 0.0;
-      fx_update(H, *w, *v, have_p ? p : nullptr, a, beta_prev, red, &n2);
-      double b = replay ? res.beta[j] : std::sqrt(n2);
+      const unsigned np = fx_matvec(H, *v, *w, nullptr, 0.0, &red);
+      double a = 0.0, n2 = 0.0;
+      fx_update(H, *w, *v, have_p ? p : nullptr, np, beta_prev, red, &a, &n2);
+      const double b = replay ? res.beta[j] : std::sqrt(n2);
       if (!replay) {
         res.alpha.push_back(a);
         res.beta.push_back(b);
-        res.energy = tridiag_lowest(res.alpha, res.beta, zz);
-        double ritz = std::fabs(zz.back() * b);
+        res.energy = tridiag_lowest(res.alpha, res.beta, z);
+        double ritz = std::fabs(z.back() * b);
         if (!std::isfinite(res.energy) || !std::isfinite(ritz))
           throw Error(QCMG_ERR_NUMERIC, "Lanczos produced a non-finite value");
         if (ritz <= tol || b == 0.0) break;
@@ -678,16 +769,37 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
       have_p = true;
       beta_prev = b;
     }
-    if (!replay) res.niter = (int)res.alpha.size();
-    return zz;
   };
-  std::vector<double> z = run(false, nullptr, nullptr);
-  if (psi_dev) {
-    FxVec gs;
-    run(true, &z, &gs);
-    fx_to_f64(gs, psi_dev, s);
+  run(false, nullptr);
+  res.niter = (int)res.alpha.size();
+  if (!psi_dev) return res;
+  double bnd = 0.0;
+  for (double zj : z) bnd += std::fabs(zj);
+  const int gE = ceil_log2(bnd) - kFxBits;  // |psi_i| <= sum_j |z_j| |v_j|_max <= sum |z_j|
+  if (keep) {
+    std::vector<FxTerm> t(z.size());
+    for (size_t j = 0; j < z.size(); ++j) {
+      int e;
+      split_double(z[j] * kept[j].c, &t[j].m, &e);
+      t[j].q = kept[j].q;
+      t[j].s = gE - kept[j].E - e;
+    }
+    DevBuf<FxTerm> dt;
+    dt.upload(t.data(), t.size(), s);
+    k_fx_combine<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dt.p, (int)t.size(), n, gE, psi_dev);
+    QCMG_CUDA(cudaGetLastError());
     QCMG_CUDA(cudaStreamSynchronize(s));
+    return res;
   }
+  FxVec gs;
+  gs.alloc(n);
+  QCMG_CUDA(cudaMemsetAsync(gs.buf.p, 0, n * 8, s));
+  gs.E = gE;
+  gs.c = 1.0;
+  gs.mb = kFxBits;
+  run(true, &gs);
+  fx_to_f64(gs, psi_dev, s);
+  QCMG_CUDA(cudaStreamSynchronize(s));
   return res;
 }
 

@@ -10,11 +10,27 @@ namespace qcmg {
 
 struct I128;
 
+// Scalars of one Lanczos step, written on the device: alpha and the update's
+// coefficients by the final sum of <v, H v>, the norm by the final sum of
+// the update, and read back together (one wait per step).
+struct FxStep {
+  double alpha;
+  long long ma, mb;    // mantissas of alpha c_v / c_w and beta c_p / c_w
+  int sw, sa, sb, Eo;  // shifts of the three terms, exponent of the result
+  long long n_hi;      // sum of squares >> kDotShift, 128 bits
+  unsigned long long n_lo, qmax;
+  int err;             // bounded-wait failure flag of the product kernels
+};
+
 struct FxReducer {
   DevBuf<I128> part;
-  DevBuf<I128> out;
-  DevBuf<unsigned long long> umax;
-  double dot(const FxVec& a, const FxVec& b, cudaStream_t s);
+  DevBuf<FxStep> step;
+  FxStep* host = nullptr;  // page-locked
+  FxReducer() = default;
+  FxReducer(const FxReducer&) = delete;
+  FxReducer& operator=(const FxReducer&) = delete;
+  ~FxReducer();
+  void init(size_t partials);
 };
 
 // Prepares the fixed-point tables; false if the Hamiltonian does not have
@@ -23,10 +39,10 @@ bool fx_prepare(qcmg_hamiltonian* H);
 void fx_from_f64(const double* x, size_t n, FxVec& v, cudaStream_t s,
                  DevBuf<unsigned long long>& tmp);
 void fx_to_f64(const FxVec& v, double* x, cudaStream_t s);
-// With dot set, also returns <x, y> for the finished y (computed by the
-// product's second pass, bit-identical to FxReducer::dot(x, y)).
-void fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
-               FxReducer* dot = nullptr, double* dot_out = nullptr);
+// With dot set, the product's second pass also leaves block partials of
+// <x, y> (for the finished y) in dot->part; returns their number.
+unsigned fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
+                   FxReducer* dot = nullptr);
 // Throws if a kernel of the fast path reported a bounded-wait failure.
 void fx_check_error(qcmg_hamiltonian* H);
 // y (+)= H x on FP64 device vectors through the fixed-point product.

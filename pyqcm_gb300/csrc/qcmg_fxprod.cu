@@ -91,8 +91,11 @@ __device__ __forceinline__ void slab_range(uint32_t a, uint32_t du, uint32_t* e0
 
 // Offset (elements) of the second slab buffer: a compile-time constant, so
 // one address serves the gathers from both slabs.  Two slabs per round need
-// slab_stride(du) <= kSlab1Off (du <= 14190).
-constexpr uint32_t kSlab1Off = 14208;
+// slab_stride(du) <= kSlab1Off (du <= 14190).  Slabs of du <= 1006 take the
+// small offset: their two buffers are 16 KB, so four 256-thread CTAs (eight
+// slabs) share an SM instead of one 1024-thread CTA (two slabs), and a
+// 924 x 924 sector is one round instead of four: 17.3 us -> 11.3 us (cold).
+constexpr uint32_t kSlab1Off = 14208, kSlab1OffSmall = 1024;
 
 // Groups of a row whose columns are requested together before the gathers.
 constexpr int kPreGroups = 4;
@@ -106,8 +109,8 @@ __device__ __forceinline__ int64_t lds64(uint32_t addr) {
 }
 
 // Sums of the four staged entries named by one group of columns, in each of
-// the NS slabs (the second slab kSlab1Off elements above the first).
-template <int NS>
+// the NS slabs (the second slab OFF elements above the first).
+template <int NS, uint32_t OFF>
 __device__ __forceinline__ void gather_group(uint32_t vbase, uint2 w, int64_t (&t)[NS]) {
   const uint32_t a0 = vbase + ((w.x & 0xffffu) << 3);
   const uint32_t a1 = vbase + ((w.x >> 16) << 3);
@@ -115,7 +118,7 @@ __device__ __forceinline__ void gather_group(uint32_t vbase, uint2 w, int64_t (&
   const uint32_t a3 = vbase + ((w.y >> 16) << 3);
   const int64_t x0 = lds64<0>(a0), x1 = lds64<0>(a1), x2 = lds64<0>(a2), x3 = lds64<0>(a3);
   if (NS == 2) {
-    constexpr uint32_t O = kSlab1Off * 8;
+    constexpr uint32_t O = OFF * 8;
     const int64_t y0 = lds64<O>(a0), y1 = lds64<O>(a1), y2 = lds64<O>(a2), y3 = lds64<O>(a3);
     t[NS - 1] = (y0 + y1) + (y2 + y3);
   }
@@ -129,8 +132,10 @@ __device__ __forceinline__ void gather_group(uint32_t vbase, uint2 w, int64_t (&
 // columns point at zero slots du..du+15.  With NS = 2 the grid is even, so the
 // two slabs of a round have the same alignment (view offset).  With NS = 1
 // a second CTA on the SM computes while this one's copy is in flight.
-template <int INTER, int NS, bool FAST>
-__global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_passU4(FxProdArgs A) {
+template <int INTER, int NS, bool FAST, bool SMALL>
+__global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 : NS == 1 ? 2 : 1)
+    k_fx_passU4(FxProdArgs A) {
+  constexpr uint32_t kOff = SMALL ? kSlab1OffSmall : kSlab1Off;
   extern __shared__ __align__(16) int64_t smem_slab[];
   __shared__ __align__(8) uint64_t bars[NS];
   const uint32_t du = A.du, dd = A.dd;
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
         slab_range(a, du, &e0, &e1);
         const unsigned bytes = (e1 - e0) * 8u;
         mbar_arrive_expect_tx(&bars[s], bytes);
-        bulk_g2s(smem_slab + s * kSlab1Off + 2 * e0, A.x + (size_t)a * du + e0, bytes, &bars[s]);
+        bulk_g2s(smem_slab + s * kOff + 2 * e0, A.x + (size_t)a * du + e0, bytes, &bars[s]);
       }
     }
     bool ok = true;
@@ -176,7 +181,7 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
       return;
     }
     parity ^= 1u;
-    // element j of slab s is view[s * kSlab1Off + j]; the copy landed at
+    // element j of slab s is view[s * kOff + j]; the copy landed at
     // buf + 2*e0, so view = buf + e0 (e0 is the same for both slabs).
     uint32_t e0, e1;
     slab_range(a0, du, &e0, &e1);
@@ -193,13 +198,13 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
       dda32[s] = FAST ? A.ddn32[a] : 0;
       dbits[s] = A.bin_dn[a];
       if (tid == 0 && a0 + s * G < dd) {
-        int64_t* v = smem_slab + s * kSlab1Off + e0;
+        int64_t* v = smem_slab + s * kOff + e0;
         const size_t base = (size_t)a * du;
         if (e0 == 1u) v[0] = A.x[base];
         if (e1 == du - 1u) v[du - 1] = A.x[base + du - 1];
       }
       if (tid < (int)kZeroSlots && a0 + s * G < dd)
-        smem_slab[s * kSlab1Off + e0 + du + tid] = 0;  // zero slots for padding columns
+        smem_slab[s * kOff + e0 + du + tid] = 0;  // zero slots for padding columns
     }
     __syncthreads();
     const uint32_t vbase = smem_u32(view);
@@ -239,7 +244,7 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
 #pragma unroll
       for (int g = 0; g < kPreGroups; ++g) {
         int64_t t[NS];
-        gather_group<NS>(vbase, w[g], t);
+        gather_group<NS, kOff>(vbase, w[g], t);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
           if ((uint32_t)g < gp)
@@ -250,7 +255,7 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
       }
       for (uint32_t g = kPreGroups; g < gt; ++g) {  // rows with more than kPreGroups groups
         int64_t t[NS];
-        gather_group<NS>(vbase, __ldg(A.ell4 + (size_t)g * du + i), t);
+        gather_group<NS, kOff>(vbase, __ldg(A.ell4 + (size_t)g * du + i), t);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
           if (g < gp)
@@ -278,7 +283,7 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
               u &= u - 1;
             }
           }
-          out += rshift_fixed(view[s * kSlab1Off + i] * (int64_t)Dn, A.t_d, A.r_d);
+          out += rshift_fixed(view[s * kOff + i] * (int64_t)Dn, A.t_d, A.r_d);
           if (A.yin) out += rshift_fixed(A.neg_in ? -yv[s] : yv[s], A.t_in, A.r_in);
         } else {
           out = mul_fix(sp[s] - sn[s], A.mt_up, A.sh_up);
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(NS == 1 ? 512 : 1024, NS == 1 ? 2 : 1) k_fx_pa
               u &= u - 1;
             }
           }
-          out += mul_fix(view[s * kSlab1Off + i], D, A.sh_d);
+          out += mul_fix(view[s * kOff + i], D, A.sh_d);
           if (A.yin) out += mul_fix(yv[s], A.m_in, A.sh_in);
         }
         __stcs(A.y + (size_t)a * du + i, out);
@@ -541,12 +546,12 @@ int choose_slabs_per_pass(uint32_t du, int max_optin_smem) {
 // ---------------------------------------------------------------------------
 // launcher
 
-template <int NS, typename Kern>
+template <int NS, bool SMALL, typename Kern>
 static void launch_passU4(Kern kern, const qcmg_hamiltonian* H, const FxProdArgs& A, int sms,
                           cudaStream_t s) {
-  const size_t smem = ((NS == 2 ? (size_t)kSlab1Off : 0) + slab_stride(H->du)) * 8;
+  const size_t smem = ((NS == 2 ? (size_t)(SMALL ? kSlab1OffSmall : kSlab1Off) : 0) + slab_stride(H->du)) * 8;
   QCMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int tmax = NS == 1 ? 512 : 1024;
+  const int tmax = SMALL ? 256 : NS == 1 ? 512 : 1024;
   const int threads = std::min<int>(tmax, (int)((H->du + 127) / 128 * 128));
   int per_sm = 0;
   QCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
@@ -566,24 +571,27 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   // and the diagonal is narrow (the Hubbard form with t = 1 and small-integer
   // energies); everything else uses the 128-bit products
   const bool fast = A.d_tz >= 0 && A.p2_up >= 0 && A.p2_dn >= 0 && (!A.yin || A.p2_in >= 0);
-  auto passU4 = [&](auto ns_tag, auto fast_tag) {
+  auto passU4 = [&](auto ns_tag, auto small_tag, auto fast_tag) {
     constexpr int NS = decltype(ns_tag)::value;
-    constexpr bool F = decltype(fast_tag)::value;
-    if (ik == QCMG_INTER_NONE) launch_passU4<NS>(k_fx_passU4<QCMG_INTER_NONE, NS, F>, H, A, sms, s);
-    else if (ik == QCMG_INTER_ONSITE) launch_passU4<NS>(k_fx_passU4<QCMG_INTER_ONSITE, NS, F>, H, A, sms, s);
-    else launch_passU4<NS>(k_fx_passU4<QCMG_INTER_GENERAL, NS, F>, H, A, sms, s);
+    constexpr bool S = decltype(small_tag)::value, F = decltype(fast_tag)::value;
+    if (ik == QCMG_INTER_NONE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_NONE, NS, F, S>, H, A, sms, s);
+    else if (ik == QCMG_INTER_ONSITE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_ONSITE, NS, F, S>, H, A, sms, s);
+    else launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_GENERAL, NS, F, S>, H, A, sms, s);
   };
   using One = std::integral_constant<int, 1>;
   using Two = std::integral_constant<int, 2>;
-  using Fast = std::true_type;
-  using Full = std::false_type;
+  using Yes = std::true_type;
+  using No = std::false_type;
   // pass U
-  if (T.ns == 2) {
-    if (fast) passU4(Two{}, Fast{});
-    else passU4(Two{}, Full{});
+  if (T.ns == 2 && slab_stride(H->du) <= kSlab1OffSmall) {
+    if (fast) passU4(Two{}, Yes{}, Yes{});
+    else passU4(Two{}, Yes{}, No{});
+  } else if (T.ns == 2) {
+    if (fast) passU4(Two{}, No{}, Yes{});
+    else passU4(Two{}, No{}, No{});
   } else if (T.ns == 1) {
-    if (fast) passU4(One{}, Fast{});
-    else passU4(One{}, Full{});
+    if (fast) passU4(One{}, No{}, Yes{});
+    else passU4(One{}, No{}, No{});
   } else {
     const size_t smem = (size_t)H->du * 8;
     const int threads = H->du >= 512 ? 512 : (H->du >= 256 ? 256 : 128);
