@@ -41,6 +41,7 @@ struct BatchSector {
   DevBuf<double> r, q, coef, part;  // coef: alpha (cap) then beta (cap)
   DevBuf<int> flags;                // j, done
   std::vector<double> alpha, beta, z;
+  TridiagLowest lowest;
   int checked = 0;                  // coefficients examined so far
   int niter = 0;
   double e0 = 0.0;
@@ -162,7 +163,7 @@ void lanczos_batch(int nsec, qcmg_hamiltonian* const* Hs, unsigned seed, double 
       for (int k = from; k < j && !stop; ++k) {
         b.alpha.push_back(land[1 + (k - from)]);
         b.beta.push_back(land[1 + chunk + (k - from)]);
-        b.e0 = tridiag_lowest(b.alpha, b.beta, b.z);
+        b.e0 = b.lowest(b.alpha, b.beta, b.z);
         const double ritz = std::fabs(b.z.back() * b.beta.back());
         if (!std::isfinite(b.e0) || !std::isfinite(ritz)) {
           b.status = QCMG_ERR_NUMERIC;

@@ -585,10 +585,10 @@ void fx_matvec_to_host(qcmg_hamiltonian* H, const double* x, double* yh, bool ac
 // Lanczos on FX vectors: the reference's recurrence (Lanczos.hpp:64-93)
 // written with normalized vectors, w = H v_j - alpha v_j - beta v_{j-1}.
 
-// w <- w - alpha v - beta p with alpha = <v, w> from the np partials that the
-// product left in red.part; returns alpha and |w|^2.
+// Queues w <- w - alpha v - beta p with alpha = <v, w> from the np partials
+// that the product left in red.part, and the copy of the step's scalars.
 static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec* p, unsigned np,
-                      double beta, FxReducer& red, double* alpha, double* norm2) {
+                      double beta, FxReducer& red) {
   cudaStream_t s = H->stream;
   const size_t n = w.n;
   double bp = 0.0;  // bound of the beta term, in units of c_w
@@ -606,7 +606,11 @@ static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec
   k_fx_norm<<<1, kFinalThreads, 0, s>>>(red.part.p, (int)g, H->fx.err.p, red.step.p);
   QCMG_CUDA(cudaGetLastError());
   QCMG_CUDA(cudaMemcpyAsync(red.host, red.step.p, sizeof(FxStep), cudaMemcpyDeviceToHost, s));
-  QCMG_CUDA(cudaStreamSynchronize(s));
+}
+
+// Waits for the step queued last: w's exponent and size, alpha and |w|^2.
+static void fx_collect(qcmg_hamiltonian* H, FxVec& w, FxReducer& red, double* alpha, double* norm2) {
+  QCMG_CUDA(cudaStreamSynchronize(H->stream));
   const FxStep& h = *red.host;
   if (h.err) throw Error(QCMG_ERR_CUDA, "a bulk copy into shared memory did not complete in time");
   w.E = h.Eo;
@@ -704,7 +708,13 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
     int E;
     double c;
   };
+  // a step queued in vain (or before an error) is over before its buffers go
+  struct Drain {
+    cudaStream_t s;
+    ~Drain() { cudaStreamSynchronize(s); }
+  } drain{s};
   std::vector<Kept> kept;
+  TridiagLowest lowest;
   std::vector<double> z;
   // the recurrence; replay: on the recorded coefficients, accumulating gs
   auto run = [&](bool replay, FxVec* gs) {
@@ -718,6 +728,27 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
     bool have_p = false;
     double beta_prev = 0.0;
     const int nsteps = replay ? (int)z.size() : max_iter + 1;
+    auto queue = [&](int j) {  // w <- H v - alpha v - beta p
+      if (!replay && keep) {
+        kept.push_back({v->buf.p, v->E, v->c});
+        int64_t* q = slots.get(want);
+        if (!q) {  // no room for more: a replay will follow
+          keep = false;
+          q = const_cast<int64_t*>(kept[0].q);  // neither v nor p: j >= 2 here
+        }
+        w->buf.borrow(q, n);
+      } else if (!replay && j < 2) {
+        w->buf.borrow(slots.get(want), n);
+      }
+      // alpha = <v, H v> comes out of the product's second pass
+      const unsigned np = fx_matvec(H, *v, *w, nullptr, 0.0, &red);
+      fx_update(H, *w, *v, have_p ? p : nullptr, np, beta_prev, red);
+    };
+    // On sectors whose step takes tens of microseconds the convergence test
+    // takes as long: the next step is queued first and runs meanwhile (one
+    // step is computed in vain).
+    const bool ahead = !replay && n < ((size_t)4 << 20);
+    if (!replay) queue(0);
     for (int j = 0; j < nsteps; ++j) {
       if (replay) {
         // gs += z_j v_j
@@ -727,33 +758,28 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
         k_fx_axpy<<<grid_ew(n), 256, 0, s>>>(gs->buf.p, v->buf.p, n, 0, m, gs->E - v->E - e);
         QCMG_CUDA(cudaGetLastError());
         if (j + 1 == nsteps) break;
-      } else if (keep) {
-        kept.push_back({v->buf.p, v->E, v->c});
-        int64_t* q = slots.get(want);
-        if (!q) {  // no room for more: a replay will follow
-          keep = false;
-          q = const_cast<int64_t*>(kept[0].q);  // neither v nor p: j >= 2 here
-        }
-        w->buf.borrow(q, n);
-      } else if (j < 2 && !w->buf.p) {
-        w->buf.borrow(slots.get(want), n);
+        queue(j);
       }
-      // alpha = <v, H v> comes out of the product's second pass
-      const unsigned np = fx_matvec(H, *v, *w, nullptr, 0.0, &red);
       double a = 0.0, n2 = 0.0;
-      fx_update(H, *w, *v, have_p ? p : nullptr, np, beta_prev, red, &a, &n2);
+      fx_collect(H, *w, red, &a, &n2);
       const double b = replay ? res.beta[j] : std::sqrt(n2);
-      if (!replay) {
-        res.alpha.push_back(a);
-        res.beta.push_back(b);
-        res.energy = tridiag_lowest(res.alpha, res.beta, z);
+      auto converged = [&] {
+        res.energy = lowest(res.alpha, res.beta, z);
         double ritz = std::fabs(z.back() * b);
         if (!std::isfinite(res.energy) || !std::isfinite(ritz))
           throw Error(QCMG_ERR_NUMERIC, "Lanczos produced a non-finite value");
-        if (ritz <= tol || b == 0.0) break;
+        if (ritz <= tol || b == 0.0) return true;
         if ((int)res.alpha.size() > max_iter)
           throw Error(QCMG_ERR_NOCONV,
                       "Lanczos procedure exceeded " + std::to_string(max_iter) + " iterations");
+        return false;
+      };
+      bool early = false;
+      if (!replay) {
+        res.alpha.push_back(a);
+        res.beta.push_back(b);
+        early = ahead && j + 1 < nsteps && std::isfinite(a) && std::isfinite(b) && b > 0.0;
+        if (!early && converged()) break;
       }
       // rotate: p <- v, v <- w / beta, w <- old p.  The division only changes
       // the lazy scale; its power of two moves into the exponent (exact), so
@@ -768,6 +794,8 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
       w = t;
       have_p = true;
       beta_prev = b;
+      if (!replay && j + 1 < nsteps) queue(j + 1);
+      if (early && converged()) break;
     }
   };
   run(false, nullptr);

@@ -548,14 +548,21 @@ int choose_slabs_per_pass(uint32_t du, int max_optin_smem) {
 
 template <int NS, bool SMALL, typename Kern>
 static void launch_passU4(Kern kern, const qcmg_hamiltonian* H, const FxProdArgs& A, int sms,
-                          cudaStream_t s) {
+                          int& per_sm, cudaStream_t s) {
   const size_t smem = ((NS == 2 ? (size_t)(SMALL ? kSlab1OffSmall : kSlab1Off) : 0) + slab_stride(H->du)) * 8;
-  QCMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int tmax = SMALL ? 256 : NS == 1 ? 512 : 1024;
   const int threads = std::min<int>(tmax, (int)((H->du + 127) / 128 * 128));
-  int per_sm = 0;
-  QCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-  per_sm = std::max(per_sm, 1);
+  if (per_sm == 0) {
+    // the largest size, so that one handle's setting serves every other
+    int n = 0, optin = 0;
+    cudaFuncAttributes fa;
+    QCMG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, H->device));
+    QCMG_CUDA(cudaFuncGetAttributes(&fa, kern));
+    QCMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   optin - (int)fa.sharedSizeBytes));
+    QCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+    per_sm = std::max(n, 1);
+  }
   const size_t rounds = ((size_t)H->dd + NS - 1) / NS;
   size_t grid = std::max<size_t>(1, std::min<size_t>(rounds, (size_t)sms * per_sm));
   if (NS == 2 && (grid & 1)) ++grid;  // even: the two slabs of a round share their alignment
@@ -564,8 +571,8 @@ static void launch_passU4(Kern kern, const qcmg_hamiltonian* H, const FxProdArgs
 
 unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStream_t s) {
   const FxTables& T = H->fx;
-  int sms = 0;
-  QCMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device));
+  if (T.sms == 0) QCMG_CUDA(cudaDeviceGetAttribute(&T.sms, cudaDevAttrMultiProcessorCount, H->device));
+  const int sms = T.sms;
   const int ik = H->inter_kind;
   // FAST kernels: hop magnitudes and accumulation factor are powers of two
   // and the diagonal is narrow (the Hubbard form with t = 1 and small-integer
@@ -574,9 +581,9 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   auto passU4 = [&](auto ns_tag, auto small_tag, auto fast_tag) {
     constexpr int NS = decltype(ns_tag)::value;
     constexpr bool S = decltype(small_tag)::value, F = decltype(fast_tag)::value;
-    if (ik == QCMG_INTER_NONE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_NONE, NS, F, S>, H, A, sms, s);
-    else if (ik == QCMG_INTER_ONSITE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_ONSITE, NS, F, S>, H, A, sms, s);
-    else launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_GENERAL, NS, F, S>, H, A, sms, s);
+    if (ik == QCMG_INTER_NONE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_NONE, NS, F, S>, H, A, sms, T.per_sm_u[F], s);
+    else if (ik == QCMG_INTER_ONSITE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_ONSITE, NS, F, S>, H, A, sms, T.per_sm_u[F], s);
+    else launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_GENERAL, NS, F, S>, H, A, sms, T.per_sm_u[F], s);
   };
   using One = std::integral_constant<int, 1>;
   using Two = std::integral_constant<int, 2>;
@@ -610,9 +617,12 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   const size_t items = (size_t)A.nbands * H->dd;
   if (items >= (1ull << 32)) throw Error(QCMG_ERR_ARG, "sector too large for pass D's 32-bit item numbers");
   auto go = [&](auto kern) {
-    int per_sm = 0;
-    QCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0));
-    per_sm = std::max(1, std::min(per_sm, 8));  // dot partials: at most 8 blocks per SM
+    int& per_sm = T.per_sm_d[fast ? 1 : 0][A.dot_part ? 1 : 0];
+    if (per_sm == 0) {
+      int n = 0;
+      QCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, 0));
+      per_sm = std::max(1, std::min(n, 8));  // dot partials: at most 8 blocks per SM
+    }
     const unsigned g = (unsigned)std::max<size_t>(1, std::min<size_t>((items + 7) / 8, (size_t)sms * per_sm));
     kern<<<g, 256, 0, s>>>(A);
     return g;

@@ -428,6 +428,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   QCMG_CUDA(cudaMemcpyAsync(r.p, x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
   QCMG_CUDA(cudaMemsetAsync(q.p, 0, n * 8, s));
   Reducer red;
+  TridiagLowest lowest;
   std::vector<double> z;
   double* rp = r.p;
   double* qp = q.p;
@@ -443,7 +444,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
       res.alpha.push_back(a);
       double b2 = red.axpy_norm2(rp, qp, a, n, s);
       res.beta.push_back(std::sqrt(b2));
-      res.energy = tridiag_lowest(res.alpha, res.beta, z);
+      res.energy = lowest(res.alpha, res.beta, z);
       ritz = std::fabs(z.back() * res.beta.back());
       if (!std::isfinite(res.energy) || !std::isfinite(ritz))
         throw Error(QCMG_ERR_NUMERIC, "Lanczos produced a non-finite value");
@@ -518,7 +519,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
       res.reorth_bytes += 2.0 * 16.0 * (double)Vp.size() * (double)n;  // 16 B per stored element per pass
       res.beta.push_back(b);
       ++total;
-      res.energy = tridiag_lowest(res.alpha, res.beta, z);
+      res.energy = lowest(res.alpha, res.beta, z);
       const double ritz = std::fabs(z.back() * b);
       if (!std::isfinite(res.energy) || !std::isfinite(ritz))
         throw Error(QCMG_ERR_NUMERIC, "Lanczos produced a non-finite value");

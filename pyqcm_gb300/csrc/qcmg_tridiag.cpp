@@ -21,13 +21,45 @@ static int sturm_below(const std::vector<double>& a, const std::vector<double>& 
   return count;
 }
 
-double tridiag_lowest(const std::vector<double>& a, const std::vector<double>& b,
-                      std::vector<double>& z) {
+// Adjacent doubles lo < hi with no eigenvalue below lo and one below hi,
+// from a bracket with those counts: bisection to full precision.
+static void bisect_lowest(const std::vector<double>& a, const std::vector<double>& b, double* lo,
+                          double* hi) {
+  for (int it = 0; it < 2000; ++it) {
+    const double mid = 0.5 * (*lo + *hi);
+    if (mid <= *lo || mid >= *hi) break;
+    if (sturm_below(a, b, mid) >= 1)
+      *hi = mid;
+    else
+      *lo = mid;
+  }
+}
+
+// -p'/p at x for the characteristic polynomial of T, x below every
+// eigenvalue (the pivots and their derivatives): 1/(this) is Newton's step
+// to the lowest eigenvalue, from below and without overshoot.
+static double log_slope(const std::vector<double>& a, const std::vector<double>& b, double x) {
+  double d = a[0] - x, dd = -1.0, s = -dd / d;
+  for (size_t i = 1; i < a.size(); ++i) {
+    const double q = b[i - 1] / d;
+    dd = -1.0 + q * q * dd;
+    d = a[i] - x - b[i - 1] * q;
+    s -= dd / d;
+  }
+  return s;
+}
+
+double TridiagLowest::operator()(const std::vector<double>& a, const std::vector<double>& b,
+                                 std::vector<double>& z) {
   const size_t n = a.size();
+  const size_t n0 = n_;
+  n_ = n;
   z.assign(n, 0.0);
   if (n == 0) return 0.0;
   if (n == 1) {
     z[0] = 1.0;
+    lo_ = hi_ = a[0];
+    change_ = INFINITY;
     return a[0];
   }
   // Gershgorin interval.
@@ -38,32 +70,59 @@ double tridiag_lowest(const std::vector<double>& a, const std::vector<double>& b
     hi = std::max(hi, a[i] + r);
     scale = std::max(scale, std::fabs(a[i]) + r);
   }
-  // Bisection to full precision: invariant count(lo) == 0, count(hi) >= 1.
-  for (int it = 0; it < 2000; ++it) {
-    double mid = 0.5 * (lo + hi);
-    if (mid <= lo || mid >= hi) break;
-    if (sturm_below(a, b, mid) >= 1)
-      hi = mid;
-    else
-      lo = mid;
+  // One row more than at the last call: the eigenvalue moved down, by about
+  // as much as last time.  Every end of the bracket is tested before use.
+  const bool warm = n0 >= 8 && n == n0 + 1 && std::isfinite(change_) && std::isfinite(scale);
+  if (warm) {
+    const double ulp = std::nextafter(std::fabs(hi_), INFINITY) - std::fabs(hi_);
+    double top = hi_ + 4.0 * ulp, w = std::max(4.0 * change_, 64.0 * ulp);
+    if (top < hi && sturm_below(a, b, top) >= 1) {
+      hi = top;
+      double x = hi - w;
+      while (x > lo && sturm_below(a, b, x) >= 1) {
+        hi = x;
+        w *= 16.0;
+        x = hi - w;
+      }
+      if (x > lo) lo = x;
+      for (int it = 0; it < 8 && hi - lo > 64.0 * ulp; ++it) {
+        const double step = 1.0 / log_slope(a, b, lo);
+        const double below = lo + 0.999 * step - 2.0 * ulp, above = lo + 2.0 * step + 4.0 * ulp;
+        if (!(step > 0.0) || !(below > lo)) break;
+        if (above < hi && sturm_below(a, b, above) >= 1) hi = above;
+        if (!(below < hi)) break;
+        if (sturm_below(a, b, below) >= 1)
+          hi = below;
+        else
+          lo = below;
+      }
+    }
   }
+  bisect_lowest(a, b, &lo, &hi);
   const double lam = 0.5 * (lo + hi);
-  // Inverse iteration on T - (lam - delta) I, positive definite.
+  change_ = n0 + 1 == n && n0 >= 1 ? std::fabs(lo - lo_) : INFINITY;
+  lo_ = lo;
+  hi_ = hi;
+  // Inverse iteration on T - (lam - delta) I, positive definite.  From the
+  // same vector at every call: once a copy of the eigenvalue has appeared
+  // (lost orthogonality) the vector is not unique, and one that followed the
+  // last call's would stop a run at another step.
   const double delta = std::max(scale, 1.0) * 64.0 * DBL_EPSILON;
   const double shift = lo - delta;
-  std::vector<double> d(n), l(n > 1 ? n - 1 : 1);
-  d[0] = a[0] - shift;
+  d_.resize(n);
+  l_.resize(n);
+  d_[0] = a[0] - shift;
   for (size_t i = 0; i + 1 < n; ++i) {
-    l[i] = b[i] / d[i];
-    d[i + 1] = a[i + 1] - shift - l[i] * b[i];
-    if (!(d[i + 1] > 0.0)) d[i + 1] = DBL_MIN * 1e10;
+    l_[i] = b[i] / d_[i];
+    d_[i + 1] = a[i + 1] - shift - l_[i] * b[i];
+    if (!(d_[i + 1] > 0.0)) d_[i + 1] = DBL_MIN * 1e10;
   }
   for (size_t i = 0; i < n; ++i) z[i] = 1.0 / std::sqrt((double)n) * ((i % 2) ? 0.9 : 1.1);
   for (int it = 0; it < 4; ++it) {
     // Solve L D L^T w = z in place.
-    for (size_t i = 1; i < n; ++i) z[i] -= l[i - 1] * z[i - 1];
-    for (size_t i = 0; i < n; ++i) z[i] /= d[i];
-    for (size_t i = n - 1; i-- > 0;) z[i] -= l[i] * z[i + 1];
+    for (size_t i = 1; i < n; ++i) z[i] -= l_[i - 1] * z[i - 1];
+    for (size_t i = 0; i < n; ++i) z[i] /= d_[i];
+    for (size_t i = n - 1; i-- > 0;) z[i] -= l_[i] * z[i + 1];
     double nrm = 0.0;
     for (double v : z) nrm += v * v;
     nrm = std::sqrt(nrm);
@@ -77,6 +136,11 @@ double tridiag_lowest(const std::vector<double>& a, const std::vector<double>& b
   if (z[imax] < 0)
     for (double& v : z) v = -v;
   return lam;
+}
+
+double tridiag_lowest(const std::vector<double>& a, const std::vector<double>& b,
+                      std::vector<double>& z) {
+  return TridiagLowest()(a, b, z);
 }
 
 // The band solvers read the matrix through low(r, c), the element (r, c)

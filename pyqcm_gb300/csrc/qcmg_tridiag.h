@@ -18,6 +18,23 @@ namespace qcmg {
 double tridiag_lowest(const std::vector<double>& alpha, const std::vector<double>& beta,
                       std::vector<double>& z);
 
+// The same for a Lanczos run that asks after every step: operator() called
+// with one row more than the last time looks for the eigenvalue just below
+// the last one, by Newton steps (~15 Sturm passes instead of ~64).  The
+// bracket's ends are tested, so it is the same pair of adjacent doubles, and
+// the same vector.  Over the calls with 1 to 220 rows (x86 host core): 45.0 us
+// -> 11.7 us on average.
+class TridiagLowest {
+ public:
+  double operator()(const std::vector<double>& alpha, const std::vector<double>& beta,
+                    std::vector<double>& z);
+
+ private:
+  double lo_ = 0.0, hi_ = 0.0, change_ = INFINITY;
+  size_t n_ = 0;  // rows of the last call
+  std::vector<double> d_, l_;
+};
+
 // Lowest eigenvalue of the leading n x n block of a symmetric band matrix
 // (half bandwidth b: t(r, c) = 0 for |r - c| > b), read from the lower
 // triangle of column-major t with leading dimension ld.  Bisection on
