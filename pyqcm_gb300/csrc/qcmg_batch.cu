@@ -1,5 +1,5 @@
-// Lanczos ground states of many sectors at once, each sector's steps
-// replayed from a captured CUDA graph.
+// Lanczos ground states of many sectors at once: sectors that fit on chip in
+// qcmg_chip.cu, each other sector's steps replayed from a CUDA graph.
 //
 // The recurrence is LanczosEigenvalue's (pyqcm src_ed/Hamiltonian/
 // Lanczos.hpp:41-95), with alpha/beta and the step index kept on the device
@@ -24,6 +24,7 @@
 
 #include "qcmg.h"
 #include "qcmg_blas.h"
+#include "qcmg_chip.h"
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
 #include "qcmg_tridiag.h"
@@ -72,8 +73,24 @@ static const double* seeded_start_dev(qcmg_hamiltonian* H, unsigned seed) {
   return H->seed_vec.p;
 }
 
-void lanczos_batch(int nsec, qcmg_hamiltonian* const* Hs, unsigned seed, double tol, int max_iter,
-                   int chunk, double* E0, int* niter, double* const* psi, int* status) {
+// The sectors that fit on chip (qcmg_chip.cu), in one go.
+static void lanczos_batch_chip(int nsec, qcmg_hamiltonian* const* Hs, unsigned seed, double tol,
+                               int max_iter, double* E0, int* niter, double* const* psi,
+                               int* status) {
+  std::vector<const double*> x0(nsec);
+  for (int i = 0; i < nsec; ++i) x0[i] = seeded_start_dev(Hs[i], seed);
+  std::vector<ChipResult> res(nsec);
+  chip_lanczos(nsec, Hs, x0.data(), tol, max_iter, psi, res.data());
+  for (int i = 0; i < nsec; ++i) {
+    E0[i] = res[i].energy;
+    niter[i] = res[i].niter;
+    status[i] = res[i].status;
+  }
+}
+
+static void lanczos_batch_graphs(int nsec, qcmg_hamiltonian* const* Hs, unsigned seed, double tol,
+                                 int max_iter, int chunk, double* E0, int* niter,
+                                 double* const* psi, int* status) {
   chunk = std::max(2, chunk + (chunk & 1));  // even: every chunk starts on the same buffers
   const int cap = max_iter + chunk + 1;
   std::vector<std::unique_ptr<BatchSector>> S(nsec);
@@ -208,8 +225,38 @@ void lanczos_batch(int nsec, qcmg_hamiltonian* const* Hs, unsigned seed, double 
     BatchSector& b = *S[i];
     QCMG_CUDA(cudaStreamSynchronize(b.stream));
     E0[i] = b.e0;
-    if (niter) niter[i] = b.niter;
-    if (status) status[i] = b.status;
+    niter[i] = b.niter;
+    status[i] = b.status;
+  }
+}
+
+// Small sectors on chip, the others from graphs; results in the caller's order.
+void lanczos_batch(int nsec, qcmg_hamiltonian* const* Hs, unsigned seed, double tol, int max_iter,
+                   int chunk, double* E0, int* niter, double* const* psi, int* status) {
+  for (int small = 1; small >= 0; --small) {
+    std::vector<int> at;
+    for (int i = 0; i < nsec; ++i)
+      if (chip_fits(Hs[i]) == (small != 0)) at.push_back(i);
+    const int n = (int)at.size();
+    if (n == 0) continue;
+    std::vector<qcmg_hamiltonian*> h(n);
+    std::vector<double> e(n);
+    std::vector<int> it(n), st(n);
+    std::vector<double*> ps(n, nullptr);
+    for (int k = 0; k < n; ++k) {
+      h[k] = Hs[at[k]];
+      if (psi) ps[k] = psi[at[k]];
+    }
+    const bool any = std::any_of(ps.begin(), ps.end(), [](double* p) { return p != nullptr; });
+    if (small)
+      lanczos_batch_chip(n, h.data(), seed, tol, max_iter, e.data(), it.data(), any ? ps.data() : nullptr, st.data());
+    else
+      lanczos_batch_graphs(n, h.data(), seed, tol, max_iter, chunk, e.data(), it.data(), any ? ps.data() : nullptr, st.data());
+    for (int k = 0; k < n; ++k) {
+      E0[at[k]] = e[k];
+      if (niter) niter[at[k]] = it[k];
+      if (status) status[at[k]] = st[k];
+    }
   }
 }
 

@@ -10,6 +10,7 @@
 #include <random>
 
 #include "qcmg_blas.h"
+#include "qcmg_chip.h"
 #include "qcmg_fxpath.h"
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
@@ -413,6 +414,24 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   } else {
     QCMG_CUDA(cudaMemcpyAsync(x0_own.p, x0_host, n * 8, cudaMemcpyHostToDevice, s));
     x0_dev = x0_own.p;
+  }
+  if (reorth <= 0 && chip_fits(H)) {
+    // on chip, in FP64 on either path: at these sizes a step is latency, and
+    // the fixed-point passes take five launches (8-site chain, 4,900 states:
+    // ~45 us per step, 16 us on chip)
+    if (x0_host) QCMG_CUDA(cudaStreamSynchronize(s));  // the solve has a stream of its own
+    ChipResult r;
+    chip_lanczos(1, &H, &x0_dev, tol, max_iter, psi_host ? &psi_host : nullptr, &r);
+    if (r.status == QCMG_ERR_NUMERIC)
+      throw Error(QCMG_ERR_NUMERIC, "Lanczos produced a non-finite value");
+    if (r.status == QCMG_ERR_NOCONV)
+      throw Error(QCMG_ERR_NOCONV,
+                  "Lanczos procedure exceeded " + std::to_string(max_iter) + " iterations");
+    res.alpha = r.alpha;
+    res.beta = r.beta;
+    res.energy = r.energy;
+    res.niter = r.niter;
+    return res;
   }
   if (reorth <= 0 && H->use_fx && fx_prepare(H)) {
     // fixed-point fast path (one hop magnitude per spin)

@@ -1,0 +1,74 @@
+"""On-chip Lanczos (qcmg_chip.cu) at the sizes where it can go wrong: one
+state to the largest sector that fits, tiles of 64 states with remainders,
+clusters larger than the number of tiles, vectors kept or recomputed, against
+dense diagonalization or the FP64 oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _sector(L, nup, ndn, seed):
+    """(engine Hamiltonian, oracle sector) of a random open chain."""
+    import pyqcm_gb300 as pg
+    import qcm_oracle as qo
+    rng = np.random.default_rng(seed)
+    t = [(i, i + 1, float(rng.uniform(-1, 1))) for i in range(L - 1)]
+    e = [(i, i, float(rng.uniform(-1, 1))) for i in range(L)]
+    ops = {"h": ("one-body", t + e + [(i + L, j + L, v) for i, j, v in t + e]),
+           "U": ("interaction", [(i, i + L, float(rng.uniform(1, 4))) for i in range(L)])}
+    m = pg.ClusterModel(L)
+    for name, (typ, els) in ops.items():
+        m.new_operator(name, typ, els)
+    vals = {"h": 1.0, "U": 1.0}
+    up, dn, pr = qo.combine_terms(ops, vals, L)
+    return pg.Hamiltonian(m, vals, f"R0:N{nup + ndn}:S{nup - ndn}"), qo.Sector(L, nup, ndn, up, dn, pr)
+
+
+# dims 1, 3, 9, 63 = 7 x 9, 64 = 8 x 8, 100, 1,225, 15,876, 16,170 = 210 x 77 is out of reach of a
+# chain sector; 252 x 45 = 11,340 has unequal factors
+@pytest.mark.parametrize("L,nup,ndn", [(3, 0, 3), (3, 1, 0), (3, 1, 2), (8, 1, 1), (5, 2, 3), (7, 3, 4), (9, 4, 4), (10, 5, 2)])
+def test_ground_state(L, nup, ndn):
+    H, S = _sector(L, nup, ndn, L + nup)
+    x0 = np.random.default_rng(3).normal(size=H.dim)
+    x0 /= np.linalg.norm(x0)
+    e0, psi, alpha, beta = H.lanczos(x0=x0, tol=1e-10)
+    assert abs(np.linalg.norm(psi) - 1) < 1e-6  # the replayed vector's norm, the recurrence's own accuracy
+    r = S.matvec(psi) - e0 * psi
+    # the Ritz residual is below tol at the last step; psi adds its rounding
+    assert np.linalg.norm(r) < 1e-7
+    if H.dim <= 1300:
+        A = np.array([S.matvec(v) for v in np.eye(H.dim)])
+        assert abs(e0 - np.linalg.eigvalsh(A)[0]) < 1e-10 * max(1.0, abs(e0))
+    assert len(alpha) == len(beta)
+
+
+def test_largest_sector_and_the_next():
+    """16,384 states is the limit: 126 x 126 is on chip, 210 x 120 is not;
+    both give the energy of the fully reorthogonalized recurrence."""
+    for L, nup, ndn in ((9, 4, 5), (10, 4, 3)):
+        H, _ = _sector(L, nup, ndn, 1)
+        e0 = H.lanczos(tol=1e-11, want_psi=False)[0]
+        e1 = H.lanczos(tol=1e-11, want_psi=False, reorth=200)[0]
+        assert abs(e0 - e1) < 1e-10 * abs(e1)
+
+
+def test_batch_equals_single_for_any_cluster_size():
+    """Clusters of 16 (one sector), 8, 4, 2 and 1 CTAs give the same bits."""
+    import pyqcm_gb300 as pg
+    hs = [_sector(6, 3, 3, k)[0] for k in range(320)]
+    one = [h.lanczos() for h in hs[:3]]
+    for n in (2, 40, 80, 160, 320):
+        got = pg.lanczos_batch(hs[:n], want_psi=True)
+        for (e, psi, it), (e1, psi1, al, _) in zip(got, one):
+            assert e == e1 and it == len(al) and np.array_equal(psi, psi1)
+
+
+def test_no_convergence_is_reported():
+    import pyqcm_gb300 as pg
+    H, _ = _sector(8, 4, 4, 5)
+    with pytest.raises(pg.QcmgError) as err:
+        H.lanczos(max_iter=20)
+    assert err.value.code == -4
+    res = pg.lanczos_batch([H], max_iter=20, raise_errors=False)
+    assert res[0][3] is not None and res[0][3].code == -4
