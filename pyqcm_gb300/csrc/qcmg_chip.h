@@ -27,4 +27,15 @@ struct ChipResult {
 void chip_lanczos(int n, qcmg_hamiltonian* const* Hs, const double* const* x0, double tol,
                   int max_iter, double* const* psi, ChipResult* res);
 
+// Whether the band Lanczos of p start vectors runs on chip.
+bool chip_band_fits(const qcmg_hamiltonian* H, int p);
+
+// Band Lanczos steps on chip from p start vectors phi (device memory), at most
+// M0 of them, on the handle's stream: fills the projected matrix t (M0 x M0,
+// column-major) and the start vectors' projections P (p x M0) as
+// band_lanczos does and sets *M to the steps taken. False when a vector
+// deflates (or a coefficient is not finite): the general path then decides.
+bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc_defl,
+               double acc_band, std::vector<double>& t, std::vector<double>& P, int* M);
+
 }  // namespace qcmg

@@ -822,6 +822,38 @@ BlockResult block_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool
   return out;
 }
 
+// Eigenvalues and Q = P(:, 0:k) U(0:k, :), k = min(p, M)
+// (Hamiltonian_base.hpp:249 with matrix::product's bound on the inner index):
+// all eigenvalues of the leading M x M block of t but only the leading k rows
+// of its eigenvectors.  Without in-band deflation (banded) t is a band matrix
+// and the host band solver gives exactly that; otherwise the device
+// eigensolver takes the whole block.
+static BandResult band_result(qcmg_hamiltonian* H, int p, int M0, int M,
+                              const std::vector<double>& t, const std::vector<double>& P,
+                              bool banded) {
+  BandResult out;
+  out.M = M;
+  if (M == 0) return out;
+  const int kk = std::min(p, M);
+  std::vector<double> U;  // U(k, c) = U[k * ustride_k + c * ustride_c]
+  size_t ustride_k = 1, ustride_c = (size_t)M;
+  if (!(banded && band_eigen_leading(t, M0, M, p, kk, out.evals, U))) {
+    Cusolver solver;
+    solver.syevd(t, M0, M, true, H->stream, out.evals, &U);
+  } else {
+    ustride_k = (size_t)M;
+    ustride_c = 1;
+  }
+  out.Q.assign((size_t)p * M, 0.0);
+  for (int a = 0; a < p; ++a)
+    for (int c = 0; c < M; ++c) {
+      double acc = 0.0;
+      for (int k = 0; k < kk; ++k) acc += P[a + (size_t)p * k] * U[k * ustride_k + c * ustride_c];
+      out.Q[(size_t)a * M + c] = acc;
+    }
+  return out;
+}
+
 BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool phi_on_device, int M0,
                         int max_iter,
                         double acc_defl, double acc_band) {
@@ -834,18 +866,22 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
   int M0p = (M0 / p + 1) * p;
   M0 = M0p - pc;
   QCMG_CHECK_ARG(M0 > 0, "band Lanczos needs M > 0");
-  // Device vectors: the p start vectors (the caller's own when they are on
-  // the device: they are only read) plus a pool for v[0..M0p).
+  // The p start vectors on the device (the caller's own when they are there:
+  // they are only read).
   std::vector<DevVec> phi;
+  if (!phi_on_device) {
+    phi.emplace_back((size_t)p * n);
+    QCMG_CUDA(cudaMemcpyAsync(phi[0].p, phi_in, (size_t)p * n * 8, cudaMemcpyHostToDevice, s));
+  }
+  const double* phi0 = phi_on_device ? phi_in : phi[0].p;
   std::vector<const double*> phip;
-  for (int k = 0; k < p; ++k) {
-    if (phi_on_device) {
-      phip.push_back(phi_in + (size_t)k * n);
-      continue;
-    }
-    phi.emplace_back(n);
-    QCMG_CUDA(cudaMemcpyAsync(phi[k].p, phi_in + (size_t)k * n, n * 8, cudaMemcpyHostToDevice, s));
-    phip.push_back(phi[k].p);
+  for (int k = 0; k < p; ++k) phip.push_back(phi0 + (size_t)k * n);
+  std::vector<double> t;  // column-major t(r,c) = t[r + M0*c]
+  std::vector<double> P;  // P(k,j) = P[k + p*j]
+  if (chip_band_fits(H, p)) {
+    int M = 0;
+    if (chip_band(H, p, phi0, M0, acc_defl, acc_band, t, P, &M))
+      return band_result(H, p, M0, M, t, P, true);
   }
   std::vector<double*> v(M0p, nullptr);
   std::vector<double*> pool;
@@ -867,9 +903,9 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
     v[i] = get();
     QCMG_CUDA(cudaMemcpyAsync(v[i], phip[i], n * 8, cudaMemcpyDeviceToDevice, s));
   }
-  std::vector<double> t((size_t)M0 * M0, 0.0);  // column-major t(r,c) = t[r + M0*c]
+  t.assign((size_t)M0 * M0, 0.0);
   auto T = [&](int r, int c) -> double& { return t[(size_t)r + (size_t)M0 * c]; };
-  std::vector<double> P((size_t)p * M0, 0.0);   // P(k,j) = P[k + p*j]
+  P.assign((size_t)p * M0, 0.0);
   std::vector<int> defl(M0, 0);
   std::vector<int> I;
   Reducer red;
@@ -1010,30 +1046,7 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
     }
   }
   flush();
-  out.M = j;
-  if (j == 0) return out;
-  // Q = P(:, 0:k) U(0:k, :), k = min(p, M) (Hamiltonian_base.hpp:249 with
-  // matrix::product's bound on the inner index): all eigenvalues of t but
-  // only the leading k rows of its eigenvectors.  Without in-band
-  // deflation t is a band matrix and the host band solver gives exactly
-  // that; otherwise the device eigensolver takes the whole block.
-  const int M = j, kk = std::min(p, M);
-  std::vector<double> U;  // U(k, c) = U[k * ustride_k + c * ustride_c]
-  size_t ustride_k = 1, ustride_c = (size_t)M;
-  if (!(I.empty() && band_eigen_leading(t, M0, M, p, kk, out.evals, U))) {
-    solver.syevd(t, M0, j, true, s, out.evals, &U);
-  } else {
-    ustride_k = (size_t)M;
-    ustride_c = 1;
-  }
-  out.Q.assign((size_t)p * M, 0.0);
-  for (int a = 0; a < p; ++a)
-    for (int c = 0; c < M; ++c) {
-      double acc = 0.0;
-      for (int k = 0; k < kk; ++k) acc += P[a + (size_t)p * k] * U[k * ustride_k + c * ustride_c];
-      out.Q[(size_t)a * M + c] = acc;
-    }
-  return out;
+  return band_result(H, p, M0, j, t, P, I.empty());
 }
 
 }  // namespace qcmg

@@ -72,3 +72,48 @@ def test_no_convergence_is_reported():
     assert err.value.code == -4
     res = pg.lanczos_batch([H], max_iter=20, raise_errors=False)
     assert res[0][3] is not None and res[0][3].code == -4
+
+
+def _green(e, Q, zs):
+    return np.einsum("am,zm,bm->zab", Q, 1.0 / (zs[:, None] - e), Q)
+
+
+def _oracle_green(S, phi, zs):
+    """The oracle's run of the same recurrence with the same stopping rule: a
+    random start vector's Green function at the centre of the spectrum is not
+    converged when the lowest eigenvalue is, so the exact resolvent is not
+    what a correct run gives."""
+    import qcm_oracle as qo
+    return _green(*qo.build_Q_matrix(S.mult_add, list(phi), S.dim), zs)
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4, 5, 8, 9, 12, 13])
+@pytest.mark.parametrize("L,nup,ndn", [(6, 3, 3), (7, 3, 4)])
+@pytest.mark.parametrize("start", ["free", "dependent"])
+def test_band_lanczos(p, L, nup, ndn, start):
+    """The Green function of p start vectors at imaginary frequencies: on chip
+    for p <= 12, on the general path above and where a vector deflates."""
+    H, S = _sector(L, nup, ndn, 11)
+    rng = np.random.default_rng(p)
+    phi = rng.normal(size=(p, S.dim))
+    if start == "dependent" and p > 1:
+        phi[-1] = phi[0]
+    phi /= np.linalg.norm(phi, axis=1)[:, None]
+    zs = np.array([1.0j, 4.0j, 20.0j])
+    e, Q = H.build_Q_matrix(phi)
+    G = _green(e, Q, zs)
+    ref = _oracle_green(S, phi, zs)
+    # the two runs stop at the same step; their rounding stays below 1e-8 in G
+    assert np.max(np.abs(G - ref)) < 1e-8 * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("L,nup,ndn,p", [(2, 1, 1, 2), (3, 1, 1, 3), (4, 2, 2, 4), (5, 2, 2, 4)])
+def test_band_lanczos_exhausts_small_sectors(L, nup, ndn, p):
+    """Krylov spaces that end (a vector deflates)."""
+    H, S = _sector(L, nup, ndn, 4)
+    phi = np.random.default_rng(2).normal(size=(p, S.dim))
+    zs = np.array([0.7j, 3.0j])
+    e, Q = H.build_Q_matrix(phi)
+    G = _green(e, Q, zs)
+    ref = _oracle_green(S, phi, zs)
+    assert np.max(np.abs(G - ref)) < 1e-8 * np.max(np.abs(ref))
