@@ -195,8 +195,8 @@ int qcmg_hamiltonian_create(int L, int n_up, int n_dn, int n_hop_up, const int32
       std::vector<HopElement> eu, ed;
       for (int k = 0; k < n_hop_up; ++k) eu.push_back({up_r[k], up_c[k], up_v[k]});
       for (int k = 0; k < n_hop_dn; ++k) ed.push_back({dn_r[k], dn_c[k], dn_v[k]});
-      build_halfop(H->up, L, n_up, eu, H->stream);
-      build_halfop(H->dn, L, n_dn, ed, H->stream);
+      build_halfop(H->up, L, n_up, eu, true, H->stream);
+      build_halfop(H->dn, L, n_dn, ed, false, H->stream);
       H->du = H->up.dim;
       H->dd = H->dn.dim;
       H->dim = (size_t)H->du * H->dd;

@@ -127,7 +127,8 @@ __global__ void k_halfop_count(uint32_t dim, const uint32_t* __restrict__ bin,
 __global__ void k_halfop_fill(uint32_t dim, const uint32_t* __restrict__ bin,
                               const HopElement* __restrict__ el, int nel,
                               const uint32_t* __restrict__ rowptr, uint32_t* __restrict__ col,
-                              double* __restrict__ val, double* __restrict__ diag) {
+                              double* __restrict__ val, double* __restrict__ diag,
+                              uint32_t* __restrict__ ell, uint16_t* __restrict__ len) {
   for (uint32_t I = blockIdx.x * blockDim.x + threadIdx.x; I < dim; I += gridDim.x * blockDim.x) {
     uint32_t b = bin[I];
     uint32_t pos = rowptr[I];
@@ -142,16 +143,21 @@ __global__ void k_halfop_fill(uint32_t dim, const uint32_t* __restrict__ bin,
       if (v == 0.0) continue;
       if (((b >> c) & 1u) && !((b >> r) & 1u)) {
         uint32_t bp = b ^ (1u << c) ^ (1u << r);
-        col[pos] = dev_rank(bp);
-        val[pos] = hop_parity(b, r, c) ? -v : v;
+        const uint32_t J = dev_rank(bp);
+        const int neg = hop_parity(b, r, c);
+        col[pos] = J;
+        val[pos] = neg ? -v : v;
+        if (ell) ell[(size_t)(pos - rowptr[I]) * dim + I] = J | ((uint32_t)(2 * k + neg) << 16);
         ++pos;
       }
     }
+    if (ell) len[I] = (uint16_t)(pos - rowptr[I]);
     diag[I] = d;
   }
 }
 
-void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, cudaStream_t s) {
+void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, bool slots,
+                  cudaStream_t s) {
   op.L = L;
   op.N = N;
   uint64_t dim64 = binomial(L, N);
@@ -188,10 +194,30 @@ void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, c
   QCMG_CUDA(cudaMemcpyAsync(op.rowptr.p, h_rp.data(), (op.dim + 1) * 4, cudaMemcpyHostToDevice, s));
   op.col.alloc(nnz);
   op.val.alloc(nnz);
+  // slot form
+  std::vector<double> h_vtab;
+  op.nval = 0;
+  if (slots && op.dim > 0 && op.dim <= 65536u && el.size() <= 1024) {
+    uint32_t width = 1;
+    for (uint32_t c : h_cnt) width = std::max(width, c);
+    for (const auto& e : el) {
+      h_vtab.push_back(e.v);
+      h_vtab.push_back(-e.v);
+    }
+    if (h_vtab.empty()) h_vtab.push_back(0.0);
+    op.nval = (int)h_vtab.size();
+    const size_t words = (size_t)width * op.dim;
+    op.slots.alloc(h_vtab.size() + (words + 1) / 2 + ((size_t)op.dim + 3) / 4);
+    op.vtab = op.slots.p;
+    op.ell = reinterpret_cast<uint32_t*>(op.vtab + h_vtab.size());
+    op.len = reinterpret_cast<uint16_t*>(op.vtab + h_vtab.size() + (words + 1) / 2);
+    QCMG_CUDA(cudaMemcpyAsync(op.vtab, h_vtab.data(), h_vtab.size() * 8, cudaMemcpyHostToDevice, s));
+  }
   if (op.dim) {
     k_halfop_fill<<<grid_for(op.dim, 256), 256, 0, s>>>(op.dim, op.bin.p, d_el.p, (int)el.size(),
                                                          op.rowptr.p, op.col.p, op.val.p,
-                                                         op.diag.p);
+                                                         op.diag.p, op.nval ? op.ell : nullptr,
+                                                         op.nval ? op.len : nullptr);
     QCMG_CUDA(cudaGetLastError());
   }
   // Row bounds for the fixed-point headroom: |T|_inf and |diag|_max.

@@ -168,7 +168,7 @@ static size_t chip_smem(uint32_t D, int C) {
   return (D + 2 * per * kTile + 2 * nt) * sizeof(double);
 }
 
-bool chip_fits(const qcmg_hamiltonian* H) { return H->dim > 0 && H->dim <= kChipStates; }
+bool chip_fits(const qcmg_hamiltonian* H) { return H->dim > 0 && H->dim <= kChipStates && H->up.nval > 0; }
 
 namespace {
 

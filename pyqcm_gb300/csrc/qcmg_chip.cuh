@@ -17,8 +17,10 @@ constexpr int kTile = 64;  // states per partial sum: two per lane
 struct ChipOp {
   uint32_t du, dd, D;
   int L, inter;
-  const uint32_t *rp_up, *col_up, *rp_dn, *col_dn, *bin_up, *bin_dn;
-  const double *val_up, *val_dn, *diag_up, *diag_dn, *wdn;
+  const uint32_t *ell;
+  const uint16_t* len;
+  const uint32_t *rp_dn, *col_dn, *bin_up, *bin_dn;
+  const double *vtab, *val_dn, *diag_up, *diag_dn, *wdn;
   double U;
 };
 
@@ -43,8 +45,10 @@ __device__ __forceinline__ double chip_hops(const ChipOp& A, const double* x, ui
                                             uint32_t id, double acc) {
   const double* xs = x + id * A.du;
 #pragma unroll 4
-  for (uint32_t k = __ldg(A.rp_up + iu), e = __ldg(A.rp_up + iu + 1); k < e; ++k)
-    acc = fma(__ldg(A.val_up + k), xs[__ldg(A.col_up + k)], acc);
+  for (int k = 0, n = __ldg(A.len + iu); k < n; ++k) {
+    const uint32_t e = __ldg(A.ell + k * A.du + iu);
+    acc = fma(__ldg(A.vtab + (e >> 16)), xs[e & 0xffffu], acc);
+  }
   const double* xc = x + iu;
 #pragma unroll 4
   for (uint32_t k = __ldg(A.rp_dn + id), e = __ldg(A.rp_dn + id + 1); k < e; ++k)
@@ -87,9 +91,9 @@ inline ChipOp chip_op(const qcmg_hamiltonian* H) {
   A.D = (uint32_t)H->dim;
   A.L = H->L;
   A.inter = H->inter_kind;
-  A.rp_up = H->up.rowptr.p;
-  A.col_up = H->up.col.p;
-  A.val_up = H->up.val.p;
+  A.ell = H->up.ell;
+  A.len = H->up.len;
+  A.vtab = H->up.vtab;
   A.diag_up = H->up.diag.p;
   A.bin_up = H->up.bin.p;
   A.rp_dn = H->dn.rowptr.p;

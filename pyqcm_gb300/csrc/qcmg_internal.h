@@ -91,6 +91,16 @@ struct HalfOp {
   DevBuf<uint32_t> col;     // nnz
   DevBuf<double> val;       // nnz
   DevBuf<double> diag;      // dim
+  // The same rows slot by slot (ell[k dim + I] is hop k of row I, so that
+  // neighbouring threads read neighbouring words): column in the low half,
+  // index into vtab (+-v of every element) in the high half; len[I] hops.
+  // Built on request for half bases of at most 65,536 states; the order
+  // within a row is the CSR's.  One allocation holds the three tables.
+  DevBuf<double> slots;
+  double* vtab = nullptr;
+  uint32_t* ell = nullptr;
+  uint16_t* len = nullptr;
+  int nval = 0;  // entries of vtab; 0: no slot form
   double max_row_abs = 0.0; // max_I sum_J |val| (for fixed-point headroom)
   double max_diag_abs = 0.0;
 };
@@ -104,7 +114,9 @@ struct HopElement {
 void launch_halfbasis(int L, int N, uint32_t dim, uint32_t* out, cudaStream_t s);
 void launch_rank(int L, const uint32_t* states, size_t n, uint32_t dim, uint32_t* ranks,
                  cudaStream_t s);
-void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, cudaStream_t s);
+// slots: also the slot form, where the half basis allows it.
+void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, bool slots,
+                  cudaStream_t s);
 
 uint64_t binomial(int n, int k);
 
