@@ -1,0 +1,331 @@
+// Band Lanczos steps on sectors larger than a cluster's shared memory, four
+// launches per step and no host round trip: the step's coefficients (the norm
+// of v_j, the band dots, the closing dot) stay in device memory, and the
+// host reads them p steps at a time for its convergence probe while the next
+// p steps run.
+//   k_band_dots   finishes v_{j+p-1} (the previous step's closing dot), then
+//                 |v_j|^2 and <v_{j+i}, v_j>; the last block forms z and c_i
+//   k_band_scale  v_j /= z, v_{j+i} -= c_i v_j
+//   (product)     w = H v_j
+//   k_band_recur  w -= sum_k T(k, j) v_k and <w, v_j>; the last block adds it up
+// Each is one pass with the loads of all its vectors in flight together; the
+// FP64 pipe (12 + 12 + 13 FMAs per element at p = 12, and ~37 of the product)
+// is the floor: 86 us per step at 731,808 states. Five launches with a host
+// wait and a host-side sum per step took ~190 us, this ~140 us (600 steps and
+// G: 146 -> 119 ms, 35 of them the host's eigenproblem of the 600 x 600 band).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <type_traits>
+
+#include "qcmg_band.h"
+#include "qcmg_tridiag.h"
+#include "qcmg_vec.cuh"
+
+namespace qcmg {
+
+// Coefficients of one step: z, c_1 .. c_{p-1}, d, 1/z.
+__host__ __device__ inline int row_len(int p) { return p + 2; }
+
+// True in every thread of the block that finishes last (its partials and all
+// others' are then visible); the counter is left at zero.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// Fixed-order sum of value k's nb partials, by one warp.
+__device__ __forceinline__ double sum_partials(const double* part, int nb, int m, int k) {
+  double s = 0.0;
+  for (int b = threadIdx.x & 31; b < nb; b += 32) s += __ldcg(part + (size_t)b * m + k);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// V: v_{j+p-1} first, then v_j .. v_{j+p-2} (the vector to finish at a fixed
+// place keeps the packs in registers)
+template <int MAXM, int VEC>
+__global__ void __launch_bounds__(kDotThreads, 2)
+    k_band_dots(VecList V, int p, double* fin, const double* __restrict__ u,
+                const double* __restrict__ dprev, size_t nv, double* __restrict__ part,
+                unsigned* ticket, double* __restrict__ row, int j, double acc_defl, int* flag) {
+  if (*(volatile int*)flag >= 0) return;
+  double acc[MAXM];
+#pragma unroll
+  for (int k = 0; k < MAXM; ++k) acc[k] = 0.0;
+  const double d = fin ? *dprev : 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
+       i += (size_t)gridDim.x * blockDim.x) {
+    Pack<VEC> v[MAXM];
+#pragma unroll
+    for (int k = 0; k < MAXM; ++k)
+      if (k < p) v[k] = load_pack<VEC>(V[k], i);
+    if (fin) {
+      const Pack<VEC> y = load_pack<VEC>(u, i);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) v[0].e[e] = fma(-d, y.e[e], v[0].e[e]);
+      store_pack<VEC>(fin, i, v[0]);
+    }
+    Pack<VEC> x = v[0];
+    if (p > 1) x = v[1];
+#pragma unroll
+    for (int k = 0; k < MAXM; ++k)
+      if (k < p)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[k] = fma(v[k].e[e], x.e[e], acc[k]);
+  }
+  block_sums<MAXM>(acc, p, part + (size_t)blockIdx.x * p);
+  if (!last_block(ticket)) return;
+  __shared__ double tot[MAXM];
+  for (int k = threadIdx.x >> 5; k < p; k += kDotThreads / 32) {
+    const double s = sum_partials(part, (int)gridDim.x, p, k);
+    if ((threadIdx.x & 31) == 0) tot[k ? k - 1 : p - 1] = s;  // back to v_j, v_{j+1}, ...
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double z = sqrt(tot[0]), iz = 1.0 / z;
+    row[0] = z;
+    for (int k = 1; k < p; ++k) row[k] = tot[k] * iz;
+    row[p + 1] = iz;
+    if (z < acc_defl) *flag = j;
+  }
+}
+
+template <int MAXM, int VEC>
+__global__ void __launch_bounds__(256)
+    k_band_scale(MutVecList V, int p, const double* __restrict__ row, size_t nv, const int* flag) {
+  if (*(volatile const int*)flag >= 0) return;
+  __shared__ double cs[MAXM + 2];
+  if (threadIdx.x < row_len(p)) cs[threadIdx.x] = row[threadIdx.x];
+  __syncthreads();
+  const double iz = cs[p + 1];
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
+       i += (size_t)gridDim.x * blockDim.x) {
+    Pack<VEC> v[MAXM];
+#pragma unroll
+    for (int k = 0; k < MAXM; ++k)
+      if (k < p) v[k] = load_pack<VEC>(V[k], i);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) v[0].e[e] *= iz;
+    store_pack<VEC>(V[0], i, v[0]);
+#pragma unroll
+    for (int k = 1; k < MAXM; ++k)
+      if (k < p) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) v[k].e[e] = fma(-cs[k], v[0].e[e], v[k].e[e]);
+        store_pack<VEC>(V[k], i, v[k]);
+      }
+  }
+}
+
+// V: the m = min(p, j) vectors v_{j-m} .. v_{j-1}
+template <int MAXM, int VEC>
+__global__ void __launch_bounds__(kDotThreads, 2)
+    k_band_recur(VecList V, int m, int p, double* __restrict__ w, const double* __restrict__ u,
+                 size_t nv, double* __restrict__ part, unsigned* ticket, double* __restrict__ row,
+                 const int* flag) {
+  if (*(volatile const int*)flag >= 0) return;
+  __shared__ double cs[MAXM];
+  if (threadIdx.x < m) cs[threadIdx.x] = row[p - m + threadIdx.x];
+  __syncthreads();
+  double acc[1] = {0.0};
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
+       i += (size_t)gridDim.x * blockDim.x) {
+    Pack<VEC> v[MAXM];
+#pragma unroll
+    for (int k = 0; k < MAXM; ++k)
+      if (k < m) v[k] = load_pack<VEC>(V[k], i);
+    Pack<VEC> s = load_pack<VEC>(w, i);
+    const Pack<VEC> y = load_pack<VEC>(u, i);
+#pragma unroll
+    for (int k = 0; k < MAXM; ++k)
+      if (k < m)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) s.e[e] = fma(-cs[k], v[k].e[e], s.e[e]);
+    store_pack<VEC>(w, i, s);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[0] = fma(s.e[e], y.e[e], acc[0]);
+  }
+  block_sums<1>(acc, 1, part + blockIdx.x);
+  if (!last_block(ticket)) return;
+  if (threadIdx.x < 32) {
+    const double s = sum_partials(part, (int)gridDim.x, 1, 0);
+    if (threadIdx.x == 0) row[p] = s;
+  }
+}
+
+// <phi_k, v_j> of an unnormalized v_j for k < p (the first p steps only).
+__global__ void __launch_bounds__(256) k_band_project(const double* __restrict__ phi, size_t n,
+                                                      const double* __restrict__ v,
+                                                      double* __restrict__ out) {
+  const double* f = phi + (size_t)blockIdx.x * n;
+  double s = 0.0;
+  for (size_t i = threadIdx.x; i < n; i += 256) s = fma(f[i], v[i], s);
+  __shared__ double red[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += red[q];
+    out[blockIdx.x] = t;
+  }
+}
+
+namespace {
+
+// f(integral constant) with the smallest list size of the kernels >= p
+template <class F>
+void with_size(int p, F&& f) {
+  if (p <= 4)
+    f(std::integral_constant<int, 4>{});
+  else if (p <= 8)
+    f(std::integral_constant<int, 8>{});
+  else if (p <= 12)
+    f(std::integral_constant<int, 12>{});
+  else
+    f(std::integral_constant<int, 16>{});
+}
+
+struct Landing {  // page-locked rows and their events
+  double* rows = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  cudaStream_t s;
+  explicit Landing(cudaStream_t st) : s(st) {}
+  ~Landing() {
+    cudaStreamSynchronize(s);
+    if (rows) cudaFreeHost(rows);
+    for (auto e : done)
+      if (e) cudaEventDestroy(e);
+  }
+};
+
+}  // namespace
+
+bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc_defl,
+                double acc_band, const std::vector<double*>& ring, std::vector<double>& t,
+                std::vector<double>& P, BandRun& run) {
+  const size_t n = H->dim;
+  cudaStream_t s = H->stream;
+  const int R = 2 * p + 1, rl = row_len(p);
+  uintptr_t low = 0;
+  for (double* r : ring) low |= (uintptr_t)r;
+  const bool two = (n & 1u) == 0 && (low & 15u) == 0;
+  const size_t nv = two ? n / 2 : n;
+  const unsigned gd = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
+  const unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 3 * 152));
+  const unsigned ge = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + 255) / 256, 152 * 8));
+  DevBuf<double> rows, proj, part;
+  DevBuf<int> flags;  // the deflated step, then the block counter
+  rows.alloc((size_t)(M0 + 1) * rl);
+  proj.alloc((size_t)p * p);
+  part.alloc((size_t)std::max(gd * (unsigned)p, gr));
+  flags.alloc(2);
+  const int init[2] = {-1, 0};
+  QCMG_CUDA(cudaMemcpyAsync(flags.p, init, sizeof init, cudaMemcpyHostToDevice, s));
+  int* flag = flags.p;
+  unsigned* ticket = reinterpret_cast<unsigned*>(flags.p + 1);
+  for (int k = 0; k < p; ++k)
+    QCMG_CUDA(cudaMemcpyAsync(ring[k], phi + (size_t)k * n, n * 8, cudaMemcpyDeviceToDevice, s));
+  auto at = [&](int k) { return ring[k % R]; };
+  auto step = [&](int j) {
+    double* row = rows.p + (size_t)j * rl;
+    VecList L, B;
+    MutVecList S;
+    for (int k = 0; k < p; ++k) {
+      S.v[k] = at(j + k);
+      L.v[k] = at(k ? j + k - 1 : j + p - 1);
+    }
+    const int m = std::min(p, j);
+    for (int k = 0; k < m; ++k) B.v[k] = at(j - m + k);
+    double* fin = j > 0 ? at(j + p - 1) : nullptr;
+    const double* u = j > 0 ? at(j - 1) : nullptr;
+    const double* dprev = j > 0 ? row - rl + p : nullptr;
+    double *vj = at(j), *w = at(j + p);
+    with_size(p, [&](auto size) {
+      constexpr int MX = decltype(size)::value;
+      auto go = [&](auto vec) {
+        constexpr int VC = decltype(vec)::value;
+        k_band_dots<MX, VC><<<gd, kDotThreads, 0, s>>>(L, p, fin, u, dprev, nv, part.p, ticket, row,
+                                                       j, acc_defl, flag);
+        if (j < p) k_band_project<<<p, 256, 0, s>>>(phi, n, vj, proj.p + (size_t)j * p);
+        k_band_scale<MX, VC><<<ge, 256, 0, s>>>(S, p, row, nv, flag);
+        matvec(H, vj, w, false, flag);
+        k_band_recur<MX, VC><<<gr, kDotThreads, 0, s>>>(B, m, p, w, vj, nv, part.p, ticket, row, flag);
+      };
+      if (two)
+        go(std::integral_constant<int, 2>{});
+      else
+        go(std::integral_constant<int, 1>{});
+    });
+    QCMG_CUDA(cudaGetLastError());
+  };
+  Landing land(s);  // declared after the buffers: waits before they go
+  const size_t slot = (size_t)p * rl + 1 + (size_t)p * p;
+  QCMG_CUDA(cudaMallocHost(&land.rows, 2 * slot * sizeof(double)));
+  for (auto& e : land.done) QCMG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // p steps at a time, their rows and the flag copied back
+  auto queue = [&](int c) {
+    const int j0 = c * p, j1 = std::min(M0, j0 + p);
+    if (j0 >= j1) return;
+    for (int j = j0; j < j1; ++j) step(j);
+    double* h = land.rows + (size_t)(c & 1) * slot;
+    QCMG_CUDA(cudaMemcpyAsync(h, rows.p + (size_t)j0 * rl, (size_t)(j1 - j0) * rl * 8, cudaMemcpyDeviceToHost, s));
+    QCMG_CUDA(cudaMemcpyAsync(h + (size_t)p * rl, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (c == 0)
+      QCMG_CUDA(cudaMemcpyAsync(h + (size_t)p * rl + 1, proj.p, (size_t)p * p * 8, cudaMemcpyDeviceToHost, s));
+    QCMG_CUDA(cudaEventRecord(land.done[c & 1], s));
+  };
+  auto T = [&](int r, int c) -> double& { return t[(size_t)r + (size_t)M0 * c]; };
+  queue(0);
+  for (int c = 0; c * p < M0; ++c) {
+    queue(c + 1);  // runs during the probe; computed in vain if that ends the run
+    QCMG_CUDA(cudaEventSynchronize(land.done[c & 1]));
+    const double* h = land.rows + (size_t)(c & 1) * slot;
+    int stop;
+    std::memcpy(&stop, h + (size_t)p * rl, sizeof stop);
+    for (int j = c * p; j < std::min(M0, (c + 1) * p); ++j) {
+      if (stop >= 0 && j >= stop) {
+        run.M = stop;
+        return false;
+      }
+      const double* row = h + (size_t)(j - c * p) * rl;
+      if (j >= p) T(j, j - p) = row[0];
+      for (int i = 1; i < p; ++i)
+        if (j + i >= p) T(j, j + i - p) = row[i];
+      for (int k = std::max(0, j - p); k < j; ++k) T(k, j) = T(j, k);
+      T(j, j) = row[p];
+      if (j < p)
+        for (int k = 0; k < p; ++k)
+          P[k + (size_t)p * j] = h[(size_t)p * rl + 1 + (size_t)j * p + k] * row[p + 1];
+      if (j >= 4 * p && j % p == 0) {
+        const bool warm = run.ev_old < 1e12;
+        const double width = std::isfinite(run.last_change) && warm
+                                 ? std::max(4.0 * run.last_change, 1e-12 * std::max(1.0, std::fabs(run.ev_old)))
+                                 : 1e-3 * std::max(1.0, std::fabs(run.ev_old));
+        const double e0 = warm ? band_lowest(t, M0, j, p, run.ev_old, width) : band_lowest(t, M0, j, p);
+        const double test = std::fabs(e0 - run.ev_old);
+        if (run.ev_old < 1e12) run.last_change = test;
+        run.ev_old = e0;
+        if (test < acc_band) {
+          run.M = j;
+          return true;
+        }
+      }
+    }
+  }
+  run.M = M0;
+  return true;
+}
+
+}  // namespace qcmg

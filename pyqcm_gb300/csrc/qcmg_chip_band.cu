@@ -22,6 +22,7 @@
 
 #include "qcmg_chip.cuh"
 #include "qcmg_tridiag.h"
+#include "qcmg_vec.cuh"
 
 namespace qcmg {
 
@@ -38,24 +39,6 @@ struct ChipBand {
 };
 
 constexpr int pow2_of(int n) { return n <= 1 ? 1 : 2 * pow2_of((n + 1) / 2); }
-
-// Sums each of the V values over the 32 lanes: lane l gets value l / (32 / V).
-template <int V>
-__device__ __forceinline__ double lane_sums(double (&a)[V], int lane) {
-  int o = 16;
-#pragma unroll
-  for (int n = V; n > 1; n >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < n / 2; ++i) {
-      const double give = up ? a[i] : a[i + n / 2], keep = up ? a[i + n / 2] : a[i];
-      a[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-    }
-  }
-  double s = a[0];
-  for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
-}
 
 template <int P>
 __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {

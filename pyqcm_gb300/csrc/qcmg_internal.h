@@ -198,8 +198,10 @@ struct qcmg_hamiltonian {
 };
 
 namespace qcmg {
-// Matrix-free factorized product y (+)= H x on the handle's stream.
-void matvec(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate);
+// Matrix-free factorized product y (+)= H x on the handle's stream; nothing
+// is done when *skip (device memory, may be null) is not negative.
+void matvec(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate,
+            const int* skip = nullptr);
 // A chain of kernel nodes added to a CUDA graph explicitly (no stream
 // capture, so no other host thread's device-wide synchronization can
 // invalidate it): each node depends on the previous one.

@@ -10,11 +10,13 @@
 #include <random>
 
 #include "qcmg_blas.h"
+#include "qcmg_band.h"
 #include "qcmg_chip.h"
 #include "qcmg_fxpath.h"
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
 #include "qcmg_tridiag.h"
+#include "qcmg_vec.cuh"
 
 namespace qcmg {
 
@@ -22,24 +24,6 @@ namespace qcmg {
 // multi-vector kernels used by reorthogonalization and band Lanczos
 
 constexpr int kTile = 2048;  // elements of w staged per block iteration
-
-// Vector lists and coefficients passed to the kernels by value (up to
-// kByValue entries): no host-to-device copy of a pointer array per call,
-// which on small sectors costs more than the kernel.  Longer lists go
-// through device arrays (the same kernels, instantiated on pointers).
-constexpr int kByValue = 64;
-struct VecList {
-  const double* v[kByValue];
-  __device__ const double* operator[](int k) const { return v[k]; }
-};
-struct MutVecList {
-  double* v[kByValue];
-  __device__ double* operator[](int k) const { return v[k]; }
-};
-struct CoefList {
-  double c[kByValue];
-  __device__ double operator[](int k) const { return c[k]; }
-};
 
 // part[b*m + k] = sum over block b's tiles of V_k . w
 template <class VL>
@@ -67,38 +51,74 @@ __global__ void __launch_bounds__(256) k_multidot(VL V, int m, const double* __r
   for (int k = threadIdx.x; k < m; k += blockDim.x) part[(size_t)blockIdx.x * m + k] = acc[k];
 }
 
-// The same partials for short lists, accumulated in registers: each thread
-// keeps m sums over its elements, so an element costs one load of w and m
-// independent loads and FMAs (no dependent chain per vector, no staging
-// barrier), and the block then reduces each sum in a fixed order.
-template <int MAXM>
-__global__ void __launch_bounds__(256) k_multidot_reg(VecList V, int m,
-                                                      const double* __restrict__ w, size_t n,
-                                                      double* __restrict__ part) {
+// part[b m + k] = block b's share of V_k . w, for the MAXM vectors from
+// k0 = MAXM blockIdx.y on: every thread keeps MAXM sums over its elements and
+// has the MAXM loads of an element in flight together, so the kernel runs at
+// the FP64 pipe (one FMA per element and vector, the floor) instead of one
+// load's latency per element.
+template <int MAXM, int VEC, class VL>
+__global__ void __launch_bounds__(kDotThreads, 2) k_dots(VL V, int m, const double* __restrict__ w,
+                                                        size_t nv, double* __restrict__ part) {
+  const int k0 = blockIdx.y * MAXM, mm = min(MAXM, m - k0);
   double acc[MAXM];
 #pragma unroll
   for (int k = 0; k < MAXM; ++k) acc[k] = 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
        i += (size_t)gridDim.x * blockDim.x) {
-    const double wi = w[i];
+    const Pack<VEC> x = load_pack<VEC>(w, i);
+    Pack<VEC> v[MAXM];
 #pragma unroll
     for (int k = 0; k < MAXM; ++k)
-      if (k < m) acc[k] = fma(V[k][i], wi, acc[k]);
-  }
-  __shared__ double red[8][MAXM];  // one row per warp of the 256-thread block
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+      if (k < mm) v[k] = load_pack<VEC>(V[k0 + k], i);
 #pragma unroll
-  for (int k = 0; k < MAXM; ++k) {
-    double v = acc[k];
+    for (int k = 0; k < MAXM; ++k)
+      if (k < mm)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[wp][k] = v;
+        for (int e = 0; e < VEC; ++e) acc[k] = fma(v[k].e[e], x.e[e], acc[k]);
   }
+  block_sums<MAXM>(acc, mm, part + (size_t)blockIdx.x * m + k0);
+}
+
+// out[k] = sum_b part[b m + k] in a fixed order, one warp per value.
+__global__ void __launch_bounds__(1024) k_dots_final(const double* __restrict__ part, int nb, int m,
+                                                     double* __restrict__ out) {
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int k = wp; k < m; k += nw) {
+    double s = 0.0;
+    for (int b = lane; b < nb; b += 32) s += part[(size_t)b * m + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[k] = s;
+  }
+}
+
+// w -= sum_k c_k V_k, c in device memory: eight vectors' loads in flight
+// together per element.
+template <int VEC, class VL>
+__global__ void __launch_bounds__(256) k_axpys(VL V, int m, const double* __restrict__ c,
+                                               double* __restrict__ w, size_t nv) {
+  extern __shared__ double cs[];
+  for (int k = threadIdx.x; k < m; k += blockDim.x) cs[k] = c[k];
   __syncthreads();
-  for (int k = threadIdx.x; k < m; k += blockDim.x) {
-    double t = 0.0;
-    for (int q = 0; q < 8; ++q) t += red[q][k];
-    part[(size_t)blockIdx.x * m + k] = t;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
+       i += (size_t)gridDim.x * blockDim.x) {
+    Pack<VEC> s = load_pack<VEC>(w, i);
+    int k = 0;
+    for (; k + 8 <= m; k += 8) {
+      Pack<VEC> v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = load_pack<VEC>(V[k + q], i);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) s.e[e] = fma(-cs[k + q], v[q].e[e], s.e[e]);
+    }
+    for (; k < m; ++k) {
+      const Pack<VEC> v = load_pack<VEC>(V[k], i);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) s.e[e] = fma(-cs[k], v.e[e], s.e[e]);
+    }
+    store_pack<VEC>(w, i, s);
   }
 }
 
@@ -220,53 +240,113 @@ void multidot_launch(int m, const double* const* V, const double* w, size_t n, d
 
 struct MultiOps {
   DevBuf<const double*> ptrs;
-  DevBuf<double> part, coef;
-  std::vector<double> host;
-  int nblocks = 0;
+  DevBuf<double> part, coef, sums;
+  std::vector<const double*> listed;  // what ptrs holds
+  double* host = nullptr;             // page-locked
+  size_t host_n = 0;
+  MultiOps() = default;
+  MultiOps(const MultiOps&) = delete;
+  MultiOps& operator=(const MultiOps&) = delete;
+  ~MultiOps() {
+    if (host) cudaFreeHost(host);
+  }
+  template <class T>
+  static void grow(DevBuf<T>& b, size_t need) {  // lists grow by one per Lanczos step
+    if (need > b.n) b.alloc(std::max(need, 2 * b.n));
+  }
+  static bool pairs(const std::vector<const double*>& V, const double* w, size_t n) {
+    uintptr_t a = (uintptr_t)w;
+    for (const double* v : V) a |= (uintptr_t)v;
+    return (a & 15u) == 0 && (n & 1u) == 0;
+  }
+  // f(list, device-accessible) with the vectors by value or, for long lists,
+  // in a device array
+  template <class F>
+  void with_list(const std::vector<const double*>& V, cudaStream_t s, F&& f) {
+    const int m = (int)V.size();
+    if (m <= kByValue) {
+      VecList L;
+      for (int k = 0; k < m; ++k) L.v[k] = V[k];
+      f(L);
+    } else {
+      if (listed != V) {
+        listed = V;
+        grow(ptrs, m);
+        QCMG_CUDA(cudaMemcpyAsync(ptrs.p, listed.data(), m * sizeof(double*), cudaMemcpyHostToDevice, s));
+      }
+      f((const double* const*)ptrs.p);
+    }
+  }
+  // V_k . w for every k, left in device memory (m doubles)
+  const double* dots_dev(const std::vector<const double*>& V, const double* w, size_t n, cudaStream_t s) {
+    const int m = (int)V.size();
+    const bool two = pairs(V, w, n);
+    const size_t nv = two ? n / 2 : n;
+    const int nb = (int)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
+    grow(part, (size_t)nb * m);
+    grow(sums, m);
+    with_list(V, s, [&](auto L) {
+      using VL = decltype(L);
+      auto go = [&](auto maxm) {
+        constexpr int MX = decltype(maxm)::value;
+        const dim3 grid((unsigned)nb, (unsigned)((m + MX - 1) / MX));
+        if (two)
+          k_dots<MX, 2, VL><<<grid, kDotThreads, 0, s>>>(L, m, w, nv, part.p);
+        else
+          k_dots<MX, 1, VL><<<grid, kDotThreads, 0, s>>>(L, m, w, nv, part.p);
+      };
+      // one group when it fits; eights for long lists (96 vectors of 3.3M
+      // elements: 581 us in eights, 611 in sixteens, floor 506)
+      if (m <= 4)
+        go(std::integral_constant<int, 4>{});
+      else if (m <= 8 || m > 16)
+        go(std::integral_constant<int, 8>{});
+      else if (m <= 12)
+        go(std::integral_constant<int, 12>{});
+      else
+        go(std::integral_constant<int, 16>{});
+    });
+    QCMG_CUDA(cudaGetLastError());
+    k_dots_final<<<1, std::min(1024, 32 * m), 0, s>>>(part.p, nb, m, sums.p);
+    QCMG_CUDA(cudaGetLastError());
+    return sums.p;
+  }
   void multidot(const std::vector<const double*>& V, const double* w, size_t n, cudaStream_t s,
                 std::vector<double>& out) {
     const int m = (int)V.size();
     out.assign(m, 0.0);
     if (m == 0) return;
-    nblocks = multidot_blocks(n);
-    if (m <= 32) {
-      // register accumulators: 256-thread blocks, two per SM at most
-      nblocks = (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 2 * 152));
-      part.alloc((size_t)nblocks * m);
-      VecList L;
-      for (int k = 0; k < m; ++k) L.v[k] = V[k];
-      if (m <= 4)
-        k_multidot_reg<4><<<nblocks, 256, 0, s>>>(L, m, w, n, part.p);
-      else if (m <= 8)
-        k_multidot_reg<8><<<nblocks, 256, 0, s>>>(L, m, w, n, part.p);
-      else if (m <= 16)
-        k_multidot_reg<16><<<nblocks, 256, 0, s>>>(L, m, w, n, part.p);
-      else
-        k_multidot_reg<32><<<nblocks, 256, 0, s>>>(L, m, w, n, part.p);
-    } else if (m <= kByValue) {
-      part.alloc((size_t)nblocks * m);
-      VecList L;
-      for (int k = 0; k < m; ++k) L.v[k] = V[k];
-      k_multidot<VecList><<<nblocks, 256, m * sizeof(double), s>>>(L, m, w, n, part.p);
-    } else {
-      part.alloc((size_t)nblocks * m);
-      ptrs.alloc(m);
-      QCMG_CUDA(cudaMemcpyAsync(ptrs.p, V.data(), m * sizeof(double*), cudaMemcpyHostToDevice, s));
-      k_multidot<const double* const*>
-          <<<nblocks, 256, m * sizeof(double), s>>>(ptrs.p, m, w, n, part.p);
+    const double* d = dots_dev(V, w, n, s);
+    if (host_n < (size_t)m) {
+      if (host) cudaFreeHost(host);
+      host = nullptr;
+      host_n = std::max<size_t>(m, 64);
+      QCMG_CUDA(cudaMallocHost(&host, host_n * sizeof(double)));
     }
-    QCMG_CUDA(cudaGetLastError());
-    // the partials come back and are summed here in k_multidot_final's order
-    // (one launch fewer per call; the sums are bitwise the same)
-    host.resize((size_t)nblocks * m);
-    QCMG_CUDA(cudaMemcpyAsync(host.data(), part.p, host.size() * sizeof(double),
-                              cudaMemcpyDeviceToHost, s));
+    QCMG_CUDA(cudaMemcpyAsync(host, d, m * sizeof(double), cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaStreamSynchronize(s));
-    for (int k = 0; k < m; ++k) {
-      double acc = 0.0;
-      for (int b = 0; b < nblocks; ++b) acc += host[(size_t)b * m + k];
-      out[k] = acc;
-    }
+    std::copy(host, host + m, out.begin());
+  }
+  // w -= sum_k c_k V_k with c in device memory
+  void axpys_dev(const std::vector<const double*>& V, const double* c, double* w, size_t n,
+                 cudaStream_t s) {
+    const int m = (int)V.size();
+    if (m == 0 || n == 0) return;
+    const bool two = pairs(V, w, n);
+    const size_t nv = two ? n / 2 : n;
+    with_list(V, s, [&](auto L) {
+      using VL = decltype(L);
+      if (two)
+        k_axpys<2, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv);
+      else
+        k_axpys<1, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv);
+    });
+    QCMG_CUDA(cudaGetLastError());
+  }
+  // one Gram-Schmidt pass: w -= sum_k (V_k . w) V_k, no host round trip
+  void project_out(const std::vector<const double*>& V, double* w, size_t n, cudaStream_t s) {
+    if (V.empty()) return;
+    axpys_dev(V, dots_dev(V, w, n, s), w, n, s);
   }
   // w -= sum_k c_k V_k, then d = w . u and w -= d u with d left at d_dev:
   // two launches.  False (nothing done) for lists longer than kByValue.
@@ -305,15 +385,11 @@ struct MultiOps {
       }
       k_multiaxpy<VecList, CoefList>
           <<<elementwise_grid(n), 256, m * sizeof(double), s>>>(L, m, C, w, n);
+      QCMG_CUDA(cudaGetLastError());
     } else {
-      ptrs.alloc(m);
-      coef.alloc(m);
-      QCMG_CUDA(cudaMemcpyAsync(ptrs.p, V.data(), m * sizeof(double*), cudaMemcpyHostToDevice, s));
-      QCMG_CUDA(cudaMemcpyAsync(coef.p, c.data(), m * sizeof(double), cudaMemcpyHostToDevice, s));
-      k_multiaxpy<const double* const*, const double*>
-          <<<elementwise_grid(n), 256, m * sizeof(double), s>>>(ptrs.p, m, coef.p, w, n);
+      coef.upload(c.data(), m, s);
+      axpys_dev(V, coef.p, w, n, s);
     }
-    QCMG_CUDA(cudaGetLastError());
   }
   // v <- sc v;  V_k <- V_k - c_k v  (k_scale_sub)
   DevBuf<double*> wptrs;
@@ -504,33 +580,38 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
       matvec(H, x, y, false);
   };
   const int keep = std::max(reorth, 2);
-  std::vector<DevVec> V;  // pool, reused across restarts
+  // the vectors, reused across restarts; allocated several at a time (up to
+  // 512 MB), since an allocation per step cost as much as a step
+  const size_t stride = (n + 1) & ~(size_t)1;
+  const size_t block = std::max<size_t>(1, std::min<size_t>(keep, ((size_t)512 << 20) / (stride * 8)));
+  std::vector<DevVec> blocks;
+  std::vector<double*> V;
+  auto add_vector = [&] {
+    if (V.size() == blocks.size() * block) blocks.emplace_back(std::min(block, (size_t)keep - V.size()) * stride);
+    V.push_back(blocks.back().p + (V.size() % block) * stride);
+  };
   std::vector<const double*> Vp;
   MultiOps mops;
-  std::vector<double> c;
-  V.emplace_back(n);
-  QCMG_CUDA(cudaMemcpyAsync(V[0].p, x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
+  add_vector();
+  QCMG_CUDA(cudaMemcpyAsync(V[0], x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
   double* w = r.p;  // residual
   Events ev;
   int total = 0;
   bool converged = false;
   while (!converged) {
-    Vp.assign(1, V[0].p);
+    Vp.assign(1, V[0]);
     res.alpha.clear();
     res.beta.clear();
     for (int j = 0;; ++j) {
       ev.record(0, s);
-      product(V[j].p, w);
+      product(V[j], w);
       ev.record(1, s);
-      if (j > 0) axpy(w, V[j - 1].p, -res.beta.back(), n, s);
-      double a = red.dot(V[j].p, w, n, s);
+      if (j > 0) axpy(w, V[j - 1], -res.beta.back(), n, s);
+      double a = red.dot(V[j], w, n, s);
       res.alpha.push_back(a);
-      axpy(w, V[j].p, -a, n, s);
+      axpy(w, V[j], -a, n, s);
       ev.record(2, s);
-      for (int pass = 0; pass < 2; ++pass) {
-        mops.multidot(Vp, w, n, s, c);
-        mops.multiaxpy(Vp, c, w, n, s);
-      }
+      for (int pass = 0; pass < 2; ++pass) mops.project_out(Vp, w, n, s);
       ev.record(3, s);
       double b = std::sqrt(red.dot(w, w, n, s));  // synchronizes the stream
       res.product_ms += ev.elapsed(0, 1);
@@ -550,10 +631,10 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
         throw Error(QCMG_ERR_NOCONV, "reorthogonalized Lanczos did not converge within " +
                                          std::to_string(max_iter) + " iterations");
       if ((int)Vp.size() >= keep) break;  // cap reached: restart
-      if ((int)V.size() <= j + 1) V.emplace_back(n);
-      QCMG_CUDA(cudaMemcpyAsync(V[j + 1].p, w, n * 8, cudaMemcpyDeviceToDevice, s));
-      scale(V[j + 1].p, 1.0 / b, n, s);
-      Vp.push_back(V[j + 1].p);
+      if ((int)V.size() <= j + 1) add_vector();
+      QCMG_CUDA(cudaMemcpyAsync(V[j + 1], w, n * 8, cudaMemcpyDeviceToDevice, s));
+      scale(V[j + 1], 1.0 / b, n, s);
+      Vp.push_back(V[j + 1]);
     }
     if (converged) break;
     // restart from the Ritz vector sum_k z_k V_k, normalized
@@ -563,8 +644,8 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
     mops.multiaxpy(Vp, mz, w, n, s);
     const double nrm = std::sqrt(red.dot(w, w, n, s));
     if (!(nrm > 0.0)) throw Error(QCMG_ERR_NUMERIC, "Lanczos restart vector vanished");
-    QCMG_CUDA(cudaMemcpyAsync(V[0].p, w, n * 8, cudaMemcpyDeviceToDevice, s));
-    scale(V[0].p, 1.0 / nrm, n, s);
+    QCMG_CUDA(cudaMemcpyAsync(V[0], w, n * 8, cudaMemcpyDeviceToDevice, s));
+    scale(V[0], 1.0 / nrm, n, s);
     ++res.restarts;
   }
   res.niter = total;
@@ -899,10 +980,6 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
     if (v[k]) pool.push_back(v[k]);
     v[k] = nullptr;
   };
-  for (int i = 0; i < p; ++i) {
-    v[i] = get();
-    QCMG_CUDA(cudaMemcpyAsync(v[i], phip[i], n * 8, cudaMemcpyDeviceToDevice, s));
-  }
   t.assign((size_t)M0 * M0, 0.0);
   auto T = [&](int r, int c) -> double& { return t[(size_t)r + (size_t)M0 * c]; };
   P.assign((size_t)p * M0, 0.0);
@@ -914,7 +991,34 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
   Cusolver solver;
   double ev_old = 1e12;
   double last_change = INFINITY;
-  int j;
+  // the steps up to the first deflation (usually all of them), without a
+  // host round trip per step; then the loop below takes over
+  int j = 0;
+  if (p <= kBandMax) {
+    std::vector<double*> ring(2 * p + 1);
+    for (double*& r : ring) r = get();
+    BandRun run;
+    run.ev_old = ev_old;
+    run.last_change = last_change;
+    if (band_steps(H, p, phi0, M0, acc_defl, acc_band, ring, t, P, run))
+      return band_result(H, p, M0, run.M, t, P, true);
+    j = run.M;
+    ev_old = run.ev_old;
+    last_change = run.last_change;
+    const int R = 2 * p + 1;
+    std::vector<char> used(R, 0);
+    for (int k = std::max(0, j - p); k < std::min(j + p, M0p); ++k) {
+      v[k] = ring[k % R];
+      used[k % R] = 1;
+    }
+    for (int k = 0; k < R; ++k)
+      if (!used[k]) pool.push_back(ring[k]);
+  } else {
+    for (int i = 0; i < p; ++i) {
+      v[i] = get();
+      QCMG_CUDA(cudaMemcpyAsync(v[i], phip[i], n * 8, cudaMemcpyDeviceToDevice, s));
+    }
+  }
   std::vector<const double*> tg;
   std::vector<double*> gs_vecs;
   std::vector<double> gs_coef;
@@ -945,7 +1049,7 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
     for (const Pending& q : pend) T(q.r, q.c) = T(q.c, q.r) = thost[q.slot];
     pend.clear();
   };
-  for (j = 0; j < M0; ++j) {
+  for (; j < M0; ++j) {
     // One multi-dot on the unscaled v_j gives its norm, its projections on
     // the p start vectors and its dots with the next pc-1 vectors (each of
     // those vectors is changed only by its own update below, so the dots

@@ -27,7 +27,8 @@ k_matvec_f64(uint32_t du, uint32_t dd, int L,
              const double* __restrict__ val_dn, const double* __restrict__ diag_dn,
              const uint32_t* __restrict__ bin_up, const uint32_t* __restrict__ bin_dn, double U,
              const double* __restrict__ wdn, const double* __restrict__ x, double* __restrict__ y,
-             int accumulate) {
+             int accumulate, const int* skip) {
+  if (skip && *(volatile const int*)skip >= 0) return;
   extern __shared__ double xs[];
   for (uint32_t a = blockIdx.x; a < dd; a += gridDim.x) {
     const double* xa = x + (size_t)a * du;
@@ -85,7 +86,9 @@ k_matvec_ell(uint32_t du, uint32_t dd, int L, int parts, const uint32_t* __restr
              const uint32_t* __restrict__ col_dn, const double* __restrict__ val_dn,
              const double* __restrict__ diag_dn, const uint32_t* __restrict__ bin_up,
              const uint32_t* __restrict__ bin_dn, double U, const double* __restrict__ wdn,
-             const double* __restrict__ x, double* __restrict__ y, int accumulate) {
+             const double* __restrict__ x, double* __restrict__ y, int accumulate,
+             const int* skip) {
+  if (skip && *(volatile const int*)skip >= 0) return;
   extern __shared__ double xs[];  // du, then the value table, then U popc
   double* vt = xs + du;
   double* ut = vt + nval;
@@ -133,7 +136,7 @@ k_matvec_ell(uint32_t du, uint32_t dd, int L, int parts, const uint32_t* __restr
 // to `launch(kernel, grid, threads, smem, args...)`.
 template <int INTER, class Launch>
 static void product_launch(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate,
-                           Launch&& launch) {
+                           const int* skip, Launch&& launch) {
   auto& up = H->up;
   auto& dn = H->dn;
   int sms = 0, max_optin = 0;
@@ -155,7 +158,7 @@ static void product_launch(qcmg_hamiltonian* H, const double* x, double* y, bool
            (const uint32_t*)up.ell, (const uint16_t*)up.len, (const double*)up.vtab, up.nval,
            (const double*)up.diag.p, (const uint32_t*)dn.rowptr.p, (const uint32_t*)dn.col.p,
            (const double*)dn.val.p, (const double*)dn.diag.p, (const uint32_t*)up.bin.p,
-           (const uint32_t*)dn.bin.p, H->U, (const double*)H->wdn.p, x, y, accumulate ? 1 : 0);
+           (const uint32_t*)dn.bin.p, H->U, (const double*)H->wdn.p, x, y, accumulate ? 1 : 0, skip);
     return;
   }
   // half bases too large for the slot form: rows from the CSR, the slab in
@@ -171,28 +174,28 @@ static void product_launch(qcmg_hamiltonian* H, const double* x, double* y, bool
          (const uint32_t*)up.rowptr.p, (const uint32_t*)up.col.p, (const double*)up.val.p,
          (const double*)up.diag.p, (const uint32_t*)dn.rowptr.p, (const uint32_t*)dn.col.p,
          (const double*)dn.val.p, (const double*)dn.diag.p, (const uint32_t*)up.bin.p,
-         (const uint32_t*)dn.bin.p, H->U, (const double*)H->wdn.p, x, y, accumulate ? 1 : 0);
+         (const uint32_t*)dn.bin.p, H->U, (const double*)H->wdn.p, x, y, accumulate ? 1 : 0, skip);
 }
 
 template <class Launch>
 static void product_any(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate,
-                        Launch&& launch) {
+                        const int* skip, Launch&& launch) {
   switch (H->inter_kind) {
-    case QCMG_INTER_NONE: product_launch<QCMG_INTER_NONE>(H, x, y, accumulate, launch); break;
-    case QCMG_INTER_ONSITE: product_launch<QCMG_INTER_ONSITE>(H, x, y, accumulate, launch); break;
-    default: product_launch<QCMG_INTER_GENERAL>(H, x, y, accumulate, launch); break;
+    case QCMG_INTER_NONE: product_launch<QCMG_INTER_NONE>(H, x, y, accumulate, skip, launch); break;
+    case QCMG_INTER_ONSITE: product_launch<QCMG_INTER_ONSITE>(H, x, y, accumulate, skip, launch); break;
+    default: product_launch<QCMG_INTER_GENERAL>(H, x, y, accumulate, skip, launch); break;
   }
 }
 
 void matvec_node(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate, GraphChain& gc) {
-  product_any(H, x, y, accumulate, [&](auto kern, unsigned grid, int threads, size_t smem, auto... args) {
+  product_any(H, x, y, accumulate, nullptr, [&](auto kern, unsigned grid, int threads, size_t smem, auto... args) {
     gc.add(kern, dim3(grid), dim3(threads), smem, args...);
   });
 }
 
-void matvec(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate) {
+void matvec(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate, const int* skip) {
   if (H->dim == 0) return;
-  product_any(H, x, y, accumulate, [&](auto kern, unsigned grid, int threads, size_t smem, auto... args) {
+  product_any(H, x, y, accumulate, skip, [&](auto kern, unsigned grid, int threads, size_t smem, auto... args) {
     kern<<<grid, threads, smem, H->stream>>>(args...);
     QCMG_CUDA(cudaGetLastError());
   });

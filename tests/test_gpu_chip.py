@@ -117,3 +117,16 @@ def test_band_lanczos_exhausts_small_sectors(L, nup, ndn, p):
     G = _green(e, Q, zs)
     ref = _oracle_green(S, phi, zs)
     assert np.max(np.abs(G - ref)) < 1e-8 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("cap", [2, 4, 5, 8, 9, 12, 13, 16, 17, 40, 64, 65, 90])
+@pytest.mark.parametrize("L,nup,ndn", [(6, 3, 3), (7, 3, 4)])
+def test_reorthogonalized_lists(cap, L, nup, ndn):
+    """The projection kernels at every list size they are built for and past
+    64 vectors, on 400 (pairs of elements) and 1,225 states (odd): the energy
+    of dense diagonalization, restarting at the cap."""
+    H, S = _sector(L, nup, ndn, 21)
+    e0 = H.lanczos(tol=1e-6, max_iter=4000, reorth=cap, want_psi=False)[0]
+    A = np.array([S.matvec(v) for v in np.eye(S.dim)])
+    # the energy's error is the square of the residual over the gap (> 1e-3)
+    assert abs(e0 - np.linalg.eigvalsh(A)[0]) < 1e-8
