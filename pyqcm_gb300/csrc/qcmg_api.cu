@@ -19,6 +19,7 @@
 #include "qcmg_fxpath.h"
 #include "qcmg_krylov.h"
 #include "qcmg_lattice.h"
+#include "qcmg_pool.h"
 
 namespace qcmg {
 
@@ -162,6 +163,26 @@ int qcmg_halfbasis_rank(int L, int N, const uint32_t* states, size_t n, uint32_t
   });
 }
 
+// Waits for everything that may use the handle's memory, then frees it.
+static void release_handle(qcmg_hamiltonian* H) {
+  cudaSetDevice(H->device);
+  if (H->foreign)
+    cudaDeviceSynchronize();  // an earlier stream of the caller's may still be busy
+  else if (H->own_stream)
+    cudaStreamSynchronize(H->own_stream);
+  if (H->copy_stream) {
+    cudaStreamSynchronize(H->copy_stream);
+    cudaStreamDestroy(H->copy_stream);
+  }
+  if (H->ev_x) cudaEventDestroy(H->ev_x);
+  if (H->ev_y) cudaEventDestroy(H->ev_y);
+  if (H->own_stream) cudaStreamDestroy(H->own_stream);
+  if (H->up.mem) pool_put(H->up.mem, H->up.mem_got);
+  if (H->dn.mem) pool_put(H->dn.mem, H->dn.mem_got);
+  if (H->cross_mem) pool_put(H->cross_mem, H->cross_got);
+  delete H;
+}
+
 int qcmg_hamiltonian_create(int L, int n_up, int n_dn, int n_hop_up, const int32_t* up_r,
                             const int32_t* up_c, const double* up_v, int n_hop_dn,
                             const int32_t* dn_r, const int32_t* dn_c, const double* dn_v,
@@ -185,6 +206,8 @@ int qcmg_hamiltonian_create(int L, int n_up, int n_dn, int n_hop_up, const int32
     }
     use_device();
     auto* H = new qcmg_hamiltonian();
+    // sized once by the sector, and idle when release_handle gets to them
+    H->seed_vec.pooled = H->xbuf.pooled = H->ybuf.pooled = true;
     try {
       H->device = g_device;
       H->L = L;
@@ -195,8 +218,10 @@ int qcmg_hamiltonian_create(int L, int n_up, int n_dn, int n_hop_up, const int32
       std::vector<HopElement> eu, ed;
       for (int k = 0; k < n_hop_up; ++k) eu.push_back({up_r[k], up_c[k], up_v[k]});
       for (int k = 0; k < n_hop_dn; ++k) ed.push_back({dn_r[k], dn_c[k], dn_v[k]});
-      build_halfop(H->up, L, n_up, eu, true, H->stream);
-      build_halfop(H->dn, L, n_dn, ed, false, H->stream);
+      std::vector<std::vector<double>> staging;  // read by uploads until the wait below
+      staging.reserve(2);
+      build_halfop(H->up, L, n_up, eu, true, staging, H->stream);
+      build_halfop(H->dn, L, n_dn, ed, false, staging, H->stream);
       H->du = H->up.dim;
       H->dd = H->dn.dim;
       H->dim = (size_t)H->du * H->dd;
@@ -224,29 +249,23 @@ int qcmg_hamiltonian_create(int L, int n_up, int n_dn, int n_hop_up, const int32
       }
       uint32_t mask = 0;
       H->inter_kind = (int)classify_onsite(W, L, &H->U, &mask);
-      H->max_inter_abs = 0.0;
-      for (int r = 0; r < L; ++r) {
-        double s = 0.0;
-        for (int c = 0; c < L; ++c) s += std::fabs(W[(size_t)r * L + c]);
-        H->max_inter_abs += s;
-      }
       if (H->inter_kind == QCMG_INTER_ONSITE && mask != (L >= 32 ? 0xffffffffu : (1u << L) - 1u)) {
         // masked on-site term (e.g. no U on bath orbitals): tabulate instead
         H->inter_kind = QCMG_INTER_GENERAL;
       }
       if (H->inter_kind == QCMG_INTER_GENERAL && H->dd) {
-        DevBuf<double> dW;
-        dW.upload(W.data(), W.size(), H->stream);
-        H->wdn.alloc((size_t)H->dd * L);
-        k_cross_table<<<(H->dd + 127) / 128, 128, 0, H->stream>>>(H->dd, L, H->dn.bin.p, dW.p,
-                                                                  H->wdn.p);
+        // the table, then the matrix it is built from
+        const size_t nt = (size_t)H->dd * L;
+        H->cross_mem = pool_get((nt + W.size()) * 8, &H->cross_got);
+        H->wdn.borrow(static_cast<double*>(H->cross_mem), nt);
+        QCMG_CUDA(cudaMemcpyAsync(H->wdn.p + nt, W.data(), W.size() * 8, cudaMemcpyHostToDevice, H->stream));
+        k_cross_table<<<(H->dd + 127) / 128, 128, 0, H->stream>>>(H->dd, L, H->dn.bin.p,
+                                                                  H->wdn.p + nt, H->wdn.p);
         QCMG_CUDA(cudaGetLastError());
-        QCMG_CUDA(cudaStreamSynchronize(H->stream));
       }
       QCMG_CUDA(cudaStreamSynchronize(H->stream));
     } catch (...) {
-      if (H->own_stream) cudaStreamDestroy(H->own_stream);
-      delete H;
+      release_handle(H);
       throw;
     }
     *out = H;
@@ -255,17 +274,7 @@ int qcmg_hamiltonian_create(int L, int n_up, int n_dn, int n_hop_up, const int32
 
 int qcmg_hamiltonian_destroy(qcmg_hamiltonian* H) {
   return guarded([&] {
-    if (!H) return;
-    cudaSetDevice(H->device);
-    if (H->stream) cudaStreamSynchronize(H->stream);
-    if (H->copy_stream) {
-      cudaStreamSynchronize(H->copy_stream);
-      cudaStreamDestroy(H->copy_stream);
-    }
-    if (H->ev_x) cudaEventDestroy(H->ev_x);
-    if (H->ev_y) cudaEventDestroy(H->ev_y);
-    if (H->own_stream) cudaStreamDestroy(H->own_stream);
-    delete H;
+    if (H) release_handle(H);
   });
 }
 
@@ -274,6 +283,7 @@ int qcmg_hamiltonian_set_stream(qcmg_hamiltonian* H, void* stream) {
     QCMG_CHECK_ARG(H != nullptr, "NULL handle");
     std::lock_guard<std::mutex> lock(H->mu);
     H->stream = stream ? (cudaStream_t)stream : H->own_stream;
+    if (stream) H->foreign = true;
   });
 }
 
@@ -760,7 +770,7 @@ int qcmg_apply_c(int L, int orb, int pm, int n_up, int n_dn, const double* x, do
       QCMG_CUDA(cudaStreamSynchronize(0));
       return;
     }
-    DevBuf<double> dx, dy;
+    PoolBuf<double> dx, dy;
     dx.upload(x, n1, 0);
     if (acc)
       dy.upload(y, n2, 0);
@@ -789,7 +799,7 @@ int qcmg_green_function(int L, int M, const double* e, const double* v, int nz, 
       return;
     }
     use_device();
-    DevBuf<double> de, dv, dz, dG;
+    PoolBuf<double> de, dv, dz, dG;
     de.upload(e, M, 0);
     dv.upload(v, (size_t)2 * L * M, 0);
     dz.upload(z, (size_t)2 * nz, 0);
@@ -808,7 +818,7 @@ int qcmg_self_energy(int L, int M, const double* e, const double* v, int nb, con
                    "NULL argument");
     if (nz == 0) return;
     use_device();
-    DevBuf<double> de, dv, dtcb, deb, dtc, dz, ds, dg;
+    PoolBuf<double> de, dv, dtcb, deb, dtc, dz, ds, dg;
     if (M) {
       de.upload(e, M, 0);
       dv.upload(v, (size_t)2 * L * M, 0);

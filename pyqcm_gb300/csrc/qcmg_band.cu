@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "qcmg_band.h"
+#include "qcmg_pool.h"
 #include "qcmg_tridiag.h"
 #include "qcmg_vec.cuh"
 
@@ -197,16 +198,17 @@ void with_size(int p, F&& f) {
     f(std::integral_constant<int, 16>{});
 }
 
-struct Landing {  // page-locked rows and their events
-  double* rows = nullptr;
-  cudaEvent_t done[2] = {nullptr, nullptr};
+// Waits for the stream before the buffers declared ahead of it go.
+struct Wait {
   cudaStream_t s;
-  explicit Landing(cudaStream_t st) : s(st) {}
-  ~Landing() {
+  cudaEvent_t e[2] = {nullptr, nullptr};
+  explicit Wait(cudaStream_t st) : s(st) {
+    for (auto& x : e) QCMG_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+  }
+  ~Wait() {
     cudaStreamSynchronize(s);
-    if (rows) cudaFreeHost(rows);
-    for (auto e : done)
-      if (e) cudaEventDestroy(e);
+    for (auto x : e)
+      if (x) cudaEventDestroy(x);
   }
 };
 
@@ -225,8 +227,9 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   const unsigned gd = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
   const unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 3 * 152));
   const unsigned ge = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + 255) / 256, 152 * 8));
-  DevBuf<double> rows, proj, part;
-  DevBuf<int> flags;  // the deflated step, then the block counter
+  PoolBuf<double> rows, proj, part;
+  PinnedBuf<double> landed;  // p steps' rows, the flag, the projections; twice
+  PoolBuf<int> flags;  // the deflated step, then the block counter
   rows.alloc((size_t)(M0 + 1) * rl);
   proj.alloc((size_t)p * p);
   part.alloc((size_t)std::max(gd * (unsigned)p, gr));
@@ -270,28 +273,27 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
     });
     QCMG_CUDA(cudaGetLastError());
   };
-  Landing land(s);  // declared after the buffers: waits before they go
   const size_t slot = (size_t)p * rl + 1 + (size_t)p * p;
-  QCMG_CUDA(cudaMallocHost(&land.rows, 2 * slot * sizeof(double)));
-  for (auto& e : land.done) QCMG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  landed.alloc(2 * slot);
+  Wait wait(s);
   // p steps at a time, their rows and the flag copied back
   auto queue = [&](int c) {
     const int j0 = c * p, j1 = std::min(M0, j0 + p);
     if (j0 >= j1) return;
     for (int j = j0; j < j1; ++j) step(j);
-    double* h = land.rows + (size_t)(c & 1) * slot;
+    double* h = landed.p + (size_t)(c & 1) * slot;
     QCMG_CUDA(cudaMemcpyAsync(h, rows.p + (size_t)j0 * rl, (size_t)(j1 - j0) * rl * 8, cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaMemcpyAsync(h + (size_t)p * rl, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (c == 0)
       QCMG_CUDA(cudaMemcpyAsync(h + (size_t)p * rl + 1, proj.p, (size_t)p * p * 8, cudaMemcpyDeviceToHost, s));
-    QCMG_CUDA(cudaEventRecord(land.done[c & 1], s));
+    QCMG_CUDA(cudaEventRecord(wait.e[c & 1], s));
   };
   auto T = [&](int r, int c) -> double& { return t[(size_t)r + (size_t)M0 * c]; };
   queue(0);
   for (int c = 0; c * p < M0; ++c) {
     queue(c + 1);  // runs during the probe; computed in vain if that ends the run
-    QCMG_CUDA(cudaEventSynchronize(land.done[c & 1]));
-    const double* h = land.rows + (size_t)(c & 1) * slot;
+    QCMG_CUDA(cudaEventSynchronize(wait.e[c & 1]));
+    const double* h = landed.p + (size_t)(c & 1) * slot;
     int stop;
     std::memcpy(&stop, h + (size_t)p * rl, sizeof stop);
     for (int j = c * p; j < std::min(M0, (c + 1) * p); ++j) {

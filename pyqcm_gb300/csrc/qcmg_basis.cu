@@ -15,6 +15,7 @@
 #include <mutex>
 
 #include "qcmg_internal.h"
+#include "qcmg_pool.h"
 
 namespace qcmg {
 
@@ -156,83 +157,113 @@ __global__ void k_halfop_fill(uint32_t dim, const uint32_t* __restrict__ bin,
   }
 }
 
+// rowptr from the row counts (one block; rows taken 1,024 at a time).
+__global__ void __launch_bounds__(1024) k_rowptr(uint32_t dim, uint32_t* __restrict__ rp) {
+  // on entry rp[i + 1] is row i's count
+  __shared__ uint32_t ws[32];
+  __shared__ uint32_t base;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    base = 0;
+    rp[0] = 0;
+  }
+  __syncthreads();
+  for (uint32_t i0 = 0; i0 < dim; i0 += 1024) {
+    const uint32_t i = i0 + threadIdx.x;
+    uint32_t v = i < dim ? rp[i + 1] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
+    }
+    if (lane == 31) ws[wp] = v;
+    __syncthreads();
+    if (wp == 0) {
+      uint32_t t = ws[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t q = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t += q;
+      }
+      ws[lane] = t;
+    }
+    __syncthreads();
+    const uint32_t out = base + v + (wp ? ws[wp - 1] : 0);
+    if (i < dim) rp[i + 1] = out;
+    __syncthreads();
+    if (threadIdx.x == 1023) base = out;
+    __syncthreads();
+  }
+}
+
+// No host round trip: a hop c -> r is allowed from the C(L-2, N-1) states
+// with c occupied and r empty, so the number of entries is known beforehand.
+// `staging` receives the host copies that the queued uploads read; the
+// caller keeps it until the stream is idle.
 void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, bool slots,
-                  cudaStream_t s) {
+                  std::vector<std::vector<double>>& staging, cudaStream_t s) {
   op.L = L;
   op.N = N;
   uint64_t dim64 = binomial(L, N);
   QCMG_CHECK_ARG(dim64 < (1ull << 31), "half basis too large");
   op.dim = (uint32_t)dim64;
-  op.bin.alloc(op.dim);
-  launch_halfbasis(L, N, op.dim, op.bin.p, s);
+  size_t hops = 0;
   for (auto& e : el) {
     QCMG_CHECK_ARG(e.r >= 0 && e.r < L && e.c >= 0 && e.c < L, "hop element orbital out of range");
+    if (e.r != e.c && e.v != 0.0) ++hops;
   }
-  DevBuf<HopElement> d_el;
-  d_el.upload(el.data(), el.size(), s);
-  DevBuf<uint32_t> cnt;
-  cnt.alloc(op.dim);
-  op.rowptr.alloc(op.dim + 1);
-  op.diag.alloc(op.dim);
-  if (op.dim) {
-    k_halfop_count<<<grid_for(op.dim, 256), 256, 0, s>>>(op.dim, op.bin.p, d_el.p, (int)el.size(),
-                                                          cnt.p);
-    QCMG_CUDA(cudaGetLastError());
-  }
-  std::vector<uint32_t> h_cnt(op.dim), h_rp(op.dim + 1);
-  if (op.dim)
-    QCMG_CUDA(cudaMemcpyAsync(h_cnt.data(), cnt.p, op.dim * 4, cudaMemcpyDeviceToHost, s));
-  QCMG_CUDA(cudaStreamSynchronize(s));
-  size_t nnz = 0;
-  for (uint32_t i = 0; i < op.dim; ++i) {
-    h_rp[i] = (uint32_t)nnz;
-    nnz += h_cnt[i];
-  }
-  h_rp[op.dim] = (uint32_t)nnz;
+  const uint64_t per = L >= 2 && N >= 1 ? binomial(L - 2, N - 1) : 0;
+  const uint64_t nnz = per * hops;
   QCMG_CHECK_ARG(nnz < (1ull << 32), "half operator too large");
   op.nnz = nnz;
-  QCMG_CUDA(cudaMemcpyAsync(op.rowptr.p, h_rp.data(), (op.dim + 1) * 4, cudaMemcpyHostToDevice, s));
-  op.col.alloc(nnz);
-  op.val.alloc(nnz);
-  // slot form
-  std::vector<double> h_vtab;
-  op.nval = 0;
-  if (slots && op.dim > 0 && op.dim <= 65536u && el.size() <= 1024) {
-    uint32_t width = 1;
-    for (uint32_t c : h_cnt) width = std::max(width, c);
-    for (const auto& e : el) {
-      h_vtab.push_back(e.v);
-      h_vtab.push_back(-e.v);
+  // slot form: value table +-v per element, at most one hop of a row per element
+  const bool slot = slots && op.dim > 0 && op.dim <= 65536u && el.size() <= 1024;
+  op.nval = slot ? (int)std::max<size_t>(1, 2 * el.size()) : 0;
+  const size_t width = slot ? std::max<size_t>(1, hops) : 0;
+  // the tables' places, in doubles
+  size_t at = 0;
+  auto place = [&](size_t bytes) {
+    const size_t here = at;
+    at += (bytes + 7) / 8;
+    return here;
+  };
+  const size_t o_val = place(nnz * 8), o_diag = place((size_t)op.dim * 8), o_vtab = place((size_t)op.nval * 8),
+               o_el = place(el.size() * sizeof(HopElement)), o_bin = place((size_t)op.dim * 4),
+               o_rp = place(((size_t)op.dim + 1) * 4), o_col = place(nnz * 4),
+               o_ell = place(width * op.dim * 4), o_len = place(slot ? (size_t)op.dim * 2 : 0);
+  op.mem = pool_get(at * 8, &op.mem_got);
+  double* m = static_cast<double*>(op.mem);
+  op.val.borrow(m + o_val, nnz);
+  op.diag.borrow(m + o_diag, op.dim);
+  op.bin.borrow(reinterpret_cast<uint32_t*>(m + o_bin), op.dim);
+  op.rowptr.borrow(reinterpret_cast<uint32_t*>(m + o_rp), (size_t)op.dim + 1);
+  op.col.borrow(reinterpret_cast<uint32_t*>(m + o_col), nnz);
+  if (slot) {
+    op.vtab = m + o_vtab;
+    op.ell = reinterpret_cast<uint32_t*>(m + o_ell);
+    op.len = reinterpret_cast<uint16_t*>(m + o_len);
+  }
+  // value table and elements in one upload (they are neighbours)
+  staging.emplace_back(o_bin - o_vtab, 0.0);
+  std::vector<double>& h = staging.back();
+  if (slot)
+    for (size_t k = 0; k < el.size(); ++k) {
+      h[2 * k] = el[k].v;
+      h[2 * k + 1] = -el[k].v;
     }
-    if (h_vtab.empty()) h_vtab.push_back(0.0);
-    op.nval = (int)h_vtab.size();
-    const size_t words = (size_t)width * op.dim;
-    op.slots.alloc(h_vtab.size() + (words + 1) / 2 + ((size_t)op.dim + 3) / 4);
-    op.vtab = op.slots.p;
-    op.ell = reinterpret_cast<uint32_t*>(op.vtab + h_vtab.size());
-    op.len = reinterpret_cast<uint16_t*>(op.vtab + h_vtab.size() + (words + 1) / 2);
-    QCMG_CUDA(cudaMemcpyAsync(op.vtab, h_vtab.data(), h_vtab.size() * 8, cudaMemcpyHostToDevice, s));
-  }
+  if (!el.empty()) std::memcpy(h.data() + (o_el - o_vtab), el.data(), el.size() * sizeof(HopElement));
+  if (!h.empty()) QCMG_CUDA(cudaMemcpyAsync(m + o_vtab, h.data(), h.size() * 8, cudaMemcpyHostToDevice, s));
+  const HopElement* d_el = reinterpret_cast<const HopElement*>(m + o_el);
+  launch_halfbasis(L, N, op.dim, op.bin.p, s);
   if (op.dim) {
-    k_halfop_fill<<<grid_for(op.dim, 256), 256, 0, s>>>(op.dim, op.bin.p, d_el.p, (int)el.size(),
-                                                         op.rowptr.p, op.col.p, op.val.p,
-                                                         op.diag.p, op.nval ? op.ell : nullptr,
-                                                         op.nval ? op.len : nullptr);
+    const unsigned g = grid_for(op.dim, 256);
+    k_halfop_count<<<g, 256, 0, s>>>(op.dim, op.bin.p, d_el, (int)el.size(), op.rowptr.p + 1);
+    k_rowptr<<<1, 1024, 0, s>>>(op.dim, op.rowptr.p);
+    k_halfop_fill<<<g, 256, 0, s>>>(op.dim, op.bin.p, d_el, (int)el.size(), op.rowptr.p, op.col.p,
+                                    op.val.p, op.diag.p, op.ell, op.len);
     QCMG_CUDA(cudaGetLastError());
-  }
-  // Row bounds for the fixed-point headroom: |T|_inf and |diag|_max.
-  std::vector<double> h_val(nnz), h_diag(op.dim);
-  if (nnz) QCMG_CUDA(cudaMemcpyAsync(h_val.data(), op.val.p, nnz * 8, cudaMemcpyDeviceToHost, s));
-  if (op.dim)
-    QCMG_CUDA(cudaMemcpyAsync(h_diag.data(), op.diag.p, op.dim * 8, cudaMemcpyDeviceToHost, s));
-  QCMG_CUDA(cudaStreamSynchronize(s));
-  op.max_row_abs = 0.0;
-  op.max_diag_abs = 0.0;
-  for (uint32_t i = 0; i < op.dim; ++i) {
-    double a = 0.0;
-    for (uint32_t k = h_rp[i]; k < h_rp[i + 1]; ++k) a += std::fabs(h_val[k]);
-    op.max_row_abs = std::max(op.max_row_abs, a);
-    op.max_diag_abs = std::max(op.max_diag_abs, std::fabs(h_diag[i]));
+  } else {
+    QCMG_CUDA(cudaMemsetAsync(op.rowptr.p, 0, 4, s));
   }
 }
 

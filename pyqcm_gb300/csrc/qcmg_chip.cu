@@ -32,6 +32,7 @@
 #include <thread>
 
 #include "qcmg_chip.cuh"
+#include "qcmg_pool.h"
 #include "qcmg_tridiag.h"
 
 namespace qcmg {
@@ -177,16 +178,6 @@ struct ChipGroup {
   std::vector<int> ids;  // into the caller's arrays
   int C = 1;
   size_t smem = 0;
-  cudaStream_t stream = nullptr;
-  cudaEvent_t done[2] = {nullptr, nullptr};
-  double* coef = nullptr;  // page-locked: [parity][sector][2 kChunk]
-  ~ChipGroup() {
-    if (stream) cudaStreamSynchronize(stream);  // nothing uses the buffers any more
-    for (auto e : done)
-      if (e) cudaEventDestroy(e);
-    if (stream) cudaStreamDestroy(stream);
-    if (coef) cudaFreeHost(coef);
-  }
 };
 
 }  // namespace
@@ -194,19 +185,24 @@ struct ChipGroup {
 static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* const* x0, double tol,
                        int max_iter, bool keep, double* const* psi, ChipResult* res) {
   const int n = (int)g.ids.size();
-  cudaStream_t s = g.stream;
   std::vector<size_t> at(n + 1, 0);  // offsets of the sectors' vectors
   for (int k = 0; k < n; ++k) at[k + 1] = at[k] + Hs[g.ids[k]]->dim;
   const size_t total = at[n];
-  DevBuf<double> xq, zbuf, gsbuf;
-  std::vector<std::unique_ptr<DevBuf<double>>> V;  // kSpan chunks of every sector each
+  PoolBuf<double> xq, zbuf, gsbuf;
+  std::vector<std::unique_ptr<PoolBuf<double>>> V;  // kSpan chunks of every sector each
   constexpr int kSpan = 8;
   xq.alloc(2 * total);
-  DevBuf<ChipSector> secs;
+  PoolBuf<ChipSector> secs;
   secs.alloc((size_t)2 * n);
+  PoolBuf<ChipSum> sums;
+  PinnedBuf<double> coef;  // [parity][sector][2 kChunk]
+  coef.alloc((size_t)n * 4 * kChunk);
+  std::vector<ChipSector> hs[2];  // by chunk parity: a launch still reads the other one
+  PoolStream lane;  // closed (waited for) before the buffers above go
+  lane.open();
+  cudaStream_t s = lane.s;
   std::vector<TridiagLowest> lowest(n);
   std::vector<char> running(n, 1);
-  std::vector<ChipSector> hs[2];  // by chunk parity: a launch still reads the other one
   auto chunk_vectors = [&](int c, int k) -> double* {
     if (keep && c * kChunk >= kKeepSteps) {  // a long run: it will be repeated instead
       QCMG_CUDA(cudaStreamSynchronize(s));
@@ -215,7 +211,7 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
     }
     if (!keep) return nullptr;
     while ((int)V.size() <= c / kSpan) {
-      V.emplace_back(new DevBuf<double>);
+      V.emplace_back(new PoolBuf<double>);
       V.back()->alloc(total * kChunk * kSpan);
     }
     // sector k's vectors of the span are contiguous: (step in span) x D
@@ -237,7 +233,7 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
       S.x = xq.p + at[k];
       S.q = xq.p + total + at[k];
       S.V = replay ? nullptr : chunk_vectors(c, k);
-      S.coef = replay ? nullptr : g.coef + ((size_t)(c & 1) * n + k) * 2 * kChunk;
+      S.coef = replay ? nullptr : coef.p + ((size_t)(c & 1) * n + k) * 2 * kChunk;
       S.z = nullptr;
       S.gs = nullptr;
       S.steps = kChunk;
@@ -256,16 +252,16 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
   std::vector<int> now, next;
   for (int k = 0; k < n; ++k) now.push_back(k);
   launch(0, now, false);
-  QCMG_CUDA(cudaEventRecord(g.done[0], s));
+  QCMG_CUDA(cudaEventRecord(lane.e[0], s));
   for (int c = 0; !now.empty(); ++c) {
     // the next chunk of every sector that may need one, before the test
     launch(c + 1, now, false);
-    QCMG_CUDA(cudaEventRecord(g.done[(c + 1) & 1], s));
-    QCMG_CUDA(cudaEventSynchronize(g.done[c & 1]));
+    QCMG_CUDA(cudaEventRecord(lane.e[(c + 1) & 1], s));
+    QCMG_CUDA(cudaEventSynchronize(lane.e[c & 1]));
     next.clear();
     for (int k : now) {
       ChipResult& r = res[g.ids[k]];
-      const double* co = g.coef + ((size_t)(c & 1) * n + k) * 2 * kChunk;
+      const double* co = coef.p + ((size_t)(c & 1) * n + k) * 2 * kChunk;
       bool stop = false;
       for (int t = 0; t < kChunk && !stop; ++t) {
         r.alpha.push_back(co[t]);
@@ -294,7 +290,6 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
   if (want.empty()) return;
   gsbuf.alloc(total);
   std::vector<double> hz;
-  DevBuf<ChipSum> sums;
   std::vector<ChipSum> hsum;
   if (!keep) {  // a second run, accumulating z_j v_j
     const int ld = max_iter + 2;
@@ -383,9 +378,6 @@ void chip_lanczos(int n, qcmg_hamiltonian* const* Hs, const double* const* x0, d
     for (int k = t; k < n; k += threads) g.ids.push_back(k);
     g.C = C;
     for (int k : g.ids) g.smem = std::max(g.smem, chip_smem((uint32_t)Hs[k]->dim, C));
-    QCMG_CUDA(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
-    for (auto& e : g.done) QCMG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    QCMG_CUDA(cudaMallocHost(&g.coef, g.ids.size() * 4 * kChunk * sizeof(double)));
   }
   if (threads == 1) {
     chip_group(*groups[0], Hs, x0, tol, max_iter, keep, psi, res);

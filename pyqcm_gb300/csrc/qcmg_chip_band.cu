@@ -21,6 +21,7 @@
 #include <cmath>
 
 #include "qcmg_chip.cuh"
+#include "qcmg_pool.h"
 #include "qcmg_tridiag.h"
 #include "qcmg_vec.cuh"
 
@@ -215,28 +216,22 @@ bool chip_band_fits(const qcmg_hamiltonian* H, int p) {
 bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc_defl,
                double acc_band, std::vector<double>& t, std::vector<double>& P, int* M) {
   const uint32_t D = (uint32_t)H->dim;
-  cudaStream_t s = H->stream;
   int optin = 0;
   QCMG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, H->device));
   const int per_step = 2 * p + 1, chunk_len = kBandChunk * per_step;
-  DevBuf<double> ring;
+  PoolBuf<double> ring;
   ring.alloc((size_t)(2 * p + 1) * D);
-  struct Pinned {
-    double* coef = nullptr;  // two chunks, then the flag
-    cudaEvent_t done[2] = {nullptr, nullptr};
-    cudaStream_t s;
-    explicit Pinned(cudaStream_t st) : s(st) {}
-    ~Pinned() {
-      cudaStreamSynchronize(s);  // nothing writes the buffer any more
-      if (coef) cudaFreeHost(coef);
-      for (auto e : done)
-        if (e) cudaEventDestroy(e);
-    }
-  } pin(s);
-  QCMG_CUDA(cudaMallocHost(&pin.coef, (2 * (size_t)chunk_len + 1) * sizeof(double)));
-  volatile int* deflated = reinterpret_cast<int*>(pin.coef + 2 * chunk_len);
+  PinnedBuf<double> coef;  // two chunks, then the flag
+  coef.alloc(2 * (size_t)chunk_len + 1);
+  volatile int* deflated = reinterpret_cast<int*>(coef.p + 2 * chunk_len);
   *deflated = -1;
-  for (auto& e : pin.done) QCMG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // a lane of its own, after what the handle's stream holds (the start
+  // vectors); closed (waited for) before the buffers above go
+  PoolStream lane;
+  lane.open();
+  QCMG_CUDA(cudaEventRecord(lane.e[0], H->stream));
+  QCMG_CUDA(cudaStreamWaitEvent(lane.s, lane.e[0], 0));
+  cudaStream_t s = lane.s;
   ChipBand S;
   S.op = chip_op(H);
   S.phi = phi;
@@ -248,7 +243,7 @@ bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc
     S.j0 = c * kBandChunk;
     S.steps = std::min(kBandChunk, M0 - S.j0);
     if (S.steps <= 0) return;
-    S.coef = pin.coef + (size_t)(c & 1) * chunk_len;
+    S.coef = coef.p + (size_t)(c & 1) * chunk_len;
     with_band_kernel<kBandMaxP>(p, [&](auto kern) {
       if (c == 0) {
         QCMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
@@ -256,7 +251,7 @@ bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc
       }
       launch_clusters(kern, 1, C, band_smem(D, p, C), s, S);
     });
-    QCMG_CUDA(cudaEventRecord(pin.done[c & 1], s));
+    QCMG_CUDA(cudaEventRecord(lane.e[c & 1], s));
   };
   t.assign((size_t)M0 * M0, 0.0);
   P.assign((size_t)p * M0, 0.0);
@@ -267,8 +262,8 @@ bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc
     launch(c + 1);  // computed in vain if this chunk converges
     const int j0 = c * kBandChunk, n = std::min(kBandChunk, M0 - j0);
     if (n <= 0) break;
-    QCMG_CUDA(cudaEventSynchronize(pin.done[c & 1]));
-    const double* co = pin.coef + (size_t)(c & 1) * chunk_len;
+    QCMG_CUDA(cudaEventSynchronize(lane.e[c & 1]));
+    const double* co = coef.p + (size_t)(c & 1) * chunk_len;
     const int stop = *deflated;
     for (int q = 0; q < n; ++q, co += per_step) {
       const int j = j0 + q;

@@ -37,20 +37,32 @@ void clear_error();
     if (!(cond)) throw ::qcmg::Error(QCMG_ERR_ARG, msg); \
   } while (0)
 
+// The memory pool (qcmg_pool.h).
+void* pool_get(size_t bytes, size_t* got);
+void pool_put(void* p, size_t got);
+
 // Owning device buffer.
 template <class T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
-  bool owned = true;  // false: p belongs to the caller and is never freed here
+  bool owned = true;   // false: p belongs to the caller and is never freed here
+  bool pooled = false;  // memory from the pool: the owner sees to it that no work is
+                        // pending on it when it is freed or grows
+  size_t got = 0;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p && owned) cudaFree(p);
+    if (p && owned) {
+      if (got)
+        pool_put(p, got);
+      else
+        cudaFree(p);
+    }
     p = nullptr;
-    n = 0;
+    n = got = 0;
     owned = true;
   }
   // Wraps caller-owned device memory.
@@ -65,7 +77,10 @@ struct DevBuf {
     QCMG_CHECK_ARG(owned, "cannot grow a borrowed buffer");
     release();
     size_t bytes = (count ? count : 1) * sizeof(T);
-    QCMG_CUDA(cudaMalloc(&p, bytes));
+    if (pooled)
+      p = static_cast<T*>(pool_get(bytes, &got));
+    else
+      QCMG_CUDA(cudaMalloc(&p, bytes));
     n = count;
   }
   void upload(const T* h, size_t count, cudaStream_t s) {
@@ -86,6 +101,7 @@ struct HalfOp {
   int L = 0, N = 0;
   uint32_t dim = 0;
   size_t nnz = 0;
+  // one allocation holds all tables
   DevBuf<uint32_t> bin;     // basis states, increasing
   DevBuf<uint32_t> rowptr;  // dim + 1
   DevBuf<uint32_t> col;     // nnz
@@ -95,14 +111,13 @@ struct HalfOp {
   // neighbouring threads read neighbouring words): column in the low half,
   // index into vtab (+-v of every element) in the high half; len[I] hops.
   // Built on request for half bases of at most 65,536 states; the order
-  // within a row is the CSR's.  One allocation holds the three tables.
-  DevBuf<double> slots;
+  // within a row is the CSR's.
   double* vtab = nullptr;
   uint32_t* ell = nullptr;
   uint16_t* len = nullptr;
   int nval = 0;  // entries of vtab; 0: no slot form
-  double max_row_abs = 0.0; // max_I sum_J |val| (for fixed-point headroom)
-  double max_diag_abs = 0.0;
+  void* mem = nullptr;  // from the pool; given back by the handle once idle
+  size_t mem_got = 0;
 };
 
 struct HopElement {
@@ -116,7 +131,7 @@ void launch_rank(int L, const uint32_t* states, size_t n, uint32_t dim, uint32_t
                  cudaStream_t s);
 // slots: also the slot form, where the half basis allows it.
 void build_halfop(HalfOp& op, int L, int N, const std::vector<HopElement>& el, bool slots,
-                  cudaStream_t s);
+                  std::vector<std::vector<double>>& staging, cudaStream_t s);
 
 uint64_t binomial(int n, int k);
 
@@ -174,9 +189,11 @@ struct qcmg_hamiltonian {
   int inter_kind = QCMG_INTER_NONE;
   double U = 0.0;                 // uniform on-site value (QCMG_INTER_ONSITE)
   qcmg::DevBuf<double> wdn;       // dd x L cross terms (QCMG_INTER_GENERAL)
-  double max_inter_abs = 0.0;
+  void* cross_mem = nullptr;      // their memory, from the pool
+  size_t cross_got = 0;
   cudaStream_t stream = nullptr;      // stream the handle launches on
   cudaStream_t own_stream = nullptr;  // created with the handle
+  bool foreign = false;               // a caller's stream has been used
   // staging for host-pointer calls; the copy stream and its events prefetch
   // the old y while the product runs (created on first use)
   qcmg::DevBuf<double> xbuf, ybuf;

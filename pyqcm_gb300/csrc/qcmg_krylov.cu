@@ -15,6 +15,7 @@
 #include "qcmg_fxpath.h"
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
+#include "qcmg_pool.h"
 #include "qcmg_tridiag.h"
 #include "qcmg_vec.cuh"
 
@@ -433,17 +434,22 @@ void seeded_vector(size_t dim, unsigned seed, double* out) {
   for (size_t i = 0; i < dim; ++i) out[i] *= s;
 }
 
-static void dalloc(double** p, size_t n) { QCMG_CUDA(cudaMalloc(p, std::max<size_t>(n, 1) * 8)); }
-
+// A vector from the pool. A function that owns some declares a Drain after
+// them, so that the stream is idle when they go back.
 struct DevVec {
   double* p = nullptr;
+  size_t got = 0;
   DevVec() = default;
-  explicit DevVec(size_t n) { dalloc(&p, n); }
+  explicit DevVec(size_t n) { p = static_cast<double*>(pool_get(std::max<size_t>(n, 1) * 8, &got)); }
   DevVec(const DevVec&) = delete;
-  DevVec(DevVec&& o) noexcept : p(o.p) { o.p = nullptr; }
+  DevVec(DevVec&& o) noexcept : p(o.p), got(o.got) { o.p = nullptr; }
   ~DevVec() {
-    if (p) cudaFree(p);
+    if (p) pool_put(p, got);
   }
+};
+struct Drain {
+  cudaStream_t s;
+  ~Drain() { cudaStreamSynchronize(s); }
 };
 
 // CUDA events for the per-solve device-time breakdown.
@@ -475,6 +481,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   // stream, bit for bit) and kept on the device per handle, so repeated solves
   // of a sector (VCA / CDMFT loops) generate it once.
   DevVec x0_own(x0_host ? n : 1);
+  Drain drain0{s};
   const double* x0_dev = nullptr;
   if (!x0_host) {
     if (!(H->seed_ok && H->seed_key == seed && H->seed_vec.n == n)) {
@@ -512,6 +519,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   if (reorth <= 0 && H->use_fx && fx_prepare(H)) {
     // fixed-point fast path (one hop magnitude per spin)
     DevVec psi_dev(psi_host ? n : 1);
+    Drain drain{s};
     LanczosResult fr = fx_lanczos(H, x0_dev, tol, max_iter, psi_host ? psi_dev.p : nullptr);
     if (psi_host) {
       QCMG_CUDA(cudaMemcpyAsync(psi_host, psi_dev.p, n * 8, cudaMemcpyDeviceToHost, s));
@@ -520,6 +528,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
     return fr;
   }
   DevVec r(n), q(n);
+  Drain drain1{s};
   QCMG_CUDA(cudaMemcpyAsync(r.p, x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
   QCMG_CUDA(cudaMemsetAsync(q.p, 0, n * 8, s));
   Reducer red;
@@ -551,6 +560,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
     if (psi_host) {
       // Eigenvector replay of LanczosEigenvector (Lanczos.hpp:109-131).
       DevVec gs(n);
+      Drain drain2{s};
       QCMG_CUDA(cudaMemcpyAsync(gs.p, x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
       scale(gs.p, z[0], n, s);
       QCMG_CUDA(cudaMemcpyAsync(r.p, x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
@@ -585,6 +595,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   const size_t stride = (n + 1) & ~(size_t)1;
   const size_t block = std::max<size_t>(1, std::min<size_t>(keep, ((size_t)512 << 20) / (stride * 8)));
   std::vector<DevVec> blocks;
+  Drain drain2{s};
   std::vector<double*> V;
   auto add_vector = [&] {
     if (V.size() == blocks.size() * block) blocks.emplace_back(std::min(block, (size_t)keep - V.size()) * stride);
@@ -652,6 +663,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   res.vectors = (int)V.size();
   if (psi_host) {
     DevVec gs(n);
+    Drain drain3{s};
     QCMG_CUDA(cudaMemsetAsync(gs.p, 0, n * 8, s));
     std::vector<const double*> Vz(Vp.begin(), Vp.begin() + z.size());
     std::vector<double> mz(z.size());
@@ -721,6 +733,7 @@ GreenResult lanczos_green(qcmg_hamiltonian* H, const double* psi0, bool on_devic
   out.b.push_back(1.0);
   if (n == 0) return out;
   DevVec P(n), Q(n);
+  Drain drain{s};
   QCMG_CUDA(cudaMemcpyAsync(P.p, psi0, n * 8,
                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   QCMG_CUDA(cudaMemsetAsync(Q.p, 0, n * 8, s));
@@ -761,6 +774,7 @@ BlockResult block_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool
   Reducer red;
   MultiOps mops;
   std::vector<DevVec> store;
+  Drain drain{s};
   std::vector<double*> q(p);
   for (int k = 0; k < p; ++k) {
     store.emplace_back(n);
@@ -949,7 +963,8 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
   QCMG_CHECK_ARG(M0 > 0, "band Lanczos needs M > 0");
   // The p start vectors on the device (the caller's own when they are there:
   // they are only read).
-  std::vector<DevVec> phi;
+  std::vector<DevVec> phi, owned;
+  Drain drain{s};
   if (!phi_on_device) {
     phi.emplace_back((size_t)p * n);
     QCMG_CUDA(cudaMemcpyAsync(phi[0].p, phi_in, (size_t)p * n * 8, cudaMemcpyHostToDevice, s));
@@ -966,7 +981,6 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
   }
   std::vector<double*> v(M0p, nullptr);
   std::vector<double*> pool;
-  std::vector<DevVec> owned;
   auto get = [&]() -> double* {
     if (!pool.empty()) {
       double* r = pool.back();

@@ -27,6 +27,7 @@
 #include "qcmg_krylov.h"
 #include "qcmg_lattice.h"
 #include "qcmg_points.h"
+#include "qcmg_pool.h"
 
 namespace qcmg {
 
@@ -167,12 +168,12 @@ void self_energy_batch(int L, int M, const double* e, const double* v, bool v_re
                        const double* eb, const double* tc, int nz, const double* z, double* sigma,
                        double* gamma, cudaStream_t s) {
   QCMG_CHECK_ARG(L > 0 && L <= 32, "Green function dimension must be 1..32");
-  DevBuf<double> G, ldg, mtc;
+  PoolBuf<double> G, ldg, mtc;
   G.alloc((size_t)2 * L * L * nz);
   if (M > 0)
     green_function_batch(L, M, e, v, v_real, nz, z, G.p, s);
   else
-    QCMG_CUDA(cudaMemsetAsync(G.p, 0, G.n * 8, s));
+    QCMG_CUDA(cudaMemsetAsync(G.p, 0, (size_t)2 * L * L * nz * 8, s));
   // constant block -t_c
   std::vector<double> h((size_t)2 * L * L);
   QCMG_CUDA(cudaMemcpyAsync(h.data(), tc, h.size() * 8, cudaMemcpyDeviceToHost, s));
@@ -845,8 +846,8 @@ void Lattice::inverse_means(int nz, const double* z, int gx, int gy, int gz, dou
       }
   }
   const int nrow = (int)rows.size() - 1, nf = 1 + 2 * (int)ax.size();
-  DevBuf<int> d_rows, d_fx;
-  DevBuf<double> d_yz, d_wx;
+  PoolBuf<int> d_rows, d_fx;  // idle again after the last wait below
+  PoolBuf<double> d_yz, d_wx;
   d_rows.upload(rows.data(), rows.size(), s);
   if (!which.empty()) {
     d_fx.upload(fx.data(), fx.size(), s);
