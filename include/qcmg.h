@@ -180,7 +180,8 @@ int qcmg_seeded_vector(size_t dim, unsigned seed, double* out);
  * (no reorthogonalization when reorth == 0); iteration stops when the Ritz
  * residual |s_last * beta| < tol or after max_iter steps.  With reorth > 0 the
  * Lanczos basis is kept on the device and every new vector is
- * reorthogonalized (classical Gram-Schmidt, twice) against all previous ones;
+ * reorthogonalized (classical Gram-Schmidt, a second time when the first pass
+ * took away half of its squared norm or more) against all previous ones;
  * at most `reorth` vectors are kept: when that many are held and the residual
  * has not converged, the iteration restarts from the current Ritz vector.
  * Outputs: *E0; psi (length dim, may be NULL: then no second pass);

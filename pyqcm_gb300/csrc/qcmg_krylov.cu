@@ -59,7 +59,9 @@ __global__ void __launch_bounds__(256) k_multidot(VL V, int m, const double* __r
 // load's latency per element.
 template <int MAXM, int VEC, class VL>
 __global__ void __launch_bounds__(kDotThreads, 2) k_dots(VL V, int m, const double* __restrict__ w,
-                                                        size_t nv, double* __restrict__ part) {
+                                                        size_t nv, double* __restrict__ part,
+                                                        const int* __restrict__ need) {
+  if (need && !*need) return;
   const int k0 = blockIdx.y * MAXM, mm = min(MAXM, m - k0);
   double acc[MAXM];
 #pragma unroll
@@ -80,9 +82,11 @@ __global__ void __launch_bounds__(kDotThreads, 2) k_dots(VL V, int m, const doub
   block_sums<MAXM>(acc, mm, part + (size_t)blockIdx.x * m + k0);
 }
 
-// out[k] = sum_b part[b m + k] in a fixed order, one warp per value.
+// out[k] = sum_b part[b m + k] in a fixed order, one warp per value.  With
+// need: the last value is |w|^2, the others its projections c_k, and need
+// says whether a second pass is called for.
 __global__ void __launch_bounds__(1024) k_dots_final(const double* __restrict__ part, int nb, int m,
-                                                     double* __restrict__ out) {
+                                                     double* __restrict__ out, int* need) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int k = wp; k < m; k += nw) {
     double s = 0.0;
@@ -91,13 +95,25 @@ __global__ void __launch_bounds__(1024) k_dots_final(const double* __restrict__ 
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) out[k] = s;
   }
+  if (!need) return;
+  __syncthreads();
+  if (wp == 0) {
+    double c2 = 0.0;
+    for (int k = lane; k < m - 1; k += 32) c2 = fma(out[k], out[k], c2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+    // |w - V c|^2 = |w|^2 - |c|^2 < |w|^2 / 2, or anything not finite
+    if (lane == 0) *need = !(c2 <= 0.5 * out[m - 1]);
+  }
 }
 
 // w -= sum_k c_k V_k, c in device memory: eight vectors' loads in flight
 // together per element.
 template <int VEC, class VL>
 __global__ void __launch_bounds__(256) k_axpys(VL V, int m, const double* __restrict__ c,
-                                               double* __restrict__ w, size_t nv) {
+                                               double* __restrict__ w, size_t nv,
+                                               const int* __restrict__ need) {
+  if (need && !*need) return;
   extern __shared__ double cs[];
   for (int k = threadIdx.x; k < m; k += blockDim.x) cs[k] = c[k];
   __syncthreads();
@@ -270,7 +286,7 @@ struct MultiOps {
       for (int k = 0; k < m; ++k) L.v[k] = V[k];
       f(L);
     } else {
-      if (listed != V) {
+      if (listed.size() < V.size() || !std::equal(V.begin(), V.end(), listed.begin())) {
         listed = V;
         grow(ptrs, m);
         QCMG_CUDA(cudaMemcpyAsync(ptrs.p, listed.data(), m * sizeof(double*), cudaMemcpyHostToDevice, s));
@@ -279,7 +295,9 @@ struct MultiOps {
     }
   }
   // V_k . w for every k, left in device memory (m doubles)
-  const double* dots_dev(const std::vector<const double*>& V, const double* w, size_t n, cudaStream_t s) {
+  // (only: when set, nothing is done unless *only; need: see k_dots_final)
+  const double* dots_dev(const std::vector<const double*>& V, const double* w, size_t n, cudaStream_t s,
+                         const int* only = nullptr, int* need = nullptr) {
     const int m = (int)V.size();
     const bool two = pairs(V, w, n);
     const size_t nv = two ? n / 2 : n;
@@ -292,9 +310,9 @@ struct MultiOps {
         constexpr int MX = decltype(maxm)::value;
         const dim3 grid((unsigned)nb, (unsigned)((m + MX - 1) / MX));
         if (two)
-          k_dots<MX, 2, VL><<<grid, kDotThreads, 0, s>>>(L, m, w, nv, part.p);
+          k_dots<MX, 2, VL><<<grid, kDotThreads, 0, s>>>(L, m, w, nv, part.p, only);
         else
-          k_dots<MX, 1, VL><<<grid, kDotThreads, 0, s>>>(L, m, w, nv, part.p);
+          k_dots<MX, 1, VL><<<grid, kDotThreads, 0, s>>>(L, m, w, nv, part.p, only);
       };
       // one group when it fits; eights for long lists (96 vectors of 3.3M
       // elements: 581 us in eights, 611 in sixteens, floor 506)
@@ -308,7 +326,7 @@ struct MultiOps {
         go(std::integral_constant<int, 16>{});
     });
     QCMG_CUDA(cudaGetLastError());
-    k_dots_final<<<1, std::min(1024, 32 * m), 0, s>>>(part.p, nb, m, sums.p);
+    k_dots_final<<<1, std::min(1024, 32 * m), 0, s>>>(part.p, nb, m, sums.p, need);
     QCMG_CUDA(cudaGetLastError());
     return sums.p;
   }
@@ -330,7 +348,7 @@ struct MultiOps {
   }
   // w -= sum_k c_k V_k with c in device memory
   void axpys_dev(const std::vector<const double*>& V, const double* c, double* w, size_t n,
-                 cudaStream_t s) {
+                 cudaStream_t s, const int* only = nullptr) {
     const int m = (int)V.size();
     if (m == 0 || n == 0) return;
     const bool two = pairs(V, w, n);
@@ -338,16 +356,28 @@ struct MultiOps {
     with_list(V, s, [&](auto L) {
       using VL = decltype(L);
       if (two)
-        k_axpys<2, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv);
+        k_axpys<2, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv, only);
       else
-        k_axpys<1, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv);
+        k_axpys<1, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv, only);
     });
     QCMG_CUDA(cudaGetLastError());
   }
-  // one Gram-Schmidt pass: w -= sum_k (V_k . w) V_k, no host round trip
-  void project_out(const std::vector<const double*>& V, double* w, size_t n, cudaStream_t s) {
+  // w orthogonal to V: a classical Gram-Schmidt pass and, when it took away
+  // half of |w|^2 or more, a second one (the criterion of Daniel, Gragg,
+  // Kaufman and Stewart, 1976: otherwise one pass leaves w orthogonal to
+  // rounding).  The device decides; *again (page-locked) tells the host at
+  // its next wait.
+  DevBuf<int> need;
+  std::vector<const double*> with_w;
+  void orthogonalize(const std::vector<const double*>& V, double* w, size_t n, int* again,
+                     cudaStream_t s) {
     if (V.empty()) return;
-    axpys_dev(V, dots_dev(V, w, n, s), w, n, s);
+    need.alloc(1);
+    with_w = V;
+    with_w.push_back(w);
+    axpys_dev(V, dots_dev(with_w, w, n, s, nullptr, need.p), w, n, s);
+    QCMG_CUDA(cudaMemcpyAsync(again, need.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    axpys_dev(V, dots_dev(V, w, n, s, need.p), w, n, s, need.p);
   }
   // w -= sum_k c_k V_k, then d = w . u and w -= d u with d left at d_dev:
   // two launches.  False (nothing done) for lists longer than kByValue.
@@ -576,7 +606,8 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   }
 
   // Fully reorthogonalized Lanczos: the basis is kept in HBM and every new
-  // residual is projected out of it twice (classical Gram-Schmidt x2).  At
+  // residual is made orthogonal to it (classical Gram-Schmidt, repeated when
+  // one pass is not enough: MultiOps::orthogonalize).  At
   // most `reorth` vectors are kept: when the cap is reached before the Ritz
   // residual converges, the iteration restarts from the current Ritz vector
   // (explicit restart).  The product is the fixed-point one where it applies
@@ -595,6 +626,8 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   const size_t stride = (n + 1) & ~(size_t)1;
   const size_t block = std::max<size_t>(1, std::min<size_t>(keep, ((size_t)512 << 20) / (stride * 8)));
   std::vector<DevVec> blocks;
+  PinnedBuf<int> again;
+  again.alloc(1);
   Drain drain2{s};
   std::vector<double*> V;
   auto add_vector = [&] {
@@ -622,12 +655,12 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
       res.alpha.push_back(a);
       axpy(w, V[j], -a, n, s);
       ev.record(2, s);
-      for (int pass = 0; pass < 2; ++pass) mops.project_out(Vp, w, n, s);
+      mops.orthogonalize(Vp, w, n, again.p, s);
       ev.record(3, s);
       double b = std::sqrt(red.dot(w, w, n, s));  // synchronizes the stream
       res.product_ms += ev.elapsed(0, 1);
       res.reorth_ms += ev.elapsed(2, 3);
-      res.reorth_bytes += 2.0 * 16.0 * (double)Vp.size() * (double)n;  // 16 B per stored element per pass
+      res.reorth_bytes += (*again.p ? 2.0 : 1.0) * 16.0 * (double)Vp.size() * (double)n;  // 16 B per stored element per pass
       res.beta.push_back(b);
       ++total;
       res.energy = lowest(res.alpha, res.beta, z);
