@@ -120,7 +120,9 @@ int qcmg_matvec(qcmg_hamiltonian* H, const double* x, double* y, unsigned flags)
 /* Chooses the arithmetic of the handle's products and Lanczos runs:
  * path 1 (default) uses the fixed-point fast path whenever the sector's hops
  * have one magnitude per spin (the Hubbard form), path 0 always uses the
- * FP64 kernels.  Lanczos runs without reorthogonalization on sectors of at
+ * FP64 kernels.  Products of FP64 vectors (qcmg_matvec) of less than 2^21
+ * states take the FP64 kernel on either path (the conversions cost more than
+ * they save; qcmg_matvec_fx has none).  Lanczos runs without reorthogonalization on sectors of at
  * most 16,384 states are FP64 on either path (they run on chip).  No
  * counterpart in the reference (FP64 throughout). */
 int qcmg_hamiltonian_set_path(qcmg_hamiltonian* H, int path);

@@ -179,6 +179,7 @@ static void release_handle(qcmg_hamiltonian* H) {
   if (H->own_stream) cudaStreamDestroy(H->own_stream);
   if (H->up.mem) pool_put(H->up.mem, H->up.mem_got);
   if (H->dn.mem) pool_put(H->dn.mem, H->dn.mem_got);
+  if (H->stage) pinned_put(H->stage, H->stage_got);
   if (H->cross_mem) pool_put(H->cross_mem, H->cross_got);
   delete H;
 }
@@ -321,6 +322,9 @@ __global__ void k_add_to_host(const double* __restrict__ d, double* __restrict__
     yh[i] = acc ? yh[i] + d[i] : d[i];
 }
 
+// Largest sector whose host vectors are staged (memcpy of 128 KB takes ~6 us).
+constexpr size_t kStagedStates = 16384;
+
 // cuPointerGetAttribute through the runtime's driver entry point (no link
 // against the driver library); null when the driver does not provide it.
 typedef CUresult (*PointerGetAttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
@@ -368,7 +372,7 @@ int qcmg_matvec(qcmg_hamiltonian* H, const double* x, double* y, unsigned flags)
     QCMG_CUDA(cudaSetDevice(H->device));
     const bool acc = (flags & QCMG_ACCUMULATE) != 0;
     const size_t n = H->dim;
-    const bool fx = H->use_fx && fx_prepare(H);
+    const bool fx = fx_for_f64(H);
     if (flags & QCMG_DEVICE_PTRS) {
       if (fx)
         fx_matvec_f64(H, x, y, acc);
@@ -381,6 +385,21 @@ int qcmg_matvec(qcmg_hamiltonian* H, const double* x, double* y, unsigned flags)
       return;
     }
     H->xbuf.alloc(n);
+    if (!fx && n <= kStagedStates) {
+      // Small host vectors go through page-locked staging of the handle's:
+      // one copy in, one launch that reads and writes y in host memory, one
+      // wait (pageable copies of x and y each way took three driver calls
+      // with a wait each; 4,900 states: 35.7 us -> 23.8 us).
+      if (!H->stage) H->stage = static_cast<double*>(pinned_get(2 * n * 8, &H->stage_got));
+      double *px = H->stage, *py = H->stage + n;
+      std::memcpy(px, x, n * 8);
+      if (acc) std::memcpy(py, y, n * 8);
+      QCMG_CUDA(cudaMemcpyAsync(H->xbuf.p, px, n * 8, cudaMemcpyHostToDevice, H->stream));
+      matvec(H, H->xbuf.p, py, acc);
+      QCMG_CUDA(cudaStreamSynchronize(H->stream));
+      std::memcpy(y, py, n * 8);
+      return;
+    }
     // QCMG_VERBOSE: which form ran, and its phases timed with events
     static const bool verbose = std::getenv("QCMG_VERBOSE") != nullptr;
     cudaEvent_t ev[4] = {};

@@ -45,6 +45,15 @@ unsigned fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* y
                    FxReducer* dot = nullptr);
 // Throws if a kernel of the fast path reported a bounded-wait failure.
 void fx_check_error(qcmg_hamiltonian* H);
+// Whether a product of FP64 vectors takes the fixed-point passes: where they
+// apply, from 2^21 states on.  Below, converting x and y there and back (five
+// launches and two host waits) costs more than the FP64 product: 4,900
+// states 61 us against 6 us, 853,776 states 88 against 52 us, 2,944,656
+// states (13-site chain) 149 against 119 us; the 4x4 sector of 165,636,900
+// states ~4.5 ms against 9.95 ms.
+inline bool fx_for_f64(qcmg_hamiltonian* H) {
+  return H->use_fx && H->dim >= ((size_t)1 << 21) && fx_prepare(H);
+}
 // y (+)= H x on FP64 device vectors through the fixed-point product.
 void fx_matvec_f64(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate);
 // y (+)= H x with x on the device and y in page-locked host memory, written

@@ -199,6 +199,9 @@ struct qcmg_hamiltonian {
   qcmg::DevBuf<double> xbuf, ybuf;
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t ev_x = nullptr, ev_y = nullptr;
+  // page-locked staging of small host products (x, then y), from the pool
+  double* stage = nullptr;
+  size_t stage_got = 0;
   // the seeded Lanczos start vector of the last seed used (generated once)
   qcmg::DevBuf<double> seed_vec;
   unsigned seed_key = 0;

@@ -613,7 +613,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   // (explicit restart).  The product is the fixed-point one where it applies
   // (the vectors stay FP64).  Device time of the products and of the
   // reorthogonalization is recorded with events (qcmg_lanczos_last_stats).
-  const bool fx = H->use_fx && fx_prepare(H);
+  const bool fx = fx_for_f64(H);
   auto product = [&](const double* x, double* y) {
     if (fx)
       fx_matvec_f64(H, x, y, false);
