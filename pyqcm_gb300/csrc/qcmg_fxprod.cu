@@ -89,6 +89,30 @@ __device__ __forceinline__ void slab_range(uint32_t a, uint32_t du, uint32_t* e0
   *e1 = (du & 1u) ? (odd_start ? du : du - 1u) : du;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// Asks L2 for the whole 16-byte units inside n elements at v.
+__device__ __forceinline__ void prefetch_slab(const int64_t* v, uint32_t n) {
+  const uintptr_t p = (uintptr_t)v, q = (p + 15) & ~(uintptr_t)15;
+  const unsigned bytes = (unsigned)((p + (size_t)n * 8 - q) & ~(size_t)15);
+  if (bytes) prefetch_l2((const void*)q, bytes);
+}
+
+// round(v / 2^t) with 1 <= t <= 31 (NARROW: two funnel shifts instead of the
+// general 64-bit shift and its test), else as rshift_fixed.
+template <bool NARROW>
+__device__ __forceinline__ int64_t rshift_term(int64_t v, int t, int64_t r) {
+  if (NARROW) {
+    v += r;
+    const unsigned lo = (unsigned)(uint64_t)v;
+    const int hi = (int)(v >> 32);
+    return ((int64_t)(hi >> t) << 32) | __funnelshift_r(lo, (unsigned)hi, t);
+  }
+  return rshift_fixed(v, t, r);
+}
+
 // Offset (elements) of the second slab buffer: a compile-time constant, so
 // one address serves the gathers from both slabs.  Two slabs per round need
 // slab_stride(du) <= kSlab1Off (du <= 14190).  Slabs of du <= 1006 take the
@@ -132,7 +156,7 @@ __device__ __forceinline__ void gather_group(uint32_t vbase, uint2 w, int64_t (&
 // columns point at zero slots du..du+15.  With NS = 2 the grid is even, so the
 // two slabs of a round have the same alignment (view offset).  With NS = 1
 // a second CTA on the SM computes while this one's copy is in flight.
-template <int INTER, int NS, bool FAST, bool SMALL>
+template <int INTER, int NS, bool FAST, bool NARROW, bool SMALL>
 __global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 : NS == 1 ? 2 : 1)
     k_fx_passU4(FxProdArgs A) {
   constexpr uint32_t kOff = SMALL ? kSlab1OffSmall : kSlab1Off;
@@ -206,6 +230,14 @@ __global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 
       if (tid < (int)kZeroSlots && a0 + s * G < dd)
         smem_slab[s * kOff + e0 + du + tid] = 0;  // zero slots for padding columns
     }
+    // the next round's slabs into L2 meanwhile: its copies then wait for L2
+    // only (with the narrow shifts: 2,556 -> 2,526 us for the 4x4 sector,
+    // 1,043 -> 982 us for its 12-electron one; asking for y too fills L2 and
+    // costs 140 us)
+    if (tid < NS) {
+      const uint32_t a = a0 + (uint32_t)NS * G + tid * G;
+      if (a < dd) prefetch_slab(A.x + (size_t)a * du, du);
+    }
     __syncthreads();
     const uint32_t vbase = smem_u32(view);
     const uint32_t bd = blockDim.x;
@@ -271,7 +303,7 @@ __global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 
         int64_t out;
         if (FAST) {
           // small-integer diagonal D >> tz in 32 bits, shifts fixed per launch
-          out = rshift_fixed(sp[s] - sn[s], A.t_up, A.r_up);
+          out = rshift_term<NARROW>(sp[s] - sn[s], A.t_up, A.r_up);
           int32_t Dn = dui32 + dda32[s];
           if (INTER == QCMG_INTER_ONSITE) {
             Dn += A.U32 * __popc(ubits & dbits[s]);
@@ -283,8 +315,8 @@ __global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 
               u &= u - 1;
             }
           }
-          out += rshift_fixed(view[s * kOff + i] * (int64_t)Dn, A.t_d, A.r_d);
-          if (A.yin) out += rshift_fixed(A.neg_in ? -yv[s] : yv[s], A.t_in, A.r_in);
+          out += rshift_term<NARROW>(view[s * kOff + i] * (int64_t)Dn, A.t_d, A.r_d);
+          if (A.yin) out += rshift_term<NARROW>(A.neg_in ? -yv[s] : yv[s], A.t_in, A.r_in);
         } else {
           out = mul_fix(sp[s] - sn[s], A.mt_up, A.sh_up);
           int64_t D = dui + dda[s];
@@ -336,7 +368,7 @@ __device__ __forceinline__ void passD5_accum(const int64_t* __restrict__ x, uint
 // Items (band, down state) are numbered in 32 bits (launch contract:
 // nbands * dd < 2^32).  A row's hops are summed with their signs into one
 // accumulator per element (exact: |sum| < 2^61).
-template <int VEC, bool FAST, bool DOT, int MINB>
+template <int VEC, bool FAST, bool NARROW, bool DOT, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_fx_passD5(FxProdArgs A) {
   const uint32_t du = A.du, dd = A.dd;
   const uint32_t lane = threadIdx.x & 31u;
@@ -366,7 +398,7 @@ __global__ void __launch_bounds__(256, MINB) k_fx_passD5(FxProdArgs A) {
       if (ia >= r1) continue;
       const size_t at = (size_t)a * du + ia;
       auto term = [&](int64_t v) {
-        return FAST ? rshift_fixed(v, A.t_dn, A.r_dn) : mul_fix(v, A.mt_dn, A.sh_dn);
+        return FAST ? rshift_term<NARROW>(v, A.t_dn, A.r_dn) : mul_fix(v, A.mt_dn, A.sh_dn);
       };
       if constexpr (VEC == 2) {
         longlong2* yp = reinterpret_cast<longlong2*>(A.y + at);
@@ -578,27 +610,31 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   // and the diagonal is narrow (the Hubbard form with t = 1 and small-integer
   // energies); everything else uses the 128-bit products
   const bool fast = A.d_tz >= 0 && A.p2_up >= 0 && A.p2_dn >= 0 && (!A.yin || A.p2_in >= 0);
-  auto passU4 = [&](auto ns_tag, auto small_tag, auto fast_tag) {
+  auto passU4 = [&](auto ns_tag, auto small_tag, auto fast_tag, auto narrow_tag) {
     constexpr int NS = decltype(ns_tag)::value;
-    constexpr bool S = decltype(small_tag)::value, F = decltype(fast_tag)::value;
-    if (ik == QCMG_INTER_NONE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_NONE, NS, F, S>, H, A, sms, T.per_sm_u[F], s);
-    else if (ik == QCMG_INTER_ONSITE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_ONSITE, NS, F, S>, H, A, sms, T.per_sm_u[F], s);
-    else launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_GENERAL, NS, F, S>, H, A, sms, T.per_sm_u[F], s);
+    constexpr bool S = decltype(small_tag)::value, F = decltype(fast_tag)::value, N = decltype(narrow_tag)::value;
+    if (ik == QCMG_INTER_NONE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_NONE, NS, F, N, S>, H, A, sms, T.per_sm_u[F + N], s);
+    else if (ik == QCMG_INTER_ONSITE) launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_ONSITE, NS, F, N, S>, H, A, sms, T.per_sm_u[F + N], s);
+    else launch_passU4<NS, S>(k_fx_passU4<QCMG_INTER_GENERAL, NS, F, N, S>, H, A, sms, T.per_sm_u[F + N], s);
   };
   using One = std::integral_constant<int, 1>;
   using Two = std::integral_constant<int, 2>;
   using Yes = std::true_type;
   using No = std::false_type;
   // pass U
+  auto narrow_shift = [](int t) { return t >= 1 && t <= 31; };
+  const bool nar = fast && narrow_shift(A.t_up) && narrow_shift(A.t_d) && (!A.yin || narrow_shift(A.t_in));
+  auto form = [&](auto ns_tag, auto small_tag) {
+    if (nar) passU4(ns_tag, small_tag, Yes{}, Yes{});
+    else if (fast) passU4(ns_tag, small_tag, Yes{}, No{});
+    else passU4(ns_tag, small_tag, No{}, No{});
+  };
   if (T.ns == 2 && slab_stride(H->du) <= kSlab1OffSmall) {
-    if (fast) passU4(Two{}, Yes{}, Yes{});
-    else passU4(Two{}, Yes{}, No{});
+    form(Two{}, Yes{});
   } else if (T.ns == 2) {
-    if (fast) passU4(Two{}, No{}, Yes{});
-    else passU4(Two{}, No{}, No{});
+    form(Two{}, No{});
   } else if (T.ns == 1) {
-    if (fast) passU4(One{}, No{}, Yes{});
-    else passU4(One{}, No{}, No{});
+    form(One{}, No{});
   } else {
     const size_t smem = (size_t)H->du * 8;
     const int threads = H->du >= 512 ? 512 : (H->du >= 256 ? 256 : 128);
@@ -617,7 +653,7 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   const size_t items = (size_t)A.nbands * H->dd;
   if (items >= (1ull << 32)) throw Error(QCMG_ERR_ARG, "sector too large for pass D's 32-bit item numbers");
   auto go = [&](auto kern) {
-    int& per_sm = T.per_sm_d[fast ? 1 : 0][A.dot_part ? 1 : 0];
+    int& per_sm = T.per_sm_d[fast ? (narrow_shift(A.t_dn) ? 2 : 1) : 0][A.dot_part ? 1 : 0];
     if (per_sm == 0) {
       int n = 0;
       QCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, 0));
@@ -629,15 +665,21 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   };
   // six 256-thread blocks per SM (40 registers) for the product; five for
   // the Lanczos form, whose 128-bit dot accumulator needs the registers
-  const bool even = (H->du & 1u) == 0u;
+  const bool even = (H->du & 1u) == 0u, nard = fast && narrow_shift(A.t_dn);
   unsigned gD;
-  if (A.dot_part) {
-    if (even) gD = fast ? go(k_fx_passD5<2, true, true, 5>) : go(k_fx_passD5<2, false, true, 5>);
-    else gD = fast ? go(k_fx_passD5<1, true, true, 5>) : go(k_fx_passD5<1, false, true, 5>);
-  } else {
-    if (even) gD = fast ? go(k_fx_passD5<2, true, false, 6>) : go(k_fx_passD5<2, false, false, 6>);
-    else gD = fast ? go(k_fx_passD5<1, true, false, 6>) : go(k_fx_passD5<1, false, false, 6>);
-  }
+  auto form_d = [&](auto vec_tag) {
+    constexpr int V = decltype(vec_tag)::value;
+    if (A.dot_part)
+      gD = nard ? go(k_fx_passD5<V, true, true, true, 5>)
+                : fast ? go(k_fx_passD5<V, true, false, true, 5>) : go(k_fx_passD5<V, false, false, true, 5>);
+    else
+      gD = nard ? go(k_fx_passD5<V, true, true, false, 6>)
+                : fast ? go(k_fx_passD5<V, true, false, false, 6>) : go(k_fx_passD5<V, false, false, false, 6>);
+  };
+  if (even)
+    form_d(Two{});
+  else
+    form_d(One{});
   QCMG_CUDA(cudaGetLastError());
   return gD;
 }

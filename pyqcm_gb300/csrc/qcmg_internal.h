@@ -171,8 +171,8 @@ struct FxTables {
   DevBuf<uint16_t> cnt4;  // groups per row of ell4
   int ns = 0;             // slabs per pass U round: 0 (threads stage the slab), 1 or 2
   // resident blocks per SM of the passes, asked for once per handle (0: not
-  // yet): pass U by [fast], pass D by [fast][dot]
-  mutable int per_sm_u[2] = {0, 0}, per_sm_d[2][2] = {{0, 0}, {0, 0}};
+  // yet), by [full, fast, fast with narrow shifts]; pass D also by [dot]
+  mutable int per_sm_u[3] = {0, 0, 0}, per_sm_d[3][2] = {{0, 0}, {0, 0}, {0, 0}};
   mutable int sms = 0;
   DevBuf<int> err;                  // bounded-wait failure flag of the kernels
   FxVec x, y;         // staging of the FP64-interface product

@@ -1,7 +1,7 @@
 """The fixed-point product on its own vectors (qcmg_matvec_fx) over the forms
 of its passes, on sectors whose FP64-vector products take the FP64 kernel:
-slabs staged by threads (du < 64), two small slabs per block (du <= 1006), two
-large ones, one per block; even and odd half bases, unequal spins; narrow
+slabs staged by threads (du < 64), two small slabs per block (du <= 1006), a
+slab and its negative (above), two large slabs, one per block; even and odd half bases, unequal spins; narrow
 (integer) and wide diagonals; bands of pass D down to one sweep."""
 import numpy as np
 import pytest
@@ -12,14 +12,15 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("mu", [4.0, 3.7])
-@pytest.mark.parametrize("slabs", ["1", "2"])
+@pytest.mark.parametrize("slabs", ["1", "2", ""])
 @pytest.mark.parametrize("shape,nup,ndn", [((5, 1), 2, 3), ((7, 1), 3, 4), ((8, 1), 4, 4), ((3, 3), 4, 5), ((11, 1), 2, 5),
                                            ((4, 3), 6, 6), ((13, 1), 5, 5), ((12, 1), 2, 1)])
 def test_fixed_point_product(monkeypatch, shape, nup, ndn, slabs, mu):
     import models
     import pyqcm_gb300 as pg
     import torch
-    monkeypatch.setenv("QCMG_FX_SLABS", slabs)
+    if slabs:
+        monkeypatch.setenv("QCMG_FX_SLABS", slabs)
     ns, nb, ops = models.hubbard_cluster(*shape)
     params = {"t": 1.0, "U": 8.0, "mu": mu}
     ops = {k: v for k, v in ops.items() if k in params}
