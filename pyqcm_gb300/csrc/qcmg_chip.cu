@@ -3,20 +3,22 @@
 // A sector of a few thousand states is bound by latency when every step is a
 // chain of six launches (3 to 7 us each on the device, and the host's share
 // of launching them): 48 impurity sectors of 3,920 and 4,900 states took
-// BATCH_OLD ms for their ground states, one of 4,900 states SINGLE_OLD us per step.
-// Here the whole recurrence stays inside a cluster of up to eight CTAs:
+// 146 ms for their ground states (104 ms of it not the host's convergence
+// test), here 4.6 ms.
+// The whole recurrence stays inside a cluster of up to sixteen CTAs:
 //  - every CTA holds the full basis vector x in shared memory (8 D bytes), so
 //    all hops are local gathers, and its own part of the second vector and of
 //    the diagonal;
-//  - dot products leave one partial per tile of 64 states in every CTA's
+//  - dot products leave one partial per tile of 32 states in every CTA's
 //    shared memory (distributed shared memory stores) and each CTA adds them
 //    in the same order, so the result depends on neither the cluster's size
 //    nor the tile's owner, and a batch gives the same bits as a single solve;
 //  - the new basis vector is stored to all CTAs by its owners.
-// Three cluster barriers per step and the FP64 pipe (two FMAs per SM and
-// cycle, ~23 instructions per state and step) are what a step costs: 16 us
+// Two cluster barriers per step and the FP64 pipe (two FMAs per SM and
+// cycle, ~25 instructions per state and step) are what a step costs: 10.3 us
 // for one sector of 4,900 states on sixteen CTAs with the host's test after
-// every step, 23 us for 15,876 states.
+// every step, 22 us for 15,876 states. (With three barriers and 64 states a
+// tile the batch took 4.73 ms; 33.5 us a step at 15,876 states on eight CTAs.)
 // Up to 16,384 states: x then takes 128 KB of a CTA's 227 KB. Above, the
 // grid-wide kernels have enough work per launch.
 //
@@ -42,7 +44,8 @@ constexpr int kKeepSteps = 320;  // basis vectors kept at most
 
 struct ChipSector {
   ChipOp op;
-  double *x, *q;     // state between launches
+  double *x, *q;     // raw and v_{j-1} between launches
+  double* scale;     // beta, 1/beta between launches
   double* V;         // basis vectors of this chunk (kChunk x D), or null
   double* coef;      // page-locked: alpha then beta of this chunk
   const double* z;   // replay: coefficients of the ground state, from this chunk's first step on
@@ -51,6 +54,12 @@ struct ChipSector {
   int first;         // the first launch of the run: q is zero
 };
 
+// Step j, with v_j = inv raw (raw in every CTA):
+//   w = H v_j - beta v_{j-1};  alpha = <v_j, w>           one barrier
+//   raw' = w - alpha v_j, stored to every CTA; beta' = |raw'|, inv' = 1/beta'
+//                                                         one barrier
+// The basis vector goes out before its norm is known and the product is
+// scaled instead, so normalizing and sending it needs no barrier of its own.
 __global__ void __launch_bounds__(kChipThreads, 1) k_chip_lanczos(const ChipSector* __restrict__ secs) {
   extern __shared__ double sm[];
   cg::cluster_group cl = cg::this_cluster();
@@ -60,90 +69,75 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_lanczos(const ChipSect
   const uint32_t D = A.D;
   const int nt = (int)((D + kTile - 1) / kTile), per = (nt + C - 1) / C;
   const int t0 = min(nt, rank * per), t1 = min(nt, t0 + per);
-  double* x = sm;                      // D
-  double* q = x + D;                   // per x kTile
+  double* x = sm;                      // D: raw
+  double* v = x + D;                   // per x kTile: v_{j-1}, then v_j
+  double* q = v + per * kTile;         // per x kTile: w
   double* dg = q + per * kTile;        // per x kTile
   double* part = dg + per * kTile;     // 2 x nt
   __shared__ double slot[3];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = kChipThreads / 32;
   for (uint32_t i = threadIdx.x; i < D; i += kChipThreads) x[i] = S.x[i];
-  for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-      q[a] = (i < D && !S.first) ? S.q[i] : 0.0;
-      dg[a] = i < D ? chip_diag(A, i % A.du, i / A.du) : 0.0;
-    }
+  for (int t = t0 + wp; t < t1; t += nw) {
+    const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
+    v[a] = (i < D && !S.first) ? S.q[i] : 0.0;
+    dg[a] = i < D ? chip_diag(A, i % A.du, i / A.du) : 0.0;
+  }
+  double beta = S.first ? 0.0 : S.scale[0], inv = S.first ? 1.0 : S.scale[1];
   // lane r of a warp stores a tile's partial to CTA r
   double* peer_part = lane < C ? cl.map_shared_rank(part, lane) : part;
   cl.sync();
   for (int s = 0; s < S.steps; ++s) {
-    // q += H x, <x, q>
     for (int t = t0 + wp; t < t1; t += nw) {
+      const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
       double d = 0.0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-        if (i < D) {
-          const uint32_t id = i / A.du, iu = i - id * A.du;
-          const double xi = x[i];
-          const double v = fma(dg[a], xi, chip_hops(A, x, iu, id, q[a]));
-          q[a] = v;
-          d = fma(xi, v, d);
-          if (S.V) S.V[(size_t)s * D + i] = xi;
-          if (S.gs) S.gs[i] = fma(S.z[s], xi, S.gs[i]);
-        }
+      if (i < D) {
+        const uint32_t id = i / A.du, iu = i - id * A.du;
+        const double xi = x[i], vi = xi * inv;
+        const double h = fma(dg[a], xi, chip_hops(A, x, iu, id, 0.0));
+        const double w = fma(-beta, v[a], h * inv);
+        v[a] = vi;
+        q[a] = w;
+        d = vi * w;
+        if (S.V) S.V[(size_t)s * D + i] = vi;
+        if (S.gs) S.gs[i] = fma(S.z[s], vi, S.gs[i]);
       }
       d = warp_total(d);
       if (lane < C) peer_part[t] = d;
     }
-    cl.sync();
+    cl.sync();  // all gathers from x are over, too
     tile_total<false>(part, nt, slot);
     const double alpha = slot[0];
-    // q -= alpha x, |q|^2
     for (int t = t0 + wp; t < t1; t += nw) {
+      const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
       double d = 0.0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-        if (i < D) {
-          const double v = fma(-alpha, x[i], q[a]);
-          q[a] = v;
-          d = fma(v, v, d);
-        }
+      if (i < D) {
+        const double w = fma(-alpha, v[a], q[a]);
+        d = w * w;
+        for (int r = 0; r < C; ++r) cl.map_shared_rank(x, r)[i] = w;
       }
       d = warp_total(d);
       if (lane < C) peer_part[nt + t] = d;
     }
     cl.sync();
     tile_total<true>(part + nt, nt, slot + 1);
-    const double beta = slot[1], inv = slot[2];
+    beta = slot[1];
+    inv = slot[2];
     if (rank == 0 && threadIdx.x == 0 && S.coef) {
       S.coef[s] = alpha;
       S.coef[kChunk + s] = beta;
     }
-    // x <- q / beta in every CTA, q <- -beta x
-    for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-        if (i < D) {
-          const double xi = x[i], xn = q[a] * inv;
-          q[a] = -beta * xi;
-          for (int r = 0; r < C; ++r) cl.map_shared_rank(x, r)[i] = xn;
-        }
-      }
-    cl.sync();
   }
-  for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-      if (i < D) {
-        S.x[i] = x[i];
-        S.q[i] = q[a];
-      }
+  for (int t = t0 + wp; t < t1; t += nw) {
+    const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
+    if (i < D) {
+      S.x[i] = x[i];
+      S.q[i] = v[a];
     }
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    S.scale[0] = beta;
+    S.scale[1] = inv;
+  }
 }
 
 // psi_i (+)= sum_j z_j v_j,i over a span of a sector's kept vectors.
@@ -166,7 +160,7 @@ __global__ void __launch_bounds__(256) k_chip_combine(const ChipSum* __restrict_
 
 static size_t chip_smem(uint32_t D, int C) {
   const size_t nt = (D + kTile - 1) / kTile, per = (nt + C - 1) / C;
-  return (D + 2 * per * kTile + 2 * nt) * sizeof(double);
+  return (D + 3 * per * kTile + 2 * nt) * sizeof(double);
 }
 
 bool chip_fits(const qcmg_hamiltonian* H) { return H->dim > 0 && H->dim <= kChipStates && H->up.nval > 0; }
@@ -191,7 +185,7 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
   PoolBuf<double> xq, zbuf, gsbuf;
   std::vector<std::unique_ptr<PoolBuf<double>>> V;  // kSpan chunks of every sector each
   constexpr int kSpan = 8;
-  xq.alloc(2 * total);
+  xq.alloc(2 * total + 2 * (size_t)n);
   PoolBuf<ChipSector> secs;
   secs.alloc((size_t)2 * n);
   PoolBuf<ChipSum> sums;
@@ -232,6 +226,7 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
       S.op = chip_op(Hs[g.ids[k]]);
       S.x = xq.p + at[k];
       S.q = xq.p + total + at[k];
+      S.scale = xq.p + 2 * total + 2 * k;
       S.V = replay ? nullptr : chunk_vectors(c, k);
       S.coef = replay ? nullptr : coef.p + ((size_t)(c & 1) * n + k) * 2 * kChunk;
       S.z = nullptr;

@@ -12,7 +12,8 @@ namespace qcmg {
 
 constexpr uint32_t kChipStates = 16384;  // largest sector
 constexpr int kChipThreads = 512;
-constexpr int kTile = 64;  // states per partial sum: two per lane
+constexpr int kTile = 32;  // states per partial sum: one per lane, so that a few hundred
+                           // states per CTA still fill the four sub-partitions's FP64 pipes
 
 struct ChipOp {
   uint32_t du, dd, D;
@@ -66,7 +67,13 @@ __device__ __forceinline__ double warp_total(double v) {
 // slot[0], or with NORM its square root and the root's inverse in slot[0] and
 // slot[1].  The block's warp 0 does it: an FP64 instruction costs the SM 16
 // cycles per warp (a square root and a division by all 16 warps 3 us), so the
-// others wait instead of repeating it.
+// others wait instead of repeating it.  The root comes from its inverse (a
+// third of the latency of a square root and a division).
+__device__ __forceinline__ void root_and_inverse(double s, double* root) {
+  const double r = rsqrt(s);
+  root[0] = s > 0.0 ? s * r : s;  // 0, or NaN as it came
+  root[1] = r;
+}
 template <bool NORM>
 __device__ __forceinline__ void tile_total(const double* part, int nt, double* slot) {
   if (threadIdx.x < 32) {
@@ -74,11 +81,10 @@ __device__ __forceinline__ void tile_total(const double* part, int nt, double* s
     for (int t = threadIdx.x; t < nt; t += 32) s += part[t];
     s = warp_total(s);
     if (threadIdx.x == 0) {
-      if (NORM) {
-        s = sqrt(s);
-        slot[1] = 1.0 / s;
-      }
-      slot[0] = s;
+      if (NORM)
+        root_and_inverse(s, slot);
+      else
+        slot[0] = s;
     }
   }
   __syncthreads();

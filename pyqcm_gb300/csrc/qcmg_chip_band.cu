@@ -4,13 +4,14 @@
 // manner of qcmg_chip.cu.
 //
 // On a 3,920-state impurity sector a step was five launches and a host wait,
-// ~63 us; here it is three cluster barriers: the norm and the band dots of
-// v_j (one reduction for all of them), the scaled v_j to every CTA with the
-// Gram-Schmidt update of the next p - 1 vectors, and the product with the
-// band recurrence and its closing dot. The 2p + 1 vectors of the band live
+// ~63 us; here it is two cluster barriers: after the norm and the band dots of
+// v_j (one reduction for all of them), and after the Gram-Schmidt update of
+// the next p - 1 vectors (v_{j+1} going out to every CTA), the product and the
+// band recurrence with its closing dot. The 2p + 1 vectors of the band live
 // in shared memory, each CTA's part of them; only v_j is held whole (the
 // hops gather from it). One impurity of the 2x2 + 4 bath model from its
-// parameters to G (two runs of ~111 steps among it): 11.4 ms -> 6.9 ms.
+// parameters to G (two runs of ~111 steps among it): 11.4 ms -> 6.9 ms;
+// two barriers instead of three and 32 states a tile 5.49 -> 5.13 ms later.
 // The dots of a tile are added over the lanes together, by a reduction that
 // halves the values per lane at each step (2p - 1 additions instead of 5p).
 //
@@ -41,7 +42,15 @@ struct ChipBand {
 
 constexpr int pow2_of(int n) { return n <= 1 ? 1 : 2 * pow2_of((n + 1) / 2); }
 
-template <int P>
+// Step j (u_j: v_j before normalization, in every CTA's x):
+//   z = |u_j| and <u_{j+i}, u_j>                                  one barrier
+//   v_j = u_j / z; v_{j+i} -= c_i v_j; w = H v_j - sum_k T(k, j) v_k;
+//   d = <w, v_j>                                                  one barrier
+//   w -= d v_j
+// TWO: x has two buffers and u_{j+1} goes out to all CTAs in the second part
+// (P > 1: it is final then). Otherwise, where two do not fit or for P = 1, it
+// goes out at the start of its own step, with a barrier more.
+template <int P, bool TWO>
 __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
   constexpr int R = 2 * P + 1;
   extern __shared__ double sm[];
@@ -52,24 +61,27 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
   const int nt = (int)((D + kTile - 1) / kTile), per = (nt + C - 1) / C;
   const int t0 = min(nt, rank * per), t1 = min(nt, t0 + per);
   const int seg = per * kTile;
-  double* x = sm;                // D: v_j
-  double* v = x + D;             // R x seg: the band's vectors, this CTA's part
-  double* dg = v + R * seg;      // seg
-  double* part = dg + seg;       // (2 P + 1) x nt
+  double* xb = sm;                         // D, or 2 x D: u_j, u_{j+1}
+  double* v = xb + (TWO ? 2 : 1) * D;      // R x seg: the band's vectors, this CTA's part
+  double* dg = v + R * seg;                // seg
+  double* part = dg + seg;                 // (2 P + 1) x nt
   __shared__ double tot[2 * P + 1], zs[2], ds;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = kChipThreads / 32;
   if (*(volatile int*)S.deflated >= 0) return;  // an earlier launch ended the run
-  for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-      dg[a] = i < D ? chip_diag(A, i % A.du, i / A.du) : 0.0;
-      for (int k = 0; k < R; ++k) {
-        double y = 0.0;
-        if (i < D) y = S.j0 > 0 ? S.ring[(size_t)k * D + i] : (k < P ? S.phi[(size_t)k * D + i] : 0.0);
-        v[k * seg + a] = y;
-      }
+  for (int t = t0 + wp; t < t1; t += nw) {
+    const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
+    dg[a] = i < D ? chip_diag(A, i % A.du, i / A.du) : 0.0;
+    for (int k = 0; k < R; ++k) {
+      double y = 0.0;
+      if (i < D) y = S.j0 > 0 ? S.ring[(size_t)k * D + i] : (k < P ? S.phi[(size_t)k * D + i] : 0.0);
+      v[k * seg + a] = y;
     }
+  }
+  if (TWO) {  // u_{j0} whole
+    const double* u = S.j0 > 0 ? S.ring + (size_t)(S.j0 % R) * D : S.phi;
+    double* x = xb + (S.j0 & 1) * D;
+    for (uint32_t i = threadIdx.x; i < D; i += kChipThreads) x[i] = u[i];
+  }
   // the V sums of tile t to every CTA: value m goes to part[m nt + t]
   auto send = [&](auto& acc, int count, int first, int t) {
     constexpr int V = sizeof(acc) / sizeof(double), sub = 32 / V;
@@ -83,26 +95,28 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
     for (int t = lane; t < nt; t += 32) s += part[m * nt + t];
     return warp_total(s);
   };
+  auto publish = [&](double* x, uint32_t i, double y) {
+    for (int r = 0; r < C; ++r) cl.map_shared_rank(x, r)[i] = y;
+  };
   cl.sync();
   for (int s = 0; s < S.steps; ++s) {
     const int j = S.j0 + s;
+    double* x = xb + (TWO ? (j & 1) * D : 0);
     int slot[R];  // slot[k]: v_{j - P + k}
 #pragma unroll
     for (int k = 0; k < R; ++k) slot[k] = ((j + k + P + 1) % R) * seg;  // j - P + k + R, mod R
     const bool proj = j < P;
-    // |v_j|^2, <v_{j+i}, v_j>, and while j < p <phi_k, v_j>
+    // |u_j|^2, <u_{j+i}, u_j>, and while j < p <phi_k, u_j>
     for (int t = t0 + wp; t < t1; t += nw) {
       double acc[pow2_of(P)] = {}, pr[pow2_of(P)] = {};
+      const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
+      const double vj = v[slot[P] + a];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-        const double vj = v[slot[P] + a];
+      for (int k = 0; k < P; ++k) acc[k] = v[slot[P + k] + a] * vj;
+      if (proj && i < D)
 #pragma unroll
-        for (int k = 0; k < P; ++k) acc[k] = fma(v[slot[P + k] + a], vj, acc[k]);
-        if (proj && i < D)
-#pragma unroll
-          for (int k = 0; k < P; ++k) pr[k] = fma(S.phi[(size_t)k * D + i], vj, pr[k]);
-      }
+        for (int k = 0; k < P; ++k) pr[k] = S.phi[(size_t)k * D + i] * vj;
+      if (!TWO && i < D) publish(x, i, vj);
       send(acc, P, 0, t);
       if (proj) send(pr, P, P, t);
     }
@@ -111,10 +125,7 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
       const double y = total(m);
       if (lane == 0) {
         tot[m] = y;
-        if (m == 0) {
-          zs[0] = sqrt(y);
-          zs[1] = 1.0 / zs[0];
-        }
+        if (m == 0) root_and_inverse(y, zs);
       }
     }
     __syncthreads();
@@ -129,42 +140,33 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
       for (int k = 1; k < P; ++k) co[k] = tot[k] * iz;
       for (int k = 0; k < P; ++k) co[P + 1 + k] = proj ? tot[P + k] * iz : 0.0;
     }
-    // v_j /= z, to every CTA; v_{j+i} -= c_i v_j
-    double c[P];
+    double c[P];  // T(j - p + k, j): c_0 = z
 #pragma unroll
     for (int k = 0; k < P; ++k) c[k] = k ? tot[k] * iz : z;
-    for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-        const double y = v[slot[P] + a] * iz;
-        v[slot[P] + a] = y;
-        if (i < D)
-          for (int r = 0; r < C; ++r) cl.map_shared_rank(x, r)[i] = y;
-#pragma unroll
-        for (int k = 1; k < P; ++k) v[slot[P + k] + a] = fma(-c[k], y, v[slot[P + k] + a]);
-      }
-    cl.sync();
-    // w = H v_j - sum_k T(k, j) v_k, <w, v_j>; T(j - p + k, j) = c_k (c_0 = z)
+    double* xn = xb + (TWO ? ((j + 1) & 1) * D : 0);
     for (int t = t0 + wp; t < t1; t += nw) {
-      double acc[1] = {0.0};
+      const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
+      double acc[1] = {0.0}, w = 0.0;
+      const double y = v[slot[P] + a] * iz;
+      v[slot[P] + a] = y;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-        double w = 0.0;
-        if (i < D) {
-          const uint32_t id = i / A.du, iu = i - id * A.du;
-          w = fma(dg[a], x[i], chip_hops(A, x, iu, id, 0.0));
-#pragma unroll
-          for (int k = 0; k < P; ++k)
-            if (j - P + k >= 0) w = fma(-c[k], v[slot[k] + a], w);
-          acc[0] = fma(w, x[i], acc[0]);
-        }
-        v[slot[2 * P] + a] = w;
+      for (int k = 1; k < P; ++k) {
+        const double t2 = fma(-c[k], y, v[slot[P + k] + a]);
+        v[slot[P + k] + a] = t2;
+        if (TWO && k == 1 && i < D) publish(xn, i, t2);
       }
+      if (i < D) {
+        const uint32_t id = i / A.du, iu = i - id * A.du;
+        w = fma(dg[a], y, chip_hops(A, x, iu, id, 0.0) * iz);
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+          if (j - P + k >= 0) w = fma(-c[k], v[slot[k] + a], w);
+        acc[0] = w * y;
+      }
+      v[slot[2 * P] + a] = w;
       send(acc, 1, 2 * P, t);
     }
-    cl.sync();
+    cl.sync();  // all gathers from x are over, too
     if (wp == 0) {
       const double y = total(2 * P);
       if (lane == 0) ds = y;
@@ -172,45 +174,42 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
     __syncthreads();
     const double d = ds;
     if (rank == 0 && threadIdx.x == 0) co[P] = d;
-    for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t a = (t - t0) * kTile + h * 32 + lane;
-        v[slot[2 * P] + a] = fma(-d, v[slot[P] + a], v[slot[2 * P] + a]);
-      }
+    for (int t = t0 + wp; t < t1; t += nw) {
+      const uint32_t a = (t - t0) * kTile + lane;
+      v[slot[2 * P] + a] = fma(-d, v[slot[P] + a], v[slot[2 * P] + a]);
+    }
     // a thread reads and writes its own elements only, so the next step needs
     // no barrier here
   }
-  for (int t = t0 + wp; t < t1; t += nw)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t i = t * kTile + h * 32 + lane, a = (t - t0) * kTile + h * 32 + lane;
-      if (i < D)
-        for (int k = 0; k < R; ++k) S.ring[(size_t)k * D + i] = v[k * seg + a];
-    }
+  for (int t = t0 + wp; t < t1; t += nw) {
+    const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
+    if (i < D)
+      for (int k = 0; k < R; ++k) S.ring[(size_t)k * D + i] = v[k * seg + a];
+  }
 }
 
-static size_t band_smem(uint32_t D, int p, int C) {
+static size_t band_smem(uint32_t D, int p, int C, bool two) {
   const size_t nt = (D + kTile - 1) / kTile, per = (nt + C - 1) / C;
-  return (D + (2 * p + 2) * per * kTile + (2 * p + 1) * nt) * sizeof(double);
+  return ((two ? 2 : 1) * (size_t)D + (2 * p + 2) * per * kTile + (2 * p + 1) * nt) * sizeof(double);
 }
 
 constexpr int kBandMaxP = 12;
 
 template <int P, class F>
-static void with_band_kernel(int p, F&& f) {
+static void with_band_kernel(int p, bool two, F&& f) {
   if constexpr (P > 0) {
-    if (p == P)
-      f(k_chip_band<P>);
-    else
-      with_band_kernel<P - 1>(p, f);
+    if (p != P) return with_band_kernel<P - 1>(p, two, f);
+    if constexpr (P > 1) {
+      if (two) return f(k_chip_band<P, true>);
+    }
+    f(k_chip_band<P, false>);
   }
 }
 
 bool chip_band_fits(const qcmg_hamiltonian* H, int p) {
   int optin = 0;
   QCMG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, H->device));
-  return chip_fits(H) && p <= kBandMaxP && band_smem((uint32_t)H->dim, p, 8) <= (size_t)optin - 1024;
+  return chip_fits(H) && p <= kBandMaxP && band_smem((uint32_t)H->dim, p, 8, false) <= (size_t)optin - 1024;
 }
 
 bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc_defl,
@@ -239,17 +238,18 @@ bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc
   S.deflated = const_cast<int*>(deflated);
   S.acc_defl = acc_defl;
   int C = 8;
+  bool two = p > 1 && band_smem(D, p, 8, true) <= (size_t)optin - 1024;
   auto launch = [&](int c) {
     S.j0 = c * kBandChunk;
     S.steps = std::min(kBandChunk, M0 - S.j0);
     if (S.steps <= 0) return;
     S.coef = coef.p + (size_t)(c & 1) * chunk_len;
-    with_band_kernel<kBandMaxP>(p, [&](auto kern) {
+    with_band_kernel<kBandMaxP>(p, two, [&](auto kern) {
       if (c == 0) {
         QCMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-        if (clusters_run(kern, 16, band_smem(D, p, 16))) C = 16;
+        if (clusters_run(kern, 16, band_smem(D, p, 16, two))) C = 16;
       }
-      launch_clusters(kern, 1, C, band_smem(D, p, C), s, S);
+      launch_clusters(kern, 1, C, band_smem(D, p, C, two), s, S);
     });
     QCMG_CUDA(cudaEventRecord(lane.e[c & 1], s));
   };
