@@ -133,82 +133,21 @@ __global__ void k_fx_to_host(const int64_t* __restrict__ q, double* __restrict__
   }
 }
 
-constexpr int kRedBlocksFx = 1024;
-constexpr int kFinalThreads = 512;
-
-// log2 rounded up, as ceil_log2 (x > 0)
-__device__ __forceinline__ int ceil_log2_dev(double x) {
-  if (!(x > 0.0)) return 0;
-  int ex;
-  const double m = frexp(x, &ex);
-  return m == 0.5 ? ex - 1 : ex;
-}
-
-// Sum of one block's share of the 128-bit partials, complete in thread 0.
-__device__ __forceinline__ I128 final_sum128(const I128* __restrict__ part, int np) {
-  __shared__ I128 total;
-  I128 s = {0, 0};
-  for (int i = threadIdx.x; i < np; i += kFinalThreads) s = add128(s, part[i]);
-  block_store128(s, &total - blockIdx.x);
-  __syncthreads();
-  return total;
-}
-
-// alpha = <v, w> from pass D's partials, and from it the coefficients of the
-// update w - alpha v - beta p: the same IEEE operations in the same order as
-// on the host (explicit roundings, no contraction), so the host need not
-// wait between the product and the update.  A single warp walking the ~1,000
-// partials took 12.1 us, this block 5.2 us (the norm's 3.8 us).
-__global__ void __launch_bounds__(kFinalThreads)
-    k_fx_alpha(const I128* __restrict__ part, int np, double vc, int vE, int vmb, double wc, int wE,
-               int wmb, double bp, long long mb, int pEe, FxStep* __restrict__ st) {
-  const I128 h = final_sum128(part, np);
-  if (threadIdx.x != 0) return;
-  const double r = __dadd_rn(ldexp((double)h.hi, 64), (double)h.lo);
-  const double alpha = __dmul_rn(__dmul_rn(vc, wc), ldexp(r, kDotShift + vE + wE));
-  const double k = __ddiv_rn(__dmul_rn(alpha, vc), wc);
-  const double bw = ldexp(1.0, wE + wmb), bv = __dmul_rn(fabs(k), ldexp(1.0, vE + vmb));
-  const int Eo = ceil_log2_dev(__dadd_rn(__dadd_rn(bw, bv), bp)) - kFxBits;
-  long long ma = 0;
-  int e = 0;
-  if (k != 0.0 && isfinite(k)) {
-    int ex;
-    const double m = frexp(k, &ex);
-    ma = llrint(ldexp(m, 53));  // an integer already
-    e = ex - 53;
-  }
-  st->alpha = alpha;
-  st->ma = ma;
-  st->mb = mb;
-  st->sw = Eo - wE;
-  st->sa = Eo - vE - e;
-  st->sb = Eo - pEe;
-  st->Eo = Eo;
-  st->qmax = 0;
-}
-
-// The update's norm from its partials.
-__global__ void __launch_bounds__(kFinalThreads) k_fx_norm(const I128* __restrict__ part, int np,
-                                                          const int* __restrict__ err,
-                                                          FxStep* __restrict__ st) {
-  const I128 h = final_sum128(part, np);
-  if (threadIdx.x != 0) return;
-  st->n_hi = h.hi;
-  st->n_lo = h.lo;
-  st->err = err ? *err : 0;
-}
-
 // Fused Lanczos update:
 //   q_o = round(q_w * 2^-sw) - round(q_v * ma 2^-sa) - round(q_p * mb 2^-sb)
-// written over q_w, with exact |q_o|^2 partials and max|q_o|.
-__global__ void __launch_bounds__(256) k_fx_update(int64_t* __restrict__ w,
+// written over q_w, with exact |q_o|^2 and max|q_o|.  The block that finishes
+// last adds the partials and writes the step's scalars straight into the
+// host's page-locked copy, seq after everything else: the host polls it and
+// queues the next product while this kernel retires.
+__global__ void __launch_bounds__(256, 4) k_fx_update(int64_t* __restrict__ w,
                                                    const int64_t* __restrict__ v,
                                                    const int64_t* __restrict__ p, size_t n,
                                                    FxStep* __restrict__ st,
-                                                   I128* __restrict__ part) {
+                                                   I128* __restrict__ part,
+                                                   const int* __restrict__ err,
+                                                   FxStep* host, unsigned long long seq) {
   const int sw = st->sw, sa = st->sa, sb = st->sb;
   const int64_t ma = st->ma, mb = st->mb;
-  unsigned long long* qmax = &st->qmax;
   I128 s = {0, 0};
   unsigned long long m = 0;
   auto one = [&](int64_t wi, int64_t vi, int64_t pi) {
@@ -237,9 +176,26 @@ __global__ void __launch_bounds__(256) k_fx_update(int64_t* __restrict__ w,
   }
   if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0)
     w[n - 1] = one(w[n - 1], v[n - 1], p ? p[n - 1] : 0);
+  // one atomic per block (one per warp queue up at the single address)
+  __shared__ unsigned long long bmax[8];
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(qmax, m);
-  block_store128(s, part);
+  if ((threadIdx.x & 31) == 0) bmax[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) m = max(m, bmax[k]);
+    atomicMax(&st->qmax, m);
+  }
+  I128 h;
+  if (!last_block_sum128(s, part, &st->ticket, &h) || threadIdx.x != 0) return;
+  volatile FxStep* out = host;
+  out->alpha = st->alpha;
+  out->Eo = st->Eo;
+  out->n_hi = h.hi;
+  out->n_lo = h.lo;
+  out->qmax = __ldcg(&st->qmax);
+  out->err = err ? *err : 0;
+  __threadfence_system();
+  out->seq = seq;
 }
 
 // g = round(g * 2^-sg) + round(q * m 2^-s)   (eigenvector accumulation)
@@ -440,14 +396,13 @@ void fx_to_f64(const FxVec& v, double* x, cudaStream_t s) {
   QCMG_CUDA(cudaGetLastError());
 }
 
-FxReducer::~FxReducer() {
-  if (host) cudaFreeHost(host);
-}
-
-void FxReducer::init(size_t partials) {
-  part.alloc(partials);
+void FxReducer::init(int sms, cudaStream_t s) {
+  update_blocks = 4u * (unsigned)sms;
+  part.alloc(std::max(update_blocks, product_dot_partials(sms)));
   step.alloc(1);
-  if (!host) QCMG_CUDA(cudaMallocHost(&host, sizeof(FxStep)));
+  QCMG_CUDA(cudaMemsetAsync(step.p, 0, sizeof(FxStep), s));
+  host.alloc(1);
+  host.p->seq = seq = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -456,8 +411,8 @@ void FxReducer::init(size_t partials) {
 // y = H x  (or y = H x + gamma * yin with yin != nullptr, yin may be &y).
 // The output exponent follows from the bound |H|_inf (T.b) and the input's
 // largest component; c_y = c_x.
-unsigned fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
-                   FxReducer* dot) {
+void fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
+               FxReducer* dot, const FxVec* p, double beta) {
   FxTables& T = H->fx;
   cudaStream_t s = H->stream;
   const size_t n = H->dim;
@@ -524,17 +479,32 @@ unsigned fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* y
   A.ell4 = T.ell4.p;
   A.cnt4 = T.cnt4.p;
   A.err = T.err.p;
+  y.E = Eo;
+  y.mb = kFxBits;
+  y.c = x.c;
   A.dot_x = nullptr;
   A.dot_part = nullptr;
   if (dot) {
     A.dot_x = x.buf.p;
     A.dot_part = dot->part.p;
+    A.dot_step = dot->step.p;
+    A.dot_xc = x.c;
+    A.dot_xE = x.E;
+    A.dot_xmb = x.mb;
+    A.dot_yc = y.c;
+    A.dot_yE = y.E;
+    A.dot_ymb = y.mb;
+    A.dot_bp = 0.0;
+    A.dot_pE = 0;
+    int64_t mb = 0;
+    if (p) {
+      A.dot_bp = std::fabs(beta * p->c / y.c) * std::ldexp(1.0, p->E + p->mb);
+      split_double(beta * p->c / y.c, &mb, &e);
+      A.dot_pE = e + p->E;
+    }
+    A.dot_mb = mb;
   }
-  const unsigned np = launch_product(H, A, s);
-  y.E = Eo;
-  y.mb = kFxBits;
-  y.c = x.c;
-  return np;
+  launch_product(H, A, s);
 }
 
 void fx_check_error(qcmg_hamiltonian* H) {
@@ -585,33 +555,33 @@ void fx_matvec_to_host(qcmg_hamiltonian* H, const double* x, double* yh, bool ac
 // Lanczos on FX vectors: the reference's recurrence (Lanczos.hpp:64-93)
 // written with normalized vectors, w = H v_j - alpha v_j - beta v_{j-1}.
 
-// Queues w <- w - alpha v - beta p with alpha = <v, w> from the np partials
-// that the product left in red.part, and the copy of the step's scalars.
-static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec* p, unsigned np,
-                      double beta, FxReducer& red) {
-  cudaStream_t s = H->stream;
+// Queues w <- w - alpha v - beta p with the coefficients that the product
+// left in red.step.
+static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec* p, FxReducer& red) {
   const size_t n = w.n;
-  double bp = 0.0;  // bound of the beta term, in units of c_w
-  int64_t mb = 0;
-  int e = 0;
-  if (p) {
-    bp = std::fabs(beta * p->c / w.c) * std::ldexp(1.0, p->E + p->mb);
-    split_double(beta * p->c / w.c, &mb, &e);
-    e += p->E;
-  }
-  k_fx_alpha<<<1, kFinalThreads, 0, s>>>(red.part.p, (int)np, v.c, v.E, v.mb, w.c, w.E, w.mb, bp,
-                                         (long long)mb, e, red.step.p);
-  unsigned g = (unsigned)std::min<size_t>(kRedBlocksFx, std::max<size_t>(1, (n + 255) / 256));
-  k_fx_update<<<g, 256, 0, s>>>(w.buf.p, v.buf.p, p ? p->buf.p : nullptr, n, red.step.p, red.part.p);
-  k_fx_norm<<<1, kFinalThreads, 0, s>>>(red.part.p, (int)g, H->fx.err.p, red.step.p);
+  // all blocks resident, four per SM
+  const unsigned g = (unsigned)std::min<size_t>(red.update_blocks, std::max<size_t>(1, (n / 2 + 255) / 256));
+  k_fx_update<<<g, 256, 0, H->stream>>>(w.buf.p, v.buf.p, p ? p->buf.p : nullptr, n, red.step.p,
+                                        red.part.p, H->fx.err.p, red.host.p, ++red.seq);
   QCMG_CUDA(cudaGetLastError());
-  QCMG_CUDA(cudaMemcpyAsync(red.host, red.step.p, sizeof(FxStep), cudaMemcpyDeviceToHost, s));
 }
 
 // Waits for the step queued last: w's exponent and size, alpha and |w|^2.
+// A stream that ran empty, or failed, without that step's number ends the wait.
 static void fx_collect(qcmg_hamiltonian* H, FxVec& w, FxReducer& red, double* alpha, double* norm2) {
-  QCMG_CUDA(cudaStreamSynchronize(H->stream));
-  const FxStep& h = *red.host;
+  const FxStep& h = *red.host.p;
+  auto arrived = [&] { return __atomic_load_n(&red.host.p->seq, __ATOMIC_ACQUIRE) == red.seq; };
+  for (unsigned spin = 1; !arrived(); ++spin) {
+    if (spin % 4096) continue;
+    const cudaError_t q = cudaStreamQuery(H->stream);
+    if (q == cudaErrorNotReady) {
+      cudaGetLastError();
+      continue;
+    }
+    QCMG_CUDA(q);
+    if (arrived()) break;
+    throw Error(QCMG_ERR_CUDA, "a Lanczos step did not report its scalars");
+  }
   if (h.err) throw Error(QCMG_ERR_CUDA, "a bulk copy into shared memory did not complete in time");
   w.E = h.Eo;
   w.mb = bitlen(h.qmax);
@@ -686,7 +656,7 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
   FxReducer red;
   int sms = 0;
   QCMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device));
-  red.init(std::max<size_t>(kRedBlocksFx, product_dot_partials(sms)));
+  red.init(sms, s);
   DevBuf<unsigned long long> tmp;
   FxSlots slots(n);
   // The Lanczos vectors are kept when the ground state is wanted and 300 of
@@ -741,8 +711,8 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
         w->buf.borrow(slots.get(want), n);
       }
       // alpha = <v, H v> comes out of the product's second pass
-      const unsigned np = fx_matvec(H, *v, *w, nullptr, 0.0, &red);
-      fx_update(H, *w, *v, have_p ? p : nullptr, np, beta_prev, red);
+      fx_matvec(H, *v, *w, nullptr, 0.0, &red, have_p ? p : nullptr, beta_prev);
+      fx_update(H, *w, *v, have_p ? p : nullptr, red);
     };
     // On sectors whose step takes tens of microseconds the convergence test
     // takes as long: the next step is queued first and runs meanwhile (one

@@ -101,6 +101,35 @@ __device__ __forceinline__ void block_store128(I128 s, I128* part) {
   }
 }
 
+// Stores a block's sum with the other blocks' in part[]. The block that
+// finishes last gets true, with the sum over all blocks (integers: the order
+// does not matter) in thread 0's total, and resets the ticket.
+__device__ __forceinline__ bool last_block_sum128(I128 s, I128* part, unsigned* ticket, I128* total) {
+  __shared__ unsigned last;
+  block_store128(s, part);  // thread 0 stores
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  I128 t = {0, 0};
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+    const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(part) + i);
+    I128 q;
+    memcpy(&q, &v, sizeof q);
+    t = add128(t, q);
+  }
+  __shared__ I128 sum;
+  block_store128(t, &sum - blockIdx.x);  // thread 0 stores
+  if (threadIdx.x == 0) {
+    *total = sum;
+    *ticket = 0;
+  }
+  return true;
+}
+
 // round(a * m / 2^s)
 __device__ __forceinline__ int64_t mul_fix(int64_t a, int64_t m, int s) {
   return shr128_round(mul_s64(a, m), s);
@@ -203,6 +232,14 @@ __device__ __forceinline__ double fx_to_f64(int64_t q, int E) {
   if (bexp <= 0) return 0.0;  // below the normal range: flush (never reached in practice)
   const uint64_t bits = sign | ((uint64_t)bexp << 52) | (frac & ((1ull << 52) - 1));
   return __longlong_as_double((long long)bits);
+}
+
+// log2 rounded up, as ceil_log2 (x > 0)
+__device__ __forceinline__ int ceil_log2_dev(double x) {
+  if (!(x > 0.0)) return 0;
+  int ex;
+  const double m = frexp(x, &ex);
+  return m == 0.5 ? ex - 1 : ex;
 }
 
 }  // namespace qcmg

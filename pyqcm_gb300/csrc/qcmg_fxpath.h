@@ -5,14 +5,15 @@
 
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
+#include "qcmg_pool.h"
 
 namespace qcmg {
 
 struct I128;
 
 // Scalars of one Lanczos step, written on the device: alpha and the update's
-// coefficients by the final sum of <v, H v>, the norm by the final sum of
-// the update, and read back together (one wait per step).
+// coefficients by the last block of the product's second pass, the norm by
+// the last block of the update.
 struct FxStep {
   double alpha;
   long long ma, mb;    // mantissas of alpha c_v / c_w and beta c_p / c_w
@@ -20,17 +21,18 @@ struct FxStep {
   long long n_hi;      // sum of squares >> kDotShift, 128 bits
   unsigned long long n_lo, qmax;
   int err;             // bounded-wait failure flag of the product kernels
+  unsigned ticket;     // blocks of the running kernel that are done
+  // the host's copy: number of the step whose values stand above
+  unsigned long long seq;
 };
 
 struct FxReducer {
   DevBuf<I128> part;
   DevBuf<FxStep> step;
-  FxStep* host = nullptr;  // page-locked
-  FxReducer() = default;
-  FxReducer(const FxReducer&) = delete;
-  FxReducer& operator=(const FxReducer&) = delete;
-  ~FxReducer();
-  void init(size_t partials);
+  PinnedBuf<FxStep> host;  // written by the device
+  unsigned long long seq = 0;  // of the step queued last
+  unsigned update_blocks = 0;
+  void init(int sms, cudaStream_t s);
 };
 
 // Prepares the fixed-point tables; false if the Hamiltonian does not have
@@ -39,10 +41,11 @@ bool fx_prepare(qcmg_hamiltonian* H);
 void fx_from_f64(const double* x, size_t n, FxVec& v, cudaStream_t s,
                  DevBuf<unsigned long long>& tmp);
 void fx_to_f64(const FxVec& v, double* x, cudaStream_t s);
-// With dot set, the product's second pass also leaves block partials of
-// <x, y> (for the finished y) in dot->part; returns their number.
-unsigned fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
-                   FxReducer* dot = nullptr);
+// With dot set, the product's second pass also computes alpha = <x, y> (for
+// the finished y) and the coefficients of y - alpha x - beta p into
+// dot->step (p may be null).
+void fx_matvec(qcmg_hamiltonian* H, const FxVec& x, FxVec& y, const FxVec* yin, double gamma,
+               FxReducer* dot = nullptr, const FxVec* p = nullptr, double beta = 0.0);
 // Throws if a kernel of the fast path reported a bounded-wait failure.
 void fx_check_error(qcmg_hamiltonian* H);
 // Whether a product of FP64 vectors takes the fixed-point passes: where they

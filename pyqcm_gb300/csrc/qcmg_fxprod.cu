@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "qcmg_fx.cuh"
+#include "qcmg_fxpath.h"
 #include "qcmg_fxprod.h"
 #include "qcmg_tma.cuh"
 
@@ -365,6 +366,38 @@ __device__ __forceinline__ void passD5_accum(const int64_t* __restrict__ x, uint
   }
 }
 
+// alpha = <x, y> from its exact sum h, and from it the coefficients of the
+// update y - alpha x - beta p: the same IEEE operations in the same order as
+// on a host (explicit roundings, no contraction).  By the last block of the
+// second pass: a launch of its own for the sums (5 us here, 4 us for the
+// norm) and a copy and a stream wait per step made a solve of 853,776 states
+// 62 us a step, 50 us now.
+__device__ __noinline__ void lanczos_coefficients(I128 h, double vc, int vE, int vmb, double wc, int wE,
+                                                  int wmb, double bp, long long mb, int pEe,
+                                                  FxStep* __restrict__ st) {
+  const double r = __dadd_rn(ldexp((double)h.hi, 64), (double)h.lo);
+  const double alpha = __dmul_rn(__dmul_rn(vc, wc), ldexp(r, kDotShift + vE + wE));
+  const double k = __ddiv_rn(__dmul_rn(alpha, vc), wc);
+  const double bw = ldexp(1.0, wE + wmb), bv = __dmul_rn(fabs(k), ldexp(1.0, vE + vmb));
+  const int Eo = ceil_log2_dev(__dadd_rn(__dadd_rn(bw, bv), bp)) - kFxBits;
+  long long ma = 0;
+  int e = 0;
+  if (k != 0.0 && isfinite(k)) {
+    int ex;
+    const double m = frexp(k, &ex);
+    ma = llrint(ldexp(m, 53));  // an integer already
+    e = ex - 53;
+  }
+  st->alpha = alpha;
+  st->ma = ma;
+  st->mb = mb;
+  st->sw = Eo - wE;
+  st->sa = Eo - vE - e;
+  st->sb = Eo - pEe;
+  st->Eo = Eo;
+  st->qmax = 0;
+}
+
 // Items (band, down state) are numbered in 32 bits (launch contract:
 // nbands * dd < 2^32).  A row's hops are summed with their signs into one
 // accumulator per element (exact: |sum| < 2^61).
@@ -418,7 +451,12 @@ __global__ void __launch_bounds__(256, MINB) k_fx_passD5(FxProdArgs A) {
       }
     }
   }
-  if (DOT) block_store128(dot, A.dot_part);  // every thread of the block gets here
+  if (DOT) {  // every thread of the block gets here
+    I128 h;
+    if (last_block_sum128(dot, A.dot_part, &A.dot_step->ticket, &h) && threadIdx.x == 0)
+      lanczos_coefficients(h, A.dot_xc, A.dot_xE, A.dot_xmb, A.dot_yc, A.dot_yE, A.dot_ymb, A.dot_bp,
+                           A.dot_mb, A.dot_pE, A.dot_step);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -601,7 +639,7 @@ static void launch_passU4(Kern kern, const qcmg_hamiltonian* H, const FxProdArgs
   kern<<<(unsigned)grid, threads, smem, s>>>(A);
 }
 
-unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStream_t s) {
+void launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStream_t s) {
   const FxTables& T = H->fx;
   if (T.sms == 0) QCMG_CUDA(cudaDeviceGetAttribute(&T.sms, cudaDevAttrMultiProcessorCount, H->device));
   const int sms = T.sms;
@@ -661,19 +699,17 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
     }
     const unsigned g = (unsigned)std::max<size_t>(1, std::min<size_t>((items + 7) / 8, (size_t)sms * per_sm));
     kern<<<g, 256, 0, s>>>(A);
-    return g;
   };
   // six 256-thread blocks per SM (40 registers) for the product; five for
   // the Lanczos form, whose 128-bit dot accumulator needs the registers
   const bool even = (H->du & 1u) == 0u, nard = fast && narrow_shift(A.t_dn);
-  unsigned gD;
   auto form_d = [&](auto vec_tag) {
     constexpr int V = decltype(vec_tag)::value;
     if (A.dot_part)
-      gD = nard ? go(k_fx_passD5<V, true, true, true, 5>)
+      nard ? go(k_fx_passD5<V, true, true, true, 5>)
                 : fast ? go(k_fx_passD5<V, true, false, true, 5>) : go(k_fx_passD5<V, false, false, true, 5>);
     else
-      gD = nard ? go(k_fx_passD5<V, true, true, false, 6>)
+      nard ? go(k_fx_passD5<V, true, true, false, 6>)
                 : fast ? go(k_fx_passD5<V, true, false, false, 6>) : go(k_fx_passD5<V, false, false, false, 6>);
   };
   if (even)
@@ -681,7 +717,6 @@ unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStre
   else
     form_d(One{});
   QCMG_CUDA(cudaGetLastError());
-  return gD;
 }
 
 }  // namespace qcmg

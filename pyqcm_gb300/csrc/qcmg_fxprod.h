@@ -9,6 +9,7 @@
 namespace qcmg {
 
 struct I128;
+struct FxStep;
 
 struct FxProdArgs {
   uint32_t du, dd;
@@ -58,6 +59,12 @@ struct FxProdArgs {
   // 128-bit partial per pass-D block into dot_part (the Lanczos alpha)
   const int64_t* dot_x;
   I128* dot_part;
+  // the last of those blocks to finish adds the partials and writes the
+  // Lanczos step's coefficients to it
+  FxStep* dot_step;
+  double dot_xc, dot_yc, dot_bp;  // lazy scales of x and y, bound of the beta term
+  int dot_xE, dot_xmb, dot_yE, dot_ymb, dot_pE;
+  long long dot_mb;
 };
 
 // Builds the grouped ELL form of the up-spin hops from the unit-magnitude
@@ -73,11 +80,10 @@ int choose_slabs_per_pass(uint32_t du, int max_optin_smem);
 // log2 |m| when |m| is a power of two, else -1 (for FxProdArgs::p2_*).
 int pow2_exponent(int64_t m);
 
-// Launches pass U then pass D for y (+)= H x; returns pass D's block count
-// (the number of dot partials when A.dot_part is set).
-unsigned launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStream_t s);
+// Launches pass U then pass D for y (+)= H x.
+void launch_product(const qcmg_hamiltonian* H, const FxProdArgs& A, cudaStream_t s);
 
-// Upper bound of launch_product's return value on a device with sms SMs.
+// Upper bound of pass D's blocks (dot partials) on a device with sms SMs.
 inline unsigned product_dot_partials(int sms) { return (unsigned)sms * 8u; }
 
 }  // namespace qcmg
