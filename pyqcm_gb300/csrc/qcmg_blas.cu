@@ -61,6 +61,12 @@ __global__ void __launch_bounds__(kRedThreads) k_axpy_norm(double* __restrict__ 
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
+__global__ void k_scaled_copy(double* __restrict__ y, const double* __restrict__ x, double a, size_t n) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    y[i] = a * x[i];
+}
+
 __global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, double a, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
@@ -252,6 +258,12 @@ void axpy_neg_dev(double* y, const double* x, const double* a_dev, size_t n, cud
 void axpy(double* y, const double* x, double a, size_t n, cudaStream_t s) {
   if (!n) return;
   k_axpy<<<ew_grid(n), 256, 0, s>>>(y, x, a, n);
+  QCMG_CUDA(cudaGetLastError());
+}
+
+void scaled_copy(double* y, const double* x, double a, size_t n, cudaStream_t s) {
+  if (!n) return;
+  k_scaled_copy<<<ew_grid(n), 256, 0, s>>>(y, x, a, n);
   QCMG_CUDA(cudaGetLastError());
 }
 

@@ -31,6 +31,7 @@ struct Reducer {
 void axpy(double* y, const double* x, double a, size_t n, cudaStream_t s);
 // y -= (*a_dev) x, bitwise the same as axpy(y, x, -(*a_dev), ...).
 void axpy_neg_dev(double* y, const double* x, const double* a_dev, size_t n, cudaStream_t s);
+void scaled_copy(double* y, const double* x, double a, size_t n, cudaStream_t s);  // y = a x
 void scale2(double* r, double s1, double* q, double s2, size_t n, cudaStream_t s);
 void scale(double* x, double a, size_t n, cudaStream_t s);
 void replay_step(double* r, double* q, double* gs, double alpha, double beta, double c, size_t n,

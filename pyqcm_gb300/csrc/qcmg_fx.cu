@@ -368,16 +368,18 @@ void FxVec::alloc(size_t count) {
   n = count;
 }
 
-void fx_from_f64(const double* x, size_t n, FxVec& v, cudaStream_t s, DevBuf<unsigned long long>& tmp) {
+void fx_from_f64(const double* x, size_t n, FxVec& v, cudaStream_t s, DevBuf<unsigned long long>& tmp,
+                 double mx) {
   v.alloc(n);
-  tmp.alloc(1);
-  QCMG_CUDA(cudaMemsetAsync(tmp.p, 0, 8, s));
-  k_absmax_f64<<<grid_ew(n), 256, 0, s>>>(x, n, tmp.p);
-  unsigned long long hb = 0;
-  QCMG_CUDA(cudaMemcpyAsync(&hb, tmp.p, 8, cudaMemcpyDeviceToHost, s));
-  QCMG_CUDA(cudaStreamSynchronize(s));
-  double mx;
-  std::memcpy(&mx, &hb, 8);
+  if (!(mx >= 0.0)) {
+    tmp.alloc(1);
+    QCMG_CUDA(cudaMemsetAsync(tmp.p, 0, 8, s));
+    k_absmax_f64<<<grid_ew(n), 256, 0, s>>>(x, n, tmp.p);
+    unsigned long long hb = 0;
+    QCMG_CUDA(cudaMemcpyAsync(&hb, tmp.p, 8, cudaMemcpyDeviceToHost, s));
+    QCMG_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(&mx, &hb, 8);
+  }
   v.c = 1.0;
   if (mx == 0.0) {
     v.E = 0;
@@ -515,10 +517,10 @@ void fx_check_error(qcmg_hamiltonian* H) {
   if (err) throw Error(QCMG_ERR_CUDA, "a bulk copy into shared memory did not complete in time");
 }
 
-void fx_matvec_f64(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate) {
+void fx_matvec_f64(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate, double absmax) {
   FxTables& T = H->fx;
   cudaStream_t s = H->stream;
-  fx_from_f64(x, H->dim, T.x, s, T.tmp);
+  fx_from_f64(x, H->dim, T.x, s, T.tmp, absmax);
   if (accumulate) {
     fx_from_f64(y, H->dim, T.y, s, T.tmp);
     fx_matvec(H, T.x, T.y, &T.y, 1.0);

@@ -38,8 +38,10 @@ struct FxReducer {
 // Prepares the fixed-point tables; false if the Hamiltonian does not have
 // one hop magnitude per spin (then the FP64 path is used).
 bool fx_prepare(qcmg_hamiltonian* H);
+// (absmax: the largest |x_i| where it is known, else negative and found here
+// with a wait for the stream)
 void fx_from_f64(const double* x, size_t n, FxVec& v, cudaStream_t s,
-                 DevBuf<unsigned long long>& tmp);
+                 DevBuf<unsigned long long>& tmp, double absmax = -1.0);
 void fx_to_f64(const FxVec& v, double* x, cudaStream_t s);
 // With dot set, the product's second pass also computes alpha = <x, y> (for
 // the finished y) and the coefficients of y - alpha x - beta p into
@@ -58,7 +60,8 @@ inline bool fx_for_f64(qcmg_hamiltonian* H) {
   return H->use_fx && H->dim >= ((size_t)1 << 21) && fx_prepare(H);
 }
 // y (+)= H x on FP64 device vectors through the fixed-point product.
-void fx_matvec_f64(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate);
+void fx_matvec_f64(qcmg_hamiltonian* H, const double* x, double* y, bool accumulate,
+                   double absmax = -1.0);
 // y (+)= H x with x on the device and y in page-locked host memory, written
 // through its device-side address yh (zero copy); product_done (optional) is
 // recorded between the product and the pass into y.  With m > 0, the old

@@ -15,8 +15,8 @@
 // is bound by the FP64 pipe of the few SMs it has (most of it the table u of
 // the block's 32 F / elements frequencies): F = 2 or 1 then, a quarter of the
 // work per block. L = 4, 480 poles, 200 frequencies: 79 us with F = 4
-// (16 blocks, tiles of 32 poles), 28 us with F = 1 (63 blocks, tiles of 128). The sums of an element, and their
-// order, are the same for every F.
+// (16 blocks, tiles of 32 poles), 28 us with F = 1 (63 blocks, tiles of 128).
+// The sums of an element, and their order, are the same for every F.
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
 

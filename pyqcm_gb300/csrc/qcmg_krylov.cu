@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <random>
 
@@ -86,7 +87,9 @@ __global__ void __launch_bounds__(kDotThreads, 2) k_dots(VL V, int m, const doub
 // need: the last value is |w|^2, the others its projections c_k, and need
 // says whether a second pass is called for.
 __global__ void __launch_bounds__(1024) k_dots_final(const double* __restrict__ part, int nb, int m,
-                                                     double* __restrict__ out, int* need) {
+                                                     double* __restrict__ out, int* need,
+                                                     const int* __restrict__ only) {
+  if (only && !*only) return;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int k = wp; k < m; k += nw) {
     double s = 0.0;
@@ -107,16 +110,36 @@ __global__ void __launch_bounds__(1024) k_dots_final(const double* __restrict__ 
   }
 }
 
+// Fixed-order block sum; the result is valid in thread 0.
+__device__ __forceinline__ double block_sum_fixed(double v) {
+  __shared__ double ws[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __syncthreads();
+  if (lane == 0) ws[w] = v;
+  __syncthreads();
+  v = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0.0;
+  if (w == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  return v;
+}
+
 // w -= sum_k c_k V_k, c in device memory: eight vectors' loads in flight
-// together per element.
-template <int VEC, class VL>
+// together per element.  STATS: every block also leaves its share of |w|^2
+// and its largest |w_i| (stat[b] and stat[grid + b]).
+template <int VEC, bool STATS, class VL>
 __global__ void __launch_bounds__(256) k_axpys(VL V, int m, const double* __restrict__ c,
                                                double* __restrict__ w, size_t nv,
-                                               const int* __restrict__ need) {
+                                               const int* __restrict__ need,
+                                               double* __restrict__ stat) {
   if (need && !*need) return;
   extern __shared__ double cs[];
   for (int k = threadIdx.x; k < m; k += blockDim.x) cs[k] = c[k];
   __syncthreads();
+  double sq = 0.0, mx = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
        i += (size_t)gridDim.x * blockDim.x) {
     Pack<VEC> s = load_pack<VEC>(w, i);
@@ -136,6 +159,25 @@ __global__ void __launch_bounds__(256) k_axpys(VL V, int m, const double* __rest
       for (int e = 0; e < VEC; ++e) s.e[e] = fma(-cs[k], v.e[e], s.e[e]);
     }
     store_pack<VEC>(w, i, s);
+    if (STATS)
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        sq = fma(s.e[e], s.e[e], sq);
+        mx = fmax(mx, fabs(s.e[e]));
+      }
+  }
+  if (STATS) {
+    __shared__ double bmax[8];
+    sq = block_sum_fixed(sq);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) bmax[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int q = 1; q < 8; ++q) mx = fmax(mx, bmax[q]);
+      stat[blockIdx.x] = sq;
+      stat[gridDim.x + blockIdx.x] = mx;
+    }
   }
 }
 
@@ -178,23 +220,6 @@ __global__ void __launch_bounds__(256) k_scale_sub(double* __restrict__ v, doubl
     v[i] = x;
     for (int k = 0; k < m; ++k) V[k][i] = fma(-cs[k], x, V[k][i]);
   }
-}
-
-// Fixed-order block sum; the result is valid in thread 0.
-__device__ __forceinline__ double block_sum_fixed(double v) {
-  __shared__ double ws[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) ws[w] = v;
-  __syncthreads();
-  v = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0.0;
-  if (w == 0) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  }
-  return v;
 }
 
 // w -= sum_k c_k V_k (the band recurrence), then one partial of w . u per
@@ -326,7 +351,7 @@ struct MultiOps {
         go(std::integral_constant<int, 16>{});
     });
     QCMG_CUDA(cudaGetLastError());
-    k_dots_final<<<1, std::min(1024, 32 * m), 0, s>>>(part.p, nb, m, sums.p, need);
+    k_dots_final<<<1, std::min(1024, 32 * m), 0, s>>>(part.p, nb, m, sums.p, need, only);
     QCMG_CUDA(cudaGetLastError());
     return sums.p;
   }
@@ -346,19 +371,23 @@ struct MultiOps {
     QCMG_CUDA(cudaStreamSynchronize(s));
     std::copy(host, host + m, out.begin());
   }
-  // w -= sum_k c_k V_k with c in device memory
+  // w -= sum_k c_k V_k with c in device memory (stat: see k_axpys; room for
+  // 2 elementwise_grid(n) values)
   void axpys_dev(const std::vector<const double*>& V, const double* c, double* w, size_t n,
-                 cudaStream_t s, const int* only = nullptr) {
+                 cudaStream_t s, const int* only = nullptr, double* stat = nullptr) {
     const int m = (int)V.size();
     if (m == 0 || n == 0) return;
     const bool two = pairs(V, w, n);
     const size_t nv = two ? n / 2 : n;
     with_list(V, s, [&](auto L) {
       using VL = decltype(L);
-      if (two)
-        k_axpys<2, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv, only);
+      auto go = [&](auto kern) {
+        kern<<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv, only, stat);
+      };
+      if (stat)
+        two ? go(k_axpys<2, true, VL>) : go(k_axpys<1, true, VL>);
       else
-        k_axpys<1, VL><<<elementwise_grid(nv), 256, m * sizeof(double), s>>>(L, m, c, w, nv, only);
+        two ? go(k_axpys<2, false, VL>) : go(k_axpys<1, false, VL>);
     });
     QCMG_CUDA(cudaGetLastError());
   }
@@ -367,17 +396,45 @@ struct MultiOps {
   // Kaufman and Stewart, 1976: otherwise one pass leaves w orthogonal to
   // rounding).  The device decides; *again (page-locked) tells the host at
   // its next wait.
+  // |w|^2 and max|w_i| of the result come from the pass that wrote it:
+  // collect() reads them, and alpha, after the stream was waited for.
   DevBuf<int> need;
   std::vector<const double*> with_w;
-  void orthogonalize(const std::vector<const double*>& V, double* w, size_t n, int* again,
-                     cudaStream_t s) {
-    if (V.empty()) return;
-    need.alloc(1);
+  DevBuf<double> stat;      // two lists of stat_n values, then alpha
+  PinnedBuf<double> hstat;  // the same, then need
+  size_t stat_n = 0;
+  void orthogonalize(const std::vector<const double*>& V, double* w, size_t n, cudaStream_t s) {
     with_w = V;
     with_w.push_back(w);
-    axpys_dev(V, dots_dev(with_w, w, n, s, nullptr, need.p), w, n, s);
-    QCMG_CUDA(cudaMemcpyAsync(again, need.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    axpys_dev(V, dots_dev(V, w, n, s, need.p), w, n, s, need.p);
+    axpys_dev(V, dots_dev(with_w, w, n, s, nullptr, need.p), w, n, s, nullptr, stat.p);
+    axpys_dev(V, dots_dev(V, w, n, s, need.p), w, n, s, need.p, stat.p);
+    QCMG_CUDA(cudaMemcpyAsync(hstat.p, stat.p, (2 * stat_n + 1) * 8, cudaMemcpyDeviceToHost, s));
+    QCMG_CUDA(cudaMemcpyAsync(hstat.p + 2 * stat_n + 1, need.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  }
+  // the step's scalars for vectors of n elements; where alpha goes
+  double* stat_init(const std::vector<const double*>& V, const double* w, size_t n) {
+    need.alloc(1);
+    stat_n = elementwise_grid(pairs(V, w, n) ? n / 2 : n);
+    stat.alloc(2 * stat_n + 1);
+    hstat.alloc(2 * stat_n + 2);
+    return stat.p + 2 * stat_n;
+  }
+  struct Scalars {
+    double alpha, norm2, absmax;
+    bool again;
+  };
+  Scalars collect(cudaStream_t s) {
+    QCMG_CUDA(cudaStreamSynchronize(s));
+    double* h = hstat.p;
+    Scalars r{h[2 * stat_n], 0.0, 0.0, false};
+    int twice;
+    std::memcpy(&twice, h + 2 * stat_n + 1, sizeof twice);
+    r.again = twice != 0;
+    for (size_t b = 0; b < stat_n; ++b) r.absmax = std::max(r.absmax, h[stat_n + b]);
+    for (size_t m = stat_n; m > 1; m = (m + 1) / 2)  // pairwise
+      for (size_t b = 0; b < m / 2; ++b) h[b] += h[(m + 1) / 2 + b];
+    r.norm2 = h[0];
+    return r;
   }
   // w -= sum_k c_k V_k, then d = w . u and w -= d u with d left at d_dev:
   // two launches.  False (nothing done) for lists longer than kByValue.
@@ -607,16 +664,21 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
 
   // Fully reorthogonalized Lanczos: the basis is kept in HBM and every new
   // residual is made orthogonal to it (classical Gram-Schmidt, repeated when
-  // one pass is not enough: MultiOps::orthogonalize).  At
+  // one pass is not enough: MultiOps::orthogonalize).  One wait per step: the
+  // local recurrence is two fused launches with alpha left on the device,
+  // |w|^2 and max|w_i| (which the next product's conversion needs) come out
+  // of the projection's last pass; with separate passes and three waits the
+  // 3,312,400-state sector of a 4x4 cluster took 208 ms (193 steps), now 199.  At
   // most `reorth` vectors are kept: when the cap is reached before the Ritz
   // residual converges, the iteration restarts from the current Ritz vector
   // (explicit restart).  The product is the fixed-point one where it applies
   // (the vectors stay FP64).  Device time of the products and of the
   // reorthogonalization is recorded with events (qcmg_lanczos_last_stats).
   const bool fx = fx_for_f64(H);
-  auto product = [&](const double* x, double* y) {
+  // absmax: the largest |x_i| where it is known, else negative
+  auto product = [&](const double* x, double* y, double absmax) {
     if (fx)
-      fx_matvec_f64(H, x, y, false);
+      fx_matvec_f64(H, x, y, false, absmax);
     else
       matvec(H, x, y, false);
   };
@@ -626,8 +688,7 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   const size_t stride = (n + 1) & ~(size_t)1;
   const size_t block = std::max<size_t>(1, std::min<size_t>(keep, ((size_t)512 << 20) / (stride * 8)));
   std::vector<DevVec> blocks;
-  PinnedBuf<int> again;
-  again.alloc(1);
+  MultiOps mops;
   Drain drain2{s};
   std::vector<double*> V;
   auto add_vector = [&] {
@@ -635,7 +696,6 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
     V.push_back(blocks.back().p + (V.size() % block) * stride);
   };
   std::vector<const double*> Vp;
-  MultiOps mops;
   add_vector();
   QCMG_CUDA(cudaMemcpyAsync(V[0], x0_dev, n * 8, cudaMemcpyDeviceToDevice, s));
   double* w = r.p;  // residual
@@ -646,21 +706,29 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
     Vp.assign(1, V[0]);
     res.alpha.clear();
     res.beta.clear();
+    double absmax = -1.0;
+    double* alpha = mops.stat_init(Vp, w, n);
     for (int j = 0;; ++j) {
       ev.record(0, s);
-      product(V[j], w);
+      product(V[j], w, absmax);
       ev.record(1, s);
-      if (j > 0) axpy(w, V[j - 1], -res.beta.back(), n, s);
-      double a = red.dot(V[j], w, n, s);
-      res.alpha.push_back(a);
-      axpy(w, V[j], -a, n, s);
+      // w -= beta v_{j-1}, alpha = <v_j, w>, w -= alpha v_j
+      std::vector<const double*> last;
+      std::vector<double> lastc;
+      if (j > 0) {
+        last.push_back(V[j - 1]);
+        lastc.push_back(res.beta.back());
+      }
+      mops.multiaxpy_orth(last, lastc, w, V[j], n, alpha, s);
       ev.record(2, s);
-      mops.orthogonalize(Vp, w, n, again.p, s);
+      mops.orthogonalize(Vp, w, n, s);
       ev.record(3, s);
-      double b = std::sqrt(red.dot(w, w, n, s));  // synchronizes the stream
+      const MultiOps::Scalars step = mops.collect(s);
+      const double b = std::sqrt(step.norm2);
+      res.alpha.push_back(step.alpha);
       res.product_ms += ev.elapsed(0, 1);
       res.reorth_ms += ev.elapsed(2, 3);
-      res.reorth_bytes += (*again.p ? 2.0 : 1.0) * 16.0 * (double)Vp.size() * (double)n;  // 16 B per stored element per pass
+      res.reorth_bytes += (step.again ? 2.0 : 1.0) * 16.0 * (double)Vp.size() * (double)n;  // 16 B per stored element per pass
       res.beta.push_back(b);
       ++total;
       res.energy = lowest(res.alpha, res.beta, z);
@@ -676,8 +744,8 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
                                          std::to_string(max_iter) + " iterations");
       if ((int)Vp.size() >= keep) break;  // cap reached: restart
       if ((int)V.size() <= j + 1) add_vector();
-      QCMG_CUDA(cudaMemcpyAsync(V[j + 1], w, n * 8, cudaMemcpyDeviceToDevice, s));
-      scale(V[j + 1], 1.0 / b, n, s);
+      scaled_copy(V[j + 1], w, 1.0 / b, n, s);
+      absmax = step.absmax * (1.0 / b);  // rounding is monotone: the copy's largest element
       Vp.push_back(V[j + 1]);
     }
     if (converged) break;
