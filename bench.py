@@ -236,7 +236,7 @@ def run_gpu(args):
     else:
         y = x.clone()
         step = lambda: H.matvec_device(x.data_ptr(), y.data_ptr(), asynchronous=True, accumulate=True)
-        kernels = ["k_matvec_f64"]
+        kernels = ["k_matvec_ell"]
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize()
@@ -272,7 +272,7 @@ def run_gpu(args):
     achieved = bytes_step / (avg_launch_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peak()
 
-    # The FP64 product (k_matvec_f64, any hop values) on the same sector and
+    # The FP64 product (k_matvec_ell, any hop values) on the same sector and
     # vectors: the arithmetic the reference's mult_add performs, timed the
     # same way; the fixed-point line above is the fast path of this product.
     fp64 = None
@@ -296,7 +296,7 @@ def run_gpu(args):
         ms_f = f0.elapsed_time(f1) / nf
         gbs_f = bytes_step / (ms_f * 1e-3) / 1e9
         fp64 = {"value": gbs_f, "unit": UNIT, "ms_per_step": ms_f, "steps": nf,
-                "frac": gbs_f / peak, "kernels": ["k_matvec_f64"], "dtype": "f64"}
+                "frac": gbs_f / peak, "kernels": ["k_matvec_ell"], "dtype": "f64"}
         del yf
 
     # e2e through the public host API (Hamiltonian.mult_add, the reference's
@@ -364,7 +364,7 @@ def run_lanczos(args):
     recurrence (no reorthogonalization), energy only, on the fixed-point
     path: time to solution and the per-iteration bytes (product 24 D + fused
     update/norm 16 D).  --reorth R: full reorthogonalization (classical
-    Gram-Schmidt twice per step) against at most R vectors held in HBM, with
+    Gram-Schmidt, a second pass where needed) against at most R vectors held in HBM, with
     an explicit restart from the Ritz vector at the cap; the products and
     the Gram-Schmidt sweeps are timed apart on the device."""
     import numpy as np
@@ -404,7 +404,7 @@ def run_lanczos(args):
             "reorth_bytes": st["reorth_bytes"], "reorth_gbs": rgbs,
             "reorth_roofline": {"bound": "hbm", "achieved": rgbs, "peak": peak, "unit": "GB/s",
                                 "frac": rgbs / peak, "peak_kind": kind,
-                                "kernels": ["k_multidot", "k_multiaxpy"]},
+                                "kernels": ["k_dots", "k_axpys"]},
             "dtype": "f64 (vectors, Gram-Schmidt); int64 (product)", "data": "synthetic",
             "config": cfg}))
         return
@@ -699,9 +699,8 @@ def run_lanczos_batch(args):
     instances of the 2x2 plaquette + 4 bath orbitals (U ~ U[0,12],
     mu ~ U[0,U], eb ~ U[-3,3], tb ~ U[0,1]), each in its sectors N = 7, 8, 9
     (3,920, 4,900 and 3,920 states), solved by Lanczos to 1e-12: all sectors
-    at once (qcmg_lanczos_batch: each sector's steps replayed from a captured
-    CUDA graph, all sectors side by side) against one sector at a time
-    through the host-driven recurrence (the same FP64 arithmetic); sector
+    at once (qcmg_lanczos_batch: on chip, all sectors side by side) against one
+    sector at a time (the same FP64 arithmetic); sector
     solves per second both ways, and the energies must agree bit for bit."""
     import numpy as np
     import torch
@@ -835,7 +834,7 @@ def main():
                          "the warm-start workload (default 512)")
     ap.add_argument("--seed", type=int, default=0, help="seed of the CDMFT instances")
     ap.add_argument("--chunk", type=int, default=16,
-                    help="lanczos-batch: recurrence steps per captured graph")
+                    help="lanczos-batch: recurrence steps per captured graph (sectors above 16,384 states)")
     ap.add_argument("--groups", type=int, default=1,
                     help="cdmft --batched: lockstep groups driven from their own threads")
     ap.add_argument("--batched", action="store_true",

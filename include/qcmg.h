@@ -199,9 +199,10 @@ int qcmg_lanczos_ground_state(qcmg_hamiltonian* H, const double* x0, unsigned se
 /* Lanczos ground states of n sectors (handles H[0..n-1], one device, no
  * handle twice) at once: the three-term recurrence of
  * qcmg_lanczos_ground_state (no reorthogonalization, FP64 product, seeded
- * start `seed`) with alpha, beta and the step index kept on the device, each
- * sector's steps captured once as a CUDA graph of `chunk` steps (rounded up
- * to even) on a stream of its own and relaunched until the Ritz residual is
+ * start `seed`), sectors of at most 16,384 states on chip (a thread-block
+ * cluster each), larger ones with alpha, beta and the step index kept on the
+ * device and the steps captured once as a CUDA graph of `chunk` steps (rounded
+ * up to even) on a stream of its own, run until the Ritz residual is
  * below tol (tested after every step, as the reference does) or max_iter
  * steps; sectors of any sizes run side by side.  Outputs per sector: E0[i],
  * niter[i] (may be NULL), status[i] (QCMG_OK, QCMG_ERR_NOCONV or

@@ -420,8 +420,7 @@ def run_batched(loops, workers=8, chunk=16, groups=1):
 def _lockstep(loops, workers=8, chunk=16):
     """Runs CDMFT loops in lockstep, one step of every unfinished loop at a
     time, with the device work of each step batched across the loops:
-      1. every loop's impurity ground states in one lanczos_batch call (each
-         sector's Lanczos steps replayed from a captured CUDA graph, all
+      1. every loop's impurity ground states in one lanczos_batch call (all
          sectors side by side);
       2. the Green and host functions of each loop, in host threads (their
          device work overlaps);

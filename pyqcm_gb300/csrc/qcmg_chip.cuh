@@ -63,7 +63,7 @@ __device__ __forceinline__ double warp_total(double v) {
   return v;
 }
 
-// Sum of the tile partials in a fixed order, for every thread of the block:
+// Sum of the tile partials in a fixed order (last tile first), for every thread of the block:
 // slot[0], or with NORM its square root and the root's inverse in slot[0] and
 // slot[1].  The block's warp 0 does it: an FP64 instruction costs the SM 16
 // cycles per warp (a square root and a division by all 16 warps 3 us), so the
@@ -78,7 +78,7 @@ template <bool NORM>
 __device__ __forceinline__ void tile_total(const double* part, int nt, double* slot) {
   if (threadIdx.x < 32) {
     double s = 0.0;
-    for (int t = threadIdx.x; t < nt; t += 32) s += part[t];
+    for (int t = nt - 1 - (int)threadIdx.x; t >= 0; t -= 32) s += part[t];
     s = warp_total(s);
     if (threadIdx.x == 0) {
       if (NORM)

@@ -135,9 +135,6 @@ __device__ __forceinline__ int64_t mul_fix(int64_t a, int64_t m, int s) {
   return shr128_round(mul_s64(a, m), s);
 }
 
-// mul_fix with a multiplier known to be +-2^p when p >= 0 (hop magnitude 1,
-// accumulation factor 1): a shift with the same rounding, bit-identical to
-// mul_fix for |a| < 2^62.  p < 0 falls back to the 128-bit product.
 // round(v / 2^t) with mul_fix's rounding, for |v| < 2^62 (t <= 0: v * 2^-t).
 __device__ __forceinline__ int64_t round_shift(int64_t v, int t) {
   if (t <= 0) return (int64_t)((uint64_t)v << (-t));
@@ -150,26 +147,6 @@ __device__ __forceinline__ int64_t round_shift(int64_t v, int t) {
 // gives 0 as round_shift does.
 __device__ __forceinline__ int64_t rshift_fixed(int64_t v, int t, int64_t r) {
   return t > 0 ? (v + r) >> t : (int64_t)((uint64_t)v << (-t));
-}
-
-__device__ __forceinline__ int64_t mul_fix_p2(int64_t a, int64_t m, int s, int p) {
-  if (p >= 0) return round_shift(m < 0 ? -a : a, s - p);
-  return mul_fix(a, m, s);
-}
-
-// Compile-time forms for kernels specialized on the multipliers: FAST = the
-// multiplier is +-2^p and the diagonal is narrow, so no 128-bit code is
-// generated at all (a runtime test alone leaves both forms in the kernel).
-template <bool FAST>
-__device__ __forceinline__ int64_t scale_term(int64_t a, int64_t m, int s, int p) {
-  if (FAST) return round_shift(m < 0 ? -a : a, s - p);
-  return mul_fix(a, m, s);
-}
-
-template <bool FAST>
-__device__ __forceinline__ int64_t diag_term(int64_t x, int64_t D, int s, int tz) {
-  if (FAST) return round_shift(x * (D >> tz), s - tz);
-  return mul_fix(x, D, s);
 }
 
 // The diagonal term round(x * D / 2^s).  tz >= 0 means D is a multiple of
