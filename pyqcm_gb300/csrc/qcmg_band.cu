@@ -1,18 +1,21 @@
-// Band Lanczos steps on sectors larger than a cluster's shared memory, four
+// Band Lanczos steps on sectors larger than a cluster's shared memory, three
 // launches per step and no host round trip: the step's coefficients (the norm
 // of v_j, the band dots, the closing dot) stay in device memory, and the
 // host reads them p steps at a time for its convergence probe while the next
 // p steps run.
-//   k_band_dots   finishes v_{j+p-1} (the previous step's closing dot), then
+//   k_band_dots   applies the last step's coefficients (v_{j-1} /= z,
+//                 v_{j-1+k} -= c_k v_{j-1}, the closing dot on v_{j+p-1}), then
 //                 |v_j|^2 and <v_{j+i}, v_j>; the last block forms z and c_i
-//   k_band_scale  v_j /= z, v_{j+i} -= c_i v_j
-//   (product)     w = H v_j
-//   k_band_recur  w -= sum_k T(k, j) v_k and <w, v_j>; the last block adds it up
+//   (product)     w = H u, u = z v_j as it stands
+//   k_band_recur  w = w / z - sum_k T(k, j) v_k and <w, v_j>; the last block
+//                 adds it up
 // Each is one pass with the loads of all its vectors in flight together; the
-// FP64 pipe (12 + 12 + 13 FMAs per element at p = 12, and ~37 of the product)
-// is the floor: 86 us per step at 731,808 states. Five launches with a host
-// wait and a host-side sum per step took ~190 us, this ~140 us (600 steps and
-// G: 146 -> 119 ms, 35 of them the host's eigenproblem of the 600 x 600 band).
+// FP64 pipe (12 + 12 + 14 FMAs per element at p = 12, and ~37 of the product)
+// is the floor: 87 us per step at 731,808 states. Five launches with a host
+// wait and a host-side sum per step took ~190 us, four (the scaling and the
+// updates in a pass of their own) ~140 us, these ~136 us (600 steps and
+// G: 146 -> 117 -> 115 ms, 35 of them the host's eigenproblem of the
+// 600 x 600 band).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -52,29 +55,40 @@ __device__ __forceinline__ double sum_partials(const double* part, int nb, int m
   return s;
 }
 
-// V: v_{j+p-1} first, then v_j .. v_{j+p-2} (the vector to finish at a fixed
-// place keeps the packs in registers)
+// V: v_{j+p-1} first, then v_j .. v_{j+p-2} (the vector with the closing dot
+// at a fixed place keeps the packs in registers); u = v_{j-1} (null at j = 0)
+// and prev its row: c_k is the coefficient of v_{j-1+k}, prev[p] the closing
+// dot's.
 template <int MAXM, int VEC>
 __global__ void __launch_bounds__(kDotThreads, 2)
-    k_band_dots(VecList V, int p, double* fin, const double* __restrict__ u,
-                const double* __restrict__ dprev, size_t nv, double* __restrict__ part,
-                unsigned* ticket, double* __restrict__ row, int j, double acc_defl, int* flag) {
+    k_band_dots(MutVecList V, int p, double* u, const double* __restrict__ prev, size_t nv,
+                double* __restrict__ part, unsigned* ticket, double* __restrict__ row, int j,
+                double acc_defl, int* flag) {
   if (*(volatile int*)flag >= 0) return;
+  __shared__ double cs[MAXM + 1];  // of V's vectors, in V's order; then 1/z
+  if (u && threadIdx.x <= p) cs[threadIdx.x] = prev[threadIdx.x == 0 ? p : threadIdx.x == p ? p + 1 : threadIdx.x];
+  __syncthreads();
   double acc[MAXM];
 #pragma unroll
   for (int k = 0; k < MAXM; ++k) acc[k] = 0.0;
-  const double d = fin ? *dprev : 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
        i += (size_t)gridDim.x * blockDim.x) {
     Pack<VEC> v[MAXM];
 #pragma unroll
     for (int k = 0; k < MAXM; ++k)
       if (k < p) v[k] = load_pack<VEC>(V[k], i);
-    if (fin) {
-      const Pack<VEC> y = load_pack<VEC>(u, i);
+    if (u) {
+      Pack<VEC> y = load_pack<VEC>(u, i);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) v[0].e[e] = fma(-d, y.e[e], v[0].e[e]);
-      store_pack<VEC>(fin, i, v[0]);
+      for (int e = 0; e < VEC; ++e) y.e[e] *= cs[p];
+      store_pack<VEC>(u, i, y);
+#pragma unroll
+      for (int k = 0; k < MAXM; ++k)
+        if (k < p) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) v[k].e[e] = fma(-cs[k], y.e[e], v[k].e[e]);
+          store_pack<VEC>(V[k], i, v[k]);
+        }
     }
     Pack<VEC> x = v[0];
     if (p > 1) x = v[1];
@@ -101,43 +115,18 @@ __global__ void __launch_bounds__(kDotThreads, 2)
   }
 }
 
-template <int MAXM, int VEC>
-__global__ void __launch_bounds__(256)
-    k_band_scale(MutVecList V, int p, const double* __restrict__ row, size_t nv, const int* flag) {
-  if (*(volatile const int*)flag >= 0) return;
-  __shared__ double cs[MAXM + 2];
-  if (threadIdx.x < row_len(p)) cs[threadIdx.x] = row[threadIdx.x];
-  __syncthreads();
-  const double iz = cs[p + 1];
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
-       i += (size_t)gridDim.x * blockDim.x) {
-    Pack<VEC> v[MAXM];
-#pragma unroll
-    for (int k = 0; k < MAXM; ++k)
-      if (k < p) v[k] = load_pack<VEC>(V[k], i);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) v[0].e[e] *= iz;
-    store_pack<VEC>(V[0], i, v[0]);
-#pragma unroll
-    for (int k = 1; k < MAXM; ++k)
-      if (k < p) {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) v[k].e[e] = fma(-cs[k], v[0].e[e], v[k].e[e]);
-        store_pack<VEC>(V[k], i, v[k]);
-      }
-  }
-}
-
-// V: the m = min(p, j) vectors v_{j-m} .. v_{j-1}
+// V: the m = min(p, j) vectors v_{j-m} .. v_{j-1}; u = z v_j, w = H u
 template <int MAXM, int VEC>
 __global__ void __launch_bounds__(kDotThreads, 2)
     k_band_recur(VecList V, int m, int p, double* __restrict__ w, const double* __restrict__ u,
                  size_t nv, double* __restrict__ part, unsigned* ticket, double* __restrict__ row,
                  const int* flag) {
   if (*(volatile const int*)flag >= 0) return;
-  __shared__ double cs[MAXM];
+  __shared__ double cs[MAXM + 1];
   if (threadIdx.x < m) cs[threadIdx.x] = row[p - m + threadIdx.x];
+  if (threadIdx.x == 0) cs[MAXM] = row[p + 1];
   __syncthreads();
+  const double iz = cs[MAXM];
   double acc[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -146,7 +135,12 @@ __global__ void __launch_bounds__(kDotThreads, 2)
     for (int k = 0; k < MAXM; ++k)
       if (k < m) v[k] = load_pack<VEC>(V[k], i);
     Pack<VEC> s = load_pack<VEC>(w, i);
-    const Pack<VEC> y = load_pack<VEC>(u, i);
+    Pack<VEC> y = load_pack<VEC>(u, i);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      s.e[e] *= iz;
+      y.e[e] *= iz;
+    }
 #pragma unroll
     for (int k = 0; k < MAXM; ++k)
       if (k < m)
@@ -226,7 +220,6 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   const size_t nv = two ? n / 2 : n;
   const unsigned gd = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
   const unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 3 * 152));
-  const unsigned ge = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + 255) / 256, 152 * 8));
   PoolBuf<double> rows, proj, part;
   PinnedBuf<double> landed;  // p steps' rows, the flag, the projections; twice
   PoolBuf<int> flags;  // the deflated step, then the block counter
@@ -243,26 +236,21 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   auto at = [&](int k) { return ring[k % R]; };
   auto step = [&](int j) {
     double* row = rows.p + (size_t)j * rl;
-    VecList L, B;
-    MutVecList S;
-    for (int k = 0; k < p; ++k) {
-      S.v[k] = at(j + k);
-      L.v[k] = at(k ? j + k - 1 : j + p - 1);
-    }
+    VecList B;
+    MutVecList L;
+    for (int k = 0; k < p; ++k) L.v[k] = at(k ? j + k - 1 : j + p - 1);
     const int m = std::min(p, j);
     for (int k = 0; k < m; ++k) B.v[k] = at(j - m + k);
-    double* fin = j > 0 ? at(j + p - 1) : nullptr;
-    const double* u = j > 0 ? at(j - 1) : nullptr;
-    const double* dprev = j > 0 ? row - rl + p : nullptr;
+    double* u = j > 0 ? at(j - 1) : nullptr;
+    const double* prev = j > 0 ? row - rl : nullptr;
     double *vj = at(j), *w = at(j + p);
     with_size(p, [&](auto size) {
       constexpr int MX = decltype(size)::value;
       auto go = [&](auto vec) {
         constexpr int VC = decltype(vec)::value;
-        k_band_dots<MX, VC><<<gd, kDotThreads, 0, s>>>(L, p, fin, u, dprev, nv, part.p, ticket, row,
-                                                       j, acc_defl, flag);
+        k_band_dots<MX, VC><<<gd, kDotThreads, 0, s>>>(L, p, u, prev, nv, part.p, ticket, row, j,
+                                                       acc_defl, flag);
         if (j < p) k_band_project<<<p, 256, 0, s>>>(phi, n, vj, proj.p + (size_t)j * p);
-        k_band_scale<MX, VC><<<ge, 256, 0, s>>>(S, p, row, nv, flag);
         matvec(H, vj, w, false, flag);
         k_band_recur<MX, VC><<<gr, kDotThreads, 0, s>>>(B, m, p, w, vj, nv, part.p, ticket, row, flag);
       };
