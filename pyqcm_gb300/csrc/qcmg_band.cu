@@ -14,7 +14,7 @@
 // is the floor: 87 us per step at 731,808 states. Five launches with a host
 // wait and a host-side sum per step took ~190 us, four (the scaling and the
 // updates in a pass of their own) ~140 us, these ~136 us (600 steps and
-// G: 146 -> 117 -> 115 ms, 35 of them the host's eigenproblem of the
+// G: 146 -> 117 -> 107 ms, 35 of them the host's eigenproblem of the
 // 600 x 600 band).
 #include <algorithm>
 #include <cmath>
@@ -158,23 +158,19 @@ __global__ void __launch_bounds__(kDotThreads, 2)
   }
 }
 
-// <phi_k, v_j> of an unnormalized v_j for k < p (the first p steps only).
+// <phi_k, v_j> of an unnormalized v_j for k < p (the first p steps only):
+// block (k, b)'s share, which the host adds up.  With a block per k, 731,808
+// states took 677 us a step, 27 us this way.
+constexpr int kProjBlocks = 32;
 __global__ void __launch_bounds__(256) k_band_project(const double* __restrict__ phi, size_t n,
                                                       const double* __restrict__ v,
                                                       double* __restrict__ out) {
   const double* f = phi + (size_t)blockIdx.x * n;
-  double s = 0.0;
-  for (size_t i = threadIdx.x; i < n; i += 256) s = fma(f[i], v[i], s);
-  __shared__ double red[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += red[q];
-    out[blockIdx.x] = t;
-  }
+  double acc[1] = {0.0};
+#pragma unroll 4
+  for (size_t i = blockIdx.y * 256u + threadIdx.x; i < n; i += 256u * kProjBlocks)
+    acc[0] = fma(f[i], v[i], acc[0]);
+  block_sums<1>(acc, 1, out + blockIdx.x * kProjBlocks + blockIdx.y);
 }
 
 namespace {
@@ -221,10 +217,10 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   const unsigned gd = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
   const unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 3 * 152));
   PoolBuf<double> rows, proj, part;
-  PinnedBuf<double> landed;  // p steps' rows, the flag, the projections; twice
+  PinnedBuf<double> landed;  // p steps' rows and the flag, twice; the projections
   PoolBuf<int> flags;  // the deflated step, then the block counter
   rows.alloc((size_t)(M0 + 1) * rl);
-  proj.alloc((size_t)p * p);
+  proj.alloc((size_t)p * p * kProjBlocks);
   part.alloc((size_t)std::max(gd * (unsigned)p, gr));
   flags.alloc(2);
   const int init[2] = {-1, 0};
@@ -250,7 +246,8 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
         constexpr int VC = decltype(vec)::value;
         k_band_dots<MX, VC><<<gd, kDotThreads, 0, s>>>(L, p, u, prev, nv, part.p, ticket, row, j,
                                                        acc_defl, flag);
-        if (j < p) k_band_project<<<p, 256, 0, s>>>(phi, n, vj, proj.p + (size_t)j * p);
+        if (j < p)
+          k_band_project<<<dim3(p, kProjBlocks), 256, 0, s>>>(phi, n, vj, proj.p + (size_t)j * p * kProjBlocks);
         matvec(H, vj, w, false, flag);
         k_band_recur<MX, VC><<<gr, kDotThreads, 0, s>>>(B, m, p, w, vj, nv, part.p, ticket, row, flag);
       };
@@ -261,8 +258,8 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
     });
     QCMG_CUDA(cudaGetLastError());
   };
-  const size_t slot = (size_t)p * rl + 1 + (size_t)p * p;
-  landed.alloc(2 * slot);
+  const size_t slot = (size_t)p * rl + 1, pp = (size_t)p * p * kProjBlocks;
+  landed.alloc(2 * slot + pp);
   Wait wait(s);
   // p steps at a time, their rows and the flag copied back
   auto queue = [&](int c) {
@@ -273,7 +270,7 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
     QCMG_CUDA(cudaMemcpyAsync(h, rows.p + (size_t)j0 * rl, (size_t)(j1 - j0) * rl * 8, cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaMemcpyAsync(h + (size_t)p * rl, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (c == 0)
-      QCMG_CUDA(cudaMemcpyAsync(h + (size_t)p * rl + 1, proj.p, (size_t)p * p * 8, cudaMemcpyDeviceToHost, s));
+      QCMG_CUDA(cudaMemcpyAsync(landed.p + 2 * slot, proj.p, pp * 8, cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaEventRecord(wait.e[c & 1], s));
   };
   auto T = [&](int r, int c) -> double& { return t[(size_t)r + (size_t)M0 * c]; };
@@ -296,8 +293,13 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
       for (int k = std::max(0, j - p); k < j; ++k) T(k, j) = T(j, k);
       T(j, j) = row[p];
       if (j < p)
-        for (int k = 0; k < p; ++k)
-          P[k + (size_t)p * j] = h[(size_t)p * rl + 1 + (size_t)j * p + k] * row[p + 1];
+        for (int k = 0; k < p; ++k) {
+          double part[kProjBlocks];
+          std::memcpy(part, landed.p + 2 * slot + ((size_t)j * p + k) * kProjBlocks, sizeof part);
+          for (int w = kProjBlocks / 2; w > 0; w /= 2)  // pairwise
+            for (int b = 0; b < w; ++b) part[b] += part[b + w];
+          P[k + (size_t)p * j] = part[0] * row[p + 1];
+        }
       if (j >= 4 * p && j % p == 0) {
         const bool warm = run.ev_old < 1e12;
         const double width = std::isfinite(run.last_change) && warm
