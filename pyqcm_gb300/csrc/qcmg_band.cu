@@ -13,8 +13,8 @@
 // FP64 pipe (12 + 12 + 14 FMAs per element at p = 12, and ~37 of the product)
 // is the floor: 87 us per step at 731,808 states. Five launches with a host
 // wait and a host-side sum per step took ~190 us, four (the scaling and the
-// updates in a pass of their own) ~140 us, these ~136 us (600 steps and
-// G: 146 -> 117 -> 107 ms, 35 of them the host's eigenproblem of the
+// updates in a pass of their own) ~140 us, these ~115 us (600 steps and
+// G: 146 -> 117 -> 103 ms, 35 of them the host's eigenproblem of the
 // 600 x 600 band).
 #include <algorithm>
 #include <cmath>
@@ -214,14 +214,15 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   for (double* r : ring) low |= (uintptr_t)r;
   const bool two = (n & 1u) == 0 && (low & 15u) == 0;
   const size_t nv = two ? n / 2 : n;
-  const unsigned gd = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
-  const unsigned gr = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 3 * 152));
+  // the two blocks per SM that are resident (registers): one round of equal
+  // shares; three took the recurrence 1.5 rounds (green run 106.8 ms, 102.5)
+  const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
   PoolBuf<double> rows, proj, part;
   PinnedBuf<double> landed;  // p steps' rows and the flag, twice; the projections
   PoolBuf<int> flags;  // the deflated step, then the block counter
   rows.alloc((size_t)(M0 + 1) * rl);
   proj.alloc((size_t)p * p * kProjBlocks);
-  part.alloc((size_t)std::max(gd * (unsigned)p, gr));
+  part.alloc((size_t)grid * p);
   flags.alloc(2);
   const int init[2] = {-1, 0};
   QCMG_CUDA(cudaMemcpyAsync(flags.p, init, sizeof init, cudaMemcpyHostToDevice, s));
@@ -244,12 +245,12 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
       constexpr int MX = decltype(size)::value;
       auto go = [&](auto vec) {
         constexpr int VC = decltype(vec)::value;
-        k_band_dots<MX, VC><<<gd, kDotThreads, 0, s>>>(L, p, u, prev, nv, part.p, ticket, row, j,
+        k_band_dots<MX, VC><<<grid, kDotThreads, 0, s>>>(L, p, u, prev, nv, part.p, ticket, row, j,
                                                        acc_defl, flag);
         if (j < p)
           k_band_project<<<dim3(p, kProjBlocks), 256, 0, s>>>(phi, n, vj, proj.p + (size_t)j * p * kProjBlocks);
         matvec(H, vj, w, false, flag);
-        k_band_recur<MX, VC><<<gr, kDotThreads, 0, s>>>(B, m, p, w, vj, nv, part.p, ticket, row, flag);
+        k_band_recur<MX, VC><<<grid, kDotThreads, 0, s>>>(B, m, p, w, vj, nv, part.p, ticket, row, flag);
       };
       if (two)
         go(std::integral_constant<int, 2>{});
