@@ -139,7 +139,8 @@ __global__ void k_fx_to_host(const int64_t* __restrict__ q, double* __restrict__
 // last adds the partials and writes the step's scalars straight into the
 // host's page-locked copy, seq after everything else: the host polls it and
 // queues the next product while this kernel retires.
-__global__ void __launch_bounds__(256, 4) k_fx_update(int64_t* __restrict__ w,
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) k_fx_update(int64_t* __restrict__ w,
                                                    const int64_t* __restrict__ v,
                                                    const int64_t* __restrict__ p, size_t n,
                                                    FxStep* __restrict__ st,
@@ -399,7 +400,7 @@ void fx_to_f64(const FxVec& v, double* x, cudaStream_t s) {
 }
 
 void FxReducer::init(int sms, cudaStream_t s) {
-  update_blocks = 4u * (unsigned)sms;
+  update_blocks = 32u * (unsigned)sms;
   part.alloc(std::max(update_blocks, product_dot_partials(sms)));
   step.alloc(1);
   QCMG_CUDA(cudaMemsetAsync(step.p, 0, sizeof(FxStep), s));
@@ -561,10 +562,20 @@ void fx_matvec_to_host(qcmg_hamiltonian* H, const double* x, double* yh, bool ac
 // left in red.step.
 static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec* p, FxReducer& red) {
   const size_t n = w.n;
-  // all blocks resident, four per SM
-  const unsigned g = (unsigned)std::min<size_t>(red.update_blocks, std::max<size_t>(1, (n / 2 + 255) / 256));
-  k_fx_update<<<g, 256, 0, H->stream>>>(w.buf.p, v.buf.p, p ? p->buf.p : nullptr, n, red.step.p,
-                                        red.part.p, H->fx.err.p, red.host.p, ++red.seq);
+  // Up to one pair of elements per thread of the large grid, the latency of
+  // the few rounds counts: four resident blocks per SM (64 registers), one
+  // round (853,776 states: 11.4 ms a solve, 13.1 ms with the other form). Above,
+  // HBM: three blocks resident and 32 per SM launched, for an even last
+  // round (165,636,900 states: 3.92 ms a step, 4.10 ms with the small form).
+  const size_t blocks = std::max<size_t>(1, (n / 2 + 255) / 256);
+  auto go = [&](auto kern, unsigned g) {
+    kern<<<g, 256, 0, H->stream>>>(w.buf.p, v.buf.p, p ? p->buf.p : nullptr, n, red.step.p, red.part.p,
+                                   H->fx.err.p, red.host.p, ++red.seq);
+  };
+  if (blocks <= red.update_blocks)
+    go(k_fx_update<4>, (unsigned)std::min<size_t>(blocks, red.update_blocks / 8));
+  else
+    go(k_fx_update<3>, red.update_blocks);
   QCMG_CUDA(cudaGetLastError());
 }
 
@@ -612,14 +623,14 @@ __global__ void __launch_bounds__(256) k_fx_combine(const FxTerm* __restrict__ t
 }
 
 // Device memory for the Lanczos vectors of one solve: slots of n elements,
-// 16-byte aligned, allocated many at a time.  get() returns null when the
+// 256-byte aligned, allocated many at a time.  get() returns null when the
 // next allocation would take more than a quarter of the memory that was free
 // at the start, or fails.
 struct FxSlots {
   std::deque<DevBuf<int64_t>> blocks;
   size_t stride = 0, left = 0, budget = 0;
   int64_t* next = nullptr;
-  explicit FxSlots(size_t n) : stride((n + 1) & ~(size_t)1) {}
+  explicit FxSlots(size_t n) : stride((n + 31) & ~(size_t)31) {}
   void measure() {
     size_t fr = 0, total = 0;
     QCMG_CUDA(cudaMemGetInfo(&fr, &total));

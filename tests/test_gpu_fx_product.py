@@ -1,7 +1,7 @@
 """The fixed-point product on its own vectors (qcmg_matvec_fx) over the forms
 of its passes, on sectors whose FP64-vector products take the FP64 kernel:
-slabs staged by threads (du < 64), two small slabs per block (du <= 1006), a
-slab and its negative (above), two large slabs, one per block; even and odd half bases, unequal spins; narrow
+slabs staged by threads (du < 64), two small slabs per block (du <= 1006), two
+large slabs, one per block; even and odd half bases, unequal spins; narrow
 (integer) and wide diagonals; bands of pass D down to one sweep."""
 import numpy as np
 import pytest
@@ -73,3 +73,28 @@ def test_small_host_products_are_staged(n):
         H.mult_add(x, y)
         assert np.max(np.abs(y - y0 - ref)) <= 1e-13 * np.max(np.abs(ref))
         assert np.max(np.abs(H.matvec(x) - ref)) <= 1e-13 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("shape,nup,ndn", [((10, 1), 5, 5), ((15, 1), 3, 2)])
+@pytest.mark.parametrize("mu", [1.0, 4.0, 1e3, 1e6, -1e6])
+def test_fixed_point_lanczos_with_a_shifted_diagonal(shape, nup, ndn, mu):
+    """The update's usual shifts and, as a large multiple of the identity makes
+    alpha outweigh beta, its general form; an even and an odd number of states."""
+    import models
+    import pyqcm_gb300 as pg
+    ns, nb, ops = models.hubbard_cluster(*shape)
+    E = []
+    for value in (0.0, mu):
+        params = {"t": 1.0, "U": 8.0, "mu": value}
+        m = pg.ClusterModel(ns, nb)
+        for name, (typ, els) in ops.items():
+            if name in params:
+                m.new_operator(name, typ, els)
+        H = pg.Hamiltonian(m, params, f"R0:N{nup + ndn}:S{nup - ndn}")
+        assert H.dim > 16384 and H.fx_available()
+        E.append(H.lanczos(tol=1e-5, want_psi=False)[0])
+    shift = mu * (nup + ndn)
+    # each run: the residual squared over the gap (> 1e-2); and the format's
+    # rounding of |H| times the ~100 steps
+    bound = 2e-8 + 100 * 2.0 ** -53 * abs(shift)
+    assert abs(E[0] - shift - E[1]) < bound
