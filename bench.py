@@ -515,7 +515,7 @@ def run_sef(args):
     L = 12
     points = 128 * 128 * len(w) * len(blocks)
     flops = points * (8 * L ** 3 + 8 * L ** 3 / 3)  # per-point count of the reference's integrand
-    lu = points * 8 * L ** 3 / 3  # executed FP64 flops of one complex LU per point
+    lu = points * 8 * L ** 3 / 3  # FP64 flops of one complex LU per point (K and -K share one here)
     peak = _fp64_peak()
     line = {"metric": "vca_sef_s_per_M_value", "value": t_total, "unit": "s",
             "higher_is_better": False, "omega": omega, "sef_grid_s": t_grid,
