@@ -234,10 +234,11 @@ __global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 
     // the next round's slabs into L2 meanwhile: its copies then wait for L2
     // only (with the narrow shifts: 2,556 -> 2,526 us for the 4x4 sector,
     // 1,043 -> 982 us for its 12-electron one; asking for y too fills L2 and
-    // costs 140 us)
+    // costs 140 us). Not with an accumulated input, whose reads compete: 200
+    // products y += H x back to back 2,575 us each with it, 2,540 without
     if (tid < NS) {
       const uint32_t a = a0 + (uint32_t)NS * G + tid * G;
-      if (a < dd) prefetch_slab(A.x + (size_t)a * du, du);
+      if (a < dd && !A.yin) prefetch_slab(A.x + (size_t)a * du, du);
     }
     __syncthreads();
     const uint32_t vbase = smem_u32(view);
