@@ -34,6 +34,7 @@
 #include <thread>
 
 #include "qcmg_chip.cuh"
+#include "qcmg_memo.h"
 #include "qcmg_pool.h"
 #include "qcmg_tridiag.h"
 
@@ -356,8 +357,10 @@ void chip_lanczos(int n, qcmg_hamiltonian* const* Hs, const double* const* x0, d
   // For one sector alone sixteen, where the chip allows it.
   int C = 8;
   if (n == 1) {
-    static const bool wide = clusters_run(k_chip_lanczos, 16, chip_smem(kChipStates, 16));
-    if (wide) C = 16;
+    // (the kernel's consent to more than eight holds for one device's context)
+    static DeviceMemo<bool> wide;
+    if (wide.get(dev, context_id(), [] { return clusters_run(k_chip_lanczos, 16, chip_smem(kChipStates, 16)); }))
+      C = 16;
   }
   while (C > 1 && n * C > 2 * sms && chip_smem(most, C / 2) <= (size_t)optin - 64) C /= 2;
   size_t fr = 0, total = 0;

@@ -35,8 +35,8 @@ int device() {
   return d;
 }
 
-// Number of the current context: another one after a device reset, when the
-// addresses of the old one mean nothing (or somebody else's memory).
+}  // namespace
+
 unsigned long long context_id() {
   typedef CUresult (*Fn)(CUcontext, unsigned long long*);
   static Fn fn = [] {
@@ -51,6 +51,8 @@ unsigned long long context_id() {
   if (!fn || fn(nullptr, &id) != 0) return 0;
   return id;
 }
+
+namespace {
 
 // The device's lists, under g_mu; emptied when they are of another context.
 Lists& lists_of(int dev, unsigned long long ctx) {

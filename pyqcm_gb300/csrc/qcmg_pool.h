@@ -22,6 +22,10 @@ namespace qcmg {
 constexpr size_t kPoolBytes = (size_t)512 << 20;
 constexpr size_t kPinnedBytes = (size_t)8 << 20;
 
+// Number of the current context: another one after a device reset, when the
+// addresses of the old one mean nothing (or somebody else's memory).
+unsigned long long context_id();
+
 // pool_get, pool_put: qcmg_internal.h; on the current device
 void* pinned_get(size_t bytes, size_t* got);
 void pinned_put(void* p, size_t got);
