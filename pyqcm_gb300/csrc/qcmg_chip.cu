@@ -29,13 +29,13 @@
 // than a quarter of the free memory, recomputed by a second run.
 #include <algorithm>
 #include <cmath>
-#include <exception>
 #include <memory>
 #include <thread>
 
 #include "qcmg_chip.cuh"
 #include "qcmg_memo.h"
 #include "qcmg_pool.h"
+#include "qcmg_shares.h"
 #include "qcmg_tridiag.h"
 
 namespace qcmg {
@@ -381,20 +381,10 @@ void chip_lanczos(int n, qcmg_hamiltonian* const* Hs, const double* const* x0, d
     chip_group(*groups[0], Hs, x0, tol, max_iter, keep, psi, res);
     return;
   }
-  std::vector<std::exception_ptr> err(threads);
-  std::vector<std::thread> pool;
-  for (int t = 0; t < threads; ++t)
-    pool.emplace_back([&, t] {
-      try {
-        QCMG_CUDA(cudaSetDevice(dev));
-        chip_group(*groups[t], Hs, x0, tol, max_iter, keep, psi, res);
-      } catch (...) {
-        err[t] = std::current_exception();
-      }
-    });
-  for (auto& th : pool) th.join();
-  for (auto& e : err)
-    if (e) std::rethrow_exception(e);
+  run_shares(threads, [&](int t) {
+    QCMG_CUDA(cudaSetDevice(dev));
+    chip_group(*groups[t], Hs, x0, tol, max_iter, keep, psi, res);
+  });
 }
 
 }  // namespace qcmg
