@@ -27,6 +27,7 @@
 #include "qcmg_chip.h"
 #include "qcmg_internal.h"
 #include "qcmg_krylov.h"
+#include "qcmg_pool.h"
 #include "qcmg_tridiag.h"
 
 namespace qcmg {
@@ -145,7 +146,7 @@ static void lanczos_batch_graphs(int nsec, qcmg_hamiltonian* const* Hs, unsigned
   // beta (the coefficients from the last examined step on)
   const size_t slot = 1 + 2 * (size_t)chunk;  // doubles: the two ints fit in the first
   double* pinned = nullptr;
-  QCMG_CUDA(cudaMallocHost(&pinned, (size_t)nsec * slot * sizeof(double)));
+  QCMG_CUDA(pinned_alloc(reinterpret_cast<void**>(&pinned), (size_t)nsec * slot * sizeof(double)));
   struct FreePinned {
     double* p;
     ~FreePinned() {

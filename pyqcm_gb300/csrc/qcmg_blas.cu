@@ -4,6 +4,7 @@
 // a Lanczos run are bitwise reproducible run to run (replaces the BLAS-1 calls
 // of src_util/vector_num.cpp:37-106 used by src_ed/Hamiltonian/Lanczos.hpp).
 #include "qcmg_blas.h"
+#include "qcmg_pool.h"
 
 namespace qcmg {
 
@@ -211,7 +212,7 @@ static unsigned red_grid(size_t n) {
 void Reducer::init() {
   part.alloc(kRedBlocks);
   out.alloc(8);
-  QCMG_CUDA(cudaMallocHost(&host, 8 * sizeof(double)));
+  QCMG_CUDA(pinned_alloc(reinterpret_cast<void**>(&host), 8 * sizeof(double)));
 }
 
 Reducer::~Reducer() {

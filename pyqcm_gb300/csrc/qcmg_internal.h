@@ -40,6 +40,8 @@ void clear_error();
 // The memory pool (qcmg_pool.h).
 void* pool_get(size_t bytes, size_t* got);
 void pool_put(void* p, size_t got);
+// cudaMalloc; out of memory, once more after the pool gave back what it keeps.
+cudaError_t device_alloc(void** p, size_t bytes);
 
 // Owning device buffer.
 template <class T>
@@ -80,7 +82,7 @@ struct DevBuf {
     if (pooled)
       p = static_cast<T*>(pool_get(bytes, &got));
     else
-      QCMG_CUDA(cudaMalloc(&p, bytes));
+      QCMG_CUDA(device_alloc(reinterpret_cast<void**>(&p), bytes));
     n = count;
   }
   void upload(const T* h, size_t count, cudaStream_t s) {

@@ -365,7 +365,7 @@ struct MultiOps {
       if (host) cudaFreeHost(host);
       host = nullptr;
       host_n = std::max<size_t>(m, 64);
-      QCMG_CUDA(cudaMallocHost(&host, host_n * sizeof(double)));
+      QCMG_CUDA(pinned_alloc(reinterpret_cast<void**>(&host), host_n * sizeof(double)));
     }
     QCMG_CUDA(cudaMemcpyAsync(host, d, m * sizeof(double), cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaStreamSynchronize(s));

@@ -84,7 +84,27 @@ void* take(std::multimap<size_t, void*>& m, size_t& held, size_t want, size_t* g
   return p;
 }
 
+// Runs an allocation; when there is no memory, once more with the pool empty.
+template <class Alloc>
+cudaError_t alloc_or_trim(Alloc&& alloc) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // not the next call's error
+    pool_trim();
+    e = alloc();
+  }
+  return e;
+}
+
 }  // namespace
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  return alloc_or_trim([&] { return cudaMalloc(p, bytes); });
+}
+
+cudaError_t pinned_alloc(void** p, size_t bytes) {
+  return alloc_or_trim([&] { return cudaMallocHost(p, bytes); });
+}
 
 void pool_trim() {
   std::vector<void*> d, h;
@@ -113,12 +133,7 @@ void* pool_get(size_t bytes, size_t* got) {
     if (void* p = take(l.dev, l.dev_bytes, want, got)) return p;
   }
   void* p = nullptr;
-  if (cudaMalloc(&p, want) == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    pool_trim();
-    QCMG_CUDA(cudaMalloc(&p, want));
-  }
-  if (!p) QCMG_CUDA(cudaGetLastError());
+  QCMG_CUDA(device_alloc(&p, want));
   *got = want;
   return p;
 }
@@ -155,7 +170,7 @@ void* pinned_get(size_t bytes, size_t* got) {
     if (void* p = take(l.pinned, l.pinned_bytes, want, got)) return p;
   }
   void* p = nullptr;
-  QCMG_CUDA(cudaMallocHost(&p, want));
+  QCMG_CUDA(pinned_alloc(&p, want));
   *got = want;
   return p;
 }

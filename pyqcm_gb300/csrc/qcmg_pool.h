@@ -8,8 +8,9 @@
 // memory is pending on any stream (declare a guard that waits after them).
 // The lists hold at most kPoolBytes per device (kPinnedBytes of page-locked
 // memory); blocks beyond that, and blocks above a quarter of it, go back to
-// the driver at once, and all of them when an allocation fails. After a
-// device reset (another context) the lists are forgotten. Safe for any number
+// the driver at once, and all of them when an allocation of the library finds
+// no memory, which is then tried once more. After a device reset (another
+// context) the lists are forgotten. Safe for any number
 // of threads and streams.
 #pragma once
 
@@ -29,6 +30,7 @@ unsigned long long context_id();
 // pool_get, pool_put: qcmg_internal.h; on the current device
 void* pinned_get(size_t bytes, size_t* got);
 void pinned_put(void* p, size_t got);
+cudaError_t pinned_alloc(void** p, size_t bytes);  // cudaMallocHost, as device_alloc
 void pool_trim();                            // the current device's lists back to the driver
 
 template <class T>
