@@ -197,7 +197,7 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
   lane.open();
   cudaStream_t s = lane.s;
   std::vector<TridiagLowest> lowest(n);
-  std::vector<char> running(n, 1);
+  std::vector<size_t> zat(n, 0);  // replay: offsets of the sectors' coefficients
   auto chunk_vectors = [&](int c, int k) -> double* {
     if (keep && c * kChunk >= kKeepSteps) {  // a long run: it will be repeated instead
       QCMG_CUDA(cudaStreamSynchronize(s));
@@ -235,7 +235,7 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
       S.steps = kChunk;
       S.first = c == 0;
       if (replay) {
-        S.z = zbuf.p + (size_t)k * (max_iter + 2) + (size_t)c * kChunk;
+        S.z = zbuf.p + zat[k] + (size_t)c * kChunk;
         S.gs = gsbuf.p + at[k];
         S.steps = std::min(kChunk, res[g.ids[k]].niter - c * kChunk);
       }
@@ -288,9 +288,10 @@ static void chip_group(ChipGroup& g, qcmg_hamiltonian* const* Hs, const double* 
   std::vector<double> hz;
   std::vector<ChipSum> hsum;
   if (!keep) {  // a second run, accumulating z_j v_j
-    const int ld = max_iter + 2;
-    hz.assign((size_t)n * ld, 0.0);
-    for (int k : want) std::copy(res[g.ids[k]].z.begin(), res[g.ids[k]].z.end(), hz.begin() + (size_t)k * ld);
+    for (int k : want) {
+      zat[k] = hz.size();
+      hz.insert(hz.end(), res[g.ids[k]].z.begin(), res[g.ids[k]].z.end());
+    }
     zbuf.upload(hz.data(), hz.size(), s);
     QCMG_CUDA(cudaMemsetAsync(gsbuf.p, 0, total * 8, s));
     start();
@@ -366,7 +367,7 @@ void chip_lanczos(int n, qcmg_hamiltonian* const* Hs, const double* const* x0, d
   size_t fr = 0, total = 0;
   const bool want = psi != nullptr;
   if (want) QCMG_CUDA(cudaMemGetInfo(&fr, &total));
-  const bool keep = want && states * 8 * (size_t)std::min(max_iter + 2 * kChunk, kKeepSteps) <= fr / 4;
+  const bool keep = want && states * 8 * std::min<size_t>((size_t)max_iter + 2 * kChunk, kKeepSteps) <= fr / 4;
   // the test after every step is host work: share it out
   const int threads = std::max(1, std::min({8, n, (int)std::thread::hardware_concurrency() / 2}));
   std::vector<std::unique_ptr<ChipGroup>> groups;
