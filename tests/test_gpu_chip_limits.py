@@ -2,6 +2,7 @@
 limits of their ranges: the largest step counts and sectors around a tile of
 32 states."""
 import numpy as np
+import pytest
 
 pytestmark = pytest.mark.gpu
 
