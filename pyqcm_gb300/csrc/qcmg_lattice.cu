@@ -641,20 +641,29 @@ double Lattice::sef_grid(int nw, const double* w, const double* wt, int nkx, int
     QCMG_CUDA(cudaGetLastError());
   };
   if (L <= kMaxPointL) {
+    // as many frequencies at a time as leave 128 MB of warps' sums (a launch
+    // then stays within a grid's 2^31 blocks)
     const int np = grid_points(nkx, nky, nkz, 0.0, s), nkb = (np + 31) / 32;
-    ws_part.alloc((size_t)nw * nkb);
+    const int fpl = (int)std::max<size_t>(1, std::min<size_t>(nw, ((size_t)16 << 20) / nkb));
+    ws_part.alloc((size_t)fpl * nkb);
     const int step = points_per_launch(nnz, np);
-    for (int h0 = 0; h0 < np; h0 += step) {
-      const int n = std::min(step, np - h0);
-      point_tables(h0, n, nullptr, nkx, nky, nkz, 0.0, false, s);
-      LuArgs A = lu_args(*this, nw);
-      A.nk = n;
-      A.wgt = wgt.p + h0;
-      A.part = ws_part.p + h0 / 32;
-      A.part_ld = nkb;
-      launch_sef_points(L, A, s);
+    for (int i0 = 0; i0 < nw; i0 += fpl) {
+      const int nf = std::min(fpl, nw - i0);
+      for (int h0 = 0; h0 < np; h0 += step) {
+        const int n = std::min(step, np - h0);
+        if (step < np || i0 == 0) point_tables(h0, n, nullptr, nkx, nky, nkz, 0.0, false, s);
+        LuArgs A = lu_args(*this, nf);
+        A.base += (size_t)i0 * L * L;
+        A.det2 += i0;
+        A.dexp += i0;
+        A.nk = n;
+        A.wgt = wgt.p + h0;
+        A.part = ws_part.p + h0 / 32;
+        A.part_ld = nkb;
+        launch_sef_points(L, A, s);
+      }
+      sums(ws_part.p, nkb, i0, nf);
     }
-    sums(ws_part.p, nkb, 0, nw);
   } else {
     // a full matrix per thread in shared memory, several frequencies per
     // launch (enough blocks for many waves on every SM)
