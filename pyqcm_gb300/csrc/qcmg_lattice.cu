@@ -808,19 +808,46 @@ void Lattice::kmean(int nz, const double* z, int gx, int gy, int gz, double off,
   kmoments(nz, z, gx, gy, gz, off, 0, nullptr, out_host, s);
 }
 
+// Whether every translation is one of the lattice; pairing takes
+// e^{2 pi i (1 - K).R} for e^{-2 pi i K.R}.
+static bool integer_translations(int nmom, const double* Rm) {
+  for (int k = 0; k < 3 * nmom; ++k)
+    if (Rm[k] != std::rint(Rm[k])) return false;
+  return true;
+}
+
+// Whether the means with phases go row by row (inverse_means).  A warp takes
+// points of one (ky, kz), so a row of less than 32 points, or the end of a
+// longer one, leaves lanes idle; below, every point's inverse is stored and
+// added up afterwards, as for L > 16 (k_points, k_mean_moments).  The row form
+// does that work 28 / L times as fast per lane (measured where both cost the
+// same, 64 frequencies, 1,024 points: L = 8 complex 8 x 128 x 1 1.8 ms against
+// 2.0, 4 x 16 x 16 3.5 against 2.0; L = 12 complex 8 x 128 x 1 11.2 against
+// 6.7, 1 x 1024 x 1 88.9 against 6.6), so it is taken where the lanes that its
+// batches occupy are at most 28 / L times the grid's points.
+bool Lattice::long_rows(int gx, int gy, int gz, double off, bool may_pair, cudaStream_t s) {
+  const int np = grid_points(gx, gy, gz, off, s, may_pair);
+  size_t lanes = 0;
+  for (int h = 0, h0 = 0; h < np; ++h)
+    if (h + 1 == np || rep_host[h + 1] / gx != rep_host[h] / gx) {
+      lanes += (size_t)(h - h0 + 32) / 32 * 32;
+      h0 = h + 1;
+    }
+  return lanes * L <= (size_t)28 * gx * gy * gz;
+}
+
 // The means of the translations `which` of Rm (empty: the plain mean) into
 // their places of out_host, nz x max(nmom, 1) x L x L.
 void Lattice::inverse_means(int nz, const double* z, int gx, int gy, int gz, double off, int nmom,
                             const std::vector<int>& which, const double* Rm, double* out_host,
                             cudaStream_t s) {
   const int nk = gx * gy * gz, LL = L * L, nm = std::max<int>(1, (int)which.size());
-  bool integer = true;  // pairing takes e^{2 pi i (1 - K).R} for e^{-2 pi i K.R}
-  for (int m : which)
-    for (int a = 0; a < 3; ++a) integer = integer && Rm[3 * m + a] == std::rint(Rm[3 * m + a]);
-  const int np = grid_points(gx, gy, gz, off, s, integer);
+  const int np = grid_points(gx, gy, gz, off, s, integer_translations(which.empty() ? 0 : nmom, Rm));
   const bool pair = rep_paired;
-  // rows: with translations, the points of each (ky, kz); else equal parts,
-  // about 4,096 warps over all frequencies but whole batches of 32
+  // rows: with translations, the points of each (ky, kz), in parts of whole
+  // batches of 32 that make about 2,048 warps over all frequencies (a 1,024 x
+  // 1 x 1 grid in one row per frequency: 13 ms for one frequency at L = 12,
+  // 0.5 ms in parts); else equal parts, about 4,096 warps
   std::vector<int> rows{0}, fx(nm, 0);
   std::vector<double> yz, wx, ax;
   if (which.empty()) {
@@ -829,8 +856,9 @@ void Lattice::inverse_means(int nz, const double* z, int gx, int gy, int gz, dou
     for (int b = per; b < batches; b += per) rows.push_back(32 * b);
     rows.push_back(np);
   } else {
+    const int per = 32 * (int)std::max<size_t>(1, std::min<size_t>((size_t)(np + 31) / 32, (size_t)np * nz / (32 * 2048)));
     for (int h = 1; h < np; ++h)
-      if (rep_host[h] / gx != rep_host[h - 1] / gx) rows.push_back(h);
+      if (rep_host[h] / gx != rep_host[h - 1] / gx || h - rows.back() == per) rows.push_back(h);
     rows.push_back(np);
     for (size_t q = 0; q < which.size(); ++q) {
       const double r = Rm[3 * which[q]];
@@ -906,7 +934,7 @@ void Lattice::inverse_means(int nz, const double* z, int gx, int gy, int gz, dou
 void Lattice::kmoments(int nz, const double* z, int gx, int gy, int gz, double off, int nmom,
                        const double* Rm, double* out_host, cudaStream_t s) {
   QCMG_CHECK_ARG(nmom >= 0 && nmom <= kMaxMoments, "at most 16 translations per call");
-  if (L <= kMaxPointL) {
+  if (L <= kMaxPointL && (nmom == 0 || long_rows(gx, gy, gz, off, integer_translations(nmom, Rm), s))) {
     // translations in groups of at most (kMaxInvFuncs - 1)/2 distinct |R_x|
     if (nmom == 0) return inverse_means(nz, z, gx, gy, gz, off, 0, {}, nullptr, out_host, s);
     std::vector<int> todo(nmom);

@@ -45,6 +45,7 @@ struct Lattice {
   bool rep_paired = false;
   std::vector<int> rep_host;
   int grid_points(int gx, int gy, int gz, double off, cudaStream_t s, bool may_pair = true);
+  bool long_rows(int gx, int gy, int gz, double off, bool may_pair, cudaStream_t s);
   void inverse_means(int nz, const double* z, int gx, int gy, int gz, double off, int nmom,
                      const std::vector<int>& which, const double* Rm, double* out_host,
                      cudaStream_t s);

@@ -1,11 +1,31 @@
-"""Lattice integrals on grids of unusual size: more points than one launch
-holds."""
+"""Lattice integrals on grids of unusual shape: one long row, rows shorter
+than a warp, cubes (the means with translations' phases take one of two ways
+by the rows' length), and more points than one launch holds."""
 import numpy as np
 import pytest
 
 from test_gpu_lattice_points import TOL, Problem, grid
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("L", [2, 8, 12, 16])
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("g", [(1024, 1, 1, 0.0), (997, 1, 1, 0.25), (1, 70, 1, 0.5), (2, 65, 1, 0.0), (8, 8, 8, 0.5),
+                               (16, 5, 3, 0.0), (100, 9, 1, 0.5)])
+def test_means_with_phases(L, kind, g):
+    from pyqcm_gb300 import _lib
+    p = Problem(L, kind, 4)
+    z = np.array([0.3 + 0.3j, 2.0j])
+    blk = p.block()
+    out = np.zeros(2 * len(z) * len(p.R) * L * L)
+    _lib.check(_lib.lib().qcmg_lattice_kmoments(blk._h, len(z), _lib.ptr(z.view(np.float64)), *g[:3], g[3], len(p.R),
+                                                _lib.ptr(np.ascontiguousarray(p.R)), _lib.ptr(out)))
+    K = grid(*g)
+    X = np.linalg.inv(p.matrices(z, K)[0])
+    ref = np.einsum("km,zkab->zmab", np.exp(2j * np.pi * (K @ p.R.T)), X) / len(K)
+    got = out.view(np.complex128).reshape(ref.shape)
+    assert np.max(np.abs(got - ref)) < TOL * max(1.0, np.max(np.abs(X)))
 
 
 class OneWay(Problem):
