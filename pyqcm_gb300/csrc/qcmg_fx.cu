@@ -14,6 +14,7 @@
 // shared memory and L2.  Hop values must share one magnitude per spin
 // (the Hubbard form: hops are +-t); other Hamiltonians use the FP64 path.
 #include <algorithm>
+#include <chrono>
 #include <cfloat>
 #include <cmath>
 #include <cstdlib>
@@ -580,18 +581,18 @@ static void fx_update(qcmg_hamiltonian* H, FxVec& w, const FxVec& v, const FxVec
 }
 
 // Waits for the step queued last: w's exponent and size, alpha and |w|^2.
-// A stream that ran empty, or failed, without that step's number ends the wait.
+// The host's copy is polled for as long as a small sector's step takes, where
+// the few microseconds of a stream wait count (step 50 us at 853,776 states); a
+// longer step is left to the stream wait, which spins, yields or blocks as the
+// caller set its device to do (165,636,900 states: 4 ms a step).
+constexpr std::chrono::microseconds kPollFor(200);
 static void fx_collect(qcmg_hamiltonian* H, FxVec& w, FxReducer& red, double* alpha, double* norm2) {
   const FxStep& h = *red.host.p;
   auto arrived = [&] { return __atomic_load_n(&red.host.p->seq, __ATOMIC_ACQUIRE) == red.seq; };
+  const auto start = std::chrono::steady_clock::now();
   for (unsigned spin = 1; !arrived(); ++spin) {
-    if (spin % 4096) continue;
-    const cudaError_t q = cudaStreamQuery(H->stream);
-    if (q == cudaErrorNotReady) {
-      cudaGetLastError();
-      continue;
-    }
-    QCMG_CUDA(q);
+    if (spin % 64 || std::chrono::steady_clock::now() - start < kPollFor) continue;
+    QCMG_CUDA(cudaStreamSynchronize(H->stream));
     if (arrived()) break;
     throw Error(QCMG_ERR_CUDA, "a Lanczos step did not report its scalars");
   }
