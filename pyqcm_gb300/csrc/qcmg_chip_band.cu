@@ -5,13 +5,16 @@
 //
 // On a 3,920-state impurity sector a step was five launches and a host wait,
 // ~63 us; here it is two cluster barriers: after the norm and the band dots of
-// v_j (one reduction for all of them), and after the Gram-Schmidt update of
-// the next p - 1 vectors (v_{j+1} going out to every CTA), the product and the
+// v_j (one reduction for all of them; v_j goes out to every CTA meanwhile), and
+// after the Gram-Schmidt update of the next p - 1 vectors, the product and the
 // band recurrence with its closing dot. The 2p + 1 vectors of the band live
 // in shared memory, each CTA's part of them; only v_j is held whole (the
 // hops gather from it). One impurity of the 2x2 + 4 bath model from its
 // parameters to G (two runs of ~111 steps among it): 11.4 ms -> 6.9 ms;
 // two barriers instead of three and 32 states a tile 5.49 -> 5.13 ms later.
+// (A second buffer for the whole vector, so that v_{j+1} goes out with its
+// update, makes no difference: 3,920 states, p = 4, 272 steps 5.68 ms with
+// one as with two, 10,584 states, p = 8 18.4 ms.)
 // The dots of a tile are added over the lanes together, by a reduction that
 // halves the values per lane at each step (2p - 1 additions instead of 5p).
 //
@@ -42,15 +45,12 @@ struct ChipBand {
 
 constexpr int pow2_of(int n) { return n <= 1 ? 1 : 2 * pow2_of((n + 1) / 2); }
 
-// Step j (u_j: v_j before normalization, in every CTA's x):
-//   z = |u_j| and <u_{j+i}, u_j>                                  one barrier
+// Step j (u_j: v_j before normalization):
+//   u_j to every CTA's x; z = |u_j| and <u_{j+i}, u_j>             one barrier
 //   v_j = u_j / z; v_{j+i} -= c_i v_j; w = H v_j - sum_k T(k, j) v_k;
 //   d = <w, v_j>                                                  one barrier
 //   w -= d v_j
-// TWO: x has two buffers and u_{j+1} goes out to all CTAs in the second part
-// (P > 1: it is final then). Otherwise, where two do not fit or for P = 1, it
-// goes out at the start of its own step, with a barrier more.
-template <int P, bool TWO>
+template <int P>
 __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
   constexpr int R = 2 * P + 1;
   extern __shared__ double sm[];
@@ -61,8 +61,8 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
   const int nt = (int)((D + kTile - 1) / kTile), per = (nt + C - 1) / C;
   const int t0 = min(nt, rank * per), t1 = min(nt, t0 + per);
   const int seg = per * kTile;
-  double* xb = sm;                         // D, or 2 x D: u_j, u_{j+1}
-  double* v = xb + (TWO ? 2 : 1) * D;      // R x seg: the band's vectors, this CTA's part
+  double* x = sm;                          // D: u_j
+  double* v = x + D;                       // R x seg: the band's vectors, this CTA's part
   double* dg = v + R * seg;                // seg
   double* part = dg + seg;                 // (2 P + 1) x nt
   __shared__ double tot[2 * P + 1], zs[2], ds;
@@ -77,11 +77,6 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
       v[k * seg + a] = y;
     }
   }
-  if (TWO) {  // u_{j0} whole
-    const double* u = S.j0 > 0 ? S.ring + (size_t)(S.j0 % R) * D : S.phi;
-    double* x = xb + (S.j0 & 1) * D;
-    for (uint32_t i = threadIdx.x; i < D; i += kChipThreads) x[i] = u[i];
-  }
   // the V sums of tile t to every CTA: value m goes to part[m nt + t]
   auto send = [&](auto& acc, int count, int first, int t) {
     constexpr int V = sizeof(acc) / sizeof(double), sub = 32 / V;
@@ -95,13 +90,9 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
     for (int t = lane; t < nt; t += 32) s += part[m * nt + t];
     return warp_total(s);
   };
-  auto publish = [&](double* x, uint32_t i, double y) {
-    for (int r = 0; r < C; ++r) cl.map_shared_rank(x, r)[i] = y;
-  };
   cl.sync();
   for (int s = 0; s < S.steps; ++s) {
     const int j = S.j0 + s;
-    double* x = xb + (TWO ? (j & 1) * D : 0);
     int slot[R];  // slot[k]: v_{j - P + k}
 #pragma unroll
     for (int k = 0; k < R; ++k) slot[k] = ((j + k + P + 1) % R) * seg;  // j - P + k + R, mod R
@@ -116,7 +107,8 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
       if (proj && i < D)
 #pragma unroll
         for (int k = 0; k < P; ++k) pr[k] = S.phi[(size_t)k * D + i] * vj;
-      if (!TWO && i < D) publish(x, i, vj);
+      if (i < D)
+        for (int r = 0; r < C; ++r) cl.map_shared_rank(x, r)[i] = vj;
       send(acc, P, 0, t);
       if (proj) send(pr, P, P, t);
     }
@@ -143,18 +135,13 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
     double c[P];  // T(j - p + k, j): c_0 = z
 #pragma unroll
     for (int k = 0; k < P; ++k) c[k] = k ? tot[k] * iz : z;
-    double* xn = xb + (TWO ? ((j + 1) & 1) * D : 0);
     for (int t = t0 + wp; t < t1; t += nw) {
       const uint32_t i = t * kTile + lane, a = (t - t0) * kTile + lane;
       double acc[1] = {0.0}, w = 0.0;
       const double y = v[slot[P] + a] * iz;
       v[slot[P] + a] = y;
 #pragma unroll
-      for (int k = 1; k < P; ++k) {
-        const double t2 = fma(-c[k], y, v[slot[P + k] + a]);
-        v[slot[P + k] + a] = t2;
-        if (TWO && k == 1 && i < D) publish(xn, i, t2);
-      }
+      for (int k = 1; k < P; ++k) v[slot[P + k] + a] = fma(-c[k], y, v[slot[P + k] + a]);
       if (i < D) {
         const uint32_t id = i / A.du, iu = i - id * A.du;
         w = fma(dg[a], y, chip_hops(A, x, iu, id, 0.0) * iz);
@@ -188,28 +175,25 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_chip_band(ChipBand S) {
   }
 }
 
-static size_t band_smem(uint32_t D, int p, int C, bool two) {
+static size_t band_smem(uint32_t D, int p, int C) {
   const size_t nt = (D + kTile - 1) / kTile, per = (nt + C - 1) / C;
-  return ((two ? 2 : 1) * (size_t)D + (2 * p + 2) * per * kTile + (2 * p + 1) * nt) * sizeof(double);
+  return (D + (2 * p + 2) * per * kTile + (2 * p + 1) * nt) * sizeof(double);
 }
 
 constexpr int kBandMaxP = 12;
 
 template <int P, class F>
-static void with_band_kernel(int p, bool two, F&& f) {
+static void with_band_kernel(int p, F&& f) {
   if constexpr (P > 0) {
-    if (p != P) return with_band_kernel<P - 1>(p, two, f);
-    if constexpr (P > 1) {
-      if (two) return f(k_chip_band<P, true>);
-    }
-    f(k_chip_band<P, false>);
+    if (p != P) return with_band_kernel<P - 1>(p, f);
+    f(k_chip_band<P>);
   }
 }
 
 bool chip_band_fits(const qcmg_hamiltonian* H, int p) {
   int optin = 0;
   QCMG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, H->device));
-  return chip_fits(H) && p <= kBandMaxP && band_smem((uint32_t)H->dim, p, 8, false) <= (size_t)optin - 1024;
+  return chip_fits(H) && p <= kBandMaxP && band_smem((uint32_t)H->dim, p, 8) <= (size_t)optin - 1024;
 }
 
 bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc_defl,
@@ -238,18 +222,17 @@ bool chip_band(qcmg_hamiltonian* H, int p, const double* phi, int M0, double acc
   S.deflated = const_cast<int*>(deflated);
   S.acc_defl = acc_defl;
   int C = 8;
-  bool two = p > 1 && band_smem(D, p, 8, true) <= (size_t)optin - 1024;
   auto launch = [&](int c) {
     S.j0 = c * kBandChunk;
     S.steps = std::min(kBandChunk, M0 - S.j0);
     if (S.steps <= 0) return;
     S.coef = coef.p + (size_t)(c & 1) * chunk_len;
-    with_band_kernel<kBandMaxP>(p, two, [&](auto kern) {
+    with_band_kernel<kBandMaxP>(p, [&](auto kern) {
       if (c == 0) {
         QCMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-        if (clusters_run(kern, 16, band_smem(D, p, 16, two))) C = 16;
+        if (clusters_run(kern, 16, band_smem(D, p, 16))) C = 16;
       }
-      launch_clusters(kern, 1, C, band_smem(D, p, C, two), s, S);
+      launch_clusters(kern, 1, C, band_smem(D, p, C), s, S);
     });
     QCMG_CUDA(cudaEventRecord(lane.e[c & 1], s));
   };
