@@ -790,6 +790,7 @@ int qcmg_apply_c(int L, int orb, int pm, int n_up, int n_dn, const double* x, do
       return;
     }
     PoolBuf<double> dx, dy;
+    Drain drain{0};
     dx.upload(x, n1, 0);
     if (acc)
       dy.upload(y, n2, 0);
@@ -819,6 +820,7 @@ int qcmg_green_function(int L, int M, const double* e, const double* v, int nz, 
     }
     use_device();
     PoolBuf<double> de, dv, dz, dG;
+    Drain drain{0};
     de.upload(e, M, 0);
     dv.upload(v, (size_t)2 * L * M, 0);
     dz.upload(z, (size_t)2 * nz, 0);
@@ -838,6 +840,7 @@ int qcmg_self_energy(int L, int M, const double* e, const double* v, int nb, con
     if (nz == 0) return;
     use_device();
     PoolBuf<double> de, dv, dtcb, deb, dtc, dz, ds, dg;
+    Drain drain{0};
     if (M) {
       de.upload(e, M, 0);
       dv.upload(v, (size_t)2 * L * M, 0);

@@ -188,15 +188,16 @@ void with_size(int p, F&& f) {
     f(std::integral_constant<int, 16>{});
 }
 
-// Waits for the stream before the buffers declared ahead of it go.
+// The events of two chunks of steps; the stream is waited for before they, and
+// the buffers declared ahead of them, go.
 struct Wait {
-  cudaStream_t s;
   cudaEvent_t e[2] = {nullptr, nullptr};
-  explicit Wait(cudaStream_t st) : s(st) {
+  Drain drain;
+  explicit Wait(cudaStream_t st) : drain(st) {
     for (auto& x : e) QCMG_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   }
   ~Wait() {
-    cudaStreamSynchronize(s);
+    cudaStreamSynchronize(drain.s);
     for (auto x : e)
       if (x) cudaEventDestroy(x);
   }
@@ -224,6 +225,9 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   proj.alloc((size_t)p * p * kProjBlocks);
   part.alloc((size_t)grid * p);
   flags.alloc(2);
+  const size_t slot = (size_t)p * rl + 1, pp = (size_t)p * p * kProjBlocks;
+  landed.alloc(2 * slot + pp);
+  Wait wait(s);
   const int init[2] = {-1, 0};
   QCMG_CUDA(cudaMemcpyAsync(flags.p, init, sizeof init, cudaMemcpyHostToDevice, s));
   int* flag = flags.p;
@@ -259,9 +263,6 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
     });
     QCMG_CUDA(cudaGetLastError());
   };
-  const size_t slot = (size_t)p * rl + 1, pp = (size_t)p * p * kProjBlocks;
-  landed.alloc(2 * slot + pp);
-  Wait wait(s);
   // p steps at a time, their rows and the flag copied back
   auto queue = [&](int c) {
     const int j0 = c * p, j1 = std::min(M0, j0 + p);

@@ -693,10 +693,7 @@ LanczosResult fx_lanczos(qcmg_hamiltonian* H, const double* x0_dev, double tol, 
     double c;
   };
   // a step queued in vain (or before an error) is over before its buffers go
-  struct Drain {
-    cudaStream_t s;
-    ~Drain() { cudaStreamSynchronize(s); }
-  } drain{s};
+  Drain drain{s};
   std::vector<Kept> kept;
   TridiagLowest lowest;
   std::vector<double> z;

@@ -534,10 +534,6 @@ struct DevVec {
     if (p) pool_put(p, got);
   }
 };
-struct Drain {
-  cudaStream_t s;
-  ~Drain() { cudaStreamSynchronize(s); }
-};
 
 // CUDA events for the per-solve device-time breakdown.
 struct Events {

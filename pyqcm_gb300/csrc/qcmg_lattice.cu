@@ -169,6 +169,7 @@ void self_energy_batch(int L, int M, const double* e, const double* v, bool v_re
                        double* gamma, cudaStream_t s) {
   QCMG_CHECK_ARG(L > 0 && L <= 32, "Green function dimension must be 1..32");
   PoolBuf<double> G, ldg, mtc;
+  Drain drain{s};
   G.alloc((size_t)2 * L * L * nz);
   if (M > 0)
     green_function_batch(L, M, e, v, v_real, nz, z, G.p, s);
@@ -190,7 +191,7 @@ void self_energy_batch(int L, int M, const double* e, const double* v, bool v_re
     k_gamma<<<nz, 128, 0, s>>>(L, nz, (const double2*)z, nb, (const double2*)tcb, eb,
                                (double2*)gamma);
   QCMG_CUDA(cudaGetLastError());
-  QCMG_CUDA(cudaStreamSynchronize(s));  // mtc, G go out of scope
+  QCMG_CUDA(cudaStreamSynchronize(s));
 }
 
 // ---------------------------------------------------------------------------
@@ -883,8 +884,9 @@ void Lattice::inverse_means(int nz, const double* z, int gx, int gy, int gz, dou
       }
   }
   const int nrow = (int)rows.size() - 1, nf = 1 + 2 * (int)ax.size();
-  PoolBuf<int> d_rows, d_fx;  // idle again after the last wait below
+  PoolBuf<int> d_rows, d_fx;
   PoolBuf<double> d_yz, d_wx;
+  Drain drain{s};
   d_rows.upload(rows.data(), rows.size(), s);
   if (!which.empty()) {
     d_fx.upload(fx.data(), fx.size(), s);

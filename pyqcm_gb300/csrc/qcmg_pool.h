@@ -75,6 +75,16 @@ struct PinnedBuf {
   }
 };
 
+// Waits for a stream when the scope is left, by an exception too: declared
+// after the buffers whose work the stream holds.
+struct Drain {
+  cudaStream_t s;
+  explicit Drain(cudaStream_t st) : s(st) {}
+  Drain(const Drain&) = delete;
+  Drain& operator=(const Drain&) = delete;
+  ~Drain() { cudaStreamSynchronize(s); }
+};
+
 // A non-blocking stream and events of the current device, kept likewise.
 struct PoolStream {
   cudaStream_t s = nullptr;
