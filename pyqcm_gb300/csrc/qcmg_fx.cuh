@@ -81,7 +81,8 @@ __device__ __forceinline__ I128 shr128(I128 v, int s) {  // arithmetic, 0 < s < 
 
 constexpr int kDotShift = 20;
 
-__device__ __forceinline__ void block_store128(I128 s, I128* part) {
+// The block's sum, stored by thread 0.
+__device__ __forceinline__ void block_store128(I128 s, I128* dst) {
   __shared__ int64_t shi[32];
   __shared__ uint64_t slo[32];
   s = warp_sum128(s);
@@ -97,7 +98,7 @@ __device__ __forceinline__ void block_store128(I128 s, I128* part) {
     t.hi = lane < nw ? shi[lane] : 0;
     t.lo = lane < nw ? slo[lane] : 0;
     t = warp_sum128(t);
-    if (lane == 0) part[blockIdx.x] = t;
+    if (lane == 0) *dst = t;
   }
 }
 
@@ -106,7 +107,7 @@ __device__ __forceinline__ void block_store128(I128 s, I128* part) {
 // does not matter) in thread 0's total, and resets the ticket.
 __device__ __forceinline__ bool last_block_sum128(I128 s, I128* part, unsigned* ticket, I128* total) {
   __shared__ unsigned last;
-  block_store128(s, part);  // thread 0 stores
+  block_store128(s, part + blockIdx.x);
   if (threadIdx.x == 0) {
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
@@ -122,7 +123,7 @@ __device__ __forceinline__ bool last_block_sum128(I128 s, I128* part, unsigned* 
     t = add128(t, q);
   }
   __shared__ I128 sum;
-  block_store128(t, &sum - blockIdx.x);  // thread 0 stores
+  block_store128(t, &sum);
   if (threadIdx.x == 0) {
     *total = sum;
     *ticket = 0;
