@@ -1071,7 +1071,14 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
   for (int k = 0; k < p; ++k) phip.push_back(phi0 + (size_t)k * n);
   std::vector<double> t;  // column-major t(r,c) = t[r + M0*c]
   std::vector<double> P;  // P(k,j) = P[k + p*j]
-  if (chip_band_fits(H, p)) {
+  // A sector of a few states is exhausted in as many steps: both fast forms
+  // would end in a deflation and the loop below do it again (dimer, 4 states:
+  // p = 1 0.81 ms against 0.78 by the loop alone, p = 4 0.95 against 0.82; 9
+  // states the same within 3%; 24 states, p = 1 2.08 ms against 2.37, 36 states,
+  // p = 4 3.19 against 3.39, and 1.0 against 4.2 at 100 states, where nothing
+  // deflates).
+  const bool tiny = n <= 9;
+  if (!tiny && chip_band_fits(H, p)) {
     int M = 0;
     if (chip_band(H, p, phi0, M0, acc_defl, acc_band, t, P, &M))
       return band_result(H, p, M0, M, t, P, true);
@@ -1105,7 +1112,7 @@ BandResult band_lanczos(qcmg_hamiltonian* H, int p, const double* phi_in, bool p
   // the steps up to the first deflation (usually all of them), without a
   // host round trip per step; then the loop below takes over
   int j = 0;
-  if (p <= kBandMax) {
+  if (!tiny && p <= kBandMax) {
     std::vector<double*> ring(2 * p + 1);
     for (double*& r : ring) r = get();
     BandRun run;
