@@ -680,16 +680,32 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   };
   const int keep = std::max(reorth, 2);
   // the vectors, reused across restarts; allocated several at a time (up to
-  // 512 MB), since an allocation per step cost as much as a step
+  // 512 MB), since an allocation per step cost as much as a step; one by one
+  // when the device has no room for several
   const size_t stride = (n + 1) & ~(size_t)1;
-  const size_t block = std::max<size_t>(1, std::min<size_t>(keep, ((size_t)512 << 20) / (stride * 8)));
+  size_t block = std::max<size_t>(1, std::min<size_t>(keep, ((size_t)512 << 20) / (stride * 8)));
   std::vector<DevVec> blocks;
   MultiOps mops;
   Drain drain2{s};
   std::vector<double*> V;
+  double* next = nullptr;  // the last block's vectors not yet handed out
+  size_t left = 0;
   auto add_vector = [&] {
-    if (V.size() == blocks.size() * block) blocks.emplace_back(std::min(block, (size_t)keep - V.size()) * stride);
-    V.push_back(blocks.back().p + (V.size() % block) * stride);
+    if (left == 0) {
+      left = std::min(block, (size_t)keep - V.size());
+      try {
+        blocks.emplace_back(left * stride);
+      } catch (const Error& e) {
+        if (e.code != QCMG_ERR_NOMEM || left == 1) throw;
+        cudaGetLastError();
+        left = block = 1;
+        blocks.emplace_back(stride);
+      }
+      next = blocks.back().p;
+    }
+    V.push_back(next);
+    next += stride;
+    --left;
   };
   std::vector<const double*> Vp;
   add_vector();

@@ -57,3 +57,38 @@ def test_a_plain_run_finds_copies():
         q = q - a[-1] * r
         b.append(np.linalg.norm(q))
     assert _copies(np.array(a), np.array(b), ev) > 0
+
+
+def test_vectors_one_by_one_when_memory_is_short():
+    """The kept vectors are allocated 512 MB at a time; where the device has no
+    room for that the run goes on with single ones (3,312,400 states, 19 vectors
+    a time, 22 steps: the limit ends the run, not the memory)."""
+    import models
+    import pyqcm_gb300 as pg
+    import torch
+    ns, _, ops = models.hubbard_cluster(4, 4)
+    params = {"t": 1.0, "U": 8.0, "mu": 4.0}
+    m = pg.ClusterModel(ns)
+    for name, (typ, els) in ops.items():
+        if name in params:
+            m.new_operator(name, typ, els)
+    H = pg.Hamiltonian(m, params, "R0:N8:S0")
+    x0 = np.random.default_rng(1).normal(size=H.dim)
+    x0 /= np.linalg.norm(x0)
+
+    def steps():
+        with pytest.raises(pg.QcmgError) as err:
+            H.lanczos(x0=x0, tol=1e-300, max_iter=22, reorth=100)
+        return err.value.code
+
+    assert steps() == -4  # also allocates the product's buffers
+    torch.cuda.empty_cache()
+    vector = 8 * H.dim
+    span = (512 << 20) // vector * vector
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - span - 8 * vector, dtype=torch.uint8, device="cuda")
+    try:
+        assert span < torch.cuda.mem_get_info()[0] < 2 * span
+        assert steps() == -4
+    finally:
+        del fill
+        torch.cuda.empty_cache()
