@@ -284,14 +284,8 @@ struct MultiOps {
   DevBuf<const double*> ptrs;
   DevBuf<double> part, coef, sums;
   std::vector<const double*> listed;  // what ptrs holds
-  double* host = nullptr;             // page-locked
-  size_t host_n = 0;
-  MultiOps() = default;
-  MultiOps(const MultiOps&) = delete;
-  MultiOps& operator=(const MultiOps&) = delete;
-  ~MultiOps() {
-    if (host) cudaFreeHost(host);
-  }
+  PinnedBuf<double> host;             // from the pool: cudaMallocHost and cudaFreeHost
+                                      // take 0.3 ms, ten steps of a small sector
   template <class T>
   static void grow(DevBuf<T>& b, size_t need) {  // lists grow by one per Lanczos step
     if (need > b.n) b.alloc(std::max(need, 2 * b.n));
@@ -361,15 +355,10 @@ struct MultiOps {
     out.assign(m, 0.0);
     if (m == 0) return;
     const double* d = dots_dev(V, w, n, s);
-    if (host_n < (size_t)m) {
-      if (host) cudaFreeHost(host);
-      host = nullptr;
-      host_n = std::max<size_t>(m, 64);
-      QCMG_CUDA(pinned_alloc(reinterpret_cast<void**>(&host), host_n * sizeof(double)));
-    }
-    QCMG_CUDA(cudaMemcpyAsync(host, d, m * sizeof(double), cudaMemcpyDeviceToHost, s));
+    host.alloc(std::max<size_t>(m, 64));
+    QCMG_CUDA(cudaMemcpyAsync(host.p, d, m * sizeof(double), cudaMemcpyDeviceToHost, s));
     QCMG_CUDA(cudaStreamSynchronize(s));
-    std::copy(host, host + m, out.begin());
+    std::copy(host.p, host.p + m, out.begin());
   }
   // w -= sum_k c_k V_k with c in device memory (stat: see k_axpys; room for
   // 2 elementwise_grid(n) values)
