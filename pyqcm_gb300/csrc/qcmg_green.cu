@@ -128,19 +128,28 @@ static void launch_green(int L, int M, const double* e, const double* v, bool re
 void green_function_batch(int L, int M, const double* e, const double* v, bool real, int nz,
                           const double* z, double* G, cudaStream_t s) {
   if (nz <= 0 || L <= 0) return;
-  QCMG_CHECK_ARG((size_t)std::max(M, 1) * sizeof(double2) <= 200 * 1024, "too many poles for one shared-memory pass");
+  // the interface's limit, which the kernel itself does not need: poles go
+  // through shared memory a tile at a time
+  QCMG_CHECK_ARG(M <= 12800, "more than 12,800 poles");
   const size_t nel = real ? L * (L + 1) / 2 : L * L;
-  auto threads = [&](int F) { return (size_t)((nz + F - 1) / F) * nel; };
-  QCMG_CHECK_ARG(threads(4) < (1u << 31), "too many frequencies for one call");
   int dev = 0, sms = 0;
   QCMG_CUDA(cudaGetDevice(&dev));
   QCMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (threads(4) >= (size_t)32 * sms)
-    launch_green<4>(L, M, e, v, real, nz, z, G, s);
-  else if (threads(2) >= (size_t)32 * sms)
-    launch_green<2>(L, M, e, v, real, nz, z, G, s);
-  else
-    launch_green<1>(L, M, e, v, real, nz, z, G, s);
+  // a launch numbers its threads (elements x frequency groups) in 31 bits
+  const int most = (int)std::min<size_t>(nz, std::max<size_t>(1, (((size_t)1 << 31) - 32) / nel / 4 * 4));
+  for (int z0 = 0; z0 < nz;) {
+    const int n = std::min(most, nz - z0);
+    const double* zc = z + 2 * (size_t)z0;
+    double* Gc = G + (size_t)2 * L * L * z0;
+    auto threads = [&](int F) { return ((size_t)n + F - 1) / F * nel; };
+    if (threads(4) >= (size_t)32 * sms)
+      launch_green<4>(L, M, e, v, real, n, zc, Gc, s);
+    else if (threads(2) >= (size_t)32 * sms)
+      launch_green<2>(L, M, e, v, real, n, zc, Gc, s);
+    else
+      launch_green<1>(L, M, e, v, real, n, zc, Gc, s);
+    z0 += n;
+  }
 }
 
 }  // namespace qcmg
