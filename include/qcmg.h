@@ -204,7 +204,7 @@ int qcmg_lanczos_ground_state(qcmg_hamiltonian* H, const double* x0, unsigned se
  * device and the steps captured once as a CUDA graph of `chunk` steps (rounded
  * up to even) on a stream of its own, run until the Ritz residual is
  * below tol (tested after every step, as the reference does) or max_iter
- * steps; sectors of any sizes run side by side.  Outputs per sector: E0[i],
+ * steps; sectors on chip run side by side, then the larger ones.  Outputs per sector: E0[i],
  * niter[i] (may be NULL), status[i] (QCMG_OK, QCMG_ERR_NOCONV or
  * QCMG_ERR_NUMERIC; may be NULL) and, where psi[i] is not NULL (psi itself
  * may be NULL), the ground-state vector (host array of length dim).  The

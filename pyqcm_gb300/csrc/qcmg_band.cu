@@ -215,8 +215,11 @@ bool band_steps(qcmg_hamiltonian* H, int p, const double* phi, int M0, double ac
   for (double* r : ring) low |= (uintptr_t)r;
   const bool two = (n & 1u) == 0 && (low & 15u) == 0;
   const size_t nv = two ? n / 2 : n;
-  // the two blocks per SM that are resident (registers): one round of equal
-  // shares; three took the recurrence 1.5 rounds (green run 106.8 ms, 102.5)
+  // two blocks per SM, at p = 12 those that the registers leave resident: one
+  // round of equal shares; three took the recurrence 1.5 rounds (green run
+  // 106.8 ms, 102.5). Smaller bands could hold three or four; with two,
+  // 731,808 states take 112 to 118 us a step at p = 1 to 4 and 144 at p = 8
+  // (168 to 172 and 223 by the host-driven loop)
   const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((nv + kDotThreads - 1) / kDotThreads, 2 * 152));
   PoolBuf<double> rows, proj, part;
   PinnedBuf<double> landed;  // p steps' rows and the flag, twice; the projections

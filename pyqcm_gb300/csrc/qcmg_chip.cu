@@ -352,10 +352,11 @@ void chip_lanczos(int n, qcmg_hamiltonian* const* Hs, const double* const* x0, d
     most = std::max(most, (uint32_t)Hs[k]->dim);
     states += Hs[k]->dim;
   }
-  // the largest cluster (at most the portable 8) with which all sectors are
-  // resident at once, two CTAs per SM; larger where a smaller one's share of
-  // the vectors does not fit
-  // For one sector alone sixteen, where the chip allows it.
+  // The portable 8, halved while the sectors ask for more than two CTAs per SM
+  // and a smaller cluster's share of the vectors fits. One CTA is resident per
+  // SM (103 registers and 512 threads), so some clusters of a launch may wait
+  // for others to finish: 48 sectors take C = 4, 192 CTAs on 152 SMs, 4.5 ms.
+  // For one sector alone sixteen, where the chip allows it
   int C = 8;
   if (n == 1) {
     // (the kernel's consent to more than eight holds for one device's context)

@@ -232,10 +232,11 @@ __global__ void __launch_bounds__(SMALL ? 256 : NS == 1 ? 512 : 1024, SMALL ? 4 
         smem_slab[s * kOff + e0 + du + tid] = 0;  // zero slots for padding columns
     }
     // the next round's slabs into L2 meanwhile: its copies then wait for L2
-    // only (with the narrow shifts: 2,556 -> 2,526 us for the 4x4 sector,
-    // 1,043 -> 982 us for its 12-electron one; asking for y too fills L2 and
-    // costs 140 us). Not with an accumulated input, whose reads compete: 200
-    // products y += H x back to back 2,575 us each with it, 2,540 without
+    // only. y = H x back to back, with it and without: 196 and 201 us (11.8M
+    // states), 890 and 914 (41.4M), 950 and 968 (64.1M), 2,380 and 2,379
+    // (165.6M). Not with an accumulated input, whose reads compete on the
+    // largest sector: y += H x 204 and 207 us, 919 and 931, 1,005 and 1,006,
+    // 2,542 and 2,500 (asking for y too fills L2: 140 us more)
     if (tid < NS) {
       const uint32_t a = a0 + (uint32_t)NS * G + tid * G;
       if (a < dd && !A.yin) prefetch_slab(A.x + (size_t)a * du, du);

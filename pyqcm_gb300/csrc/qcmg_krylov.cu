@@ -383,8 +383,7 @@ struct MultiOps {
   // w orthogonal to V: a classical Gram-Schmidt pass and, when it took away
   // half of |w|^2 or more, a second one (the criterion of Daniel, Gragg,
   // Kaufman and Stewart, 1976: otherwise one pass leaves w orthogonal to
-  // rounding).  The device decides; *again (page-locked) tells the host at
-  // its next wait.
+  // rounding).  The device decides; collect() tells the host.
   // |w|^2 and max|w_i| of the result come from the pass that wrote it:
   // collect() reads them, and alpha, after the stream was waited for.
   DevBuf<int> need;
@@ -572,8 +571,11 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
   }
   if (reorth <= 0 && chip_fits(H)) {
     // on chip, in FP64 on either path: at these sizes a step is latency, and
-    // the fixed-point passes take five launches (8-site chain, 4,900 states:
-    // ~45 us per step, 16 us on chip)
+    // the fixed-point passes take several launches (8-site chain, 4,900 states:
+    // ~45 us per step, 10.3 us on chip). No less accurate against 64-bit
+    // references over 114 solves of 49 to 15,876 states: energies 2.8e-16 rms relative
+    // (fixed point 2.9e-16), residuals up to 1.0e-12 (1.5e-12) at tol 1e-12,
+    // |psi|^2 - 1 up to 4e-14 (1.9e-13)
     if (x0_host) QCMG_CUDA(cudaStreamSynchronize(s));  // the solve has a stream of its own
     ChipResult r;
     chip_lanczos(1, &H, &x0_dev, tol, max_iter, psi_host ? &psi_host : nullptr, &r);

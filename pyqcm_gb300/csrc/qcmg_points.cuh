@@ -19,7 +19,8 @@
 // 3x4 cluster, 128x128 K x 256 frequencies x 2 spins: 8.39M points (4.20M
 // with K and -K paired): 114.1 ms with a full matrix per thread in shared
 // memory, 21.8 ms now for the whole call (FP64 pipe floor of the paired
-// points: 18 ms).  8-site chain, 256 K x 512 z: 1,120 -> 609 us per call.
+// points: 18 ms; 20.2 ms with the later Green function kernel).  8-site chain,
+// 256 K x 512 z: 1,120 -> 609 us per call, 427 with that kernel.
 #pragma once
 
 #include "qcmg_points.h"

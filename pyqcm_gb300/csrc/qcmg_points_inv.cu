@@ -19,7 +19,8 @@
 // 2x4 cluster, 64x64 K x 64 w x 2 spins, 9 translations: writing the inverses
 // (537 MB per spin) and reading them back once per element and translation
 // took 16.9 ms per call, 4.7 ms now; the plaquette's host function (64x64 K x
-// 200 w) 2.63 ms, 1.28 ms now. Bound by the FP64 pipe.
+// 200 w) 2.63 ms, 1.28 ms (0.85 ms with the later Green function kernel). Bound
+// by the FP64 pipe.
 #include "qcmg_points.h"
 
 namespace qcmg {

@@ -337,7 +337,7 @@ def lanczos_batch(hamiltonians, want_psi=False, tol=None, max_iter=None, chunk=1
                   raise_errors=True):
     """Lanczos ground states of several sectors at once (qcmg_lanczos_batch):
     sectors of at most 16,384 states run on chip, larger ones from captured
-    CUDA graphs of `chunk` steps, all side by side; results
+    CUDA graphs of `chunk` steps, each kind side by side; results
     equal Hamiltonian.lanczos() on the FP64 path.  Returns a list of
     (E0, psi or None, iterations) in the order of `hamiltonians`; a sector
     that did not converge raises QcmgError, or with raise_errors=False each
