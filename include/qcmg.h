@@ -122,9 +122,10 @@ int qcmg_matvec(qcmg_hamiltonian* H, const double* x, double* y, unsigned flags)
  * have one magnitude per spin (the Hubbard form), path 0 always uses the
  * FP64 kernels.  Products of FP64 vectors (qcmg_matvec) of less than 2^21
  * states take the FP64 kernel on either path (the conversions cost more than
- * they save; qcmg_matvec_fx has none).  Lanczos runs without reorthogonalization on sectors of at
- * most 16,384 states are FP64 on either path (they run on chip).  No
- * counterpart in the reference (FP64 throughout). */
+ * they save; qcmg_matvec_fx has none).  Lanczos runs without reorthogonalization
+ * on sectors of at most 16,384 states run on chip in FP64 on either path; on path
+ * 1 one that has not converged after max_iter steps is repeated in fixed point.
+ * No counterpart in the reference (FP64 throughout). */
 int qcmg_hamiltonian_set_path(qcmg_hamiltonian* H, int path);
 
 /* *available = 1 when the fixed-point fast path applies to this sector. */

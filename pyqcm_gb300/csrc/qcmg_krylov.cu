@@ -581,14 +581,20 @@ LanczosResult lanczos_ground_state(qcmg_hamiltonian* H, const double* x0_host, u
     chip_lanczos(1, &H, &x0_dev, tol, max_iter, psi_host ? &psi_host : nullptr, &r);
     if (r.status == QCMG_ERR_NUMERIC)
       throw Error(QCMG_ERR_NUMERIC, "Lanczos produced a non-finite value");
-    if (r.status == QCMG_ERR_NOCONV)
+    // A tolerance below the rounding of FP64 steps (|H| eps: 2e-8 for energies
+    // of 1e8) can still be met by the fixed-point path's exact sums, in a
+    // sector that a few steps exhaust: its run decides where it applies.
+    const bool decided = r.status == QCMG_OK || !(H->use_fx && fx_prepare(H));
+    if (decided && r.status == QCMG_ERR_NOCONV)
       throw Error(QCMG_ERR_NOCONV,
                   "Lanczos procedure exceeded " + std::to_string(max_iter) + " iterations");
-    res.alpha = r.alpha;
-    res.beta = r.beta;
-    res.energy = r.energy;
-    res.niter = r.niter;
-    return res;
+    if (decided) {
+      res.alpha = r.alpha;
+      res.beta = r.beta;
+      res.energy = r.energy;
+      res.niter = r.niter;
+      return res;
+    }
   }
   if (reorth <= 0 && H->use_fx && fx_prepare(H)) {
     // fixed-point fast path (one hop magnitude per spin)

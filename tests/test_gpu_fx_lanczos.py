@@ -132,3 +132,26 @@ def test_large_products_on_host_vectors(offset, pinned):
     xd, yd = torch.from_numpy(x).cuda(), torch.full((H.dim,), 0.75, dtype=torch.float64, device="cuda")
     H.matvec_device(xd.data_ptr(), yd.data_ptr(), accumulate=True)
     assert np.max(np.abs(yd.cpu().numpy() - 0.75 - ref)) <= tol
+
+
+@pytest.mark.parametrize("scale", [1e8, 3e10])
+@pytest.mark.parametrize("nup,ndn", [(0, 1), (1, 1), (2, 1)])
+def test_small_sectors_beyond_fp64(scale, nup, ndn):
+    """A dimer with energies of 1e8 to 3e10 at a tolerance of 1e-12, below the
+    rounding of an FP64 step: the on-chip run does not meet it, the fixed-point
+    run that then decides does (its exact sums end the Krylov space); on the
+    FP64 path the run ends with NOCONV."""
+    import pyqcm_gb300 as pg
+    m = pg.ClusterModel(2)
+    m.new_operator("t", "one-body", [(0, 1, -1.0), (2, 3, -1.0)])
+    m.new_operator("U", "interaction", [(0, 2, 1.0), (1, 3, 1.0)])
+    m.new_operator("e", "one-body", [(0, 0, 1.0), (2, 2, 1.0)])
+    H = pg.Hamiltonian(m, {"t": 0.921 * scale, "U": 3.0 * scale, "e": 0.37 * scale}, f"R0:N{nup + ndn}:S{nup - ndn}")
+    assert H.fx_available()
+    A = np.array([H.matvec(v) for v in np.eye(H.dim)])
+    x0 = np.random.default_rng(5).normal(size=H.dim)
+    x0 /= np.linalg.norm(x0)
+    e0, psi, _, _ = H.lanczos(x0=x0, tol=1e-12, max_iter=300, reorth=0)
+    e = np.linalg.eigvalsh(A)
+    assert abs(e0 - e[0]) < 1e-13 * np.max(np.abs(e))
+    assert np.linalg.norm(A @ psi - e0 * psi) < 1e-13 * np.max(np.abs(e))
